@@ -172,7 +172,8 @@ int sftg_light_vis_noalloc(sftg_ctx* ctx, const sftg_frame_desc* frame, uint8_t*
  * the 64x64 tile stays fixed here too, because the per-tile payload lists are part of the
  * render path's observable output). */
 typedef struct sftg_tuning {
-    int32_t resolve_split[3];     /* resolve CTAs per 64x64 tile at 1x, 2x, 4x: 1, 2, 4, 8 or 16 (default 16, 8, 16) */
+    int32_t resolve_split[3];     /* most resolve CTAs per 64x64 tile at 1x, 2x, 4x: 1, 2, 4, 8 or 16 (default 16); 8 and
+                                     16 are halved, down to 4, where the tiles alone fill the GPU */
     int32_t raster_slab_rows[3];  /* tile rows per raster work item at 1x, 2x, 4x: 4..64 (default 8, 8, 4) */
     int32_t geom_job_width;       /* meshlets per geometry warp: 1..8 (default 1; the reference's job is 8) */
     int32_t occl_ray_prune;       /* 1: also cull BLAS children no unblocked shadow ray reaches (faster; can differ
@@ -183,8 +184,7 @@ typedef struct sftg_tuning {
                                      1, 2 or 4 = every tile (at 4x at least 2) */
     int32_t tile_lights[3];       /* where a tile's light list and proxy selection are made at 1x, 2x, 4x: 1 = by each of
                                      its resolve CTAs, 2 = once per tile by a launch before the resolve (its CTAs read
-                                     the result), 0 = 2 where the range has 16 CTAs per tile and at least 256 tiles,
-                                     else 1 (default) */
+                                     the result), 0 = 2 where the range has at least 128 tiles, else 1 (default) */
     int32_t tile_queue;           /* bit 0 raster, bit 1 resolve: set, the phase is one persistent launch of as many CTAs
                                      as are resident at once, which take its (tile, band) / (tile, part) items, heaviest
                                      tiles first, from a device counter; clear (default 0), one CTA per item */

@@ -109,7 +109,7 @@ struct sftg_ctx {
     uint32_t blas_items = 0, blas_launches = 0; /* and its triangles and kernels */
     cudaEvent_t ev_blas[2] = { nullptr, nullptr };
     bool use_graphs = true;
-    sftg_tuning tuning = { { 16, 8, 16 }, { 8, 8, 4 }, 1, 0, { 0, 0, 0 }, { 0, 0, 0 }, 0 };   /* measured best on the single-view workloads */
+    sftg_tuning tuning = { { 16, 16, 16 }, { 8, 8, 4 }, 1, 0, { 0, 0, 0 }, { 0, 0, 0 }, 0 };   /* measured best on the single-view workloads */
     /* transient models (one frame's dynamic meshes): pool marks where they start */
     bool tr_live = false, tr_pinned = false;
     uint32_t tr_meshlets = 0, tr_skin = 0, tr_blas = 0;
@@ -918,15 +918,14 @@ static int launch_batch(sftg_ctx* ctx, sftg_lane& ln, const batch_bufs& B) {
      * launch on the critical path) or by every resolve CTA of the tile (split-fold work) */
     bool records[3];
     for (int si = 0; si < 3; si++) {
-        const int m = ctx->tuning.tile_lights[si];
-        records[si] = m == 2 || (m == 0 && ctx->tuning.resolve_split[si] >= 16 && B.s_tiles[si] >= 256);
+        records[si] = sftg_resolve_records(ctx->tuning.tile_lights[si], B.s_tiles[si]);
         if (records[si] && B.s_tiles[si]) {   /* on st: every range's resolve waits for it (per_range forks after it) */
             sftg_launch_tile_lights(B.s_tile0[si], B.s_tiles[si], st, A);
             ln.launches++;
         }
     }
     prc = per_range(1, [&](int si, cudaStream_t s) {
-        sftg_launch_resolve(1 << si, B.s_tile0[si], B.s_tiles[si], ctx->tuning.resolve_split[si], records[si],
+        sftg_launch_resolve(1 << si, B.s_tile0[si], B.s_tiles[si], sftg_resolve_split(ctx->tuning.resolve_split[si], B.total_tiles), records[si],
                             queue_resolve ? B.queue + 3 + si : nullptr, s, A);
     });
     if (prc) return prc;

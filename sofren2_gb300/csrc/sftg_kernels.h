@@ -84,6 +84,9 @@ int sftg_raster_bands(void);   /* raster CTAs (row bands) per 64x64 tile */
 /* order[] = the batch's tiles, heaviest first inside each sample-count range; scratch holds 192 words */
 int sftg_launch_tile_order(const sftg_frame* frames, const uint16_t* tile_view, const uint32_t* tile_count, uint32_t n_tiles,
                             uint32_t* scratch, uint32_t* order, cudaStream_t st);
+/* resolve CTAs per tile and where its light lists are made, from the tuning knobs and the tile count */
+int sftg_resolve_split(int knob, uint32_t tiles);
+bool sftg_resolve_records(int knob, uint32_t tiles);
 /* slab_rows: rows of one raster work item (4..64); split: resolve CTAs per tile (1, 2, 4, 8 or 16) */
 void sftg_launch_raster(int S, uint32_t tile0, uint32_t tiles, int slab_rows, int bands, uint32_t* queue, cudaStream_t st,
                         const sftg_tile_args& A);

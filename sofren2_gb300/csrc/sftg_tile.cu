@@ -16,12 +16,10 @@
  * guard-band choices; the AA chunk skip is a group ballot.  The decoded visibility buffer
  * (depth, vid) goes to global memory, where it stays L2-resident, with the tile's depth range.
  *
- * k_resolve: 1 to 16 CTAs per tile (a tuning knob per sample count), each a share of its 4x2
- * blocks, small shared memory for high occupancy.  A group of 8 threads is one 4x2 block (the reference's AVX2 lanes).  For
- * each distinct triangle in the block (peeled in the reference's order) all 8 lanes shade it,
- * because the reference's LOD uses the first covered lane's screen derivatives (neighbour
- * lanes via shuffles) and its proxy loop skips a proxy for the whole block when no lane is
- * affected (a ballot), which changes the smooth-max shadow of every lane.
+ * k_resolve: 1 to 16 CTAs per tile (sftg_resolve_split), each a share of its 4x2 blocks (the
+ * reference's AVX2 lanes).  A warp lists the covered (pixel, triangle) fragments of 4 to 16
+ * neighbouring blocks, in the reference's order per block, and shades them 32 at a time, one per
+ * lane (resolve_item).
  */
 #include "sftg_types.h"
 #include "sftg_lane.cuh"
@@ -86,11 +84,6 @@ SFTG_D tri_setup unpack_setup(const tri_setup_packed& P, int tmx, int tmy) {
     return T;
 }
 
-struct proxy_cache {   /* sft_light_proxy_cache (sofren2.c:991-998) */
-    float pa[3], pb[3], ab[3], W[3];
-    float abdab, wdw, rb2, pr, pr2, vis_mult;
-};
-
 struct tri_verts {
     float sx[3], sy[3], iw[3], u[3], v[3], lu[3], lv[3], px[3], py[3], pz[3], nx[3], ny[3], nz[3];
     uint32_t inst, m;
@@ -143,52 +136,6 @@ SFTG_D void fetch_tri(const sftg_frame* F, const float* ss, const sftg_clip_tri*
         t.nx[k] = b4.z; t.ny[k] = b4.w; t.nz[k] = c4.x;
     }
     t.inst = ii; t.m = m;
-}
-
-/* Grows [mn, mx] by the world position the resolve interpolates on triangle `vid` at pixel
- * centre (pxf, pyf): the same barycentrics, MSAA clamp, perspective weights and interpolation as
- * the shading loop (D6 below), so the box holds exactly the points the proxy tests use. */
-template <int S>
-SFTG_D void pixel_pos_acc(const sftg_frame* F, const float* ss, const sftg_clip_tri* clips, uint32_t vid, float pxf, float pyf,
-                          float* mn, float* mx) {
-    float sx[3], sy[3], iw[3], px[3], py[3], pz[3];
-    if (vid & 0x80000000u) {
-        const sftg_clip_tri* c = &clips[vid & 0x7FFFFFFFu];
-#pragma unroll
-        for (int k = 0; k < 3; k++) { sx[k] = c->sx[k]; sy[k] = c->sy[k]; iw[k] = c->iw[k]; px[k] = c->px[k]; py[k] = c->py[k]; pz[k] = c->pz[k]; }
-    } else {
-        const uint32_t ii = (vid >> 25) & 63, m = (vid >> 7) & 0x3FFFF, tri = vid & 127;
-        const sftg_inst* I = &F->inst[ii];
-        const uint32_t g = I->meshlet_base + m;
-        const uint8_t* ind = F->ml_inds + (size_t)g * 512;
-        const float* Sc = ss + (size_t)(I->ss_offset + m) * SFTG_SS_FLOATS;
-        const uint32_t b = tri >> 3, l = tri & 7;
-#pragma unroll
-        for (int k = 0; k < 3; k++) {
-            const uint32_t v = ind[b * 32 + 8 * k + l];
-            const float4 a = ((const float4*)(Sc + SFTG_SS_A))[v], b4 = ((const float4*)(Sc + SFTG_SS_B))[v];
-            sx[k] = a.x; sy[k] = a.y; iw[k] = a.z; px[k] = a.w; py[k] = b4.x; pz[k] = b4.y;
-        }
-    }
-    const float dx1 = sx[1] - sx[0], dx2 = sx[2] - sx[0], dy1 = sy[1] - sy[0], dy2 = sy[2] - sy[0];
-    const float idet = rcpr(dx1 * dy2 - dx2 * dy1);
-    const float pxs = pxf - sx[0], pys = pyf - sy[0];
-    const float rbu = (pxs * dy2 - pys * dx2) * idet;
-    const float rbv = (pys * dx1 - pxs * dy1) * idet;
-    const float rbw = (1.f - rbu) - rbv;
-    float bu = rbu, bv = rbv, bw = rbw;
-    if (S > 1) {
-        bu = vmax(0.f, rbu); bv = vmax(0.f, rbv); bw = vmax(0.f, rbw);
-        const float bs = rcpr(bu + (bv + bw));
-        bu = bu * bs; bv = bv * bs; bw = bw * bs;
-    }
-    const float iz = fma_(bw, iw[0], fma_(bu, iw[1], bv * iw[2]));
-    const float z = rcpr(iz);
-    const float w0 = (bw * iw[0]) * z, w1 = (bu * iw[1]) * z, w2 = (bv * iw[2]) * z;
-    const float P[3] = { fma_(w0, px[0], fma_(w1, px[1], w2 * px[2])), fma_(w0, py[0], fma_(w1, py[1], w2 * py[2])),
-                         fma_(w0, pz[0], fma_(w1, pz[1], w2 * pz[2])) };
-#pragma unroll
-    for (int a = 0; a < 3; a++) { mn[a] = fminf(mn[a], P[a]); mx[a] = fmaxf(mx[a], P[a]); }
 }
 
 /* edge / depth setup of one triangle lane (5211-5311), false when culled or off-tile */
@@ -615,33 +562,77 @@ k_tile_lights(const sftg_tile_args A, uint32_t tile0)
     }
 }
 
-/* the tile's 4x2 block that a resolve CTA's b-th block is: at 4x the CTAs of a tile take every
- * split-th block, so the costly ones (many triangles, many lights) spread over all of them
- * (measured on the atrium at 4x: the slowest CTA of a tile took twice the mean with contiguous
- * ranges); at 1x and 2x a contiguous range of rows keeps each CTA's surface points close together,
- * which tightens the per-CTA proxy filter */
-template <int S>
-SFTG_D int block_of(int part, int split, int nblk, int b) { return S == 4 ? b * split + part : part * nblk + b; }
 #define TILE_BLOCKS (16 * 32)                 /* 4x2 blocks per 64x64 tile; a CTA resolves 1/split of them */
+#define RESOLVE_WARPS (TILE_THREADS / 32)
+#define LIGHT_SLOTS (SFTG_MAX_TILE_LIGHTS * SFTG_MAX_LIGHT_PROXIES)
 
-/* One CTA per quarter tile: tile light list (5855-5934) and proxy cache (5936-5990), then one
- * 8-thread group per 4x2 block for the per-triangle shading and MSAA resolve (6029-6745). */
+/* A warp resolves `set` neighbouring 4x2 blocks at a time: up to max_set, fewer where a tile's
+ * split leaves its 8 warps less.  Its fragments (covered pixel, distinct triangle) number at most
+ * max_set * 8 * S; a chunk of 32 is closed when the next (block, triangle) pair does not fit, so
+ * it holds at least 25 of them, which bounds the chunks. */
+template <int S> struct resolve_plan {
+    static constexpr int max_set = S == 1 ? 16 : 8;
+    static constexpr int pixels = max_set * 8, chunks = pixels * S / 25 + 2, cap = chunks * 32;
+};
+
+/* A fragment: bits 0-2 pixel of its 4x2 block, 3-6 block of the set, 7-9 samples hit, 10-11 how
+ * many triangles of the block covered this pixel before it, 12-16 lane where its (block, triangle)
+ * pair starts, 17-24 the pair's covered pixels; FRAG_NONE pads a chunk. */
+#define FRAG_NONE 0x80000000u
+
+/* the OR of v over the lanes [start, end) of this lane's pair (at most 8 lanes, any offset) */
+SFTG_D uint32_t pair_or(uint32_t v, int lane, int start, int end) {
+    uint32_t t = __shfl_down_sync(0xFFFFFFFFu, v, 1); if (lane + 1 < end) v |= t;
+    t = __shfl_down_sync(0xFFFFFFFFu, v, 2); if (lane + 2 < end) v |= t;
+    t = __shfl_down_sync(0xFFFFFFFFu, v, 4); if (lane + 4 < end) v |= t;
+    return __shfl_sync(0xFFFFFFFFu, v, start);
+}
+
+SFTG_D float warp_min(float v) { float r; asm volatile("redux.sync.min.f32 %0, %1, 0xffffffff;" : "=f"(r) : "f"(v)); return r; }
+SFTG_D float warp_max(float v) { float r; asm volatile("redux.sync.max.f32 %0, %1, 0xffffffff;" : "=f"(r) : "f"(v)); return r; }
+
+/* Bound by instruction issue.  With 8 lanes on each (block, triangle) pair, covered or not, 24 of 32
+ * threads were active and a frame of few tiles waited for the block with the most triangles; a
+ * lane per covered fragment and the proxies selected per 32 fragments instead of per CTA (which
+ * also took a second interpolation of every pixel) measured: skinned characters 1080p 2x 0.252 ->
+ * 0.172 ms, atrium 1080p 4x 0.541 -> 0.381, atrium 1279x719 1x 0.272 -> 0.103, mixed materials
+ * 1333x717 2x 0.213 -> 0.143, skinned 320x180 2x 0.516 -> 0.074, a batch of 48 views 12.3 -> 8.0.
+ * Sets of 16 blocks at 2x cost 3-15 %, contiguous sets per CTA at 4x 7 %.
+ *
+ * One (tile, part) item, run by one CTA.  The CTA makes the tile's light list and proxy cache
+ * (5855-5990); then each warp resolves its sets of 4x2 blocks on its own (6029-6745):
+ *   peel     one 8-thread group per block finds the block's distinct triangles in the reference's
+ *            order and appends a fragment per covered pixel to the warp's list, four blocks at once
+ *   shade    a lane per fragment, 32 at a time.  The reference shades the block's 8 pixels for
+ *            every triangle; only covered pixels reach the image, and what the block shares is the
+ *            LOD (the first covered pixel's derivatives: its neighbours' texture coordinates come
+ *            from their lanes or are interpolated again) and the set of proxies that some covered
+ *            pixel's segment to the light comes near (an OR over the pair's lanes)
+ *   blend    a pixel's fragments follow one another in peel order, so the MSAA sum is accumulated
+ *            in the reference's order
+ * Uncovered pixels also keep a light from being skipped for their block.  That shows only where a
+ * covered pixel's zero attenuation meets a value that is not finite (a light's colour, a proxy of
+ * zero size, an interpolated position): such chunks are shaded again 8 lanes per pair, the
+ * uncovered pixels among them, as the reference does (`full` below). */
 template <int S>
 SFTG_D void resolve_item(const sftg_tile_args& A, uint32_t tile0, int split, bool records, uint32_t item)
 {
-    __shared__ proxy_cache pcache[SFTG_MAX_TILE_LIGHTS * SFTG_MAX_LIGHT_PROXIES];
-    /* the per-lane "between" test's operands of each cached proxy, in pcache's order: W (proxy
-     * centre minus light) with |W|^2 as one 16-byte load, and the squared bounding radius */
-    __shared__ float4 s_btw[SFTG_MAX_TILE_LIGHTS * SFTG_MAX_LIGHT_PROXIES];
-    __shared__ float s_rb2[SFTG_MAX_TILE_LIGHTS * SFTG_MAX_LIGHT_PROXIES];
+    using plan = resolve_plan<S>;
+    /* proxy cache, entry light * 16 + slot: pa with |ab|^2, ab with radius^2, visibility factor; for
+     * the per-lane "between" test W (proxy centre minus light) with |W|^2 and the squared bounding
+     * radius; for the chunk filter the bounding radius grown by its share of the rounding margin */
+    __shared__ float4 s_pa[LIGHT_SLOTS], s_ab[LIGHT_SLOTS], s_btw[LIGHT_SLOTS];
+    __shared__ float s_vm[LIGHT_SLOTS], s_rb2[LIGHT_SLOTS], s_rbm[LIGHT_SLOTS];
     __shared__ uint16_t s_lights[SFTG_MAX_TILE_LIGHTS];
-    __shared__ sftg_point_light s_pl[SFTG_MAX_TILE_LIGHTS];   /* the tile's lights, in list order */
-    __shared__ int s_nlights;
+    __shared__ float4 s_lp[SFTG_MAX_TILE_LIGHTS], s_lc[SFTG_MAX_TILE_LIGHTS];   /* position with 1/r^2, colour */
+    __shared__ int s_nlights, s_odd;
     __shared__ uint8_t s_npc[SFTG_MAX_TILE_LIGHTS];
+    __shared__ uint32_t s_meta[RESOLVE_WARPS][plan::cap], s_vid[RESOLVE_WARPS][plan::cap];
+    __shared__ float s_acc[RESOLVE_WARPS][S > 1 ? plan::pixels * 3 : 1];
+    __shared__ uint32_t s_wm[RESOLVE_WARPS][SFTG_MAX_TILE_LIGHTS / 2];
 
     const uint32_t gtile = A.tile_order[tile0 + item / (uint32_t)split];   /* batch-wide tile index, heaviest first */
     const int part = (int)(item % (uint32_t)split);
-    const int nblk = TILE_BLOCKS / split;
     const sftg_frame* F = A.frames + A.tile_view[gtile];
     const int tile = (int)(gtile - F->tile_base);
     const float* ss = A.ss + (size_t)F->ss_base * SFTG_SS_FLOATS;
@@ -652,102 +643,72 @@ SFTG_D void resolve_item(const sftg_tile_args& A, uint32_t tile0, int split, boo
     float* shadow_out = A.shadow_out;
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
     const int tmx = (tile % F->cols) * SFTG_TILE, tmy = (tile / F->cols) * SFTG_TILE;
-    const float2 zr = tile_zrange(A.zrange, gtile);
-    const float zmin = zr.x, zmax = zr.y;
     const float2* vis = A.vis + F->vis_base + (size_t)tile * S * SFTG_TILE_PX;
 
     const sftg_tile_lights* TL = A.tile_lights + gtile;
+    if (tid == 0) s_odd = shadow_out != nullptr;
     if (records) {   /* D2 and D3's selection come from the tile's record (k_tile_lights) */
         if (tid < SFTG_MAX_TILE_LIGHTS) { s_lights[tid] = TL->light[tid]; s_npc[tid] = TL->npc[tid]; }
         if (tid == 0) s_nlights = (int)TL->nlights;
-    } else {
-        if (warp == 0) {   /* D2 */
-            const int n = tile_light_list(F, zmin, zmax, tmx, tmy, lane, s_lights);
-            if (lane == 0) {
-                s_nlights = n;
-                if (part == 0) A.tile_nlights[gtile] = (uint8_t)n;
-            }
+    } else if (warp == 0) {   /* D2 */
+        const float2 zr = tile_zrange(A.zrange, gtile);
+        const int n = tile_light_list(F, zr.x, zr.y, tmx, tmy, lane, s_lights);
+        if (lane == 0) {
+            s_nlights = n;
+            if (part == 0) A.tile_nlights[gtile] = (uint8_t)n;
         }
     }
     __syncthreads();
     const int ntl = s_nlights;
-    if (tid < ntl) s_pl[tid] = F->point[s_lights[tid]];
-
-    /* World box of every surface point this CTA shades (per covered pixel and distinct sample
-     * triangle, interpolated as the shading loop does), for the proxy filter below. */
-    __shared__ float s_bnd[TILE_THREADS / 32][6];
-    const int sw = (int)(F->hw * 2.f), sh = (int)(F->hh * 2.f);
-    const int lim_x = min(tmx + SFTG_TILE, sw), lim_y = min(tmy + SFTG_TILE, sh);
-    const bool cull_proxies = F->shadows && F->n_proxies > 0 && ntl > 0;
-    if (cull_proxies) {
-        float mn[3] = { 1e30f, 1e30f, 1e30f }, mx[3] = { -1e30f, -1e30f, -1e30f };
-        uint32_t last = SFTG_INVALID;
-        const int ix0 = tid & 3, iy0 = (tid >> 2) & 1;
-        for (int b = tid >> 3; b < nblk; b += TILE_THREADS / 8) {
-            const int blk = block_of<S>(part, split, nblk, b);
-            const int gx = tmx + (blk & 15) * 4 + ix0, gy = tmy + (blk >> 4) * 2 + iy0;
-            if (gx >= lim_x || gy >= lim_y) continue;
-            const int pind = (gy - tmy) * SFTG_TILE + (gx - tmx);
-            const float pxf = ((float)(gx - ix0) + 0.5f) + (float)ix0, pyf = ((float)(gy - iy0) + 0.5f) + (float)iy0;
-            last = SFTG_INVALID;
-#pragma unroll
-            for (int s = 0; s < S; s++) {
-                const uint32_t vid = __float_as_uint(vis[s * SFTG_TILE_PX + pind].y);
-                if (vid != SFTG_INVALID && vid != last) { last = vid; pixel_pos_acc<S>(F, ss, clips, vid, pxf, pyf, mn, mx); }
-            }
-        }
-#pragma unroll
-        for (int o = 16; o; o >>= 1)
-#pragma unroll
-            for (int a = 0; a < 3; a++) {
-                mn[a] = fminf(mn[a], __shfl_xor_sync(0xFFFFFFFFu, mn[a], o));
-                mx[a] = fmaxf(mx[a], __shfl_xor_sync(0xFFFFFFFFu, mx[a], o));
-            }
-        if (lane == 0) { s_bnd[warp][0] = mn[0]; s_bnd[warp][1] = mn[1]; s_bnd[warp][2] = mn[2]; s_bnd[warp][3] = mx[0]; s_bnd[warp][4] = mx[1]; s_bnd[warp][5] = mx[2]; }
+    /* `odd`: a light or proxy with which a product with zero could be other than zero */
+    if (tid < ntl) {
+        const sftg_point_light L = F->point[s_lights[tid]];
+        s_lp[tid] = make_float4(L.pos[0], L.pos[1], L.pos[2], L.inv_radius_sqr);
+        s_lc[tid] = make_float4(L.color[0], L.color[1], L.color[2], 0.f);
+        if (!(fabsf(L.pos[0]) + fabsf(L.pos[1]) + fabsf(L.pos[2]) <= 1e15f && fabsf(L.color[0]) + fabsf(L.color[1]) + fabsf(L.color[2]) <= 1e30f &&
+              L.inv_radius_sqr >= 0.f && L.inv_radius_sqr <= 1e30f)) s_odd = 1;
     }
-
-    if (records) {
-        /* D3's proxy cache (5936-5990): the tile's selected proxies, one thread per (light, slot), the
-         * entries computed as the selection computed them */
-        for (int t = tid; t < SFTG_MAX_TILE_LIGHTS * SFTG_MAX_LIGHT_PROXIES; t += TILE_THREADS) {
+    /* D3's cache entry of proxy p in slot t (5936-5990) */
+    auto cache = [&](int t, const sftg_proxy& px, uint8_t vs, const sftg_point_light& L, v3 ab, v3 Wv, float br, float d2) {
+        s_pa[t] = make_float4(px.posa[0], px.posa[1], px.posa[2], sdot(ab, ab));
+        s_ab[t] = make_float4(ab.x, ab.y, ab.z, px.radius * px.radius);
+        s_vm[t] = (float)vs * 0.3333333f;
+        s_btw[t] = make_float4(Wv.x, Wv.y, Wv.z, d2);
+        s_rb2[t] = br * br;
+        s_rbm[t] = sqrtf(br * br) + 2e-3f * sqrtf(d2) + 1e-3f + 1e-6f * (fabsf(L.pos[0]) + fabsf(L.pos[1]) + fabsf(L.pos[2]));
+        if (!(fabsf(px.posa[0]) + fabsf(px.posa[1]) + fabsf(px.posa[2]) + fabsf(px.posb[0]) + fabsf(px.posb[1]) + fabsf(px.posb[2]) <= 1e15f &&
+              px.radius >= 1e-15f && px.radius <= 1e15f)) s_odd = 1;
+    };
+    if (records) {   /* the tile's selected proxies, one thread per (light, slot) */
+        for (int t = tid; t < LIGHT_SLOTS; t += TILE_THREADS) {
             const int i = t / SFTG_MAX_LIGHT_PROXIES, k = t % SFTG_MAX_LIGHT_PROXIES;
             if (i >= ntl || k >= s_npc[i]) continue;
             const uint32_t p = TL->proxy[i][k];
-            const sftg_point_light L = F->point[s_lights[i]];   /* s_pl is read only after the next barrier */
+            const sftg_point_light L = F->point[s_lights[i]];   /* s_lp is read only after the next barrier */
             const sftg_proxy px = F->proxies[p];
             const uint8_t vs = light_vis[(size_t)p * 64 + s_lights[i]];
             const v3 cc = mk3((px.posa[0] + px.posb[0]) * 0.5f, (px.posa[1] + px.posb[1]) * 0.5f, (px.posa[2] + px.posb[2]) * 0.5f);
             const v3 ab = mk3(px.posb[0] - px.posa[0], px.posb[1] - px.posa[1], px.posb[2] - px.posa[2]);
-            const float cl = fsqrt(sdot(ab, ab));
-            const float br = px.radius + (cl * 0.5f);
+            const float br = px.radius + (fsqrt(sdot(ab, ab)) * 0.5f);
             const v3 Wv = sub3(cc, mk3(L.pos[0], L.pos[1], L.pos[2]));
-            const float d2 = sdot(Wv, Wv);
-            proxy_cache* q = &pcache[t];
-            q->pa[0] = px.posa[0]; q->pa[1] = px.posa[1]; q->pa[2] = px.posa[2];
-            q->pb[0] = px.posb[0]; q->pb[1] = px.posb[1]; q->pb[2] = px.posb[2];
-            q->ab[0] = ab.x; q->ab[1] = ab.y; q->ab[2] = ab.z;
-            q->W[0] = Wv.x; q->W[1] = Wv.y; q->W[2] = Wv.z;
-            q->abdab = sdot(ab, ab); q->wdw = d2; q->rb2 = br * br; q->pr = px.radius; q->pr2 = px.radius * px.radius;
-            q->vis_mult = (float)vs * 0.3333333f;
-            s_btw[t] = make_float4(Wv.x, Wv.y, Wv.z, d2);
-            s_rb2[t] = q->rb2;
+            cache(t, px, vs, L, ab, Wv, br, sdot(Wv, Wv));
         }
     } else {
         /* D3: per light, the first 16 proxies that see it and can reach it (5936-5990) */
-        for (int i = warp; i < SFTG_MAX_TILE_LIGHTS; i += TILE_THREADS / 32) {
+        for (int i = warp; i < SFTG_MAX_TILE_LIGHTS; i += RESOLVE_WARPS) {
             int n = 0;
             if (i < ntl && F->shadows && F->n_proxies > 0) {
                 const sftg_point_light L = F->point[s_lights[i]];
                 for (uint32_t base = 0; base < F->n_proxies && n < SFTG_MAX_LIGHT_PROXIES; base += 32) {
                     const uint32_t p = base + lane;
                     bool take = false; uint8_t vs = 0;
-                    v3 cc, ab, Wv; float br = 0.f, d2 = 0.f;
+                    v3 ab, Wv; float br = 0.f, d2 = 0.f;
                     sftg_proxy px;
                     if (p < F->n_proxies) {
                         px = F->proxies[p];
                         vs = light_vis[(size_t)p * 64 + s_lights[i]];
                         if (vs) {
-                            cc = mk3((px.posa[0] + px.posb[0]) * 0.5f, (px.posa[1] + px.posb[1]) * 0.5f, (px.posa[2] + px.posb[2]) * 0.5f);
+                            const v3 cc = mk3((px.posa[0] + px.posb[0]) * 0.5f, (px.posa[1] + px.posb[1]) * 0.5f, (px.posa[2] + px.posb[2]) * 0.5f);
                             ab = mk3(px.posb[0] - px.posa[0], px.posb[1] - px.posa[1], px.posb[2] - px.posa[2]);
                             const float cl = fsqrt(sdot(ab, ab));
                             br = px.radius + (cl * 0.5f);
@@ -759,17 +720,7 @@ SFTG_D void resolve_item(const sftg_tile_args& A, uint32_t tile0, int split, boo
                     }
                     const uint32_t bal = __ballot_sync(0xFFFFFFFFu, take);
                     const int rank = __popc(bal & ((1u << lane) - 1u));
-                    if (take && n + rank < SFTG_MAX_LIGHT_PROXIES) {
-                        proxy_cache* q = &pcache[i * SFTG_MAX_LIGHT_PROXIES + n + rank];
-                        q->pa[0] = px.posa[0]; q->pa[1] = px.posa[1]; q->pa[2] = px.posa[2];
-                        q->pb[0] = px.posb[0]; q->pb[1] = px.posb[1]; q->pb[2] = px.posb[2];
-                        q->ab[0] = ab.x; q->ab[1] = ab.y; q->ab[2] = ab.z;
-                        q->W[0] = Wv.x; q->W[1] = Wv.y; q->W[2] = Wv.z;
-                        q->abdab = sdot(ab, ab); q->wdw = d2; q->rb2 = br * br; q->pr = px.radius; q->pr2 = px.radius * px.radius;
-                        s_btw[i * SFTG_MAX_LIGHT_PROXIES + n + rank] = make_float4(Wv.x, Wv.y, Wv.z, d2);
-                        s_rb2[i * SFTG_MAX_LIGHT_PROXIES + n + rank] = q->rb2;
-                        q->vis_mult = (float)vs * 0.3333333f;
-                    }
+                    if (take && n + rank < SFTG_MAX_LIGHT_PROXIES) cache(i * SFTG_MAX_LIGHT_PROXIES + n + rank, px, vs, L, ab, Wv, br, d2);
                     n = min(SFTG_MAX_LIGHT_PROXIES, n + __popc(bal));
                 }
             }
@@ -778,176 +729,207 @@ SFTG_D void resolve_item(const sftg_tile_args& A, uint32_t tile0, int split, boo
     }
     __syncthreads();
 
-    /* Conservative filter of the cached proxies (order kept).  Every pixel this CTA shades lies
-     * in the ball (Bc, Br) around the bounds above.  The per-block skip (6520-6540) drops a
-     * proxy unless some lane's segment pixel -> light passes within the proxy's bounding radius
-     * of its centre; for pixels in the ball that segment stays within Br of the segment
-     * Bc -> light.  So a proxy farther than rb + Br (+ a rounding margin) from that segment is
-     * skipped by every block, and removing it here leaves every pixel unchanged. */
-    if (cull_proxies) {
-        float mn[3], mx[3];
-#pragma unroll
-        for (int a = 0; a < 3; a++) { mn[a] = s_bnd[0][a]; mx[a] = s_bnd[0][3 + a]; }
-        for (int w = 1; w < TILE_THREADS / 32; w++)
-#pragma unroll
-            for (int a = 0; a < 3; a++) { mn[a] = fminf(mn[a], s_bnd[w][a]); mx[a] = fmaxf(mx[a], s_bnd[w][3 + a]); }
-        const bool empty = !(mn[0] <= mx[0] && mn[1] <= mx[1] && mn[2] <= mx[2]);
-        const v3 bc = mk3((mn[0] + mx[0]) * 0.5f, (mn[1] + mx[1]) * 0.5f, (mn[2] + mx[2]) * 0.5f);
-        const v3 he = mk3((mx[0] - mn[0]) * 0.5f, (mx[1] - mn[1]) * 0.5f, (mx[2] - mn[2]) * 0.5f);
-        const float br = sqrtf(he.x * he.x + he.y * he.y + he.z * he.z);
-        const bool usable = isfinite(br) && isfinite(bc.x) && isfinite(bc.y) && isfinite(bc.z);
-        for (int i = warp; i < ntl; i += TILE_THREADS / 32) {
-            const int n = s_npc[i];
-            if (n == 0 || (usable == false && !empty)) continue;
-            const sftg_point_light L = F->point[s_lights[i]];
-            bool keep = false;
-            proxy_cache q;
-            if (lane < n) {
-                q = pcache[i * SFTG_MAX_LIGHT_PROXIES + lane];
-                if (!empty) {
-                    const v3 Wv = mk3(q.W[0], q.W[1], q.W[2]);
-                    const v3 D = mk3(bc.x - L.pos[0], bc.y - L.pos[1], bc.z - L.pos[2]);
-                    const float dd = D.x * D.x + D.y * D.y + D.z * D.z;
-                    const float t = dd > 0.f ? fminf(fmaxf((Wv.x * D.x + Wv.y * D.y + Wv.z * D.z) / dd, 0.f), 1.f) : 0.f;
-                    const v3 E = mk3(Wv.x - t * D.x, Wv.y - t * D.y, Wv.z - t * D.z);
-                    const float dist = sqrtf(E.x * E.x + E.y * E.y + E.z * E.z);
-                    const float m = 2e-3f * (sqrtf(q.wdw) + sqrtf(dd) + br) + 1e-3f;
-                    keep = !(dist > sqrtf(q.rb2) + br + m);
-                }
-            }
-            const uint32_t bal = __ballot_sync(0xFFFFFFFFu, keep);
-            __syncwarp();
-            if (keep) {
-                const int k = i * SFTG_MAX_LIGHT_PROXIES + __popc(bal & ((1u << lane) - 1u));
-                pcache[k] = q;
-                s_btw[k] = make_float4(q.W[0], q.W[1], q.W[2], q.wdw);
-                s_rb2[k] = q.rb2;
-            }
-            if (lane == 0) s_npc[i] = (uint8_t)__popc(bal);
-        }
-        __syncthreads();
-    }
-
-    /* ---------------- resolve: one 8-thread group per 4x2 block ---------------- */
     const int W = F->width;
-    const int grp = tid >> 3, gl = tid & 7, gshift = lane & ~7;
-    const uint32_t gmask = 0xFFu << gshift;
-    const int ix = gl & 3, iy = gl >> 2;
+    const int sw = (int)(F->hw * 2.f), sh = (int)(F->hh * 2.f);
+    const int lim_x = min(tmx + SFTG_TILE, sw), lim_y = min(tmy + SFTG_TILE, sh);
+    const bool proxies = F->shadows && F->n_proxies > 0 && ntl > 0;
+    const bool clear = F->clear != 0;
+    const int gl = lane & 7, gshift = lane & ~7;
     const float inv_s = 1.f / (float)S;
+    const float i255 = 1.f / 255.f;
+    const int ix = gl & 3, iy = gl >> 2;
     const uint32_t cc = F->clear_color;
-    const float clr[3] = { (float)((cc >> 16) & 0xFF) * (1.f / 255.f), (float)((cc >> 8) & 0xFF) * (1.f / 255.f), (float)(cc & 0xFF) * (1.f / 255.f) };
-    const v3 cam = mk3(F->cam[0], F->cam[1], F->cam[2]);
+    uint32_t* const metas = s_meta[warp];
+    uint32_t* const vidl = s_vid[warp];
+    float* const accs = s_acc[warp];
+    uint32_t* const wm = s_wm[warp];
 
-    for (int b = grp; b < nblk; b += TILE_THREADS / 8) {
-        const int blk = block_of<S>(part, split, nblk, b);
-        const int x = tmx + (blk & 15) * 4, y = tmy + (blk >> 4) * 2;
-        if (x >= lim_x || y >= lim_y) continue;
-        const int gx = x + ix, gy = y + iy;
-        const bool inb = (sw > gx) && (sh > gy);
-        const int pind = (gy - tmy) * SFTG_TILE + (gx - tmx);
-        const float pxf = ((float)x + 0.5f) + (float)ix, pyf = ((float)y + 0.5f) + (float)iy;
-        uint32_t vids[S];
-        uint32_t asm_[S];
-        int ecount = 0;
+    /* the CTA's 512 / split blocks in sets of `set`: a set is 2 or 4 blocks wide */
+    const int set = min(plan::max_set, TILE_BLOCKS / RESOLVE_WARPS / split);   /* 4, 8 or 16: split is at most 16 */
+    const int bw = set >= 8 ? 4 : 2, across = 16 / bw, bh = set / bw;
+    const int nsets = TILE_BLOCKS / set / split;
+    for (int q0 = warp; q0 < nsets; q0 += RESOLVE_WARPS) {
+        const int q = S == 4 ? q0 * split + part : part * nsets + q0;
+        const int X0 = tmx + (q % across) * bw * 4, Y0 = tmy + (q / across) * bh * 2;
+        if (X0 >= lim_x || Y0 >= lim_y) continue;   /* whole warp */
+
+        /* ---------------- peel ---------------- */
+        int cur = 0;             /* list position, uniform over the warp */
+        uint32_t stores = 0;     /* bit k: this lane's pixel of its k-th block is written at the end */
+        for (int k = 0; k < set / 4; k++) {
+            const int bl = k * 4 + (lane >> 3);
+            const int x = X0 + (bl % bw) * 4, y = Y0 + (bl / bw) * 2;
+            const int gx = x + ix, gy = y + iy;
+            const bool inb = sw > gx && sh > gy && x < lim_x && y < lim_y;
+            const int pind = (gy - tmy) * SFTG_TILE + (gx - tmx);
+            uint32_t vids[S], open[S];
+            int ecount = 0;
+            uint32_t act = 0;
 #pragma unroll
-        for (int s = 0; s < S; s++) {
-            vids[s] = __float_as_uint(vis[s * SFTG_TILE_PX + pind].y);
-            const bool empty = vids[s] == SFTG_INVALID;
-            asm_[s] = (__ballot_sync(gmask, !empty && inb) >> gshift) & 0xFFu;
-            ecount += (empty && inb);
-        }
-        uint32_t act = 0;
-#pragma unroll
-        for (int s = 0; s < S; s++) act |= asm_[s];
-        float acc[3] = { 0.f, 0.f, 0.f };
-        if (S == 1) {
-            if (F->clear && inb && vids[0] == SFTG_INVALID) color[gy * CP + gx] = cc;
-        } else {
-            if (!act) {
-                if (F->clear && inb) color[gy * CP + gx] = cc;
-                continue;
+            for (int s = 0; s < S; s++) {
+                vids[s] = __float_as_uint(vis[s * SFTG_TILE_PX + pind].y);
+                const bool empty = vids[s] == SFTG_INVALID;
+                open[s] = (__ballot_sync(0xFFFFFFFFu, !empty && inb) >> gshift) & 0xFFu;
+                ecount += (empty && inb);
+                act |= open[s];
             }
-            const float ew = (float)ecount * inv_s;
-            const bool any_e = (__ballot_sync(gmask, ew > 0.f) & gmask) != 0;
-            if (F->clear) { acc[0] = clr[0] * ew; acc[1] = clr[1] * ew; acc[2] = clr[2] * ew; }
-            else if (any_e) {
-                float bg[3] = { 0.f, 0.f, 0.f };
-                if (gx < sw && gy < sh) {
-                    const uint32_t q = color[gy * CP + gx];
-                    bg[0] = (float)((q >> 16) & 0xFF) * (1.f / 255.f); bg[1] = (float)((q >> 8) & 0xFF) * (1.f / 255.f); bg[2] = (float)(q & 0xFF) * (1.f / 255.f);
-                }
-                acc[0] = bg[0] * ew; acc[1] = bg[1] * ew; acc[2] = bg[2] * ew;
-            }
-        }
-        const uint32_t block_write = act;
-        while (act) {
-            uint32_t target, tri_mask = 0, tri_lanes = 0; int hits = 0;
             if (S == 1) {
-                const int fl = __ffs(act) - 1;
-                target = __shfl_sync(gmask, vids[0], gshift + fl);
-                tri_mask = (__ballot_sync(gmask, vids[0] == target && inb) >> gshift) & 0xFFu;
-                tri_lanes = tri_mask & act;
-                act &= ~tri_lanes;
-            } else {
-                int fs = 0;
-                while (!asm_[fs]) fs++;
-                const int fl = __ffs(asm_[fs]) - 1;
-                uint32_t vsel = vids[0];
-#pragma unroll
-                for (int s = 1; s < S; s++) if (s == fs) vsel = vids[s];
-                target = __shfl_sync(gmask, vsel, gshift + fl);
-#pragma unroll
-                for (int s = 0; s < S; s++) {
-                    const bool match = vids[s] == target && inb;
-                    const uint32_t mb = (__ballot_sync(gmask, match) >> gshift) & 0xFFu;
-                    const uint32_t mm = mb & asm_[s];
-                    asm_[s] &= ~mm; tri_lanes |= mm; tri_mask |= mb;
-                    hits += match;
+                if (clear && inb && vids[0] == SFTG_INVALID) color[gy * CP + gx] = cc;
+            } else if (!act) {
+                if (clear && inb) color[gy * CP + gx] = cc;
+            } else {   /* the empty samples' share of the background */
+                const float ew = (float)ecount * inv_s;
+                float bg[3] = { 0.f, 0.f, 0.f };
+                if (clear || (ew > 0.f && inb)) {
+                    const uint32_t c = clear ? cc : color[gy * CP + gx];
+                    bg[0] = (float)((c >> 16) & 0xFF) * i255; bg[1] = (float)((c >> 8) & 0xFF) * i255; bg[2] = (float)(c & 0xFF) * i255;
                 }
+#pragma unroll
+                for (int c = 0; c < 3; c++) accs[(bl * 8 + gl) * 3 + c] = bg[c] * ew;
+                stores |= (uint32_t)(clear ? inb : ((act >> gl) & 1u)) << k;
+            }
+            uint32_t nj = 0;     /* triangles that covered this pixel so far */
+            while (__any_sync(0xFFFFFFFFu, act != 0)) {
+                /* the group's next triangle: the first covered pixel of its first sample plane with any left */
+                const bool have = act != 0;
+                uint32_t vsel = vids[0], osel = open[0];
+#pragma unroll
+                for (int s = 1; s < S; s++) if (!osel) { osel = open[s]; vsel = vids[s]; }
+                const uint32_t target = __shfl_sync(0xFFFFFFFFu, vsel, gshift + (have ? __ffs(osel) - 1 : 0));
+                uint32_t mask = 0, hits = 0;
                 act = 0;
 #pragma unroll
-                for (int s = 0; s < S; s++) act |= asm_[s];
+                for (int s = 0; s < S; s++) {
+                    const bool match = have && inb && vids[s] == target;
+                    const uint32_t mb = (__ballot_sync(0xFFFFFFFFu, match) >> gshift) & 0xFFu;
+                    open[s] &= ~mb; mask |= mb; act |= open[s];
+                    hits += match;
+                }
+                /* places for the four groups' pairs; a pair does not straddle two chunks */
+                const int n = __popc(mask);
+                int at = 0;
+#pragma unroll
+                for (int g = 0; g < 4; g++) {
+                    const int ng = __shfl_sync(0xFFFFFFFFu, n, g * 8);
+                    if ((cur & 31) + ng > 32) {
+                        const int nx = (cur + 31) & ~31;
+                        if (cur + lane < nx) metas[cur + lane] = FRAG_NONE;
+                        cur = nx;
+                    }
+                    if (g == (lane >> 3)) at = cur;
+                    cur += ng;
+                }
+                if ((mask >> gl) & 1u) {
+                    const int pos = at + __popc(mask & ((1u << gl) - 1u));
+                    metas[pos] = (uint32_t)gl | (uint32_t)bl << 3 | hits << 7 | nj << 10 | (uint32_t)(at & 31) << 12 | mask << 17;
+                    vidl[pos] = target;
+                    nj++;
+                }
             }
-            const bool in_tri = (tri_mask >> gl) & 1u;
+        }
+        if (cur & 31) {
+            const int nx = (cur + 31) & ~31;
+            if (cur + lane < nx) metas[cur + lane] = FRAG_NONE;
+            cur = nx;
+        }
+        __syncwarp();
+
+        /* ---------------- shade ---------------- */
+        bool full = s_odd != 0;   /* 8 lanes per pair, uncovered pixels among them */
+        int pass = 0;             /* with `full`: which four of the chunk's pairs */
+        for (int c0 = 0; c0 < cur; ) {
+            uint32_t meta = metas[c0 + lane];
+            uint32_t vid;
+            int start, end, pl, npass = 1;
+            bool in_tri;
+            if (!full) {
+                in_tri = !(meta & FRAG_NONE);
+                if (!in_tri) meta = metas[c0];     /* a padding lane repeats the first fragment, without effect */
+                vid = vidl[in_tri ? c0 + lane : c0];
+                start = in_tri ? (int)((meta >> 12) & 31u) : lane;
+                end = in_tri ? start + __popc((meta >> 17) & 0xFFu) : lane + 1;
+                pl = (int)(meta & 7u);
+            } else {
+                uint32_t lead = __ballot_sync(0xFFFFFFFFu, !(meta & FRAG_NONE) && ((meta >> 12) & 31u) == (uint32_t)lane);
+                npass = (__popc(lead) + 3) / 4;
+                int src = 0;
+                bool have = false;
+                for (int k = 0; k <= pass * 4 + (lane >> 3); k++) { have = lead != 0; if (have) src = __ffs(lead) - 1; lead &= lead - 1; }
+                const uint32_t mask = (metas[c0 + src] >> 17) & 0xFFu;
+                in_tri = have && ((mask >> gl) & 1u);
+                meta = metas[c0 + src + (in_tri ? __popc(mask & ((1u << gl) - 1u)) : 0)];
+                vid = vidl[c0 + src];
+                start = gshift; end = gshift + 8;
+                pl = gl;
+            }
+            const int bl = (int)((meta >> 3) & 15u);
+            const int x = X0 + (bl % bw) * 4, y = Y0 + (bl / bw) * 2;
+            const int gx = x + (pl & 3), gy = y + (pl >> 2);
+            const float pxf = ((float)x + 0.5f) + (float)(pl & 3), pyf = ((float)y + 0.5f) + (float)(pl >> 2);
             tri_verts T;
-            fetch_tri(F, ss, clips, target, T);
-            const sftg_inst* I = &F->inst[T.inst];
-            const sftg_meshlet_info info = F->ml_info[I->meshlet_base + T.m];
+            fetch_tri(F, ss, clips, vid, T);
+            const sftg_meshlet_info info = F->ml_info[F->inst[T.inst].meshlet_base + T.m];
             /* D6 barycentrics and perspective-correct interpolation (6282-6347) */
             const float dx1 = T.sx[1] - T.sx[0], dx2 = T.sx[2] - T.sx[0], dy1 = T.sy[1] - T.sy[0], dy2 = T.sy[2] - T.sy[0];
             const float idet = rcpr(dx1 * dy2 - dx2 * dy1);
-            const float pxs = pxf - T.sx[0], pys = pyf - T.sy[0];
-            const float rbu = (pxs * dy2 - pys * dx2) * idet;
-            const float rbv = (pys * dx1 - pxs * dy1) * idet;
-            const float rbw = (1.f - rbu) - rbv;
-            float bu = rbu, bv = rbv, bw = rbw;
-            if (S > 1) {
-                bu = vmax(0.f, rbu); bv = vmax(0.f, rbv); bw = vmax(0.f, rbw);
-                const float bs = rcpr(bu + (bv + bw));
-                bu = bu * bs; bv = bv * bs; bw = bw * bs;
-            }
-            const float iz = fma_(bw, T.iw[0], fma_(bu, T.iw[1], bv * T.iw[2]));
-            const float z = rcpr(iz);
-            const float w0 = (bw * T.iw[0]) * z, w1 = (bu * T.iw[1]) * z, w2 = (bv * T.iw[2]) * z;
-#define INTERP(a) fma_(w0, (a)[0], fma_(w1, (a)[1], w2 * (a)[2]))
-            const float cu = INTERP(T.u), cv = INTERP(T.v), clu = INTERP(T.lu), clv = INTERP(T.lv);
-            const v3 P = mk3(INTERP(T.px), INTERP(T.py), INTERP(T.pz));
-            const v3 N = vnorm_fast(mk3(INTERP(T.nx), INTERP(T.ny), INTERP(T.nz)));
-#undef INTERP
-            const v3 V = vnorm_fast(sub3(cam, P));
+            float bu, bv, bw_, w0, w1, w2;
+            auto weights = [&](float px, float py) {
+                const float pxs = px - T.sx[0], pys = py - T.sy[0];
+                const float rbu = (pxs * dy2 - pys * dx2) * idet;
+                const float rbv = (pys * dx1 - pxs * dy1) * idet;
+                const float rbw = (1.f - rbu) - rbv;
+                bu = rbu; bv = rbv; bw_ = rbw;
+                if (S > 1) {
+                    bu = vmax(0.f, rbu); bv = vmax(0.f, rbv); bw_ = vmax(0.f, rbw);
+                    const float bs = rcpr(bu + (bv + bw_));
+                    bu = bu * bs; bv = bv * bs; bw_ = bw_ * bs;
+                }
+                const float iz = fma_(bw_, T.iw[0], fma_(bu, T.iw[1], bv * T.iw[2]));
+                const float z = rcpr(iz);
+                w0 = (bw_ * T.iw[0]) * z; w1 = (bu * T.iw[1]) * z; w2 = (bv * T.iw[2]) * z;
+            };
             /* material (6350-6382) */
             uint32_t base = 0xFFFFFFFFu; int ti = -1; float shin = 4.f;
             if (info.material >= 0) { const sftg_mat mt = F->mats[info.material]; base = mt.base_color; ti = mt.tex; shin = mt.shininess; }
             if (F->debug_mode == 5) { ti = F->debug_tex; base = 0xFFFFFFFFu; }   /* checkerboard view (6373-6376) */
-            const float i255 = 1.f / 255.f;
-            const float bcol[3] = { (float)((base >> 16) & 0xFF) * i255, (float)((base >> 8) & 0xFF) * i255, (float)(base & 0xFF) * i255 };
-            /* D7 LOD from the first covered lane's derivatives (5501-5541) */
+#define INTERP(a) fma_(w0, (a)[0], fma_(w1, (a)[1], w2 * (a)[2]))
+            /* D7 LOD from the first covered lane's derivatives (5501-5541): its neighbours' coordinates from
+             * their lanes where the triangle covers them, else interpolated here */
+            const uint32_t mask = (meta >> 17) & 0xFFu;
+            const int fl = __ffs(mask) - 1;
+            const bool ok_x = full || ((mask >> (fl ^ 1)) & 1u), ok_y = full || ((mask >> (fl ^ 4)) & 1u);
+            float cu_x = 0.f, cv_x = 0.f, cu_y = 0.f, cv_y = 0.f;
+            if (__any_sync(0xFFFFFFFFu, ti >= 0 && !(ok_x && ok_y))) {
+                weights(((float)x + 0.5f) + (float)((fl ^ 1) & 3), ((float)y + 0.5f) + (float)(fl >> 2));
+                cu_x = INTERP(T.u); cv_x = INTERP(T.v);
+                weights(((float)x + 0.5f) + (float)(fl & 3), ((float)y + 0.5f) + (float)((fl ^ 4) >> 2));
+                cu_y = INTERP(T.u); cv_y = INTERP(T.v);
+            }
+            weights(pxf, pyf);
+            const float cu = INTERP(T.u), cv = INTERP(T.v), clu = INTERP(T.lu), clv = INTERP(T.lv);
+            const v3 P = mk3(INTERP(T.px), INTERP(T.py), INTERP(T.pz));
+            const v3 N = vnorm_fast(mk3(INTERP(T.nx), INTERP(T.ny), INTERP(T.nz)));
+#undef INTERP
+            if (!full && __any_sync(0xFFFFFFFFu, !(fabsf(P.x) + fabsf(P.y) + fabsf(P.z) <= 1e15f))) { full = true; continue; }
+            bool wire = false;
+            if (F->debug_mode == 1) {   /* wireframe view (6645-6671): edges where a barycentric is under its screen width */
+                const float dbu_dx = (0.f - dy2) * idet, dbu_dy = dx2 * idet;
+                const float dbv_dx = dy1 * idet, dbv_dy = (0.f - dx1) * idet;
+                const float fw_u = fabsf(dbu_dx) + fabsf(dbu_dy), fw_v = fabsf(dbv_dx) + fabsf(dbv_dy);
+                const float dbw_dx = 0.f - (dbu_dx + dbv_dx), dbw_dy = 0.f - (dbu_dy + dbv_dy);
+                const float fw_w = fabsf(dbw_dx) + fabsf(dbw_dy);
+                wire = bu < fw_u || bv < fw_v || bw_ < fw_w;
+            }
             int lod = 0;
             {
-                const int fl = __ffs(tri_mask) - 1;
-                const float cu_f = __shfl_sync(gmask, cu, gshift + fl), cv_f = __shfl_sync(gmask, cv, gshift + fl);
-                const float cu_x = __shfl_sync(gmask, cu, gshift + (fl ^ 1)), cv_x = __shfl_sync(gmask, cv, gshift + (fl ^ 1));
-                const float cu_y = __shfl_sync(gmask, cu, gshift + (fl ^ 4)), cv_y = __shfl_sync(gmask, cv, gshift + (fl ^ 4));
+                const int at_x = full ? gshift + (fl ^ 1) : start + __popc(mask & ((1u << (fl ^ 1)) - 1u));
+                const int at_y = full ? gshift + (fl ^ 4) : start + __popc(mask & ((1u << (fl ^ 4)) - 1u));
+                const int at_f = full ? gshift + fl : start;
+                const float cu_f = __shfl_sync(0xFFFFFFFFu, cu, at_f), cv_f = __shfl_sync(0xFFFFFFFFu, cv, at_f);
+                const float su_x = __shfl_sync(0xFFFFFFFFu, cu, at_x), sv_x = __shfl_sync(0xFFFFFFFFu, cv, at_x);
+                const float su_y = __shfl_sync(0xFFFFFFFFu, cu, at_y), sv_y = __shfl_sync(0xFFFFFFFFu, cv, at_y);
+                if (ok_x) { cu_x = su_x; cv_x = sv_x; }
+                if (ok_y) { cu_y = su_y; cv_y = sv_y; }
                 if (ti >= 0) {
                     const sftg_tex& tx = F->texs[ti];
                     const float ux = (cu_f - cu_x) * (float)tx.w, vx = (cv_f - cv_x) * (float)tx.h;
@@ -967,12 +949,14 @@ SFTG_D void resolve_item(const sftg_tile_args& A, uint32_t tile0, int split, boo
                 float tr, tg, tb;
                 if (lod > 1) sample_nearest(F, ti, lod, cu, cv, tr, tg, tb);
                 else sample_bilinear(F, ti, lod, cu, cv, tr, tg, tb);
-                out[0] = tr * bcol[0]; out[1] = tg * bcol[1]; out[2] = tb * bcol[2];
+                out[0] = tr * ((float)((base >> 16) & 0xFF) * i255); out[1] = tg * ((float)((base >> 8) & 0xFF) * i255);
+                out[2] = tb * ((float)(base & 0xFF) * i255);
             }
             const bool lm = info.lightmap_tex >= 0;
-            if (shin < 0.f) {
-                out[0] = out[0] * (-shin); out[1] = out[1] * (-shin); out[2] = out[2] * (-shin);
-            } else {
+            const bool lighted = !(shin < 0.f);
+            if (!lighted) { out[0] = out[0] * (-shin); out[1] = out[1] * (-shin); out[2] = out[2] * (-shin); }
+            if (__any_sync(0xFFFFFFFFu, lighted)) {
+                const v3 V = vnorm_fast(sub3(mk3(F->cam[0], F->cam[1], F->cam[2]), P));
                 const float sscale = ((shin + 8.f) / 8.f) * 0.04f;
                 float dif[3], spc[3] = { 0.f, 0.f, 0.f }, lms = 1.f;
                 if (lm) {
@@ -995,87 +979,105 @@ SFTG_D void resolve_item(const sftg_tile_args& A, uint32_t tile0, int split, boo
                         }
                     }
                 }
+                /* The chunk's own selection of the cached proxies, conservative: every shaded point lies in the
+                 * ball (bc, br) around the chunk's bounds, so its segment to a light stays within br of the
+                 * segment bc -> light, and a proxy farther than its bounding radius + br (+ a rounding margin)
+                 * from that segment passes no pixel's "between" test (6520-6540).  Bit k of a light's 16: slot k. */
+                uint32_t lb = ntl ? 0xFFFFFFFFu >> (32 - ntl) : 0u;   /* lights to visit */
+                if (!full && ntl) {
+                    uint32_t shadowing = 0;
+                    if (proxies) {
+                        const bool use = in_tri && lighted;
+                        const float lx = warp_min(use ? P.x : 1e30f), ly = warp_min(use ? P.y : 1e30f), lz = warp_min(use ? P.z : 1e30f);
+                        const float hx = warp_max(use ? P.x : -1e30f), hy = warp_max(use ? P.y : -1e30f), hz = warp_max(use ? P.z : -1e30f);
+                        const v3 bc = mk3((lx + hx) * 0.5f, (ly + hy) * 0.5f, (lz + hz) * 0.5f);
+                        const v3 he = mk3(hx - bc.x, hy - bc.y, hz - bc.z);
+                        const float br = sqrtf(he.x * he.x + he.y * he.y + he.z * he.z) * 1.002f +
+                                         1e-6f * (fabsf(bc.x) + fabsf(bc.y) + fabsf(bc.z));
+                        for (int i0 = 0; i0 < ntl; i0 += 2) {
+                            const int i = i0 + (lane >> 4), k = lane & 15;
+                            bool keep = false;
+                            if (i < ntl && k < s_npc[i]) {
+                                const float4 L = s_lp[i], Wv = s_btw[i * SFTG_MAX_LIGHT_PROXIES + k];
+                                const v3 D = mk3(bc.x - L.x, bc.y - L.y, bc.z - L.z);
+                                const float dd = D.x * D.x + D.y * D.y + D.z * D.z;
+                                const float t = dd > 0.f ? fminf(fmaxf(__fdividef(Wv.x * D.x + Wv.y * D.y + Wv.z * D.z, dd), 0.f), 1.f) : 0.f;
+                                const v3 E = mk3(Wv.x - t * D.x, Wv.y - t * D.y, Wv.z - t * D.z);
+                                const float r = s_rbm[i * SFTG_MAX_LIGHT_PROXIES + k] + br + 2e-3f * sqrtf(dd);
+                                keep = !(E.x * E.x + E.y * E.y + E.z * E.z > r * r);
+                            }
+                            const uint32_t bal = __ballot_sync(0xFFFFFFFFu, keep);
+                            if (lane == 0) wm[i0 >> 1] = bal;
+                            shadowing |= ((bal & 0xFFFFu) ? 1u : 0u) << i0 | ((bal >> 16) ? 2u : 0u) << i0;
+                        }
+                        __syncwarp();
+                    }
+                    /* a light no proxy shadows leaves a lightmapped surface as it is */
+                    if (__all_sync(0xFFFFFFFFu, lm || !in_tri || !lighted)) lb = shadowing;
+                }
                 /* D10 point lights and capsule shadows (6474-6607) */
-                /* A lightmapped surface and a light with no cached proxy: msh = 0, si = 1 and the
-                 * light multiplies lms by 1 - 0 * att, a no-op unless att is NaN (att is in [0, 1]
-                 * or NaN).  The reference's path below reaches that product only when some lane
-                 * of the block has att > 0 and some covered lane has a NaN att; such lights are
-                 * gathered as bits and applied after the loop (NaN absorbs the other factors, so
-                 * order does not matter).  Not used while per-light shadow factors are captured. */
-                const bool lm_quick = lm && shadow_out == nullptr;
-                uint32_t q_alive = 0, q_nan = 0;
-                for (int i = 0; i < ntl; i++) {
-                    const sftg_point_light& L = s_pl[i];
-                    const v3 Lr = sub3(mk3(L.pos[0], L.pos[1], L.pos[2]), P);
+                while (lb) {
+                    const int i = __ffs(lb) - 1;
+                    lb &= lb - 1;
+                    const float4 L = s_lp[i];
+                    const v3 Lr = sub3(mk3(L.x, L.y, L.z), P);
                     const float d2 = vdot(Lr, Lr);
-                    float att = vmax(0.f, fma_(-d2, L.inv_radius_sqr, 1.f));
+                    float att = vmax(0.f, fma_(-d2, L.w, 1.f));
                     att = att * att;
                     const bool alive = att > 0.f;
-                    if (lm_quick && s_npc[i] == 0) {
-                        q_alive |= (uint32_t)alive << i;
-                        q_nan |= (uint32_t)(in_tri && !(att <= 3.402823466e38f)) << i;
-                        continue;
-                    }
-                    if (!(__ballot_sync(gmask, alive) & gmask)) continue;
+                    /* a covered pixel out of the light's reach gets nothing from it; with `full`, not skipped
+                     * while any pixel of the block is in reach */
+                    bool go = alive;
+                    if (full) go = pair_or(alive, lane, start, end) != 0;
+                    go = go && lighted;
+                    if (!__any_sync(0xFFFFFFFFu, go && in_tri)) continue;
                     v3 Ln = mk3(0.f, 0.f, 0.f);
                     float ndl = 0.f;
                     bool lit = false;
                     if (!lm) {
                         Ln = vnorm_fast(Lr);
                         ndl = vmax(vdot(N, Ln), 0.f);
-                        lit = (ndl > 0.f) && alive && in_tri;
+                        lit = (ndl > 0.f) && alive && in_tri && lighted;
                     }
-                    /* every cached proxy's "between" test first (independent, so they overlap),
-                     * then the block-level skip as the OR over the block's lanes */
-                    const int np = s_npc[i];
+                    /* every selected proxy's "between" test first, then the block-level skip as the OR over
+                     * the pair's lanes */
+                    uint32_t pm = !proxies ? 0u : full ? (1u << s_npc[i]) - 1u : (wm[i >> 1] >> ((i & 1) * 16)) & 0xFFFFu;
                     uint32_t rmask = 0, bmask = 0;
-                    const bool want = lm ? in_tri : lit;
-                    /* a lane's bit needs `want`: with no lane of the block wanting, every mask is 0 */
-                    if (np > 0 && (__ballot_sync(gmask, want) & gmask)) {
-                        const float rd2 = rcpr(d2);   /* loop-invariant: the reference recomputes the same value per proxy */
+                    const bool want = lm ? in_tri && lighted : lit;
+                    if (pm && __any_sync(0xFFFFFFFFu, want)) {
+                        const float rd2 = rcpr(d2);   /* the reference recomputes the same value per proxy */
                         const float nd2 = -d2;
                         /* The reference's test with wdv = 0 - dot(W, Lr): wdv > 0 && wdv < d2, then
                          * cd2 = fma(-wdv, wdv * rd2, |W|^2) < rb2.  With v = dot(W, Lr): wdv > 0 is
                          * v < 0 (both false for a zero or NaN v), wdv < d2 is v > -d2, and for such
                          * v, wdv = -v exactly, wdv * rd2 = -(v * rd2) (round to nearest is
                          * symmetric) and cd2 = fma(-v, v * rd2, |W|^2): the same bits. */
-#pragma unroll 4
-                        for (int pi = 0; pi < np; pi++) {
+                        while (pm) {
+                            const int pi = __ffs(pm) - 1;
+                            pm &= pm - 1;
                             const float4 bt = s_btw[i * SFTG_MAX_LIGHT_PROXIES + pi];
                             const float v = vdot(mk3(bt.x, bt.y, bt.z), Lr);
                             const bool btw = v < 0.f && v > nd2;
                             const float cd2 = fma_(-v, v * rd2, bt.w);
                             rmask |= (uint32_t)(btw && (cd2 < s_rb2[i * SFTG_MAX_LIGHT_PROXIES + pi]) && want) << pi;
                         }
-                        bmask = rmask;
-                        bmask |= __shfl_xor_sync(gmask, bmask, 1);
-                        bmask |= __shfl_xor_sync(gmask, bmask, 2);
-                        bmask |= __shfl_xor_sync(gmask, bmask, 4);
+                        if (__any_sync(0xFFFFFFFFu, rmask != 0)) bmask = pair_or(rmask, lane, start, end);
                     }
-                    if (lm && !bmask) {
-                        /* lightmapped and no proxy shadows the block: si = 1, drop = 0 * att and the
-                         * light leaves lms unchanged, unless att is not finite on a covered lane */
-                        if (!(__ballot_sync(gmask, in_tri && !(att <= 3.402823466e38f)) & gmask)) {
-                            if (shadow_out && S == 1 && ((tri_lanes >> gl) & 1u) && i < 16)
-                                shadow_out[((size_t)gy * W + gx) * 16 + i] = 1.f;
-                            continue;
-                        }
-                    }
-                    if (lm) Ln = vnorm_fast(Lr);
                     float msh = 0.f;
                     if (bmask) {
+                        if (lm) Ln = vnorm_fast(Lr);
                         const float lrl = fsqrt(d2);
                         const float bk = 0.2f, b4 = 0.25f / 0.2f;
                         /* the smooth-max blend over the surviving proxies in index order */
                         while (bmask) {
                             const int pi = __ffs(bmask) - 1;
                             bmask &= bmask - 1;
-                            const proxy_cache& q = pcache[i * SFTG_MAX_LIGHT_PROXIES + pi];
+                            const float4 qa = s_pa[i * SFTG_MAX_LIGHT_PROXIES + pi], qb = s_ab[i * SFTG_MAX_LIGHT_PROXIES + pi];
                             const bool ray = (rmask >> pi) & 1u;
-                            const v3 pa = mk3(q.pa[0], q.pa[1], q.pa[2]), ab = mk3(q.ab[0], q.ab[1], q.ab[2]);
+                            const v3 pa = mk3(qa.x, qa.y, qa.z), ab = mk3(qb.x, qb.y, qb.z);
                             const v3 ao = sub3(P, pa);
                             const float abl = vdot(ab, Ln), abao = vdot(ab, ao), lao = vdot(Ln, ao);
-                            const float den = fma_(-abl, abl, q.abdab);
+                            const float den = fma_(-abl, abl, qa.w);
                             const float sden = vmax(den, 1e-6f);
                             float t2 = fma_(-abl, lao, abao) * rcpr(sden);
                             t2 = vmax(0.f, vmin(t2, 1.f));
@@ -1085,84 +1087,87 @@ SFTG_D void resolve_item(const sftg_tile_args& A, uint32_t tile0, int split, boo
                             const v3 pc = add3(pa, scl3(ab, t2));
                             const v3 dd = sub3(pr, pc);
                             const float dist2 = vdot(dd, dd);
-                            float sv = vmax(0.f, 1.f - fdiv(dist2, q.pr2));
+                            float sv = vmax(0.f, 1.f - fdiv(dist2, qb.w));
                             if (!ray || !vc) sv = 0.f;
-                            sv = sv * q.vis_mult;
+                            sv = sv * s_vm[i * SFTG_MAX_LIGHT_PROXIES + pi];
                             const float h = vmax(0.f, bk - fabsf(msh - sv));
                             const float badd = (h * h) * b4;
                             msh = vmax(msh, sv) + badd;
                         }
                     }
                     const float si = vmax(0.f, 1.f - msh);
-                    if (shadow_out && S == 1 && ((tri_lanes >> gl) & 1u) && i < 16)
-                        shadow_out[((size_t)gy * W + gx) * 16 + i] = si;
+                    if (S == 1 && shadow_out && go && in_tri && i < 16) shadow_out[((size_t)gy * W + gx) * 16 + i] = si;
                     if (lm) {
                         const float drop = (1.f - si) * att;
-                        lms = lms * (1.f - drop);
-                    } else {
+                        if (go) lms = lms * (1.f - drop);
+                    } else if (lit || (full && go)) {
+                        const float4 C = s_lc[i];
                         const float di = ndl * att;
                         const float md = lit ? (di * si) : 0.f;
-                        dif[0] = fma_(md, L.color[0], dif[0]); dif[1] = fma_(md, L.color[1], dif[1]); dif[2] = fma_(md, L.color[2], dif[2]);
+                        dif[0] = fma_(md, C.x, dif[0]); dif[1] = fma_(md, C.y, dif[1]); dif[2] = fma_(md, C.z, dif[2]);
                         if (lit) {
                             const v3 Hh = vnorm_fast(add3(Ln, V));
                             const float ndh = vmax(vdot(N, Hh), 0.f);
                             const float den = (shin - shin * ndh) + ndh;
                             const float sp = ndh * rcpr(den);
                             const float term = ((sp * sscale) * di) * si;
-                            spc[0] = fma_(term, L.color[0], spc[0]); spc[1] = fma_(term, L.color[1], spc[1]); spc[2] = fma_(term, L.color[2], spc[2]);
+                            spc[0] = fma_(term, C.x, spc[0]); spc[1] = fma_(term, C.y, spc[1]); spc[2] = fma_(term, C.z, spc[2]);
                         }
                     }
                 }
-                if (lm_quick) {   /* uniform over the block's 8 lanes, as the shuffles need */
-                    uint32_t ga = q_alive;
-                    ga |= __shfl_xor_sync(gmask, ga, 1);
-                    ga |= __shfl_xor_sync(gmask, ga, 2);
-                    ga |= __shfl_xor_sync(gmask, ga, 4);
-                    if (ga & q_nan) lms = __int_as_float(0x7FFFFFFF);
-                }
-                if (lm) {
-                    const float mod = fma_(lms, 1.f - 0.4f, 0.4f);
-                    out[0] = out[0] * (dif[0] * mod); out[1] = out[1] * (dif[1] * mod); out[2] = out[2] * (dif[2] * mod);
-                } else {
-                    out[0] = fma_(out[0], dif[0], spc[0]); out[1] = fma_(out[1], dif[1], spc[1]); out[2] = fma_(out[2], dif[2], spc[2]);
+                if (lighted) {
+                    if (lm) {
+                        const float mod = fma_(lms, 1.f - 0.4f, 0.4f);
+                        out[0] = out[0] * (dif[0] * mod); out[1] = out[1] * (dif[1] * mod); out[2] = out[2] * (dif[2] * mod);
+                    } else {
+                        out[0] = fma_(out[0], dif[0], spc[0]); out[1] = fma_(out[1], dif[1], spc[1]); out[2] = fma_(out[2], dif[2], spc[2]);
+                    }
                 }
             }
-            if (F->debug_mode == 1) {   /* wireframe view (6645-6671): edges where a barycentric is under its screen width */
-                const float dbu_dx = (0.f - dy2) * idet, dbu_dy = dx2 * idet;
-                const float dbv_dx = dy1 * idet, dbv_dy = (0.f - dx1) * idet;
-                const float fw_u = fabsf(dbu_dx) + fabsf(dbu_dy), fw_v = fabsf(dbv_dx) + fabsf(dbv_dy);
-                const float dbw_dx = 0.f - (dbu_dx + dbv_dx), dbw_dy = 0.f - (dbu_dy + dbv_dy);
-                const float fw_w = fabsf(dbw_dx) + fabsf(dbw_dy);
-                if (bu < fw_u || bv < fw_v || bw < fw_w) { out[0] = 0.f; out[1] = 1.f; out[2] = 0.f; }
-            }
+            if (wire) { out[0] = 0.f; out[1] = 1.f; out[2] = 0.f; }
             if (S == 1) {
-                if ((tri_lanes >> gl) & 1u) {
+                if (in_tri) {
                     uint32_t px = 0xFF000000u;
 #pragma unroll
                     for (int k = 0; k < 3; k++) px |= ((uint32_t)cvtt(vmax(0.f, vmin(out[k], 1.f)) * 255.f)) << (16 - 8 * k);
                     color[gy * CP + gx] = px;
                 }
             } else {
-                const float wgt = in_tri ? (float)hits * inv_s : 0.f;
+                /* a pixel's fragments of one chunk are added in turn */
+                const float wgt = (float)((meta >> 7) & 7u) * inv_s;
+                const uint32_t j = (meta >> 10) & 3u;
+                float* const a = accs + (bl * 8 + pl) * 3;
 #pragma unroll
-                for (int k = 0; k < 3; k++) acc[k] = fma_(vmax(0.f, vmin(out[k], 1.f)), wgt, acc[k]);
+                for (uint32_t jj = 0; jj < (uint32_t)S; jj++) {
+                    if (in_tri && j == jj)
+#pragma unroll
+                        for (int k = 0; k < 3; k++) a[k] = fma_(vmax(0.f, vmin(out[k], 1.f)), wgt, a[k]);
+                    __syncwarp();
+                }
             }
+            if (!full || ++pass >= npass) { c0 += 32; pass = 0; full = s_odd != 0; }
         }
+
+        /* ---------------- store ---------------- */
         if (S > 1) {
-            const bool store = F->clear ? inb : ((block_write >> gl) & 1u);
-            if (store) {
+            for (int k = 0; k < set / 4; k++) {
+                if (!((stores >> k) & 1u)) continue;
+                const int bl = k * 4 + (lane >> 3);
+                const int gx = X0 + (bl % bw) * 4 + ix, gy = Y0 + (bl / bw) * 2 + iy;
+                const float* a = accs + (bl * 8 + gl) * 3;
                 uint32_t px = 0xFF000000u;
 #pragma unroll
-                for (int k = 0; k < 3; k++) px |= ((uint32_t)cvtt(vmin(acc[k], 1.f) * 255.f)) << (16 - 8 * k);
+                for (int c = 0; c < 3; c++) px |= ((uint32_t)cvtt(vmin(a[c], 1.f) * 255.f)) << (16 - 8 * c);
                 color[gy * CP + gx] = px;
             }
         }
+        __syncwarp();   /* the next set reuses the warp's list and sums */
     }
 }
 
 /* one CTA per (tile, part) item */
 template <int S>
-__global__ void __launch_bounds__(TILE_THREADS, S == 1 ? 3 : 4)   /* 64 registers at 2x and 4x, 80 at 1x: measured best */
+__global__ void __launch_bounds__(TILE_THREADS, 4)   /* 64 registers; 80 (3 CTAs) cost 2-7 %, 48 (5 CTAs) 5-11 % */
 k_resolve(const sftg_tile_args A, uint32_t tile0, int split, bool records)
 {
     resolve_item<S>(A, tile0, split, records, blockIdx.x);
@@ -1170,7 +1175,7 @@ k_resolve(const sftg_tile_args A, uint32_t tile0, int split, bool records)
 
 /* Persistent form, as k_raster_queue: CTAs take (tile, part) items in launch order from a counter. */
 template <int S>
-__global__ void __launch_bounds__(TILE_THREADS, S == 1 ? 3 : 4)
+__global__ void __launch_bounds__(TILE_THREADS, 4)
 k_resolve_queue(const sftg_tile_args A, uint32_t tile0, int split, bool records, uint32_t n_items, uint32_t* next)
 {
     __shared__ uint32_t s_item;
@@ -1328,6 +1333,24 @@ static size_t raster_smem(int S, int slab_rows) {
 }
 
 int sftg_raster_bands(void) { return RASTER_BANDS; }
+
+/* Resolve CTAs per tile for a launch over `tiles` tiles in all: the knob's number, halved down to 4
+ * while the launch would exceed 4096 CTAs, about 7 waves of the 152 SMs x 4 resident ones.  Fewer
+ * tiles want the 16 (skinned 320x180 2x, 15 tiles: 0.074 ms against 0.139 with 8; atrium 1279x719
+ * 1x, 240 tiles: 0.103 against 0.112); with more, a CTA's light list and proxy cache should serve
+ * more blocks (1080p, 510 tiles: 0.172 ms with 8, 0.200 with 16 at 2x, 0.381 and 0.404 at 4x; 48
+ * views, 16000 tiles: 8.05 ms with 4, 8.12 with 8, 9.03 with 16).  Below 4 a warp has several sets
+ * to itself and the tail grows (1080p 2x 0.249 ms with 2). */
+int sftg_resolve_split(int knob, uint32_t tiles) {
+    while (knob > 4 && (uint64_t)tiles * (uint32_t)knob > 4096u) knob /= 2;
+    return knob;
+}
+
+/* Whether a range's light lists and proxy selections are made once per tile (k_tile_lights) or by
+ * each of its resolve CTAs: from 128 tiles on, the selections saved outweigh one more launch on the
+ * critical path (240 tiles 1x 0.103 against 0.111 ms, 510 tiles 4x 0.381 against 0.406; 60 tiles
+ * 0.0225 against 0.0205). */
+bool sftg_resolve_records(int knob, uint32_t tiles) { return knob == 2 || (knob == 0 && tiles >= 128u); }
 
 cudaError_t sftg_tile_configure(int max_dynamic_smem) {
     cudaError_t e = cudaSuccess;
