@@ -200,7 +200,7 @@ int sftg_autotune(sftg_ctx* ctx, const sftg_frame_desc* frames, uint32_t n_views
 /* Skeletal animation on the GPU (sft_pose_update, sofren2.c:8952-9108).  A skeleton (bones in
  * sft_bone's layout, sofren2.c:1000-1009) with its animations (samplers / channels,
  * sofren2.c:1023-1049) is uploaded once; sftg_pose_eval then evaluates any number of
- * (skeleton, animation, time) requests in one launch, one warp per request.  Results are the
+ * (skeleton, animation, time) requests in one launch.  Results are the
  * reference's posed bone matrices (inverse bind x global) and, optionally, the globals; they
  * equal the reference's up to the rounding of the device's acosf / sinf / cosf against the host
  * libm's inside the quaternion slerp (a few ulp). */

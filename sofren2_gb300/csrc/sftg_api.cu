@@ -115,10 +115,10 @@ struct sftg_ctx {
     uint32_t tr_meshlets = 0, tr_skin = 0, tr_blas = 0;
     size_t tr_models = 0;
     /* skeletons and animations (sftg_skeleton_upload) */
-    dpool p_skels, p_bones, p_anims, p_samplers, p_channels, p_keys, p_order, p_levels, p_pose_io;
+    dpool p_skels, p_bones, p_anims, p_samplers, p_wins, p_keys, p_order, p_pose_io;
     dpool p_ray_io;                            /* staging of sftg_raycast */
     std::vector<sftg_skel_dev> h_skels;
-    uint32_t n_bones = 0, n_anims = 0, n_samplers = 0, n_channels = 0, n_keys = 0, n_order = 0, n_levels = 0;
+    uint32_t n_bones = 0, n_anims = 0, n_samplers = 0, n_wins = 0, n_keys = 0, n_order = 0, max_bones = 0;
 };
 
 static int set_err(sftg_ctx* c, int code, const char* fmt, ...) {
@@ -223,7 +223,7 @@ extern "C" void sftg_destroy(sftg_ctx* ctx) {
     for (int l = 0; l < SFTG_MAX_LANES; l++) if (ctx->lanes[l].stream) cudaStreamSynchronize(ctx->lanes[l].stream);
     dpool* pools[] = { &ctx->texels, &ctx->texs, &ctx->mats, &ctx->ml_attr, &ctx->ml_inds, &ctx->ml_cull, &ctx->ml_info,
                        &ctx->skin_j, &ctx->skin_w, &ctx->blas, &ctx->models, &ctx->p_skels, &ctx->p_bones, &ctx->p_anims,
-                       &ctx->p_samplers, &ctx->p_channels, &ctx->p_keys, &ctx->p_order, &ctx->p_levels, &ctx->p_pose_io, &ctx->p_ray_io };
+                       &ctx->p_samplers, &ctx->p_wins, &ctx->p_keys, &ctx->p_order, &ctx->p_pose_io, &ctx->p_ray_io };
     for (dpool* p : pools) if (p->ptr) cudaFree(p->ptr);
     for (int l = 0; l < SFTG_MAX_LANES; l++) {
         sftg_lane& ln = ctx->lanes[l];
@@ -1216,13 +1216,11 @@ extern "C" int sftg_skeleton_upload(sftg_ctx* ctx, const sftg_bone_desc* bones, 
         depth[b] = d;
     }
     const int levels = *std::max_element(depth.begin(), depth.end()) + 1;
-    std::vector<uint16_t> order, lv;
-    for (int L = 0; L < levels; L++) {
-        lv.push_back((uint16_t)order.size());
-        for (uint32_t b = 0; b < bone_count; b++) if (depth[b] == L) order.push_back((uint16_t)b);
-    }
-    lv.push_back((uint16_t)order.size());
-    std::vector<sftg_bone_dev> bd(bone_count);
+    std::vector<uint32_t> order;
+    for (int L = 0; L < levels; L++)
+        for (uint32_t b = 0; b < bone_count; b++)
+            if (depth[b] == L) order.push_back(b | (bones[b].parent >= 0 ? (uint32_t)bones[b].parent : 0xFFFFu) << 16);
+    std::vector<sftg_bone_dev> bd(bone_count, sftg_bone_dev{});
     for (uint32_t b = 0; b < bone_count; b++) {
         memcpy(bd[b].inverse_bind, bones[b].inverse_bind, 64); memcpy(bd[b].local_bind, bones[b].local_bind, 64);
         bd[b].parent = bones[b].parent;
@@ -1232,17 +1230,19 @@ extern "C" int sftg_skeleton_upload(sftg_ctx* ctx, const sftg_bone_desc* bones, 
     memset(&sk, 0, sizeof(sk));
     sk.bone_base = ctx->n_bones; sk.bone_count = bone_count;
     sk.anim_base = ctx->n_anims; sk.anim_count = anim_count;
-    sk.order_base = ctx->n_order; sk.level_base = ctx->n_levels; sk.level_count = (uint32_t)levels;
+    sk.order_base = ctx->n_order;
     std::vector<sftg_anim_dev> ad(anim_count);
     std::vector<sftg_sampler_dev> sd;
-    std::vector<sftg_channel_desc> cd;
+    std::vector<int32_t> wins;
     std::vector<float> keys;
     for (uint32_t a = 0; a < anim_count; a++) {
         const sftg_animation_desc& A = anims[a];
         if (A.sampler_count < 0 || A.channel_count < 0 || (A.sampler_count && !A.samplers) || (A.channel_count && !A.channels))
             return set_err(ctx, SFTG_E_ARG, "animation %u: bad arrays", a);
-        ad[a].sampler_base = ctx->n_samplers + (uint32_t)sd.size(); ad[a].channel_base = ctx->n_channels + (uint32_t)cd.size();
-        ad[a].sampler_count = A.sampler_count; ad[a].channel_count = A.channel_count; ad[a].duration = A.duration;
+        const uint32_t sampler_base = ctx->n_samplers + (uint32_t)sd.size();
+        const size_t w0 = wins.size();
+        ad[a].win_base = ctx->n_wins + (uint32_t)w0; ad[a].duration = A.duration;
+        wins.resize(w0 + 3 * (size_t)bone_count, -1);
         for (int k = 0; k < A.sampler_count; k++) {
             const sftg_sampler_desc& S = A.samplers[k];
             if (S.count < 1 || !S.inputs || !S.outputs) return set_err(ctx, SFTG_E_ARG, "animation %u sampler %d: no keyframes", a, k);
@@ -1256,18 +1256,19 @@ extern "C" int sftg_skeleton_upload(sftg_ctx* ctx, const sftg_bone_desc* bones, 
             const sftg_channel_desc& C = A.channels[k];
             if (C.sampler < 0 || C.sampler >= A.sampler_count || C.path < 0 || C.path > 2)
                 return set_err(ctx, SFTG_E_ARG, "animation %u channel %d: bad sampler or path", a, k);
-            cd.push_back(C);
+            /* in channel order: a later channel of the same node and path wins; other nodes are skipped */
+            if (C.node >= 0 && C.node < (int)bone_count) wins[w0 + 3 * (size_t)C.node + C.path] = (int32_t)(sampler_base + (uint32_t)C.sampler);
         }
     }
     int rc;
     if ((rc = pool_push(ctx, ctx->p_bones, ctx->n_bones, bd.data(), bd.size())) ||
         (rc = pool_push(ctx, ctx->p_anims, ctx->n_anims, ad.data(), ad.size())) ||
         (rc = pool_push(ctx, ctx->p_samplers, ctx->n_samplers, sd.data(), sd.size())) ||
-        (rc = pool_push(ctx, ctx->p_channels, ctx->n_channels, cd.data(), cd.size())) ||
+        (rc = pool_push(ctx, ctx->p_wins, ctx->n_wins, wins.data(), wins.size())) ||
         (rc = pool_push(ctx, ctx->p_keys, ctx->n_keys, keys.data(), keys.size())) ||
-        (rc = pool_push(ctx, ctx->p_order, ctx->n_order, order.data(), order.size())) ||
-        (rc = pool_push(ctx, ctx->p_levels, ctx->n_levels, lv.data(), lv.size())))
+        (rc = pool_push(ctx, ctx->p_order, ctx->n_order, order.data(), order.size())))
         return rc;
+    ctx->max_bones = std::max(ctx->max_bones, bone_count);
     ctx->h_skels.push_back(sk);
     uint32_t ns = (uint32_t)ctx->h_skels.size() - 1;
     if ((rc = pool_push(ctx, ctx->p_skels, ns, &sk, 1))) return rc;
@@ -1281,8 +1282,8 @@ static sftg_pose_tables pose_tables(const sftg_ctx* ctx) {
     T.n_skels = (uint32_t)ctx->h_skels.size();
     T.skels = (const sftg_skel_dev*)ctx->p_skels.ptr; T.bones = (const sftg_bone_dev*)ctx->p_bones.ptr;
     T.anims = (const sftg_anim_dev*)ctx->p_anims.ptr; T.samplers = (const sftg_sampler_dev*)ctx->p_samplers.ptr;
-    T.channels = (const sftg_channel_desc*)ctx->p_channels.ptr; T.keys = (const float*)ctx->p_keys.ptr;
-    T.order = (const uint16_t*)ctx->p_order.ptr; T.levels = (const uint16_t*)ctx->p_levels.ptr;
+    T.wins = (const int32_t*)ctx->p_wins.ptr; T.keys = (const float*)ctx->p_keys.ptr;
+    T.order = (const uint32_t*)ctx->p_order.ptr; T.max_bones = ctx->max_bones;
     return T;
 }
 

@@ -99,24 +99,24 @@ void sftg_launch_resolve(int S, uint32_t tile0, uint32_t tiles, int split, bool 
 void sftg_launch_debug_overlay(uint32_t tiles, cudaStream_t st, const sftg_tile_args& A);
 
 /* skeletons and animations on the device (sftg_skeleton_upload) */
-struct sftg_bone_dev {
+struct __align__(16) sftg_bone_dev {   /* the matrices are read as 16-byte rows */
     float inverse_bind[16], local_bind[16];
     int32_t parent;
     float base_t[3], base_r[4], base_s[3];
 };
-struct sftg_skel_dev { uint32_t bone_base, bone_count, anim_base, anim_count, order_base, level_base, level_count, pad; };
-struct sftg_anim_dev { uint32_t sampler_base, channel_base; int32_t sampler_count, channel_count; float duration; uint32_t pad[3]; };
+struct sftg_skel_dev { uint32_t bone_base, bone_count, anim_base, anim_count, order_base, pad[3]; };
+struct sftg_anim_dev { uint32_t win_base; float duration; };
 struct sftg_sampler_dev { uint32_t input_base, output_base; int32_t count, is_step; };
 struct sftg_pose_tables {
     uint32_t n_skels;              /* requests naming another skeleton leave their matrices untouched */
+    uint32_t max_bones;            /* of any skeleton */
     const sftg_skel_dev* skels;
     const sftg_bone_dev* bones;
     const sftg_anim_dev* anims;
     const sftg_sampler_dev* samplers;
-    const sftg_channel_desc* channels;
+    const int32_t* wins;           /* per animation and bone: the samplers of its T, R and S, -1 for none */
     const float* keys;
-    const uint16_t* order;         /* per skeleton: bones parents-first */
-    const uint16_t* levels;        /* per skeleton: level_count + 1 starts into order */
+    const uint32_t* order;         /* per skeleton: bone | parent << 16 (0xFFFF: a root), parents first */
 };
 void sftg_launch_raycast(const sftg_ray* rays, uint32_t n, const sftg_model* models, uint32_t n_models, const sftg_bvh_node* blas,
                          const float* ml_attr, const uint8_t* ml_inds, sftg_ray_hit* hits, cudaStream_t st);

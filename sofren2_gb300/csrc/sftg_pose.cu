@@ -1,22 +1,28 @@
 /*
- * Skeletal pose evaluation (sft_pose_update, sofren2.c:8952-9108), one warp per request.
+ * Skeletal pose evaluation (sft_pose_update, sofren2.c:8952-9108), `per` requests per CTA.
  *
- *   channels   lanes take channels in order of their index; each finds its keyframe pair by the
- *              reference's binary search, interpolates (lerp for T and S, sft_q_slerp for R, or
- *              the step value), and the values are stored in channel order, so a later channel
- *              of the same node and path wins as in the reference's sequential loop
- *   locals     per bone S * (R * T) from the animated or rest TRS, else the local bind matrix
- *   hierarchy  parents before children, level by level (host-computed order): global =
- *              local * global[parent], each bone once, as the reference's repeated passes do
- *   posed      inverse bind * global
+ *   locals     a thread per (request, bone): the bone's T, R and S samplers (the upload keeps, per
+ *              animation, the last channel of each node and path, which is the one that wins in
+ *              the reference's sequential loop); the keyframe pair by the reference's binary
+ *              search, lerp for T and S, sft_q_slerp for R, or the step value; S * (R * T) from
+ *              the animated or rest values, else the local bind matrix
+ *   hierarchy  four threads per request, one per matrix row, take the bones parents first:
+ *              global = local * global[parent], each bone once, as the reference's repeated passes do
+ *   posed      inverse bind * global, a thread per (request, bone, row): both outputs leave as
+ *              16-byte rows, consecutive over the warp
  * Matrix products follow sft_m_mul (sofren2.c:1668): left-to-right sums of plain products.
+ *
+ * Bound by issue, most of it the slerps and the local products (a quarter of the time is the
+ * 2.8 KB of matrices a request of 22 bones writes, at the copy rate).  One warp per request, lanes
+ * on channels and whole matrices stored per lane, took 361 us for 65536 requests of 22 bones: the
+ * hierarchy ran level by level with a few lanes, and each store touched 32 lines.  Now 105 us; 1024
+ * requests 14.4 -> 12.4 us.
  */
 #include "sftg_types.h"
 #include "sftg_kernels.h"
 
-#define POSE_WARPS 1
-
-struct pose_trs { float p[3], r[4], s[3]; uint32_t mask; };
+#define POSE_THREADS 128
+#define POSE_MAX_PER 32           /* requests per CTA: POSE_THREADS / 4 rows */
 
 __device__ __forceinline__ void mmul(const float* a, const float* b, float* r) {
 #pragma unroll
@@ -59,120 +65,153 @@ __device__ void from_quat(const float* q, float* m) {   /* sft_m_from_quat (1822
     m[12] = 0.f; m[13] = 0.f; m[14] = 0.f; m[15] = 1.f;
 }
 
-__global__ void __launch_bounds__(32)
-k_pose(const sftg_pose_tables T, const sftg_pose_request* __restrict__ reqs, const uint32_t* __restrict__ out_off, uint32_t n,
-       float* __restrict__ posed, float* __restrict__ global_out)
+/* A sampler at `time`: xyz (path T or S) or the slerped quaternion (R) into val. */
+__device__ void sample(const sftg_pose_tables& T, int sampler, bool rotation, float time, float* val) {
+    const sftg_sampler_dev sm = T.samplers[sampler];
+    const float* in = T.keys + sm.input_base;
+    const float* out = T.keys + sm.output_base;
+    int f0 = 0, f1 = 0;
+    float t = 0.f;
+    if (time <= in[0]) {
+        f0 = f1 = 0;
+    } else if (time >= in[sm.count - 1]) {
+        f0 = f1 = sm.count - 1;
+    } else {
+        int low = 0, high = sm.count - 1;
+        while (low <= high) {
+            const int mid = low + (high - low) / 2;
+            if (time < in[mid]) high = mid - 1;
+            else if (time >= in[mid + 1]) low = mid + 1;
+            else { f0 = mid; f1 = mid + 1; break; }
+        }
+        const float dt = in[f1] - in[f0];
+        t = (dt > 0.0001f) ? __fdiv_rn(time - in[f0], dt) : 0.f;
+    }
+    if (rotation) {
+        if (sm.is_step) { for (int q = 0; q < 4; q++) val[q] = out[f0 * 4 + q]; }
+        else slerp(out + f0 * 4, out + f1 * 4, t, val);
+    } else {
+        for (int q = 0; q < 3; q++) {
+            const float v0 = out[f0 * 4 + q], v1 = out[f1 * 4 + q];
+            val[q] = sm.is_step ? v0 : v0 + (v1 - v0) * t;
+        }
+    }
+}
+
+/* row * m for a row and the four rows of a matrix, in mmul's order */
+__device__ __forceinline__ float4 row_mul(float4 a, const float4* m) {
+    const float4 m0 = m[0], m1 = m[1], m2 = m[2], m3 = m[3];
+#define COL(c) __fadd_rn(__fadd_rn(__fadd_rn(__fmul_rn(a.x, m0.c), __fmul_rn(a.y, m1.c)), __fmul_rn(a.z, m2.c)), __fmul_rn(a.w, m3.c))
+    return make_float4(COL(x), COL(y), COL(z), COL(w));
+#undef COL
+}
+
+/* VEC: the output arrays are 16-byte aligned */
+template <bool VEC>
+__device__ __forceinline__ void store_row(float* p, float4 v) {
+    if (VEC) *(float4*)p = v;
+    else { p[0] = v.x; p[1] = v.y; p[2] = v.z; p[3] = v.w; }
+}
+
+template <bool VEC>
+__global__ void __launch_bounds__(POSE_THREADS)
+k_pose(const sftg_pose_tables T, const sftg_pose_request* __restrict__ reqs, const uint32_t* __restrict__ out_off, uint32_t n, int per,
+       int stride, float* __restrict__ posed, float* __restrict__ global_out)
 {
-    __shared__ pose_trs s_trs[SFTG_MAX_BONES];
-    __shared__ float s_g[SFTG_MAX_BONES][16];
-    const uint32_t k = blockIdx.x;
-    const int lane = threadIdx.x;
-    if (k >= n) return;
-    const sftg_pose_request R = reqs[k];
-    if (R.skeleton < 0 || (uint32_t)R.skeleton >= T.n_skels) return;
-    const sftg_skel_dev sk = T.skels[R.skeleton];
-    if (R.animation < 0 || R.animation >= (int)sk.anim_count) return;   /* sft_pose_update returns early */
-    const sftg_anim_dev an = T.anims[sk.anim_base + R.animation];
-    const int nb = (int)sk.bone_count;
-    float time = R.time;
-    if (an.duration > 1e-6f) time = fmodf(time, an.duration);
-    for (int b = lane; b < nb; b += 32) s_trs[b].mask = 0;
-    __syncwarp();
-    /* channels, 32 at a time; values stored in channel order */
-    for (int c0 = 0; c0 < an.channel_count; c0 += 32) {
-        const int c = c0 + lane;
-        bool have = false;
-        int node = 0, path = 0;
-        float val[4] = { 0.f, 0.f, 0.f, 0.f };
-        if (c < an.channel_count) {
-            const sftg_channel_desc ch = T.channels[an.channel_base + c];
-            node = ch.node; path = ch.path;
-            if (node >= 0 && node < nb) {
-                have = true;
-                const sftg_sampler_dev sm = T.samplers[an.sampler_base + ch.sampler];
-                const float* in = T.keys + sm.input_base;
-                const float* out = T.keys + sm.output_base;
-                int f0 = 0, f1 = 0;
-                float t = 0.f;
-                if (time <= in[0]) {
-                    f0 = f1 = 0;
-                } else if (time >= in[sm.count - 1]) {
-                    f0 = f1 = sm.count - 1;
-                } else {
-                    int low = 0, high = sm.count - 1;
-                    while (low <= high) {
-                        const int mid = low + (high - low) / 2;
-                        if (time < in[mid]) high = mid - 1;
-                        else if (time >= in[mid + 1]) low = mid + 1;
-                        else { f0 = mid; f1 = mid + 1; break; }
-                    }
-                    const float dt = in[f1] - in[f0];
-                    t = (dt > 0.0001f) ? __fdiv_rn(time - in[f0], dt) : 0.f;
-                }
-                if (path == 1) {
-                    if (sm.is_step) { for (int q = 0; q < 4; q++) val[q] = out[f0 * 4 + q]; }
-                    else slerp(out + f0 * 4, out + f1 * 4, t, val);
-                } else {
-                    for (int q = 0; q < 3; q++) {
-                        const float v0 = out[f0 * 4 + q], v1 = out[f1 * 4 + q];
-                        val[q] = sm.is_step ? v0 : v0 + (v1 - v0) * t;
-                    }
+    extern __shared__ float4 s_g[];   /* [per][stride][4 rows]: local, then global matrices; stride is odd (banks) */
+    __shared__ int s_nb[POSE_MAX_PER];
+    __shared__ uint32_t s_bone[POSE_MAX_PER], s_win[POSE_MAX_PER], s_order[POSE_MAX_PER], s_off[POSE_MAX_PER];
+    __shared__ float s_time[POSE_MAX_PER];
+    const int tid = threadIdx.x;
+    if (tid < per) {
+        const uint32_t k = blockIdx.x * (uint32_t)per + tid;
+        int nb = 0;   /* 0: a request that leaves its matrices untouched */
+        if (k < n) {
+            const sftg_pose_request R = reqs[k];
+            if (R.skeleton >= 0 && (uint32_t)R.skeleton < T.n_skels) {
+                const sftg_skel_dev sk = T.skels[R.skeleton];
+                if (R.animation >= 0 && R.animation < (int)sk.anim_count) {   /* else sft_pose_update returns early */
+                    const sftg_anim_dev an = T.anims[sk.anim_base + R.animation];
+                    nb = (int)sk.bone_count;
+                    s_bone[tid] = sk.bone_base; s_order[tid] = sk.order_base; s_win[tid] = an.win_base;
+                    s_off[tid] = out_off[k];
+                    s_time[tid] = an.duration > 1e-6f ? fmodf(R.time, an.duration) : R.time;
                 }
             }
         }
-        for (int w = 0; w < 32; w++) {   /* channel order */
-            if (lane == w && have) {
-                pose_trs& d = s_trs[node];
-                if (path == 1) { d.r[0] = val[0]; d.r[1] = val[1]; d.r[2] = val[2]; d.r[3] = val[3]; d.mask |= 2u; }
-                else if (path == 0) { d.p[0] = val[0]; d.p[1] = val[1]; d.p[2] = val[2]; d.mask |= 1u; }
-                else if (path == 2) { d.s[0] = val[0]; d.s[1] = val[1]; d.s[2] = val[2]; d.mask |= 4u; }
+        s_nb[tid] = nb;
+    }
+    __syncthreads();
+    /* local matrices */
+    for (int i = tid; i < per * stride; i += POSE_THREADS) {
+        const int r = i / stride, b = i - r * stride;
+        if (b >= s_nb[r]) continue;
+        const sftg_bone_dev& bd = T.bones[s_bone[r] + b];
+        const int* win = T.wins + (size_t)s_win[r] + 3 * b;
+        const int wt = win[0], wr = win[1], ws = win[2];
+        float4* g = s_g + 4 * (size_t)i;
+        if (wt >= 0 || wr >= 0 || ws >= 0) {
+            float tp[4] = { bd.base_t[0], bd.base_t[1], bd.base_t[2], 0.f };
+            float rq[4] = { bd.base_r[0], bd.base_r[1], bd.base_r[2], bd.base_r[3] };
+            float sc[4] = { bd.base_s[0], bd.base_s[1], bd.base_s[2], 0.f };
+            const float time = s_time[r];
+            if (wr >= 0) sample(T, wr, true, time, rq);
+            if (wt >= 0) sample(T, wt, false, time, tp);
+            if (ws >= 0) sample(T, ws, false, time, sc);
+            float Tm[16] = { 1, 0, 0, 0, 0, 1, 0, 0, 0, 0, 1, 0, tp[0], tp[1], tp[2], 1 };
+            float Sm[16] = { sc[0], 0, 0, 0, 0, sc[1], 0, 0, 0, 0, sc[2], 0, 0, 0, 0, 1 };
+            float Rm[16], RT[16], L[16];
+            from_quat(rq, Rm);
+            mmul(Rm, Tm, RT);
+            mmul(Sm, RT, L);
+#pragma unroll
+            for (int q = 0; q < 4; q++) g[q] = make_float4(L[4 * q], L[4 * q + 1], L[4 * q + 2], L[4 * q + 3]);
+        } else {
+#pragma unroll
+            for (int q = 0; q < 4; q++) g[q] = ((const float4*)bd.local_bind)[q];
+        }
+    }
+    __syncthreads();
+    /* hierarchy: the order table holds bone | parent << 16 (0xFFFF: none), parents first */
+    if (tid < ((per * 4 + 31) & ~31)) {   /* whole warps */
+        const int r = tid >> 2, row = tid & 3;
+        const int nb = r < per ? s_nb[r] : 0;   /* per may be 1 or 2 */
+        const uint32_t* order = T.order + (nb ? s_order[r] : 0u);
+        float4* g = s_g + (size_t)r * stride * 4;
+        const int steps = __reduce_max_sync(0xFFFFFFFFu, nb);
+        uint32_t next = nb ? order[0] : 0u;
+        for (int q = 0; q < steps; q++) {
+            const uint32_t e = next;
+            if (q + 1 < nb) next = order[q + 1];
+            if (q < nb && (e >> 16) != 0xFFFFu) {
+                const int b = (int)(e & 0xFFFFu), p = (int)(e >> 16);
+                g[b * 4 + row] = row_mul(g[b * 4 + row], g + p * 4);
             }
             __syncwarp();
         }
     }
-    /* local matrices */
-    for (int b = lane; b < nb; b += 32) {
-        const sftg_bone_dev& bd = T.bones[sk.bone_base + b];
-        const pose_trs& tr = s_trs[b];
-        if (tr.mask) {
-            const float* tp = (tr.mask & 1u) ? tr.p : bd.base_t;
-            const float* rq = (tr.mask & 2u) ? tr.r : bd.base_r;
-            const float* sc = (tr.mask & 4u) ? tr.s : bd.base_s;
-            float Tm[16] = { 1, 0, 0, 0, 0, 1, 0, 0, 0, 0, 1, 0, tp[0], tp[1], tp[2], 1 };
-            float Sm[16] = { sc[0], 0, 0, 0, 0, sc[1], 0, 0, 0, 0, sc[2], 0, 0, 0, 0, 1 };
-            float Rm[16], RT[16];
-            from_quat(rq, Rm);
-            mmul(Rm, Tm, RT);
-            mmul(Sm, RT, s_g[b]);
-        } else {
-            for (int q = 0; q < 16; q++) s_g[b][q] = bd.local_bind[q];
-        }
-    }
-    __syncwarp();
-    /* hierarchy, level by level */
-    const uint16_t* order = T.order + sk.order_base;
-    const uint16_t* lvl = T.levels + sk.level_base;
-    for (uint32_t L = 1; L < sk.level_count; L++) {
-        for (int i = (int)lvl[L] + lane; i < (int)lvl[L + 1]; i += 32) {
-            const int b = order[i];
-            const int p = T.bones[sk.bone_base + b].parent;
-            float g[16];
-            mmul(s_g[b], s_g[p], g);
-            for (int q = 0; q < 16; q++) s_g[b][q] = g[q];
-        }
-        __syncwarp();
-    }
+    __syncthreads();
     /* posed = inverse bind * global */
-    float* po = posed + (size_t)out_off[k] * 16;
-    for (int b = lane; b < nb; b += 32) {
-        float pm[16];
-        mmul(T.bones[sk.bone_base + b].inverse_bind, s_g[b], pm);
-        for (int q = 0; q < 16; q++) po[b * 16 + q] = pm[q];
-        if (global_out) for (int q = 0; q < 16; q++) global_out[(size_t)out_off[k] * 16 + b * 16 + q] = s_g[b][q];
+    for (int i = tid; i < per * stride * 4; i += POSE_THREADS) {
+        const int m = i >> 2, row = i & 3, r = m / stride, b = m - r * stride;
+        if (b >= s_nb[r]) continue;
+        const float4 iv = ((const float4*)T.bones[s_bone[r] + b].inverse_bind)[row];
+        const size_t o = ((size_t)s_off[r] + b) * 16 + 4 * row;
+        store_row<VEC>(posed + o, row_mul(iv, s_g + 4 * (size_t)m));
+        if (global_out) store_row<VEC>(global_out + o, s_g[i]);
     }
 }
 
 void sftg_launch_pose(const sftg_pose_tables& T, const sftg_pose_request* reqs, const uint32_t* out_off, uint32_t n, float* posed,
                       float* global, cudaStream_t st) {
-    if (n) k_pose<<<n, 32, 0, st>>>(T, reqs, out_off, n, posed, global);
+    if (!n) return;
+    /* requests per CTA: as many as 24 KB of matrices hold (22 bones: 16; 65536 requests 105 us, with 48 KB
+     * 141, 16384 requests 33 us, with 12 KB 37), fewer while that leaves SMs without two CTAs */
+    const int stride = (int)(T.max_bones | 1u);
+    int per = POSE_MAX_PER;
+    while (per > 1 && ((size_t)per * stride * 64 > 24u * 1024u || (uint64_t)per * 304u > n)) per /= 2;
+    const size_t sm = (size_t)per * stride * 64;
+    const uint32_t grid = (n + per - 1) / per;
+    if ((((uintptr_t)posed | (uintptr_t)global) & 15u) == 0) k_pose<true><<<grid, POSE_THREADS, sm, st>>>(T, reqs, out_off, n, per, stride, posed, global);
+    else k_pose<false><<<grid, POSE_THREADS, sm, st>>>(T, reqs, out_off, n, per, stride, posed, global);
 }
