@@ -85,7 +85,7 @@ struct sftg_ctx {
     std::vector<void*> retired_stage;          /* outgrown pinned staging: freed at sftg_destroy (cudaFreeHost synchronises) */
     char err[512] = { 0 };
     /* resident */
-    dpool texels, texs, mats, ml_attr, ml_inds, ml_cull, ml_info, skin_j, skin_w, blas, models;
+    dpool texels, texs, mats, ml_attr, ml_inds, ml_cull, ml_info, skin_j, skin_w, blas, wslots, wtris, models;
     std::vector<sftg_tex> h_texs;
     std::vector<sftg_mat> h_mats;
     std::vector<sftg_model> h_models;
@@ -117,6 +117,7 @@ struct sftg_ctx {
     /* skeletons and animations (sftg_skeleton_upload) */
     dpool p_skels, p_bones, p_anims, p_samplers, p_wins, p_keys, p_order, p_pose_io;
     dpool p_ray_io;                            /* staging of sftg_raycast */
+    uint32_t* d_ray_next = nullptr;            /* ray counter of a large launch (lane 0's stream only) */
     std::vector<sftg_skel_dev> h_skels;
     uint32_t n_bones = 0, n_anims = 0, n_samplers = 0, n_wins = 0, n_keys = 0, n_order = 0, max_bones = 0;
 };
@@ -210,6 +211,7 @@ extern "C" int sftg_create(int device, sftg_ctx** out) {
         uint64_t keep = ~0ull;
         cudaMemPoolSetAttribute(ctx->lane_pool, cudaMemPoolAttrReleaseThreshold, &keep);
     }
+    if (cudaMalloc((void**)&ctx->d_ray_next, 256) != cudaSuccess) { ctx->d_ray_next = nullptr; sftg_destroy(ctx); return SFTG_E_CUDA; }
     sftg_tile_configure(227 * 1024);
     if (noalloc_scratch_setup(device) != cudaSuccess) { sftg_destroy(ctx); return SFTG_E_CUDA; }
     { const char* e = getenv("SFTG_NO_GRAPHS"); if (e && *e && *e != '0') ctx->use_graphs = false; }
@@ -222,9 +224,10 @@ extern "C" void sftg_destroy(sftg_ctx* ctx) {
     cudaSetDevice(ctx->device);
     for (int l = 0; l < SFTG_MAX_LANES; l++) if (ctx->lanes[l].stream) cudaStreamSynchronize(ctx->lanes[l].stream);
     dpool* pools[] = { &ctx->texels, &ctx->texs, &ctx->mats, &ctx->ml_attr, &ctx->ml_inds, &ctx->ml_cull, &ctx->ml_info,
-                       &ctx->skin_j, &ctx->skin_w, &ctx->blas, &ctx->models, &ctx->p_skels, &ctx->p_bones, &ctx->p_anims,
+                       &ctx->skin_j, &ctx->skin_w, &ctx->blas, &ctx->wslots, &ctx->wtris, &ctx->models, &ctx->p_skels, &ctx->p_bones, &ctx->p_anims,
                        &ctx->p_samplers, &ctx->p_wins, &ctx->p_keys, &ctx->p_order, &ctx->p_pose_io, &ctx->p_ray_io };
     for (dpool* p : pools) if (p->ptr) cudaFree(p->ptr);
+    if (ctx->d_ray_next) cudaFree(ctx->d_ray_next);
     for (int l = 0; l < SFTG_MAX_LANES; l++) {
         sftg_lane& ln = ctx->lanes[l];
         if (ln.arena) cudaFree(ln.arena);
@@ -287,6 +290,22 @@ extern "C" int sftg_material_set(sftg_ctx* ctx, int32_t index, int32_t texture, 
     ctx->h_mats[index].shininess = shininess;
     ctx->tables_dirty = true;
     return SFTG_OK;
+}
+
+/* Whether every node's boxes lie inside the box its parent holds for it (sftg_model.nested): true of
+ * a tree built from its triangles, not checked by the loaders of caller-built ones. */
+static uint32_t blas_nested(const sftg_bvh_node* nodes, uint32_t count) {
+    for (uint32_t i = 0; i < count; i++) {
+        if (nodes[i].leaf) continue;
+        for (int c = 0; c < nodes[i].count && c < 8; c++) {
+            const uint32_t ch = nodes[i].child[c];
+            if (ch == SFTG_INVALID || ch >= count) continue;
+            for (int q = 0; q < nodes[ch].count && q < 8; q++)
+                for (int a = 0; a < 3; a++)
+                    if (!(nodes[ch].mn[a][q] >= nodes[i].mn[a][c] && nodes[ch].mx[a][q] <= nodes[i].mx[a][c])) return 0;
+        }
+    }
+    return 1;
 }
 
 static int model_upload(sftg_ctx* ctx, const sftg_model_desc* d, int32_t* out_model, bool transient) {
@@ -360,6 +379,7 @@ static int model_upload(sftg_ctx* ctx, const sftg_model_desc* d, int32_t* out_mo
         if ((rc = pool_reserve(ctx, ctx->blas, ((size_t)ctx->n_blas + d->blas_count) * 256))) return rc;
         CK(cudaMemcpyAsync((char*)ctx->blas.ptr + (size_t)ctx->n_blas * 256, d->blas_nodes, (size_t)d->blas_count * 256, cudaMemcpyHostToDevice, ctx->stream));
         ctx->blas.size = ((size_t)ctx->n_blas + d->blas_count) * 256;
+        md.nested = blas_nested((const sftg_bvh_node*)d->blas_nodes, d->blas_count);
     } else if (d->build_blas && total) {   /* built from the meshlets just uploaded */
         md.blas_count = 0; md.blas_root = 0;
         sftg_blas_job* job = nullptr;
@@ -376,6 +396,7 @@ static int model_upload(sftg_ctx* ctx, const sftg_model_desc* d, int32_t* out_mo
             if (e == cudaSuccess && !status) {
                 ctx->blas.size = ((size_t)ctx->n_blas + n_nodes) * 256;
                 md.blas_count = n_nodes;
+                md.nested = 1;   /* a node's box is the union of its children's */
             }
         }
         ctx->blas_launches = sftg_blas_launches(job);
@@ -389,6 +410,16 @@ static int model_upload(sftg_ctx* ctx, const sftg_model_desc* d, int32_t* out_mo
         ctx->blas_items = n_items;
         if (e != cudaSuccess) return set_err(ctx, SFTG_E_CUDA, "BLAS build: %s", cudaGetErrorString(e));
         if (status) return set_err(ctx, SFTG_E_DEVICE_STATUS, "BLAS build: a device work list overflowed");
+    }
+    if (md.blas_count) {   /* the forms the walks read */
+        const size_t end = (size_t)ctx->n_blas + md.blas_count;
+        if ((rc = pool_reserve(ctx, ctx->wslots, end * 8 * sizeof(sftg_wslot))) || (rc = pool_reserve(ctx, ctx->wtris, end * 8 * sizeof(sftg_wtri)))) return rc;
+        ctx->wslots.size = end * 8 * sizeof(sftg_wslot); ctx->wtris.size = end * 8 * sizeof(sftg_wtri);
+        sftg_launch_walk_forms((const sftg_bvh_node*)ctx->blas.ptr + ctx->n_blas, md.blas_count,
+                               (const float*)((const char*)ctx->ml_attr.ptr + (size_t)md.meshlet_base * 2560),
+                               (const uint8_t*)ctx->ml_inds.ptr + (size_t)md.meshlet_base * 512, total,
+                               (sftg_wslot*)ctx->wslots.ptr + (size_t)ctx->n_blas * 8, (sftg_wtri*)ctx->wtris.ptr + (size_t)ctx->n_blas * 8, ctx->stream);
+        CK(cudaGetLastError());
     }
     CK(cudaStreamSynchronize(ctx->stream));
     ctx->n_meshlets += total; ctx->n_skin += nskin; ctx->n_blas += md.blas_count;
@@ -435,6 +466,7 @@ extern "C" void sftg_transient_reset(sftg_ctx* ctx) {
         ctx->ml_cull.size = (size_t)ctx->n_meshlets * 32; ctx->ml_info.size = (size_t)ctx->n_meshlets * sizeof(sftg_meshlet_info);
         ctx->skin_j.size = (size_t)ctx->n_skin * 512; ctx->skin_w.size = (size_t)ctx->n_skin * 256;
         ctx->blas.size = (size_t)ctx->n_blas * 256;
+        ctx->wslots.size = (size_t)ctx->n_blas * 8 * sizeof(sftg_wslot); ctx->wtris.size = (size_t)ctx->n_blas * 8 * sizeof(sftg_wtri);
         ctx->tables_dirty = true;
     }
     ctx->tr_live = false; ctx->tr_pinned = false;
@@ -792,7 +824,8 @@ static int build_batch(sftg_ctx* ctx, sftg_lane& ln, const sftg_frame_desc* fds,
         F->ml_info = (const sftg_meshlet_info*)ctx->ml_info.ptr;
         F->skin_j = (const uint16_t*)ctx->skin_j.ptr;
         F->skin_w = (const uint8_t*)ctx->skin_w.ptr;
-        F->blas = (const sftg_bvh_node*)ctx->blas.ptr;
+        F->wslots = (const sftg_wslot*)ctx->wslots.ptr;
+        F->wtris = (const sftg_wtri*)ctx->wtris.ptr;
         for (uint32_t l = 0; l < fd->n_point; l++) memcpy(hs + o_pl + (P.pl_off + l) * sizeof(sftg_point_light), fd->point_lights + 8 * l, 32);
         for (uint32_t l = 0; l < fd->n_dir; l++) memcpy(hs + o_dl + (P.dl_off + l) * sizeof(sftg_dir_light), fd->dir_lights + 6 * l, 24);
         for (uint32_t p = 0; p < fd->n_proxies; p++) memcpy(hs + o_px + (P.prox_base + p) * sizeof(sftg_proxy), fd->proxies + 8 * p, 32);
@@ -1358,8 +1391,8 @@ extern "C" int sftg_raycast_device(sftg_ctx* ctx, const sftg_ray* d_rays, uint32
     CK(cudaSetDevice(ctx->device));
     int rc = sync_tables(ctx);   /* the device model table follows uploads lazily */
     if (rc) return rc;
-    sftg_launch_raycast(d_rays, n, (const sftg_model*)ctx->models.ptr, (uint32_t)ctx->h_models.size(), (const sftg_bvh_node*)ctx->blas.ptr,
-                        (const float*)ctx->ml_attr.ptr, (const uint8_t*)ctx->ml_inds.ptr, d_hits, ctx->stream);
+    CK((cudaError_t)sftg_launch_raycast(d_rays, n, (const sftg_model*)ctx->models.ptr, (uint32_t)ctx->h_models.size(), (const sftg_wslot*)ctx->wslots.ptr,
+                        (const sftg_wtri*)ctx->wtris.ptr, ctx->d_ray_next, d_hits, ctx->stream));
     CK(cudaGetLastError());
     return SFTG_OK;
 }
@@ -1589,7 +1622,8 @@ extern "C" int sftg_light_vis_noalloc(sftg_ctx* ctx, const sftg_frame_desc* fd, 
     F.ml_attr = (const float*)ctx->ml_attr.ptr;
     F.ml_inds = (const uint8_t*)ctx->ml_inds.ptr;
     F.ml_info = (const sftg_meshlet_info*)ctx->ml_info.ptr;
-    F.blas = (const sftg_bvh_node*)ctx->blas.ptr;
+    F.wslots = (const sftg_wslot*)ctx->wslots.ptr;
+    F.wtris = (const sftg_wtri*)ctx->wtris.ptr;
     sftg_inst inst[SFTG_MAX_INSTANCES + 1];
     memset(inst, 0, sizeof(inst));
     for (uint32_t i = 0; i < fd->n_instances; i++) {

@@ -919,3 +919,44 @@ void sftg_blas_end(sftg_blas_job* J) {
     if (J->d_cnt) cudaFreeAsync(J->d_cnt, J->st);
     delete J;
 }
+
+/* The walks' forms of the nodes: a thread per (node, slot).  A walk's step waits for the node and, at
+ * a leaf, used to wait twice more, for the triangle's indices and then its vertices; here the
+ * triangle lies at the node's own index.  e1 and e2 are the differences both walks take. */
+__global__ void k_blas_walk_forms(const sftg_bvh_node* __restrict__ nodes, uint32_t count, const float* __restrict__ attr,
+                                  const uint8_t* __restrict__ inds, uint32_t meshlets, sftg_wslot* __restrict__ wslots,
+                                  sftg_wtri* __restrict__ wtris)
+{
+    const uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
+    if (i >= count * 8u) return;
+    const sftg_bvh_node* nd = nodes + (i >> 3);
+    const uint32_t c = i & 7u;
+    sftg_wslot s;
+    for (int a = 0; a < 3; a++) { s.mn[a] = nd->mn[a][c]; s.mx[a] = nd->mx[a][c]; }
+    s.child = nd->child[c];
+    s.flags = (nd->leaf ? 1u : 0u) | (c < nd->count ? 2u : 0u);
+    sftg_wtri t;
+    for (int a = 0; a < 3; a++) t.v0[a] = t.e1[a] = t.e2[a] = 0.f;
+    t.ok = 0; t.pad[0] = t.pad[1] = 0;
+    if (nd->leaf && s.child != SFTG_INVALID) {
+        const uint32_t pay = s.child & ~0x80000000u, tri = pay & 127u, m = pay >> 7;
+        if (m < meshlets) {
+            const uint8_t* ind = inds + (size_t)m * 512 + (tri >> 3) * 32 + (tri & 7);
+            const float* X = attr + (size_t)m * 640;
+            const uint32_t i0 = ind[0], i1 = ind[8], i2 = ind[16];
+            for (int a = 0; a < 3; a++) {
+                t.v0[a] = X[64 * a + i0];
+                t.e1[a] = __fsub_rn(X[64 * a + i1], X[64 * a + i0]);
+                t.e2[a] = __fsub_rn(X[64 * a + i2], X[64 * a + i0]);
+            }
+            t.ok = 1;
+        }
+    }
+    wslots[i] = s;
+    wtris[i] = t;
+}
+
+void sftg_launch_walk_forms(const sftg_bvh_node* nodes, uint32_t count, const float* attr, const uint8_t* inds, uint32_t meshlets,
+                            sftg_wslot* wslots, sftg_wtri* wtris, cudaStream_t st) {
+    if (count) k_blas_walk_forms<<<(count * 8 + 255) / 256, 256, 0, st>>>(nodes, count, attr, inds, meshlets, wslots, wtris);
+}

@@ -118,8 +118,12 @@ struct sftg_pose_tables {
     const float* keys;
     const uint32_t* order;         /* per skeleton: bone | parent << 16 (0xFFFF: a root), parents first */
 };
-void sftg_launch_raycast(const sftg_ray* rays, uint32_t n, const sftg_model* models, uint32_t n_models, const sftg_bvh_node* blas,
-                         const float* ml_attr, const uint8_t* ml_inds, sftg_ray_hit* hits, cudaStream_t st);
+/* next: a device word, the ray counter of a launch of many rays; returns a cudaError_t */
+int sftg_launch_raycast(const sftg_ray* rays, uint32_t n, const sftg_model* models, uint32_t n_models, const sftg_wslot* wslots,
+                        const sftg_wtri* wtris, uint32_t* next, sftg_ray_hit* hits, cudaStream_t st);
+/* the walks' forms of `count` BLAS nodes of a model of `meshlets` meshlets at attr and inds */
+void sftg_launch_walk_forms(const sftg_bvh_node* nodes, uint32_t count, const float* attr, const uint8_t* inds, uint32_t meshlets,
+                            sftg_wslot* wslots, sftg_wtri* wtris, cudaStream_t st);
 /* BLAS construction on the device (sftg_blas.cu): begin counts the model's triangles and lays
  * out the tree's shape (node count known on return), finish builds the node images into dst
  * (status 1: a device work list overflowed), end releases the job. */

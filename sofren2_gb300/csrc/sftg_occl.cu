@@ -41,6 +41,24 @@ SFTG_D uint32_t node_mask(const sftg_bvh_node* nd, const frustum6& fr, int lane)
     return __ballot_sync(0xFFFFFFFFu, in) & 0xFFu;
 }
 
+/* the same test for the lane's slot of a BLAS node */
+SFTG_D uint32_t slot_mask(float4 mn, float4 mx, const frustum6& fr, int lane) {
+    bool in = false;
+    if (lane < 8) {
+        const float cx = (mx.x + mn.x) * 0.5f, cy = (mx.y + mn.y) * 0.5f, cz = (mx.z + mn.z) * 0.5f;
+        const float ex = (mx.x - mn.x) * 0.5f, ey = (mx.y - mn.y) * 0.5f, ez = (mx.z - mn.z) * 0.5f;
+        in = true;
+#pragma unroll
+        for (int p = 0; p < 6; p++) {
+            const float r = fma_(fr.an[p][0], ex, fma_(fr.an[p][1], ey, fr.an[p][2] * ez));
+            const float dc = fma_(fr.n[p][0], cx, fma_(fr.n[p][1], cy, fr.n[p][2] * cz));
+            const float dist = dc + fr.d[p];
+            in = in && (dist + r >= 0.f);
+        }
+    }
+    return __ballot_sync(0xFFFFFFFFu, in) & 0xFFu;
+}
+
 /* sft_m_view_look_at (1737-1770) */
 SFTG_D void view_look_at(v3 pos, v3 target, v3 up, float* m) {
     const v3 fwd = snorm(sub3(target, pos));
@@ -254,10 +272,8 @@ struct occ_rays { float ox[8], oy[8], oz[8], ix[8], iy[8], iz[8], tmax[8]; };
  * triangle's plane (|a| just above the test's 1e-6 threshold while its true value is rounding
  * noise) the reference's u, v and t are noise and it can report a hit far from the ray, which
  * this cull would skip.  That is why it is off by default. */
-SFTG_D uint32_t ray_box_mask(const sftg_bvh_node* nd, const occ_rays& R, uint32_t open_rays, int lane) {
-    const int c = lane & 7;
-    const float lo[3] = { nd->mn[0][c], nd->mn[1][c], nd->mn[2][c] };
-    const float hi[3] = { nd->mx[0][c], nd->mx[1][c], nd->mx[2][c] };
+SFTG_D uint32_t ray_box_mask(float4 mn, float4 mx, const occ_rays& R, uint32_t open_rays, int lane) {
+    const float lo[3] = { mn.x, mn.y, mn.z }, hi[3] = { mx.x, mx.y, mx.z };   /* slot lane & 7 */
     float blo[3], bhi[3];
 #pragma unroll
     for (int a = 0; a < 3; a++) {
@@ -338,19 +354,21 @@ SFTG_D uint32_t occ_walk_from(const sftg_frame* F, const sftg_inst* I, const sft
     int top = 1;
     if (lane == 0) stack[0] = start;      /* entry: node | depth << 29 (depth only tracked when expanding) */
     __syncwarp();
-    const sftg_bvh_node* blas = F->blas + Md.blas_base;
+    const sftg_wslot* slots = F->wslots + (size_t)Md.blas_base * 8;
+    const sftg_wtri* tris = F->wtris + (size_t)Md.blas_base * 8;
     uint32_t guard = 0;
     while (top > 0 && sat != full) {
         const uint32_t ent = stack[--top];
         __syncwarp();
         const uint32_t ni = ent & 0x1FFFFFFFu, depth = ent >> 29;
-        const sftg_bvh_node* nd = &blas[ni];
-        uint32_t m = node_mask(nd, w.mf, lane);
-        if (prune && m) m &= ray_box_mask(nd, R, full & ~sat, lane);
-        if (!nd->leaf) {
+        const float4* sl = (const float4*)(slots + (size_t)ni * 8 + (lane & 7));
+        const float4 mn = sl[0], mx = sl[1];
+        uint32_t m = slot_mask(mn, mx, w.mf, lane);
+        if (prune && m) m &= ray_box_mask(mn, mx, R, full & ~sat, lane);
+        if (!(__float_as_uint(mx.w) & 1u)) {
             /* lane c < 8 takes child c: one ballot for the checks, one atomic for the items, one
              * stack write per lane (the stack keeps the children in slot order) */
-            const uint32_t ch = lane < 8 ? nd->child[lane] : SFTG_INVALID;
+            const uint32_t ch = lane < 8 ? __float_as_uint(mn.w) : SFTG_INVALID;
             const bool mine = lane < 8 && ((m >> lane) & 1u) && ch != SFTG_INVALID;
             const uint32_t tm = __ballot_sync(0xFFFFFFFFu, mine);
             guard += (uint32_t)__popc(tm);
@@ -387,20 +405,13 @@ SFTG_D uint32_t occ_walk_from(const sftg_frame* F, const sftg_inst* I, const sft
             const bool have = (__popc(m) > kq) && c >= 0;
             for (int q = 0; q < 4 && m; q++) m &= m - 1;
             bool hit = false;
-            if (have && nd->child[c] != SFTG_INVALID && ((full & ~sat) >> r & 1u)) {
-                const uint32_t pay = nd->child[c] & ~0x80000000u;
-                const uint32_t g = I->meshlet_base + (pay >> 7), t = pay & 0x7F;
-                const uint8_t* ind = F->ml_inds + (size_t)g * 512;
-                const float* at = F->ml_attr + (size_t)g * 640;
-                const uint32_t tb = t >> 3, tl = t & 7;
-                const uint32_t i0 = ind[tb * 32 + tl], i1 = ind[tb * 32 + 8 + tl], i2 = ind[tb * 32 + 16 + tl];
-                const v3 v0 = mk3(at[i0], at[64 + i0], at[128 + i0]);
-                const v3 v1 = mk3(at[i1], at[64 + i1], at[128 + i1]);
-                const v3 v2 = mk3(at[i2], at[64 + i2], at[128 + i2]);
-                const v3 e1 = sub3(v1, v0), e2 = sub3(v2, v0);
+            if (have && ((full & ~sat) >> r & 1u)) {
+                const float4* tq = (const float4*)(tris + (size_t)ni * 8 + c);
+                const float4 ta = tq[0], tb = tq[1], tc = tq[2];
+                const v3 v0 = mk3(ta.x, ta.y, ta.z), e1 = mk3(ta.w, tb.x, tb.y), e2 = mk3(tb.z, tb.w, tc.x);
                 const v3 h = cross3(w.ld, e2);
                 const float a = vdot(e1, h);
-                hit = fabsf(a) > 1e-6f;
+                hit = __float_as_uint(tc.y) != 0u && fabsf(a) > 1e-6f;
                 const float fr = rcpr(a);
                 const v3 sv = sub3(w.lo, v0);
                 const float u = fr * vdot(sv, h);

@@ -13,7 +13,9 @@
  *                     cull[g] = f32[8] (sphere centre, radius, cone axis, cone cutoff),
  *                     info[g] (culling bone, skin slot, mesh material, lightmap texture);
  *                     skinned meshlets also own skin[slot] = u16 j[4][64] + u8 w[4][64]
- *   BLAS node pool    sft_bvh_node images (256 B: SoA child AABBs, child ids, count, leaf flag)
+ *   BLAS node pool    sft_bvh_node images (256 B: SoA child AABBs, child ids, count, leaf flag),
+ *                     and beside each the two forms the walks read: its slots (sftg_wslot) and,
+ *                     for a leaf, its triangles (sftg_wtri)
  *   sftg_model        per model: meshlet range in the pool, BLAS range, bone count
  *
  * Per frame (one upload of a few KB, then a bump arena for scratch):
@@ -72,7 +74,8 @@ typedef struct sftg_model {
     uint32_t meshlet_base, total_meshlets;
     uint32_t blas_base, blas_root, blas_count;
     uint32_t bone_count;
-    uint32_t mesh_count, pad;
+    uint32_t mesh_count;
+    uint32_t nested;       /* 1: every BLAS node's boxes lie inside the box its parent holds for it */
 } sftg_model;
 
 typedef struct sftg_bvh_node {  /* sft_bvh_node, sofren2.c:967-983 */
@@ -81,6 +84,21 @@ typedef struct sftg_bvh_node {  /* sft_bvh_node, sofren2.c:967-983 */
     uint32_t child[8];
     uint8_t count, leaf, pad[30];
 } sftg_bvh_node;
+
+/* A BLAS node's child slot as the walks read it, two 16-byte loads (the image keeps the reference's
+ * bytes for read-back), and a leaf's triangle, three, in place of the meshlet's indices and then its
+ * vertices.  8 of each per node. */
+typedef struct sftg_wslot {
+    float mn[3];
+    uint32_t child;
+    float mx[3];
+    uint32_t flags;        /* bit 0: the node is a leaf, bit 1: the slot is below the node's count */
+} sftg_wslot;
+typedef struct sftg_wtri {
+    float v0[3], e1[3], e2[3];   /* e1 = v1 - v0, e2 = v2 - v0 */
+    uint32_t ok;           /* 0: no triangle, or its meshlet index is outside the model */
+    uint32_t pad[2];
+} sftg_wtri;
 
 typedef struct sftg_inst {
     float T[16];           /* row-major 4x4, row vectors (translation in row 3) */
@@ -161,7 +179,8 @@ typedef struct sftg_frame {
     const sftg_meshlet_info* ml_info;
     const uint16_t* skin_j;        /* [slot][4][64] */
     const uint8_t* skin_w;         /* [slot][4][64] */
-    const sftg_bvh_node* blas;     /* pool */
+    const sftg_wslot* wslots;      /* BLAS pools, 8 per node */
+    const sftg_wtri* wtris;
     const uint32_t* lightmaps_of_model; /* unused: lightmap textures are resolved per meshlet */
 } sftg_frame;
 
