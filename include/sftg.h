@@ -174,14 +174,14 @@ int sftg_light_vis_noalloc(sftg_ctx* ctx, const sftg_frame_desc* frame, uint8_t*
 typedef struct sftg_tuning {
     int32_t resolve_split[3];     /* most resolve CTAs per 64x64 tile at 1x, 2x, 4x: 1, 2, 4, 8 or 16 (default 16); 8 and
                                      16 are halved, down to 4, where the tiles alone fill the GPU */
-    int32_t raster_slab_rows[3];  /* tile rows per raster work item at 1x, 2x, 4x: 4..64 (default 8, 8, 4) */
+    int32_t raster_slab_rows[3];  /* rows per triangle a raster group walks at a time at 1x, 2x, 4x: 4..64 (default 8) */
     int32_t geom_job_width;       /* meshlets per geometry warp: 1..8 (default 1; the reference's job is 8) */
     int32_t occl_ray_prune;       /* 1: also cull BLAS children no unblocked shadow ray reaches (faster; can differ
                                      from the reference only where a ray grazes a triangle's plane); default 0.
                                      The only knob that is not result-neutral: sftg_autotune leaves it as set */
-    int32_t raster_bands[3];      /* raster CTAs per 64x64 tile at 1x, 2x, 4x, each a band of its rows: 0 = by the
-                                     tile's payload count (default: 1, 2 above 48 payloads, 4 above 128; at 4x 2),
-                                     1, 2 or 4 = every tile (at 4x at least 2) */
+    int32_t raster_bands[3];      /* row bands a tile's raster is cut into at 1x, 2x, 4x, each a CTA of its own: 1, 2 or 4
+                                     (at 4x at least 2); 0 = the least (default).  Apart from that a heavy tile's
+                                     payload list is cut into parts by the batch's payload counts */
     int32_t tile_lights[3];       /* where a tile's light list and proxy selection are made at 1x, 2x, 4x: 1 = by each of
                                      its resolve CTAs, 2 = once per tile by a launch before the resolve (its CTAs read
                                      the result), 0 = 2 where the range has at least 128 tiles, else 1 (default) */

@@ -109,7 +109,7 @@ struct sftg_ctx {
     uint32_t blas_items = 0, blas_launches = 0; /* and its triangles and kernels */
     cudaEvent_t ev_blas[2] = { nullptr, nullptr };
     bool use_graphs = true;
-    sftg_tuning tuning = { { 16, 16, 16 }, { 8, 8, 4 }, 1, 0, { 0, 0, 0 }, { 0, 0, 0 }, 0 };   /* measured best on the single-view workloads */
+    sftg_tuning tuning = { { 16, 16, 16 }, { 8, 8, 8 }, 1, 0, { 0, 0, 0 }, { 0, 0, 0 }, 0 };   /* measured best on the single-view workloads */
     /* transient models (one frame's dynamic meshes): pool marks where they start */
     bool tr_live = false, tr_pinned = false;
     uint32_t tr_meshlets = 0, tr_skin = 0, tr_blas = 0;
@@ -518,6 +518,7 @@ struct batch_bufs {
     sftg_clip_tri* clips; int4* clip_rect;
     uint32_t* tile_count; uint32_t* tile_start;
     uint32_t* tile_order; uint32_t* order_scratch;
+    sftg_raster_item* raster_items; uint32_t* raster_range; uint32_t* raster_done;
     uint8_t* tile_nlights;   /* per tile: its light list length (debug views) */
     sftg_tile_lights* tile_lights;   /* per tile: lights and selected proxies, shared by its resolve CTAs */
     uint32_t* queue;         /* item counters of the persistent raster and resolve launches, one per launch */
@@ -696,12 +697,15 @@ static int build_batch(sftg_ctx* ctx, sftg_lane& ln, const sftg_frame_desc* fds,
     const size_t o_xv = stage_take((size_t)total_prox * 2 + 16);
     const size_t o_sv = stage_take((size_t)total_stiles * 2 + 16);
     const size_t stage_bytes = so;
+    size_t raster_items = 1;
+    for (int si = 0; si < 3; si++) if (B.s_tiles[si]) raster_items += sftg_raster_items_max(1 << si, B.s_tiles[si], ctx->tuning.raster_bands[si]);
     /* device arena layout */
     size_t need = stage_bytes + 4096;
     auto acc = [&](size_t bytes) { need = ((need + 255) & ~(size_t)255) + bytes; };
     acc((size_t)total_ss * SFTG_SS_FLOATS * 4); acc(n_rec * sizeof(sftg_batch_rec)); acc(n_rec * 4); acc(n_rec * 4);
     acc((size_t)total_ss * 16 + 16); acc(ctx->clip_cap * sizeof(sftg_clip_tri)); acc(ctx->clip_cap * 16);
-    acc((size_t)total_tiles * 4); acc((size_t)total_tiles * 4); acc((size_t)total_tiles * 4); acc(1024); acc(total_tiles + 16);
+    acc((size_t)total_tiles * 4); acc((size_t)total_tiles * 4); acc((size_t)total_tiles * 4); acc(2048); acc(total_tiles + 16);
+    acc(raster_items * sizeof(sftg_raster_item)); acc(64); acc((size_t)total_tiles * sftg_raster_bands() * 4);
     acc(ctx->tile_cap * 8);
     acc((size_t)total_stiles * 4); acc((size_t)total_stiles * 4); acc(ctx->stile_cap * 4);
     acc((size_t)total_prox * 64 + 64); acc((size_t)total_packets * sftg_packet_bytes() + 64);
@@ -749,7 +753,10 @@ static int build_batch(sftg_ctx* ctx, sftg_lane& ln, const sftg_frame_desc* fds,
     B.tile_count = bp.take<uint32_t>(total_tiles);
     B.tile_start = bp.take<uint32_t>(total_tiles);
     B.tile_order = bp.take<uint32_t>(total_tiles);
-    B.order_scratch = bp.take<uint32_t>(256);
+    B.order_scratch = bp.take<uint32_t>(512);
+    B.raster_items = bp.take<sftg_raster_item>(raster_items);
+    B.raster_range = bp.take<uint32_t>(16);
+    B.raster_done = bp.take<uint32_t>((size_t)total_tiles * sftg_raster_bands());
     B.tile_nlights = bp.take<uint8_t>((size_t)total_tiles + 16);
     B.any_overlay = false;
     for (uint32_t v = 0; v < nv; v++) if (fds[v].debug_mode >= 2 && fds[v].debug_mode <= 4) B.any_overlay = true;
@@ -908,17 +915,21 @@ static int launch_batch(sftg_ctx* ctx, sftg_lane& ln, const batch_bufs& B) {
         CK(cudaMemsetAsync(B.totals + 2, 0, 4, st));
     }
     k_bin<<<B.total_tiles, 256, 0, st>>>(B.frames, B.tile_view, B.recs, B.clip_cnt, B.clip_base, B.clip_rect, B.mrect,
-                                         B.stile_count, B.stile_start, B.stile_list, B.tile_count, nullptr, nullptr);
+                                         B.stile_count, B.stile_start, B.stile_list, B.tile_count, nullptr, nullptr,
+                                         nullptr, nullptr, nullptr);
     scan_u32(B.tile_count, B.tile_start, B.total_tiles, B.scan_tmp, B.totals + 1, st, &ln.launches);
     k_bin<<<B.total_tiles, 256, 0, st>>>(B.frames, B.tile_view, B.recs, B.clip_cnt, B.clip_base, B.clip_rect, B.mrect,
-                                         B.stile_count, B.stile_start, B.stile_list, B.tile_count, B.tile_start, B.tile_pay);
-    ln.launches += 2 + sftg_launch_tile_order(B.frames, B.tile_view, B.tile_count, B.total_tiles, B.order_scratch, B.tile_order, st);
+                                         B.stile_count, B.stile_start, B.stile_list, B.tile_count, B.tile_start, B.tile_pay,
+                                         B.totals + 1, B.vis, B.raster_done);
+    ln.launches += 2 + sftg_launch_tile_order(B.frames, B.tile_view, B.tile_count, B.total_tiles, B.totals + 1, ctx->tuning.raster_bands,
+                                              B.order_scratch, B.tile_order, B.raster_items, B.raster_range, st);
     CK(cudaGetLastError());
     CK(record_event(ln.ev[3], st));
     if (B.shadow) CK(cudaMemsetAsync(B.shadow, 0, B.color_total * 16 * 4, st));
     sftg_tile_args A;
     A.frames = B.frames; A.tile_view = B.tile_view; A.ss = B.ss; A.clips = B.clips; A.clip_base = B.clip_base;
-    A.tile_order = B.tile_order; A.tile_nlights = B.tile_nlights; A.tile_lights = B.tile_lights;
+    A.tile_order = B.tile_order; A.raster_items = B.raster_items; A.raster_range = B.raster_range; A.raster_done = B.raster_done;
+    A.tile_nlights = B.tile_nlights; A.tile_lights = B.tile_lights;
     A.tile_start = B.tile_start; A.tile_count = B.tile_count; A.tile_pay = B.tile_pay; A.light_vis = B.light_vis;
     A.vis = B.vis; A.zrange = B.zrange; A.vis_depth = B.vis_depth; A.vis_id = B.vis_id; A.shadow_out = B.shadow;
     /* With views of several sample counts, the 4x tile range runs on the main stream and the 1x
@@ -940,7 +951,7 @@ static int launch_batch(sftg_ctx* ctx, sftg_lane& ln, const batch_bufs& B) {
     const bool queue_raster = (ctx->tuning.tile_queue & 1) != 0, queue_resolve = (ctx->tuning.tile_queue & 2) != 0;
     if (ctx->tuning.tile_queue) CK(cudaMemsetAsync(B.queue, 0, 64, st));   /* counters: raster 0-2, resolve 3-5 */
     int prc = per_range(0, [&](int si, cudaStream_t s) {
-        sftg_launch_raster(1 << si, B.s_tile0[si], B.s_tiles[si], ctx->tuning.raster_slab_rows[si], ctx->tuning.raster_bands[si],
+        sftg_launch_raster(1 << si, B.s_tiles[si], ctx->tuning.raster_slab_rows[si], ctx->tuning.raster_bands[si],
                            queue_raster ? B.queue + si : nullptr, s, A);
     });
     if (prc) return prc;
@@ -981,7 +992,8 @@ static uint64_t batch_key(const sftg_ctx* ctx, const batch_bufs& B) {
     h = fnv(h, &ov, sizeof(ov));
     const void* ptrs[] = { B.frames, B.jobs, B.tile_view, B.packet_view, B.prox_view, B.stile_view, B.stile_count, B.stile_start,
                            B.stile_list, B.ss, B.recs, B.clip_cnt, B.clip_base, B.tile_nlights, B.tile_lights, B.queue,
-                           B.mrect, B.clips, B.clip_rect, B.tile_count, B.tile_start, B.tile_order, B.order_scratch, B.tile_pay,
+                           B.mrect, B.clips, B.clip_rect, B.tile_count, B.tile_start, B.tile_order, B.order_scratch, B.raster_items,
+                           B.raster_range, B.raster_done, B.tile_pay,
                            B.light_vis, B.packets, B.pairs, B.n_pairs, B.scan_tmp, B.status, B.totals, B.vis, B.zrange,
                            B.vis_depth, B.vis_id, B.shadow };
     h = fnv(h, ptrs, sizeof(ptrs));

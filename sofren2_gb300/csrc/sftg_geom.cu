@@ -427,7 +427,7 @@ k_bin(const sftg_frame* __restrict__ frames, const uint16_t* __restrict__ tile_v
       const uint32_t* __restrict__ clip_cnt, const uint32_t* __restrict__ clip_base, const int4* __restrict__ clip_rect,
       const int4* __restrict__ mrect, const uint32_t* __restrict__ stile_count, const uint32_t* __restrict__ stile_start,
       const uint32_t* __restrict__ stile_list, uint32_t* __restrict__ tile_count, const uint32_t* __restrict__ tile_start,
-      uint64_t* __restrict__ tile_pay)
+      uint64_t* __restrict__ tile_pay, const uint32_t* __restrict__ total, float2* __restrict__ vis, uint32_t* __restrict__ raster_done)
 {
     __shared__ uint32_t s_hits[BIN_THREADS];
     __shared__ uint32_t s_cnt[BIN_THREADS];
@@ -443,6 +443,12 @@ k_bin(const sftg_frame* __restrict__ frames, const uint16_t* __restrict__ tile_v
     const uint32_t vclip = n_ss ? clip_base[(size_t)F->ss_base * 16] : 0u;
     uint64_t* out = nullptr;
     if (tile_pay) {
+        if (sftg_raster_parts(tile_count[gtile], *total, F->samples) > 1u) {   /* rastered in parts, merged into a cleared buffer */
+            const int n = F->samples * SFTG_TILE_PX / 2;
+            float4* v = (float4*)(vis + F->vis_base + (size_t)tile * F->samples * SFTG_TILE_PX);
+            for (int i = tid; i < n; i += BIN_THREADS) v[i] = make_float4(0.f, 0.f, 0.f, 0.f);
+            if (tid < 4) raster_done[gtile * 4 + tid] = 0u;
+        }
         /* over capacity: the host grows the buffer and re-renders; write nothing */
         if ((uint64_t)tile_start[gtile] + tile_count[gtile] > F->tile_cap) return;
         out = tile_pay + tile_start[gtile];

@@ -31,6 +31,26 @@ struct sftg_tile_lights {
     uint32_t pad[3];
 };
 
+/* Raster work item: a row band of a tile and a part of its payload list. */
+struct sftg_raster_item { uint32_t tile; uint8_t band, bands; uint16_t part; uint32_t parts; uint32_t pad; };
+/* Parts of a tile's list of `count` payloads, of `total` in the batch.  A frame's raster time is its
+ * slowest item's, and a small frame's few tiles hold thousands of payloads each; but every part
+ * clears a band of keys and merges them (64-bit maxima in the visibility buffer; the last part to
+ * finish decodes), so parts no smaller than the batch's share per resident CTA (2 on each of the
+ * 152 SMs; 2 items a tile at 4x), and no smaller than 32 payloads, 64 at 4x with its larger keys.
+ * Raster before (1 to 4 row bands per tile by its payloads) and with parts, 8 * S lanes per triangle in
+ * both: skinned 1080p 2x 0.110 -> 0.098 ms, atrium 1279x719 1x 0.098 -> 0.082, atrium 640x360 1x 0.098
+ * -> 0.059, skinned 320x180 2x 0.178 -> 0.047, atrium 155x106 4x 0.817 -> 0.104; 1080p 4x the same
+ * (0.228: no list is cut; cut at half the share 0.238-0.256), 48 views 3.90 -> 3.41 (no bands). */
+#define SFTG_RASTER_CTAS 304u
+static __host__ __device__ __forceinline__ uint32_t sftg_raster_parts(uint32_t count, uint32_t total, int samples) {
+    const uint32_t least = samples == 4 ? 64u : 32u;
+    const uint32_t share = (uint32_t)(((uint64_t)total * (samples == 4 ? 2u : 1u) + SFTG_RASTER_CTAS - 1) / SFTG_RASTER_CTAS);
+    const uint32_t per = share > least ? share : least;
+    const uint32_t parts = (count + per / 2u) / per;
+    return parts > 1u ? parts : 1u;
+}
+
 struct sftg_tile_args {
     const sftg_frame* frames;
     const uint16_t* tile_view;
@@ -38,6 +58,9 @@ struct sftg_tile_args {
     const sftg_clip_tri* clips;
     const uint32_t* clip_base;     /* exclusive scan of clip counts: a view's first slot is clip_base[ss_base * 16] */
     const uint32_t* tile_order;    /* launch order of the tiles (heaviest first within each sample count) */
+    const sftg_raster_item* raster_items;   /* heaviest tiles first within each sample count */
+    const uint32_t* raster_range;  /* per sample count: first item, then per sample count: items */
+    uint32_t* raster_done;         /* per tile and band: parts merged so far */
     uint8_t* tile_nlights;         /* per tile: light list length, for the debug overlays (k_tile_lights or the resolve) */
     sftg_tile_lights* tile_lights; /* per tile, written by k_tile_lights, read by every resolve CTA of the tile
                                       where the range's resolve is launched with records */
@@ -62,7 +85,7 @@ __global__ void k_coarse(const sftg_frame* frames, const uint16_t* stile_view, c
 __global__ void k_bin(const sftg_frame* frames, const uint16_t* tile_view, const sftg_batch_rec* recs, const uint32_t* clip_cnt,
                       const uint32_t* clip_base, const int4* clip_rect, const int4* mrect, const uint32_t* stile_count,
                       const uint32_t* stile_start, const uint32_t* stile_list, uint32_t* tile_count,
-                      const uint32_t* tile_start, uint64_t* tile_pay);
+                      const uint32_t* tile_start, uint64_t* tile_pay, const uint32_t* total, float2* vis, uint32_t* raster_done);
 __global__ void k_scan_reduce(const uint32_t* in, uint32_t n, uint32_t* sums);
 __global__ void k_scan_top(uint32_t* sums, uint32_t nb, uint32_t* total_out);
 __global__ void k_scan_down(const uint32_t* in, uint32_t n, const uint32_t* sums, uint32_t* out);
@@ -80,16 +103,19 @@ void sftg_launch_occlusion(const sftg_frame* frames, const uint16_t* packet_view
                            uint32_t max_pairs, uint32_t items_per_pair, uint8_t* light_vis, uint32_t* status, int ray_prune,
                            cudaStream_t st);
 cudaError_t sftg_tile_configure(int max_dynamic_smem);
-int sftg_raster_bands(void);   /* raster CTAs (row bands) per 64x64 tile */
-/* order[] = the batch's tiles, heaviest first inside each sample-count range; scratch holds 192 words */
+int sftg_raster_bands(void);   /* most row bands of a 64x64 tile */
+/* order[] = the batch's tiles, heaviest first inside each sample-count range, items[] = the raster's work
+ * items in the same order, range[] their first and number per sample count (6 words); total: the
+ * batch's payload count; bands: the raster_bands knob; scratch holds 512 words.  Returns the launches. */
 int sftg_launch_tile_order(const sftg_frame* frames, const uint16_t* tile_view, const uint32_t* tile_count, uint32_t n_tiles,
-                            uint32_t* scratch, uint32_t* order, cudaStream_t st);
+                           const uint32_t* total, const int* bands, uint32_t* scratch, uint32_t* order, sftg_raster_item* items,
+                           uint32_t* range, cudaStream_t st);
+uint32_t sftg_raster_items_max(int S, uint32_t tiles, int bands);   /* bound on the items of a sample-count range */
 /* resolve CTAs per tile and where its light lists are made, from the tuning knobs and the tile count */
 int sftg_resolve_split(int knob, uint32_t tiles);
 bool sftg_resolve_records(int knob, uint32_t tiles);
 /* slab_rows: rows of one raster work item (4..64); split: resolve CTAs per tile (1, 2, 4, 8 or 16) */
-void sftg_launch_raster(int S, uint32_t tile0, uint32_t tiles, int slab_rows, int bands, uint32_t* queue, cudaStream_t st,
-                        const sftg_tile_args& A);
+void sftg_launch_raster(int S, uint32_t tiles, int slab_rows, int bands, uint32_t* queue, cudaStream_t st, const sftg_tile_args& A);
 void sftg_launch_tile_lights(uint32_t tile0, uint32_t tiles, cudaStream_t st, const sftg_tile_args& A);
 /* queue: null for one CTA per (tile, part) item, else a zeroed counter for one persistent launch
  * whose CTAs take the items in launch order (k_resolve_queue); likewise for the raster */

@@ -2,18 +2,16 @@
  * Per-tile raster and resolve (sft__worker_phase_rasterize, sofren2.c:6756-6813,
  * sft__rast_simd_batch 5148-5499, sft__resolve_tile 5809-6753).
  *
- * k_raster: one to four CTAs per 64x64 tile, each owning a band of its rows (more for tiles with
- * more payloads; every CTA sets up the tile's whole list and keeps the triangles that reach its
- * band, whose rows it walks from the triangle's first row exactly as the one-CTA walk would).
- * The reference walks the tile's list in order and keeps a
+ * k_raster: a CTA per work item, a part of a 64x64 tile's payload list on the tile or a band of its
+ * rows (sftg_raster_parts; a band keeps the triangles that reach it, whose rows it walks from the
+ * triangle's first row exactly as the whole tile's walk would).  The reference walks the tile's list in order and keeps a
  * sample when z > stored z (strict), so a sample ends holding the largest z, and among equal z
  * the earliest triangle.  That final state does not depend on the order triangles are visited,
  * so each sample is a 64-bit shared-memory word (z bits << 32 | ~order) updated with atomicMax,
  * where order = list position * 8 + lane; only z > 0 ever wins (the buffer starts at 0).
- * Coverage and z are replayed bit-exactly: a group of 8 threads takes one triangle, thread l
- * owns pixel column l of every aligned 8-pixel chunk and performs exactly the reference's
- * incremental adds (row start + B per row, + 8A per chunk) and its trivial-accept / AA
- * guard-band choices; the AA chunk skip is a group ballot.  The decoded visibility buffer
+ * Coverage and z are replayed bit-exactly: a group of 8 * S threads takes one triangle's rows, a thread
+ * one sample of a pixel column of every aligned 8-pixel chunk (tri_raster), with the reference's
+ * trivial-accept / AA guard-band choices; the AA chunk skip is a group ballot.  The decoded visibility buffer
  * (depth, vid) goes to global memory, where it stays L2-resident, with the tile's depth range.
  *
  * k_resolve: 1 to 16 CTAs per tile (sftg_resolve_split), each a share of its 4x2 blocks (the
@@ -27,11 +25,7 @@
 
 #define TILE_THREADS 256          /* resolve CTA */
 #define RASTER_THREADS 512        /* raster CTA: 64 groups of 8 */
-/* A tile is rastered by 1, 2 or 4 CTAs, each owning a band of its rows, by its payload count: the
- * frame's raster time is set by its heaviest tiles, which one CTA would walk alone. */
-#define RASTER_BANDS 4            /* raster CTAs launched per tile; those past the tile's band count exit */
-#define BANDS2_ABOVE 48           /* payloads above which a tile gets 2 bands */
-#define BANDS4_ABOVE 128          /* and 4 (1x and 2x; measured: at 4x two bands are best for every tile) */
+#define RASTER_BANDS 4            /* most row bands of a tile */
 /* keys of one sample plane in shared memory: a whole tile, except at 4x, where every tile takes at
  * least 2 bands so that the keys (S x 32 KB per tile) leave room for 2 CTAs per SM */
 template <int S> struct raster_plan {
@@ -184,16 +178,19 @@ SFTG_D bool tri_setup_one(float sx0, float sy0, float iw0, float sx1, float sy1,
     return true;
 }
 
-/* the incremental edge walk for pixel column `l` of one triangle (5345-5497) */
+/* The incremental edge walk of one triangle's rows y0..y1 (5345-5497) by a group of 8 * S lanes: lane
+ * (sample << 3 | l) owns one sample of pixel column l of every aligned 8-pixel chunk.  All lanes of a
+ * column perform exactly the reference's adds of the pixel (row start + B per row, + 8A per chunk),
+ * then each its own sample's offset.  Bound by issue: with 8 lanes per triangle and the samples in
+ * turn, the four groups of a warp diverged over their triangles' sizes (17 of 32 threads) and the 4x
+ * raster of the 1080p atrium took 0.287 ms; a warp per triangle 0.258, and 0.228 with slabs of 8 rows,
+ * which now balance well enough (4 rows 0.251). */
 template <int S>
-SFTG_D void tri_raster(const tri_setup& T, int y0, int y1, int l, uint32_t gmask, int tmx, int ky0, unsigned long long* keys) {
-    float de0[S], de1[S], de2[S], dz[S];
-#pragma unroll
-    for (int s = 0; s < S; s++) {
-        const float ox = ms_ox<S>(s), oy = ms_oy<S>(s);
-        de0[s] = T.A[0] * ox + T.B[0] * oy; de1[s] = T.A[1] * ox + T.B[1] * oy; de2[s] = T.A[2] * ox + T.B[2] * oy;
-        dz[s] = T.dzdx * ox + T.dzdy * oy;
-    }
+SFTG_D void tri_raster(const tri_setup& T, int y0, int y1, int lane, uint32_t gmask, int tmx, int ky0, unsigned long long* keys) {
+    const int l = lane & 7, smp = (lane >> 3) & (S - 1);
+    const float ox = ms_ox<S>(smp), oy = ms_oy<S>(smp);
+    const float de0 = T.A[0] * ox + T.B[0] * oy, de1 = T.A[1] * ox + T.B[1] * oy, de2 = T.A[2] * ox + T.B[2] * oy;
+    const float dz = T.dzdx * ox + T.dzdy * oy;
     const float fl = (float)l;
     float e0r = T.se[0] + T.A[0] * fl, e1r = T.se[1] + T.A[1] * fl, e2r = T.se[2] + T.A[2] * fl;
     float zr = T.sz + T.dzdx * fl;
@@ -203,30 +200,20 @@ SFTG_D void tri_raster(const tri_setup& T, int y0, int y1, int l, uint32_t gmask
     const float a0c = T.A[0] * 8.f, a1c = T.A[1] * 8.f, a2c = T.A[2] * 8.f, zc = T.dzdx * 8.f;
     const float np0 = -T.pad[0], np1 = -T.pad[1], np2 = -T.pad[2];
     const uint32_t order = T.order;
+    unsigned long long* const kp = keys + smp * raster_plan<S>::plane + (T.ax0 - tmx) + l;   /* keys hold the band's rows from ky0 */
+    const int width = T.ax1 - T.ax0;
     for (int y = y0; y <= y1; y++) {
         float e0 = e0r, e1 = e1r, e2 = e2r, z = zr;
-        int pi = (y - ky0) * SFTG_TILE + (T.ax0 - tmx) + l;   /* keys hold the band's rows from ky0 */
-        for (int x = T.ax0; x < T.ax1; x += 8, pi += 8) {
+        unsigned long long* k = kp + (y - ky0) * SFTG_TILE;
+        for (int x = 0; x < width; x += 8, k += 8) {
             if (T.trivial) {
-#pragma unroll
-                for (int s = 0; s < S; s++) {
-                    const float zs = (S > 1) ? z + dz[s] : z;
-                    if (zs > 0.f) atomicMax(&keys[s * raster_plan<S>::plane + pi], zkey(zs, order));
-                }
+                const float zs = (S > 1) ? z + dz : z;
+                if (zs > 0.f) atomicMax(k, zkey(zs, order));
             } else if (S == 1) {
-                if (e0 >= 0.f && e1 >= 0.f && e2 >= 0.f && z > 0.f) atomicMax(&keys[pi], zkey(z, order));
-            } else {
-                const bool might = (e0 >= np0 && e1 >= np1 && e2 >= np2);
-                if (__ballot_sync(gmask, might) & gmask) {
-#pragma unroll
-                    for (int s = 0; s < S; s++) {
-                        const float a = e0 + de0[s], b = e1 + de1[s], c = e2 + de2[s];
-                        if (a >= 0.f && b >= 0.f && c >= 0.f) {
-                            const float zs = z + dz[s];
-                            if (zs > 0.f) atomicMax(&keys[s * raster_plan<S>::plane + pi], zkey(zs, order));
-                        }
-                    }
-                }
+                if (e0 >= 0.f && e1 >= 0.f && e2 >= 0.f && z > 0.f) atomicMax(k, zkey(z, order));
+            } else if (__ballot_sync(gmask, e0 >= np0 && e1 >= np1 && e2 >= np2)) {
+                const float a = e0 + de0, b = e1 + de1, c = e2 + de2, zs = z + dz;
+                if (a >= 0.f && b >= 0.f && c >= 0.f && zs > 0.f) atomicMax(k, zkey(zs, order));
             }
             e0 = e0 + a0c; e1 = e1 + a1c; e2 = e2 + a2c; z = z + zc;
         }
@@ -287,12 +274,13 @@ SFTG_D void sample_nearest(const sftg_frame* F, int ti, int lod, float cu, float
 }
 
 /* ---------------------------------------------------------------- raster */
-/* One (tile, band) item, run by one CTA: the tile's payload list into a shared-memory visibility
- * buffer (64-bit z/order words) for the band's rows, decoded into the global visibility buffer
- * (float2: depth, vid bits) plus the band's depth range over valid samples (sofren2.c:5820-5853),
- * which the resolve needs for its light culling (a tile's range is the union of its bands'). */
+/* One item, run by one CTA: its part of the tile's payload list into a shared-memory visibility buffer
+ * (64-bit z/order words) for the band's rows, merged with the list's other parts where there are any,
+ * then decoded into the global visibility buffer (float2: depth, vid bits) plus the band's depth
+ * range over valid samples (sofren2.c:5820-5853), which the resolve needs for its light culling (a
+ * tile's range is the union of its bands'). */
 template <int S>
-SFTG_D void raster_item(const sftg_tile_args& A, uint32_t tile0, int slab_rows, int fixed_bands, uint32_t item)
+SFTG_D void raster_item(const sftg_tile_args& A, int slab_rows, const sftg_raster_item W)
 {
     extern __shared__ __align__(16) unsigned char smem[];
     unsigned long long* keys = (unsigned long long*)smem;                  /* S planes, a band uses the first band_px of each */
@@ -304,8 +292,9 @@ SFTG_D void raster_item(const sftg_tile_args& A, uint32_t tile0, int slab_rows, 
      * still walking a long slab (items touch keys only through atomicMax: order is free) */
     const uint32_t items_cap = (uint32_t)SETUP_CAP * (uint32_t)((raster_plan<S>::rows + slab_rows - 1) / slab_rows);
     __shared__ float s_red[2][RASTER_THREADS / 32];
-    const uint32_t gtile = A.tile_order[tile0 + item / RASTER_BANDS];   /* batch-wide tile index, heaviest first */
-    const int band = (int)(item % RASTER_BANDS);
+    __shared__ uint32_t s_done;
+    const uint32_t gtile = W.tile;   /* batch-wide tile index */
+    const int band = W.band, bands = W.bands;
     const sftg_frame* F = A.frames + A.tile_view[gtile];
     const int tile = (int)(gtile - F->tile_base);
     const float* ss = A.ss + (size_t)F->ss_base * SFTG_SS_FLOATS;
@@ -314,12 +303,6 @@ SFTG_D void raster_item(const sftg_tile_args& A, uint32_t tile0, int slab_rows, 
     const int tmx = (tile % F->cols) * SFTG_TILE, tmy = (tile / F->cols) * SFTG_TILE;
     uint32_t count = A.tile_count[gtile];
     if ((uint64_t)A.tile_start[gtile] + count > F->tile_cap) count = 0;   /* overflowed frame, redone by the host */
-    const int bands = max(raster_plan<S>::min_bands,
-                          fixed_bands ? fixed_bands : ((S < 4 && count > BANDS4_ABOVE) ? 4 : (count > BANDS2_ABOVE ? 2 : 1)));
-    if (band >= bands) {   /* not needed for this tile: an empty depth range for the readers' union */
-        if (threadIdx.x == 0) A.zrange[(size_t)gtile * RASTER_BANDS + band] = make_float2(1e9f, -1e9f);
-        return;
-    }
     const int band_rows = SFTG_TILE / bands, band_px = band_rows * SFTG_TILE;
     const int by0 = tmy + band * band_rows, by1 = by0 + band_rows - 1;   /* this CTA's rows */
     const uint64_t* list = A.tile_pay + A.tile_start[gtile];
@@ -328,13 +311,15 @@ SFTG_D void raster_item(const sftg_tile_args& A, uint32_t tile0, int slab_rows, 
 
     for (int i = tid; i < S * band_px; i += RASTER_THREADS) keys[(i / band_px) * raster_plan<S>::plane + i % band_px] = 0ull;
     const int grp_lane = tid & 7;
-    const uint32_t gmask = 0xFFu << (lane & ~7);
+    const uint32_t wmask = (0xFFFFFFFFu >> (32 - 8 * S)) << (lane & ~(8 * S - 1));   /* the walk's group */
     /* the payloads in equal rounds of at most SETUP_CAP / 8 (a short last round would leave most
      * groups idle at its barrier) */
-    const uint32_t rounds = (count + SETUP_CAP / 8 - 1) / (SETUP_CAP / 8);
-    const uint32_t per_round = rounds ? (count + rounds - 1) / rounds : 1u;
-    for (uint32_t pbase = 0; pbase < count; pbase += per_round) {
-        const uint32_t pend = min(count, pbase + per_round);
+    const uint32_t per_part = (count + W.parts - 1) / W.parts;
+    const uint32_t part0 = min(count, W.part * per_part), part1 = min(count, part0 + per_part), mine = part1 - part0;
+    const uint32_t rounds = (mine + SETUP_CAP / 8 - 1) / (SETUP_CAP / 8);
+    const uint32_t per_round = rounds ? (mine + rounds - 1) / rounds : 1u;
+    for (uint32_t pbase = part0; pbase < part1; pbase += per_round) {
+        const uint32_t pend = min(part1, pbase + per_round);
         if (tid == 0) { s_nsetup = 0; s_nbig = 0; s_nsmall = 0; s_next = 0; }
         __syncthreads();
         {
@@ -391,25 +376,39 @@ SFTG_D void raster_item(const sftg_tile_args& A, uint32_t tile0, int slab_rows, 
         const uint32_t nbig = s_nbig, nitem = nbig + s_nsmall;
         while (true) {
             uint32_t idx = 0;
-            if (grp_lane == 0) idx = atomicAdd(&s_next, 1u);
-            idx = __shfl_sync(gmask, idx, lane & ~7);
+            if ((lane & (8 * S - 1)) == 0) idx = atomicAdd(&s_next, 1u);
+            idx = __shfl_sync(wmask, idx, lane & ~(8 * S - 1));
             if (idx >= nitem) break;
             const uint32_t it = idx < nbig ? items[idx] : items[items_cap - 1u - (idx - nbig)];
             const tri_setup T = unpack_setup<S>(setups[it >> 8], tmx, tmy);
             const int y0 = max(T.miny, by0) + (int)(it & 0xFFu) * slab_rows;   /* rows before y0 are replayed */
             const int y1 = min(y0 + slab_rows - 1, min(T.maxy, by1));
-            tri_raster<S>(T, y0, y1, grp_lane, gmask, tmx, by0, keys);
+            tri_raster<S>(T, y0, y1, lane, wmask, tmx, by0, keys);
         }
         __syncthreads();
     }
     __syncthreads();
+    float2* tv = A.vis + F->vis_base + (size_t)tile * S * SFTG_TILE_PX;
+    unsigned long long* const merged = (unsigned long long*)tv;   /* of a list in parts: cleared by k_bin */
+    if (W.parts > 1) {
+        for (int i = tid; i < S * band_px; i += RASTER_THREADS) {
+            const int sp = i / band_px, pp = i % band_px;
+            const unsigned long long k = keys[sp * raster_plan<S>::plane + pp];
+            if (k) atomicMax(&merged[sp * SFTG_TILE_PX + band * band_px + pp], k);
+        }
+        __threadfence();
+        __syncthreads();
+        if (tid == 0) s_done = atomicAdd(&A.raster_done[gtile * RASTER_BANDS + band], 1u);
+        __syncthreads();
+        if (s_done + 1 != W.parts) return;   /* the last part decodes: nobody waits */
+        __threadfence();
+    }
     /* decode, store, depth range */
     float zmin = 1e9f, zmax = -1e9f;
-    float2* tv = A.vis + F->vis_base + (size_t)tile * S * SFTG_TILE_PX;
     for (int i = tid; i < S * band_px; i += RASTER_THREADS) {
         const int sp = i / band_px, pp = i % band_px;
-        const unsigned long long k = keys[sp * raster_plan<S>::plane + pp];
         const int ti = sp * SFTG_TILE_PX + band * band_px + pp;              /* the same sample in the tile */
+        const unsigned long long k = W.parts > 1 ? __ldcg(&merged[ti]) : keys[sp * raster_plan<S>::plane + pp];
         float d = 0.f; uint32_t vid = SFTG_INVALID;
         if (k) {
             d = __uint_as_float((uint32_t)(k >> 32));
@@ -433,32 +432,36 @@ SFTG_D void raster_item(const sftg_tile_args& A, uint32_t tile0, int slab_rows, 
         zmin = 1e9f; zmax = -1e9f;
         for (int w = 0; w < RASTER_THREADS / 32; w++) { zmin = fminf(zmin, s_red[0][w]); zmax = fmaxf(zmax, s_red[1][w]); }
         A.zrange[(size_t)gtile * RASTER_BANDS + band] = make_float2(zmin, zmax);   /* combined by the readers */
+        if (band == 0) for (int b = bands; b < RASTER_BANDS; b++) A.zrange[(size_t)gtile * RASTER_BANDS + b] = make_float2(1e9f, -1e9f);
     }
 }
 
-/* one CTA per (tile, band) item */
+/* one CTA per item; the grid is the bound on their number */
 template <int S>
 __global__ void __launch_bounds__(RASTER_THREADS)
-k_raster(const sftg_tile_args A, uint32_t tile0, int slab_rows, int fixed_bands)
+k_raster(const sftg_tile_args A, int slab_rows)
 {
-    raster_item<S>(A, tile0, slab_rows, fixed_bands, blockIdx.x);
+    constexpr int si = S == 4 ? 2 : S - 1;
+    if (blockIdx.x >= A.raster_range[3 + si]) return;
+    raster_item<S>(A, slab_rows, A.raster_items[A.raster_range[si] + blockIdx.x]);
 }
 
-/* Persistent form: as many CTAs as fit on the GPU at once, each taking the next (tile, band) item
- * in launch order (heaviest tiles first) from a counter until all n_items are taken.  The loop
- * ends after at most n_items + grid counter reads: nothing waits on another CTA. */
+/* Persistent form: as many CTAs as fit on the GPU at once, each taking the next item in launch order
+ * from a counter until all are taken.  The loop ends after at most items + grid counter reads:
+ * nothing waits on another CTA. */
 template <int S>
 __global__ void __launch_bounds__(RASTER_THREADS, 2)   /* the 64 registers k_raster gets: 2 CTAs per SM */
-k_raster_queue(const sftg_tile_args A, uint32_t tile0, int slab_rows, int fixed_bands, uint32_t n_items, uint32_t* next)
+k_raster_queue(const sftg_tile_args A, int slab_rows, uint32_t* next)
 {
+    constexpr int si = S == 4 ? 2 : S - 1;
     __shared__ uint32_t s_item;
     for (;;) {
         __syncthreads();   /* the previous item is done with shared memory, and s_item has been read */
         if (threadIdx.x == 0) s_item = atomicAdd(next, 1u);
         __syncthreads();
         const uint32_t item = s_item;
-        if (item >= n_items) break;
-        raster_item<S>(A, tile0, slab_rows, fixed_bands, item);
+        if (item >= A.raster_range[3 + si]) break;
+        raster_item<S>(A, slab_rows, A.raster_items[A.raster_range[si] + item]);
     }
 }
 
@@ -1195,6 +1198,7 @@ k_resolve_queue(const sftg_tile_args A, uint32_t tile0, int split, bool records,
  * short: tiles are bucketed by floor(log2(count + 1)) inside their sample-count range and the
  * launches walk the buckets heaviest first.  Order affects scheduling only, never results. */
 #define ORDER_BUCKETS 32
+#define ORDER_ALL (3 * ORDER_BUCKETS)
 
 __device__ __forceinline__ uint32_t order_bucket(const sftg_frame* frames, const uint16_t* tile_view, const uint32_t* tile_count, uint32_t t) {
     const int S = frames[tile_view[t]].samples;
@@ -1203,70 +1207,120 @@ __device__ __forceinline__ uint32_t order_bucket(const sftg_frame* frames, const
     return si * ORDER_BUCKETS + (ORDER_BUCKETS - 1u - key);
 }
 
+struct band_knobs { int b[3]; };   /* tuning.raster_bands */
+
+/* row bands of a tile at 1x, 2x, 4x (slot si): the knob's, at 4x at least 2 (shared memory) */
+__device__ __forceinline__ uint32_t order_bands(const band_knobs& K, uint32_t si) {
+    const uint32_t b = (uint32_t)K.b[si], least = si == 2u ? 2u : 1u;
+    return b > least ? b : least;
+}
+
+/* the exclusive starts of both histograms, and the item range of every sample count */
+__device__ __forceinline__ void order_starts(const uint32_t* h, uint32_t* base, uint32_t* range) {
+    uint32_t run = 0, items = 0;
+    for (uint32_t i = 0; i < ORDER_ALL; i++) {
+        if (range && i % ORDER_BUCKETS == 0) range[i / ORDER_BUCKETS] = items;
+        base[i] = run; base[ORDER_ALL + i] = items;
+        run += h[i]; items += h[ORDER_ALL + i];
+        if (range && i % ORDER_BUCKETS == ORDER_BUCKETS - 1) range[3 + i / ORDER_BUCKETS] = items - range[i / ORDER_BUCKETS];
+    }
+}
+
+/* tile t's place in the order and its raster items, from counters that start at its bucket's */
+__device__ __forceinline__ void order_place(uint32_t t, uint32_t b, uint32_t count, uint32_t total, const band_knobs& K, uint32_t* cursor,
+                                            uint32_t* order, sftg_raster_item* items) {
+    order[atomicAdd(&cursor[b], 1u)] = t;
+    const uint32_t bands = order_bands(K, b / ORDER_BUCKETS), parts = sftg_raster_parts(count, total, 1 << (b / ORDER_BUCKETS));
+    uint32_t at = atomicAdd(&cursor[ORDER_ALL + b], bands * parts);
+    for (uint32_t p = 0; p < parts; p++)
+        for (uint32_t k = 0; k < bands; k++) {
+            sftg_raster_item w;
+            w.tile = t; w.band = (uint8_t)k; w.bands = (uint8_t)bands; w.part = (uint16_t)p; w.parts = parts; w.pad = 0;
+            items[at++] = w;
+        }
+}
+
 __global__ void k_order_count(const sftg_frame* __restrict__ frames, const uint16_t* __restrict__ tile_view,
-                              const uint32_t* __restrict__ tile_count, uint32_t n_tiles, uint32_t* __restrict__ hist)
+                              const uint32_t* __restrict__ tile_count, uint32_t n_tiles, const uint32_t* __restrict__ total,
+                              const band_knobs K, uint32_t* __restrict__ hist)
 {
-    __shared__ uint32_t h[3 * ORDER_BUCKETS];
-    for (int i = threadIdx.x; i < 3 * ORDER_BUCKETS; i += blockDim.x) h[i] = 0;
+    __shared__ uint32_t h[2 * ORDER_ALL];
+    for (int i = threadIdx.x; i < 2 * ORDER_ALL; i += blockDim.x) h[i] = 0;
     __syncthreads();
     const uint32_t t = blockIdx.x * blockDim.x + threadIdx.x;
-    if (t < n_tiles) atomicAdd(&h[order_bucket(frames, tile_view, tile_count, t)], 1u);
+    if (t < n_tiles) {
+        const uint32_t b = order_bucket(frames, tile_view, tile_count, t);
+        atomicAdd(&h[b], 1u);
+        atomicAdd(&h[ORDER_ALL + b], order_bands(K, b / ORDER_BUCKETS) * sftg_raster_parts(tile_count[t], *total, 1 << (b / ORDER_BUCKETS)));
+    }
     __syncthreads();
-    for (int i = threadIdx.x; i < 3 * ORDER_BUCKETS; i += blockDim.x) if (h[i]) atomicAdd(&hist[i], h[i]);
+    for (int i = threadIdx.x; i < 2 * ORDER_ALL; i += blockDim.x) if (h[i]) atomicAdd(&hist[i], h[i]);
+}
+
+/* one CTA: the starts, into the histogram's place */
+__global__ void k_order_starts(uint32_t* __restrict__ hist, uint32_t* __restrict__ range)
+{
+    __shared__ uint32_t h[2 * ORDER_ALL], base[2 * ORDER_ALL];
+    for (int i = threadIdx.x; i < 2 * ORDER_ALL; i += blockDim.x) h[i] = hist[i];
+    __syncthreads();
+    if (threadIdx.x == 0) order_starts(h, base, range);
+    __syncthreads();
+    for (int i = threadIdx.x; i < 2 * ORDER_ALL; i += blockDim.x) hist[i] = base[i];
 }
 
 __global__ void k_order_scatter(const sftg_frame* __restrict__ frames, const uint16_t* __restrict__ tile_view,
-                                const uint32_t* __restrict__ tile_count, uint32_t n_tiles, const uint32_t* __restrict__ hist,
-                                uint32_t* __restrict__ cursor, uint32_t* __restrict__ order)
+                                const uint32_t* __restrict__ tile_count, uint32_t n_tiles, const uint32_t* __restrict__ total,
+                                const band_knobs K, uint32_t* __restrict__ cursor, uint32_t* __restrict__ order,
+                                sftg_raster_item* __restrict__ items)
 {
-    __shared__ uint32_t base[3 * ORDER_BUCKETS];
-    if (threadIdx.x == 0) {
-        uint32_t run = 0;
-        for (int i = 0; i < 3 * ORDER_BUCKETS; i++) { base[i] = run; run += hist[i]; }
-    }
-    __syncthreads();
     const uint32_t t = blockIdx.x * blockDim.x + threadIdx.x;
-    if (t >= n_tiles) return;
-    const uint32_t b = order_bucket(frames, tile_view, tile_count, t);
-    order[base[b] + atomicAdd(&cursor[b], 1u)] = t;
+    if (t < n_tiles) order_place(t, order_bucket(frames, tile_view, tile_count, t), tile_count[t], *total, K, cursor, order, items);
 }
 
-/* the same order in one CTA for small tile counts: histogram, bucket starts and scatter in
- * shared memory */
+/* the same in one CTA for small tile counts: histogram, bucket starts and scatter in shared memory */
 __global__ void __launch_bounds__(1024)
 k_order_small(const sftg_frame* __restrict__ frames, const uint16_t* __restrict__ tile_view, const uint32_t* __restrict__ tile_count,
-              uint32_t n_tiles, uint32_t* __restrict__ order)
+              uint32_t n_tiles, const uint32_t* __restrict__ total, const band_knobs K, uint32_t* __restrict__ order,
+              sftg_raster_item* __restrict__ items, uint32_t* __restrict__ range)
 {
-    __shared__ uint32_t h[3 * ORDER_BUCKETS], base[3 * ORDER_BUCKETS];
-    for (int i = threadIdx.x; i < 3 * ORDER_BUCKETS; i += blockDim.x) h[i] = 0;
+    __shared__ uint32_t h[2 * ORDER_ALL], base[2 * ORDER_ALL];
+    for (int i = threadIdx.x; i < 2 * ORDER_ALL; i += blockDim.x) h[i] = 0;
     __syncthreads();
-    for (uint32_t t = threadIdx.x; t < n_tiles; t += blockDim.x) atomicAdd(&h[order_bucket(frames, tile_view, tile_count, t)], 1u);
-    __syncthreads();
-    if (threadIdx.x == 0) {
-        uint32_t run = 0;
-        for (int i = 0; i < 3 * ORDER_BUCKETS; i++) { base[i] = run; run += h[i]; }
-    }
-    __syncthreads();
+    const uint32_t all = *total;
     for (uint32_t t = threadIdx.x; t < n_tiles; t += blockDim.x) {
         const uint32_t b = order_bucket(frames, tile_view, tile_count, t);
-        order[atomicAdd(&base[b], 1u)] = t;
+        atomicAdd(&h[b], 1u);
+        atomicAdd(&h[ORDER_ALL + b], order_bands(K, b / ORDER_BUCKETS) * sftg_raster_parts(tile_count[t], all, 1 << (b / ORDER_BUCKETS)));
     }
+    __syncthreads();
+    if (threadIdx.x == 0) order_starts(h, base, range);
+    __syncthreads();
+    for (uint32_t t = threadIdx.x; t < n_tiles; t += blockDim.x)
+        order_place(t, order_bucket(frames, tile_view, tile_count, t), tile_count[t], all, K, base, order, items);
 }
 
 #define ORDER_SMALL 8192u   /* tile counts up to this are ordered by one CTA */
 
 int sftg_launch_tile_order(const sftg_frame* frames, const uint16_t* tile_view, const uint32_t* tile_count, uint32_t n_tiles,
-                           uint32_t* scratch, uint32_t* order, cudaStream_t st) {
+                           const uint32_t* total, const int* bands, uint32_t* scratch, uint32_t* order, sftg_raster_item* items,
+                           uint32_t* range, cudaStream_t st) {
     if (!n_tiles) return 0;
+    const band_knobs K = { { bands[0], bands[1], bands[2] } };
     if (n_tiles <= ORDER_SMALL) {
-        k_order_small<<<1, 1024, 0, st>>>(frames, tile_view, tile_count, n_tiles, order);
+        k_order_small<<<1, 1024, 0, st>>>(frames, tile_view, tile_count, n_tiles, total, K, order, items, range);
         return 1;
     }
-    cudaMemsetAsync(scratch, 0, 2 * 3 * ORDER_BUCKETS * sizeof(uint32_t), st);
+    cudaMemsetAsync(scratch, 0, 2 * ORDER_ALL * sizeof(uint32_t), st);
     const uint32_t g = (n_tiles + 255) / 256;
-    k_order_count<<<g, 256, 0, st>>>(frames, tile_view, tile_count, n_tiles, scratch);
-    k_order_scatter<<<g, 256, 0, st>>>(frames, tile_view, tile_count, n_tiles, scratch, scratch + 3 * ORDER_BUCKETS, order);
-    return 2;
+    k_order_count<<<g, 256, 0, st>>>(frames, tile_view, tile_count, n_tiles, total, K, scratch);
+    k_order_starts<<<1, 256, 0, st>>>(scratch, range);
+    k_order_scatter<<<g, 256, 0, st>>>(frames, tile_view, tile_count, n_tiles, total, K, scratch, order, items);
+    return 3;
+}
+
+uint32_t sftg_raster_items_max(int S, uint32_t tiles, int bands) {
+    const uint32_t least = S == 4 ? 2u : 1u, b = (uint32_t)bands > least ? (uint32_t)bands : least;
+    return b * (tiles + 2u * SFTG_RASTER_CTAS);   /* parts: one per tile, and one per share of the payloads */
 }
 
 /* ---------------------------------------------------------------- debug overlays
@@ -1381,20 +1435,19 @@ static uint32_t queue_grid(K kernel, int threads, size_t smem, uint32_t n_items)
     return (uint32_t)(g < n_items ? g : n_items);
 }
 
-void sftg_launch_raster(int S, uint32_t tile0, uint32_t tiles, int slab_rows, int bands, uint32_t* queue, cudaStream_t st,
-                        const sftg_tile_args& A) {
+void sftg_launch_raster(int S, uint32_t tiles, int slab_rows, int bands, uint32_t* queue, cudaStream_t st, const sftg_tile_args& A) {
     if (!tiles) return;
     const size_t sm = raster_smem(S, slab_rows);
-    const uint32_t items = tiles * RASTER_BANDS;
+    const uint32_t items = sftg_raster_items_max(S, tiles, bands);
     if (queue) {
-        if (S == 1) k_raster_queue<1><<<queue_grid(k_raster_queue<1>, RASTER_THREADS, sm, items), RASTER_THREADS, sm, st>>>(A, tile0, slab_rows, bands, items, queue);
-        else if (S == 2) k_raster_queue<2><<<queue_grid(k_raster_queue<2>, RASTER_THREADS, sm, items), RASTER_THREADS, sm, st>>>(A, tile0, slab_rows, bands, items, queue);
-        else k_raster_queue<4><<<queue_grid(k_raster_queue<4>, RASTER_THREADS, sm, items), RASTER_THREADS, sm, st>>>(A, tile0, slab_rows, bands, items, queue);
+        if (S == 1) k_raster_queue<1><<<queue_grid(k_raster_queue<1>, RASTER_THREADS, sm, items), RASTER_THREADS, sm, st>>>(A, slab_rows, queue);
+        else if (S == 2) k_raster_queue<2><<<queue_grid(k_raster_queue<2>, RASTER_THREADS, sm, items), RASTER_THREADS, sm, st>>>(A, slab_rows, queue);
+        else k_raster_queue<4><<<queue_grid(k_raster_queue<4>, RASTER_THREADS, sm, items), RASTER_THREADS, sm, st>>>(A, slab_rows, queue);
         return;
     }
-    if (S == 1) k_raster<1><<<items, RASTER_THREADS, sm, st>>>(A, tile0, slab_rows, bands);
-    else if (S == 2) k_raster<2><<<items, RASTER_THREADS, sm, st>>>(A, tile0, slab_rows, bands);
-    else k_raster<4><<<items, RASTER_THREADS, sm, st>>>(A, tile0, slab_rows, bands);
+    if (S == 1) k_raster<1><<<items, RASTER_THREADS, sm, st>>>(A, slab_rows);
+    else if (S == 2) k_raster<2><<<items, RASTER_THREADS, sm, st>>>(A, slab_rows);
+    else k_raster<4><<<items, RASTER_THREADS, sm, st>>>(A, slab_rows);
 }
 
 void sftg_launch_tile_lights(uint32_t tile0, uint32_t tiles, cudaStream_t st, const sftg_tile_args& A) {

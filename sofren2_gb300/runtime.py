@@ -275,7 +275,7 @@ class Renderer:
             k += n
         return out
 
-    def set_tuning(self, resolve_split=(16, 16, 16), raster_slab_rows=(8, 8, 4), geom_job_width=1, occl_ray_prune=0,
+    def set_tuning(self, resolve_split=(16, 16, 16), raster_slab_rows=(8, 8, 8), geom_job_width=1, occl_ray_prune=0,
                    raster_bands=(0, 0, 0), tile_lights=(0, 0, 0), tile_queue=0) -> None:
         vals = dict(resolve_split=resolve_split, raster_slab_rows=raster_slab_rows, geom_job_width=geom_job_width,
                     occl_ray_prune=occl_ray_prune, raster_bands=raster_bands, tile_lights=tile_lights, tile_queue=tile_queue)

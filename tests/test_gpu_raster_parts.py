@@ -1,0 +1,58 @@
+"""The raster's parts of a tile's payload list, merged in the visibility buffer, against the oracle:
+depth, vis ids and colour of frames whose few tiles hold far more payloads than one part, at every
+sample count, with row bands and with the persistent queue; and the tile order of a batch of more
+tiles than one CTA orders."""
+import numpy as np
+import pytest
+
+import golden_cases as gc
+from compare import compare_frames
+from oracle_lib import Oracle
+from sofren2_gb300 import runtime, scenes
+
+pytestmark = pytest.mark.gpu
+
+
+@pytest.mark.parametrize("samples", [1, 2, 4])
+@pytest.mark.parametrize("w,h,nx", [(64, 64, 8), (130, 70, 8), (100, 129, 3)])
+def test_parts_equal_oracle(renderer, w, h, nx, samples):
+    sc = scenes.atrium_scene(w, h, seed=51, nx=nx, nz=4, levels=2, arch_segments=8, n_tex=3, tex_size=32, lm_size=256, n_lights=3, n_chars=1,
+                             char_tex=32, floor_quads=(30, 15))
+    blob = sc.to_bytes()
+    o = Oracle(blob)
+    try:
+        ref = o.render_dump(0, samples)
+    finally:
+        o.close()
+    assert int(ref["tile_counts"].max()) > 2 * 64, "a tile's list has to be cut"
+    handle = renderer.load_scene(blob)
+    saved = renderer.tuning()
+    try:
+        renderer.set_samples(samples)
+        tss, npx = runtime.scene_counts(sc)
+        for knobs in ({}, {"tile_queue": 1}, {"raster_bands": (2, 4, 4), "raster_slab_rows": (4, 64, 16)}):
+            renderer.set_tuning(**dict(saved, **knobs))
+            for _ in range(2):      # a frame after another finds the last one's visibility buffer
+                out = renderer.render_debug(handle, 0, tss, npx)
+            res = compare_frames(ref, out, samples, len(sc.frames[0].point_lights))
+            assert not {k: v for k, v in res.items() if k not in ("color_max_lsb", "tlas") and v != 0}, (knobs, res)
+    finally:
+        renderer.set_tuning(**saved)
+        renderer.free_scene(handle)
+
+
+def test_order_of_many_tiles(renderer):
+    h = renderer.load_scene(gc.blob("small"))
+    try:
+        w, hh = renderer.frame_size(h, 0)
+        tiles = ((w + 63) // 64) * ((hh + 63) // 64)
+        n = 8192 // tiles + 2
+        alone = {}
+        for S in (1, 2, 4):
+            renderer.set_samples(S)
+            alone[S] = renderer.render(h, 0)
+        views = [(h, 0, (1, 2, 4)[k % 3]) for k in range(n)]
+        for k, c in enumerate(renderer.render_batch(views, [None] * n)):
+            assert np.array_equal(c, alone[views[k][2]]), f"view {k}"
+    finally:
+        renderer.free_scene(h)
