@@ -46,7 +46,8 @@ struct sftg_lane {
     cudaStream_t stream = nullptr;
     cudaStream_t stream2 = nullptr;            /* proxy occlusion runs here, beside geometry, binning and raster */
     cudaStream_t stream3 = nullptr;            /* the 1x and 2x tile ranges of raster and resolve, beside the 4x range */
-    cudaEvent_t ev_fork = nullptr, ev_join = nullptr, ev_geo = nullptr, ev_done = nullptr;
+    cudaStream_t stream_ev = nullptr;          /* capture only: the graph's event-record nodes */
+    cudaEvent_t ev_fork = nullptr, ev_join = nullptr, ev_geo = nullptr, ev_done = nullptr, ev_tap = nullptr;
     cudaEvent_t ev_split[2] = { nullptr, nullptr }, ev_merge[2] = { nullptr, nullptr };
     cudaEvent_t ev[6] = { nullptr, nullptr, nullptr, nullptr, nullptr, nullptr };
     void* arena = nullptr;
@@ -187,7 +188,8 @@ extern "C" int sftg_create(int device, sftg_ctx** out) {
         sftg_lane& ln = ctx->lanes[l];
         if (cudaStreamCreateWithPriority(&ln.stream, cudaStreamNonBlocking, prio_high) != cudaSuccess ||
             cudaStreamCreateWithPriority(&ln.stream2, cudaStreamNonBlocking, prio_low) != cudaSuccess ||
-            cudaStreamCreateWithPriority(&ln.stream3, cudaStreamNonBlocking, prio_high) != cudaSuccess) { sftg_destroy(ctx); return SFTG_E_CUDA; }
+            cudaStreamCreateWithPriority(&ln.stream3, cudaStreamNonBlocking, prio_high) != cudaSuccess ||
+            cudaStreamCreateWithFlags(&ln.stream_ev, cudaStreamNonBlocking) != cudaSuccess) { sftg_destroy(ctx); return SFTG_E_CUDA; }
         for (int k = 0; k < 2; k++) {
             cudaEventCreateWithFlags(&ln.ev_split[k], cudaEventDisableTiming);
             cudaEventCreateWithFlags(&ln.ev_merge[k], cudaEventDisableTiming);
@@ -196,6 +198,7 @@ extern "C" int sftg_create(int device, sftg_ctx** out) {
         cudaEventCreateWithFlags(&ln.ev_fork, cudaEventDisableTiming);
         cudaEventCreateWithFlags(&ln.ev_join, cudaEventDisableTiming);
         cudaEventCreateWithFlags(&ln.ev_done, cudaEventDisableTiming);
+        cudaEventCreateWithFlags(&ln.ev_tap, cudaEventDisableTiming);
         cudaEventCreate(&ln.ev_geo);
         if (cudaMallocHost((void**)&ln.h_status, 64) != cudaSuccess) { sftg_destroy(ctx); return SFTG_E_CUDA; }
     }
@@ -243,6 +246,8 @@ extern "C" void sftg_destroy(sftg_ctx* ctx) {
         if (ln.ev_geo) cudaEventDestroy(ln.ev_geo);
         if (ln.stream2) cudaStreamDestroy(ln.stream2);
         if (ln.stream3) cudaStreamDestroy(ln.stream3);
+        if (ln.stream_ev) cudaStreamDestroy(ln.stream_ev);
+        if (ln.ev_tap) cudaEventDestroy(ln.ev_tap);
         for (int k = 0; k < 2; k++) {
             if (ln.ev_split[k]) cudaEventDestroy(ln.ev_split[k]);
             if (ln.ev_merge[k]) cudaEventDestroy(ln.ev_merge[k]);
@@ -513,10 +518,11 @@ struct batch_bufs {
     uint32_t* stile_count; uint32_t* stile_start; uint32_t* stile_list;   /* super-tile meshlet lists */
     float* ss;
     sftg_batch_rec* recs;
-    uint32_t* clip_cnt; uint32_t* clip_base;
+    uint32_t* clip_cnt; uint32_t* clip_tot; uint32_t* clip_base;   /* per batch; per meshlet */
     int4* mrect;
     sftg_clip_tri* clips; int4* clip_rect;
     uint32_t* tile_count; uint32_t* tile_start;
+    uint32_t nseg; uint32_t* seg_count; uint32_t* seg_start;   /* binning segments per tile (tile_count, tile_start when 1) */
     uint32_t* tile_order; uint32_t* order_scratch;
     sftg_raster_item* raster_items; uint32_t* raster_range; uint32_t* raster_done;
     uint8_t* tile_nlights;   /* per tile: its light list length (debug views) */
@@ -531,6 +537,7 @@ struct batch_bufs {
     uint32_t* totals;    /* [0] clip total, [1] tile payload total, [2] super-tile list total */
     float* vis_depth; uint32_t* vis_id; float* shadow;
     float2* vis; float2* zrange;
+    void* stage_dev; const void* stage_host; size_t stage_bytes;   /* the frame block's upload */
     uint32_t n_views, total_ss, n_jobs, total_tiles, total_prox, total_packets, max_inst, total_stiles;
     uint32_t s_tile0[3], s_tiles[3];   /* batch-wide tile range of the views with 1, 2 and 4 samples */
     uint64_t color_total;              /* pixels over all views */
@@ -671,13 +678,22 @@ static int build_batch(sftg_ctx* ctx, sftg_lane& ln, const sftg_frame_desc* fds,
     for (uint32_t v = 0; v < nv; v++) {
         view_plan& P = B.plan[v];
         const uint32_t cols = (uint32_t)((fds[v].width + 63) / 64), rows = (uint32_t)((fds[v].height + 63) / 64);
-        /* coarse lists pay off once a tile would scan more than four chunks of meshlet slots */
-        const bool coarse = P.total_ss > 4u * 256u;
+        /* coarse lists cost three launches and pay off where many tiles would each scan many meshlet
+         * slots (48 views, 16000 tiles: binning 1.1 ms); fewer tiles cut their scans into segments */
+        const bool coarse = P.total_ss > 4u * 256u && total_tiles >= 1024u;
         P.scols = coarse ? (cols + SFTG_STILE - 1) / SFTG_STILE : 0u;
         P.stiles = P.scols * ((rows + SFTG_STILE - 1) / SFTG_STILE);
         P.stile_base = total_stiles; total_stiles += P.stiles;
     }
     B.total_stiles = total_stiles;
+    /* segments per tile of the binning: up to SFTG_BIN_CTAS in all, of at least 64 meshlets */
+    B.nseg = 1;
+    if (total_tiles && total_tiles < SFTG_BIN_CTAS) {
+        uint32_t most = 1;
+        for (uint32_t v = 0; v < nv; v++) most = std::max(most, B.plan[v].total_ss / 64u);
+        B.nseg = std::min(SFTG_BIN_CTAS / total_tiles, most);
+    }
+    const size_t n_seg = (size_t)total_tiles * B.nseg;
     B.total_ss = total_ss; B.n_jobs = (uint32_t)jobs.size(); B.total_tiles = total_tiles; B.total_prox = total_prox;
     B.total_packets = total_packets; B.max_inst = max_inst; B.max_pairs = (uint32_t)max_pairs; B.color_total = color_total;
     const size_t n_rec = (size_t)total_ss * 16;
@@ -696,20 +712,21 @@ static int build_batch(sftg_ctx* ctx, sftg_lane& ln, const sftg_frame_desc* fds,
     const size_t o_pv = stage_take((size_t)total_packets * 2 + 16);
     const size_t o_xv = stage_take((size_t)total_prox * 2 + 16);
     const size_t o_sv = stage_take((size_t)total_stiles * 2 + 16);
+    const size_t o_zero = stage_take(256);   /* status, totals, pair and item counters: zero when the batch starts */
     const size_t stage_bytes = so;
     size_t raster_items = 1;
     for (int si = 0; si < 3; si++) if (B.s_tiles[si]) raster_items += sftg_raster_items_max(1 << si, B.s_tiles[si], ctx->tuning.raster_bands[si]);
     /* device arena layout */
     size_t need = stage_bytes + 4096;
     auto acc = [&](size_t bytes) { need = ((need + 255) & ~(size_t)255) + bytes; };
-    acc((size_t)total_ss * SFTG_SS_FLOATS * 4); acc(n_rec * sizeof(sftg_batch_rec)); acc(n_rec * 4); acc(n_rec * 4);
+    acc((size_t)total_ss * SFTG_SS_FLOATS * 4); acc(n_rec * sizeof(sftg_batch_rec)); acc(n_rec * 4); acc((size_t)total_ss * 4); acc((size_t)total_ss * 4);
     acc((size_t)total_ss * 16 + 16); acc(ctx->clip_cap * sizeof(sftg_clip_tri)); acc(ctx->clip_cap * 16);
-    acc((size_t)total_tiles * 4); acc((size_t)total_tiles * 4); acc((size_t)total_tiles * 4); acc(2048); acc(total_tiles + 16);
+    acc((size_t)total_tiles * 4); acc((size_t)total_tiles * 4); acc(n_seg * 4); acc(n_seg * 4); acc((size_t)total_tiles * 4); acc(2048); acc(total_tiles + 16);
     acc(raster_items * sizeof(sftg_raster_item)); acc(64); acc((size_t)total_tiles * sftg_raster_bands() * 4);
     acc(ctx->tile_cap * 8);
     acc((size_t)total_stiles * 4); acc((size_t)total_stiles * 4); acc(ctx->stile_cap * 4);
     acc((size_t)total_prox * 64 + 64); acc((size_t)total_packets * sftg_packet_bytes() + 64);
-    acc((max_pairs * (1 + SFTG_OCC_ITEMS_PER_PAIR) + 1) * 8); acc(64); acc(((n_rec + total_tiles + total_stiles) / SFTG_SCAN_ELEMS_PER_BLOCK + 16) * 4); acc(64); acc(64);
+    acc((max_pairs * (1 + SFTG_OCC_ITEMS_PER_PAIR) + 1) * 8); acc(((total_ss + total_tiles + total_stiles) / SFTG_SCAN_ELEMS_PER_BLOCK + 16) * 4);
     acc(vis_total * 8); acc((size_t)(total_tiles + 1) * sftg_raster_bands() * sizeof(float2));
     acc((size_t)total_tiles * sizeof(sftg_tile_lights)); acc(64);
     const int W0 = fds[0].width, H0 = fds[0].height, S0 = fds[0].samples;
@@ -746,12 +763,15 @@ static int build_batch(sftg_ctx* ctx, sftg_lane& ln, const sftg_frame_desc* fds,
     B.ss = bp.take<float>((size_t)total_ss * SFTG_SS_FLOATS);
     B.recs = bp.take<sftg_batch_rec>(n_rec);
     B.clip_cnt = bp.take<uint32_t>(n_rec);
-    B.clip_base = bp.take<uint32_t>(n_rec);
+    B.clip_tot = bp.take<uint32_t>(total_ss);
+    B.clip_base = bp.take<uint32_t>(total_ss);
     B.mrect = bp.take<int4>((size_t)total_ss + 1);
     B.clips = bp.take<sftg_clip_tri>(ctx->clip_cap);
     B.clip_rect = bp.take<int4>(ctx->clip_cap);
     B.tile_count = bp.take<uint32_t>(total_tiles);
     B.tile_start = bp.take<uint32_t>(total_tiles);
+    B.seg_count = B.nseg > 1 ? bp.take<uint32_t>(n_seg) : B.tile_count;
+    B.seg_start = B.nseg > 1 ? bp.take<uint32_t>(n_seg) : B.tile_start;
     B.tile_order = bp.take<uint32_t>(total_tiles);
     B.order_scratch = bp.take<uint32_t>(512);
     B.raster_items = bp.take<sftg_raster_item>(raster_items);
@@ -767,10 +787,10 @@ static int build_batch(sftg_ctx* ctx, sftg_lane& ln, const sftg_frame_desc* fds,
     B.light_vis = bp.take<uint8_t>((size_t)total_prox * 64 + 64);
     B.packets = bp.take<char>((size_t)total_packets * sftg_packet_bytes() + 64);
     B.pairs = bp.take<uint2>((size_t)max_pairs * (1 + SFTG_OCC_ITEMS_PER_PAIR) + 1);   /* pairs, then BLAS sub-walk items */
-    B.n_pairs = bp.take<uint32_t>(16);
-    B.scan_tmp = bp.take<uint32_t>((n_rec + total_tiles + total_stiles) / SFTG_SCAN_ELEMS_PER_BLOCK + 16);
-    B.status = bp.take<uint32_t>(16);
-    B.totals = bp.take<uint32_t>(16);
+    B.scan_tmp = bp.take<uint32_t>((total_ss + total_tiles + total_stiles) / SFTG_SCAN_ELEMS_PER_BLOCK + 16);
+    B.status = (uint32_t*)(ds + o_zero);
+    B.totals = B.status + 2;
+    B.n_pairs = B.status + 16;
     B.vis = bp.take<float2>(vis_total);
     B.zrange = bp.take<float2>((size_t)(total_tiles + 1) * sftg_raster_bands());   /* per raster band of each tile */
     B.tile_lights = bp.take<sftg_tile_lights>(total_tiles);
@@ -844,6 +864,7 @@ static int build_batch(sftg_ctx* ctx, sftg_lane& ln, const sftg_frame_desc* fds,
     }
     memcpy(hs + o_inst, inst.data(), inst.size() * sizeof(sftg_inst));
     if (!bones.empty()) memcpy(hs + o_bones, bones.data(), bones.size() * 4);
+    memset(hs + o_zero, 0, 256);
     if (!jobs.empty()) memcpy(hs + o_jobs, jobs.data(), jobs.size() * sizeof(sftg_job));
     B.frames = (sftg_frame*)(ds + o_F);
     B.jobs = (const sftg_job*)(ds + o_jobs);
@@ -851,80 +872,84 @@ static int build_batch(sftg_ctx* ctx, sftg_lane& ln, const sftg_frame_desc* fds,
     B.packet_view = (const uint16_t*)(ds + o_pv);
     B.prox_view = (const uint16_t*)(ds + o_xv);
     B.stile_view = (const uint16_t*)(ds + o_sv);
-    CK(cudaMemcpyAsync(ds, hs, stage_bytes, cudaMemcpyHostToDevice, ln.stream));
+    B.stage_dev = ds; B.stage_host = hs; B.stage_bytes = stage_bytes;
     return 0;
 }
 
-/* Phase events: inside a stream capture they must become event-record nodes of the graph
- * (cudaEventRecordExternal) so that replays still time the phases. */
-static cudaError_t record_event(cudaEvent_t ev, cudaStream_t st) {
-    cudaStreamCaptureStatus cs = cudaStreamCaptureStatusNone;
-    const cudaError_t e = cudaStreamIsCapturing(st, &cs);
-    if (e != cudaSuccess) return e;
-    return cs == cudaStreamCaptureStatusActive ? cudaEventRecordWithFlags(ev, st, cudaEventRecordExternal) : cudaEventRecord(ev, st);
+/* Phase events.  Inside a stream capture they become event-record nodes of the graph
+ * (cudaEventRecordExternal), so that replays still time the phases, on a side branch: each hangs off
+ * the work before it and nothing waits for it but the graph's end (as nodes between the kernels they
+ * cost 14 us of a 126 us thumbnail frame). */
+static cudaError_t record_event(sftg_lane& ln, cudaEvent_t ev, cudaStream_t st, bool capturing) {
+    if (!capturing) return cudaEventRecord(ev, st);
+    cudaError_t e = cudaEventRecord(ln.ev_tap, st);
+    if (e == cudaSuccess) e = cudaStreamWaitEvent(ln.stream_ev, ln.ev_tap, 0);
+    return e == cudaSuccess ? cudaEventRecordWithFlags(ev, ln.stream_ev, cudaEventRecordExternal) : e;
 }
 
 static int launch_batch(sftg_ctx* ctx, sftg_lane& ln, const batch_bufs& B) {
-    const uint32_t n_rec = B.total_ss * 16;
     cudaStream_t st = ln.stream;
     ln.launches = 0;
+    cudaStreamCaptureStatus cs = cudaStreamCaptureStatusNone;
+    CK(cudaStreamIsCapturing(st, &cs));
+    const bool cap = cs == cudaStreamCaptureStatusActive;
     CK(cudaGetLastError());   /* nothing pending from earlier calls: every launch below is checked */
-    CK(cudaMemsetAsync(B.status, 0, 64, st));
-    CK(record_event(ln.ev[0], st));
+    CK(cudaMemcpyAsync(B.stage_dev, B.stage_host, B.stage_bytes, cudaMemcpyHostToDevice, st));
+    CK(record_event(ln, ln.ev[0], st, cap));
     /* proxy occlusion only feeds the resolve: it runs on the second stream, forked here and
      * joined before the resolve, overlapping geometry, binning and raster */
     const bool occl = B.total_prox || B.total_packets;
+    cudaStream_t so = ln.stream2;
     if (occl) {
-        cudaStream_t so = ln.stream2;
         CK(cudaEventRecord(ln.ev_fork, st));
         CK(cudaStreamWaitEvent(so, ln.ev_fork, 0));
-        if (B.total_prox) CK(cudaMemsetAsync(B.light_vis, 0, (size_t)B.total_prox * 64, so));   /* columns past the lights stay 0 */
-        if (B.total_packets) {
-            sftg_launch_occlusion(B.frames, B.packet_view, B.total_packets, B.prox_view, B.total_prox, B.max_inst, B.packets,
-                                  B.pairs, B.n_pairs, B.max_pairs, SFTG_OCC_ITEMS_PER_PAIR, B.light_vis, B.status,
-                                  ctx->tuning.occl_ray_prune, so);
-            ln.launches += 4;
-            CK(cudaGetLastError());
-        }
-        CK(record_event(ln.ev[1], so));
+        sftg_launch_occlusion(B.frames, B.packet_view, B.total_packets, B.prox_view, B.total_prox, B.max_inst, B.packets,
+                              B.pairs, B.n_pairs, B.max_pairs, SFTG_OCC_ITEMS_PER_PAIR, B.light_vis, B.status,
+                              ctx->tuning.occl_ray_prune, so);
+        ln.launches += B.total_packets ? 4 : 1;
+        CK(cudaGetLastError());
         CK(cudaEventRecord(ln.ev_join, so));
+        if (cap) CK(cudaEventRecordWithFlags(ln.ev[1], so, cudaEventRecordExternal));   /* after the join's tap */
+        else CK(cudaEventRecord(ln.ev[1], so));
     } else {
-        CK(record_event(ln.ev[1], st));
+        CK(record_event(ln, ln.ev[1], st, cap));
     }
-    CK(record_event(ln.ev_geo, st));
+    CK(record_event(ln, ln.ev_geo, st, cap));
     if (B.n_jobs) {
-        k_geometry<<<(B.n_jobs + 3) / 4, 128, 0, st>>>(B.frames, B.jobs, B.n_jobs, B.ss, B.recs, B.clip_cnt, B.mrect);
+        k_geometry<<<(B.n_jobs + 3) / 4, 128, 0, st>>>(B.frames, B.jobs, B.n_jobs, B.ss, B.recs, B.clip_cnt, B.clip_tot, B.mrect);
         ln.launches++;
         CK(cudaGetLastError());
     }
-    if (n_rec) {
-        scan_u32(B.clip_cnt, B.clip_base, n_rec, B.scan_tmp, B.totals + 0, st, &ln.launches);
-        k_clip<<<(n_rec + 255) / 256, 256, 0, st>>>(B.frames, B.n_views, B.ss, B.clip_cnt, B.clip_base, B.clips, B.clip_rect, B.mrect, n_rec);
+    if (B.total_ss) {
+        scan_u32(B.clip_tot, B.clip_base, B.total_ss, B.scan_tmp, B.totals + 0, st, &ln.launches);
+        k_clip<<<(B.total_ss + CLIP_MESHLETS - 1) / CLIP_MESHLETS, 128, 0, st>>>(B.frames, B.n_views, B.ss, B.clip_cnt, B.clip_tot, B.clip_base,
+                                                                                 B.clips, B.clip_rect, B.mrect, B.total_ss);
         ln.launches++;
         CK(cudaGetLastError());
-    } else {
-        CK(cudaMemsetAsync(B.totals, 0, 8, st));
     }
-    CK(record_event(ln.ev[2], st));
+    CK(record_event(ln, ln.ev[2], st, cap));
     if (B.total_stiles) {
         k_coarse<<<B.total_stiles, 1024, 0, st>>>(B.frames, B.stile_view, B.mrect, B.stile_count, nullptr, nullptr);
         scan_u32(B.stile_count, B.stile_start, B.total_stiles, B.scan_tmp, B.totals + 2, st, &ln.launches);
         k_coarse<<<B.total_stiles, 1024, 0, st>>>(B.frames, B.stile_view, B.mrect, B.stile_count, B.stile_start, B.stile_list);
         ln.launches += 2;
-    } else {
-        CK(cudaMemsetAsync(B.totals + 2, 0, 4, st));
     }
-    k_bin<<<B.total_tiles, 256, 0, st>>>(B.frames, B.tile_view, B.recs, B.clip_cnt, B.clip_base, B.clip_rect, B.mrect,
-                                         B.stile_count, B.stile_start, B.stile_list, B.tile_count, nullptr, nullptr,
-                                         nullptr, nullptr, nullptr);
-    scan_u32(B.tile_count, B.tile_start, B.total_tiles, B.scan_tmp, B.totals + 1, st, &ln.launches);
-    k_bin<<<B.total_tiles, 256, 0, st>>>(B.frames, B.tile_view, B.recs, B.clip_cnt, B.clip_base, B.clip_rect, B.mrect,
-                                         B.stile_count, B.stile_start, B.stile_list, B.tile_count, B.tile_start, B.tile_pay,
-                                         B.totals + 1, B.vis, B.raster_done);
-    ln.launches += 2 + sftg_launch_tile_order(B.frames, B.tile_view, B.tile_count, B.total_tiles, B.totals + 1, ctx->tuning.raster_bands,
-                                              B.order_scratch, B.tile_order, B.raster_items, B.raster_range, st);
+    const uint32_t bin_ctas = B.total_tiles * B.nseg;
+    k_bin<<<bin_ctas, 256, 0, st>>>(B.frames, B.tile_view, B.nseg, B.recs, B.clip_cnt, B.clip_tot, B.clip_base, B.clip_rect, B.mrect,
+                                    B.stile_count, B.stile_start, B.stile_list, B.seg_count, nullptr, nullptr, nullptr, nullptr, nullptr, nullptr);
+    const bool ordered = sftg_launch_tile_starts(B.frames, B.tile_view, B.seg_count, B.nseg, B.total_tiles, B.seg_start, B.tile_count, B.tile_start,
+                                                 B.totals + 1, ctx->tuning.raster_bands, B.tile_order, B.raster_items, B.raster_range, st,
+                                                 &ln.launches);
+    if (!ordered) scan_u32(B.tile_count, B.tile_start, B.total_tiles, B.scan_tmp, B.totals + 1, st, &ln.launches);
+    k_bin<<<bin_ctas, 256, 0, st>>>(B.frames, B.tile_view, B.nseg, B.recs, B.clip_cnt, B.clip_tot, B.clip_base, B.clip_rect, B.mrect,
+                                    B.stile_count, B.stile_start, B.stile_list, B.seg_count, B.seg_start, B.tile_count, B.tile_pay,
+                                    B.totals + 1, B.vis, B.raster_done);
+    ln.launches += 2;
+    if (!ordered)
+        sftg_launch_tile_order(B.frames, B.tile_view, B.tile_count, B.total_tiles, B.totals + 1, ctx->tuning.raster_bands, B.order_scratch,
+                               B.tile_order, B.raster_items, B.raster_range, st, &ln.launches);
     CK(cudaGetLastError());
-    CK(record_event(ln.ev[3], st));
+    CK(record_event(ln, ln.ev[3], st, cap));
     if (B.shadow) CK(cudaMemsetAsync(B.shadow, 0, B.color_total * 16 * 4, st));
     sftg_tile_args A;
     A.frames = B.frames; A.tile_view = B.tile_view; A.ss = B.ss; A.clips = B.clips; A.clip_base = B.clip_base;
@@ -956,7 +981,7 @@ static int launch_batch(sftg_ctx* ctx, sftg_lane& ln, const batch_bufs& B) {
     });
     if (prc) return prc;
     CK(cudaGetLastError());
-    CK(record_event(ln.ev[4], st));
+    CK(record_event(ln, ln.ev[4], st, cap));
     if (occl) CK(cudaStreamWaitEvent(st, ln.ev_join, 0));
     /* per sample count: the tiles' light lists and proxy selections made once per tile (one more
      * launch on the critical path) or by every resolve CTA of the tile (split-fold work) */
@@ -975,7 +1000,15 @@ static int launch_batch(sftg_ctx* ctx, sftg_lane& ln, const batch_bufs& B) {
     if (prc) return prc;
     if (B.any_overlay) { sftg_launch_debug_overlay(B.total_tiles, st, A); ln.launches++; }
     CK(cudaGetLastError());
-    CK(record_event(ln.ev[5], st));
+    CK(record_event(ln, ln.ev[5], st, cap));
+    if (cap) {   /* the side branches end with the graph */
+        CK(cudaEventRecord(ln.ev_tap, ln.stream_ev));
+        CK(cudaStreamWaitEvent(st, ln.ev_tap, 0));
+        if (occl) {
+            CK(cudaEventRecord(ln.ev_tap, so));
+            CK(cudaStreamWaitEvent(st, ln.ev_tap, 0));
+        }
+    }
     return 0;
 }
 
@@ -991,14 +1024,15 @@ static uint64_t batch_key(const sftg_ctx* ctx, const batch_bufs& B) {
     const uint32_t ov = B.any_overlay ? 1u : 0u;
     h = fnv(h, &ov, sizeof(ov));
     const void* ptrs[] = { B.frames, B.jobs, B.tile_view, B.packet_view, B.prox_view, B.stile_view, B.stile_count, B.stile_start,
-                           B.stile_list, B.ss, B.recs, B.clip_cnt, B.clip_base, B.tile_nlights, B.tile_lights, B.queue,
+                           B.stile_list, B.ss, B.recs, B.clip_cnt, B.clip_tot, B.clip_base, B.seg_count, B.seg_start, B.stage_dev,
+                           B.stage_host, (const void*)B.stage_bytes, B.tile_nlights, B.tile_lights, B.queue,
                            B.mrect, B.clips, B.clip_rect, B.tile_count, B.tile_start, B.tile_order, B.order_scratch, B.raster_items,
                            B.raster_range, B.raster_done, B.tile_pay,
                            B.light_vis, B.packets, B.pairs, B.n_pairs, B.scan_tmp, B.status, B.totals, B.vis, B.zrange,
                            B.vis_depth, B.vis_id, B.shadow };
     h = fnv(h, ptrs, sizeof(ptrs));
     const uint32_t cnt[] = { B.max_pairs, B.n_views, B.total_ss, B.n_jobs, B.total_tiles, B.total_prox, B.total_packets, B.max_inst,
-                             B.total_stiles,
+                             B.total_stiles, B.nseg,
                              B.s_tile0[0], B.s_tile0[1], B.s_tile0[2], B.s_tiles[0], B.s_tiles[1], B.s_tiles[2] };
     h = fnv(h, cnt, sizeof(cnt));
     h = fnv(h, &B.color_total, sizeof(B.color_total));
@@ -1056,8 +1090,7 @@ static int submit_batch(sftg_ctx* ctx, sftg_lane& ln, const sftg_frame_desc* fds
                                  (size_t)fds[v].width * 4, fds[v].height, cudaMemcpyHostToDevice, ln.stream));
         }
     if ((rc = (dbg || !ctx->use_graphs) ? launch_batch(ctx, ln, B) : launch_batch_graph(ctx, ln, B))) return rc;
-    CK(cudaMemcpyAsync(ln.h_status, B.status, 4, cudaMemcpyDeviceToHost, ln.stream));
-    CK(cudaMemcpyAsync(ln.h_status + 2, B.totals, 12, cudaMemcpyDeviceToHost, ln.stream));
+    CK(cudaMemcpyAsync(ln.h_status, B.status, 20, cudaMemcpyDeviceToHost, ln.stream));   /* and the totals after it */
     if (!defer_colors)
         for (uint32_t v = 0; v < nv; v++)
             if (host_color && host_color[v] && !B.plan[v].direct)
@@ -1652,6 +1685,7 @@ extern "C" int sftg_light_vis_noalloc(sftg_ctx* ctx, const sftg_frame_desc* fd, 
     CK(cudaMemcpyAsync(d + o_px, fd->proxies, (size_t)np * 32, cudaMemcpyHostToDevice, st));
     if (fd->tlas_count) CK(cudaMemcpyAsync(d + o_tl, fd->tlas_nodes, (size_t)fd->tlas_count * 256, cudaMemcpyHostToDevice, st));
     CK(cudaMemsetAsync(d + o_st, 0, 16, st));
+    CK(cudaMemsetAsync(d + o_np, 0, 16, st));
     CK(cudaMemsetAsync(d + o_lv, 0, (size_t)np * 64, st));
     if (n_packets) {
         CK(cudaMemsetAsync(d + o_pv, 0, (size_t)n_packets * 2, st));

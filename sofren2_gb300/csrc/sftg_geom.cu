@@ -9,15 +9,15 @@
  *               time (sft__geom_setup_and_bin_batch, 4775-4884): one 8-lane group per batch,
  *               shuffles build the batch's tile rectangle and lane mask.
  *   k_clip      near-plane clipping of straddling triangles (4691-4772, 4264-4381); clip
- *               slots come from an exclusive scan of per-batch clip counts, which numbers
+ *               slots come from an exclusive scan of the meshlets' clip counts, which numbers
  *               them in the reference's single-worker emission order.
  *   k_coarse    one CTA per super-tile (4 x 4 tiles) lists, in slot order, the meshlets of its
  *               view whose tile rectangle overlaps it; run once to count and once to write.
- *   k_bin       one CTA per tile builds that tile's payload list in the reference's order
+ *   k_bin       one or more CTAs per tile build that tile's payload list in the reference's order
  *               (meshlet, batch, clipped triangles before the batch payload) with ordered
- *               warp-aggregated compaction over its super-tile's meshlet list (every meshlet
- *               that touches the tile is on it, in slot order); run once to count and once
- *               to write.
+ *               warp-aggregated compaction over the view's meshlets, or its super-tile's
+ *               meshlet list (every meshlet that touches the tile is on it, in slot order);
+ *               run once to count and once to write.
  *   k_scan_*    a three-phase exclusive scan used for clip slots and tile list offsets.
  */
 #include "sftg_types.h"
@@ -30,8 +30,9 @@
 /* ----------------------------------------------------------------------------------------- */
 __global__ void __launch_bounds__(GEOM_WARPS * 32)
 k_geometry(const sftg_frame* __restrict__ frames, const sftg_job* __restrict__ jobs, uint32_t n_jobs, float* __restrict__ ss,
-           sftg_batch_rec* __restrict__ recs, uint32_t* __restrict__ clip_cnt, int4* __restrict__ mrect)
+           sftg_batch_rec* __restrict__ recs, uint32_t* __restrict__ clip_cnt, uint32_t* __restrict__ clip_tot, int4* __restrict__ mrect)
 {
+    __shared__ uint4 s_ind[GEOM_WARPS][32];    /* the meshlet's 512 index bytes */
     __shared__ float s_bones[GEOM_WARPS][GEOM_BONES * 16];
     __shared__ float s_v[GEOM_WARPS][6][64];   /* tx ty tz w sx sy */
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
@@ -92,17 +93,14 @@ k_geometry(const sftg_frame* __restrict__ frames, const sftg_job* __restrict__ j
         const uint32_t g = I->meshlet_base + m;      /* pool index */
         const uint32_t ssi = F->ss_base + I->ss_offset + m;
         if (!((alive >> ln) & 1u)) {
-            if (lane < 16) {
-                sftg_batch_rec r; r.payload = 0; r.x0 = 1; r.x1 = 0; r.y0 = 1; r.y1 = 0;
-                recs[(size_t)ssi * 16 + lane] = r;
-                clip_cnt[(size_t)ssi * 16 + lane] = 0;
-            }
-            if (lane == 0) mrect[ssi] = make_int4(1, 0, 1, 0);
+            /* its records are read only where its rectangle or its clip count says so */
+            if (lane == 0) { mrect[ssi] = make_int4(1, 0, 1, 0); clip_tot[ssi] = 0; }
             continue;
         }
         const float* at = F->ml_attr + (size_t)g * 640;
         float* S = ss + (size_t)ssi * SFTG_SS_FLOATS;
         const sftg_meshlet_info info = F->ml_info[g];
+        s_ind[warp][lane] = ((const uint4*)(F->ml_inds + (size_t)g * 512))[lane];
         /* ---- vertices: lane and lane + 32 (5015-5124) ---- */
 #pragma unroll
         for (int h = 0; h < 2; h++) {
@@ -147,10 +145,10 @@ k_geometry(const sftg_frame* __restrict__ frames, const sftg_job* __restrict__ j
         }
         __syncwarp();
         /* ---- triangle batches: 4 per round, one 8-lane group each (4775-4884) ---- */
-        const uint8_t* ind = F->ml_inds + (size_t)g * 512;
+        const uint8_t* ind = (const uint8_t*)s_ind[warp];
         const int grp = lane >> 3, tl = lane & 7;
-        const uint32_t gmask = 0xFFu << (grp * 8);
         int4 mr = make_int4(9999, -9999, 9999, -9999);
+        uint32_t clips = 0;
         for (int round = 0; round < 4; round++) {
             const int b = round * 4 + grp;
             const uint32_t i0 = ind[b * 32 + tl], i1 = ind[b * 32 + 8 + tl], i2 = ind[b * 32 + 16 + tl];
@@ -178,7 +176,7 @@ k_geometry(const sftg_frame* __restrict__ frames, const sftg_job* __restrict__ j
                 y1 = max(y1, __shfl_xor_sync(0xFFFFFFFFu, y1, o));
                 nclip += __shfl_xor_sync(0xFFFFFFFFu, nclip, o);
             }
-            (void)gmask;
+            clips += nclip;
             if (tl == 0) {
                 sftg_batch_rec r;
                 if (vm) {
@@ -198,8 +196,9 @@ k_geometry(const sftg_frame* __restrict__ frames, const sftg_job* __restrict__ j
             mr.y = max(mr.y, __shfl_xor_sync(0xFFFFFFFFu, mr.y, o));
             mr.z = min(mr.z, __shfl_xor_sync(0xFFFFFFFFu, mr.z, o));
             mr.w = max(mr.w, __shfl_xor_sync(0xFFFFFFFFu, mr.w, o));
+            clips += __shfl_xor_sync(0xFFFFFFFFu, clips, o);
         }
-        if (lane == 0) mrect[ssi] = mr;
+        if (lane == 0) { mrect[ssi] = mr; clip_tot[ssi] = clips; }
         __syncwarp();
     }
 }
@@ -215,29 +214,87 @@ SFTG_D cvert lerp_cv(const cvert& a, const cvert& b, float t) {
     return r;
 }
 
-/* Batch records with clip outputs (clipping is rare).  Each warp scans 32 records; the records
- * that clip are taken four at a time, one per 8-lane group, lane tl of the group clipping
- * triangle tl of the batch.  A triangle's clip slots follow those of the batch's earlier
- * triangles (exclusive scan over the group), the reference's order. */
-__global__ void k_clip(const sftg_frame* __restrict__ frames, uint32_t n_views, const float* __restrict__ ss,
-                       const uint32_t* __restrict__ clip_cnt, const uint32_t* __restrict__ clip_base,
-                       sftg_clip_tri* __restrict__ clips, int4* __restrict__ clip_rect, int4* __restrict__ mrect,
-                       uint32_t n_records)
+/* the first vertex of a clipped triangle and its edges' cuts, from the vertex's place in the meshlet */
+SFTG_D cvert clip_vertex(const float* S, const float* at, uint32_t v, const float* VP) {
+    cvert c;
+    const float4 sa = ((const float4*)(S + SFTG_SS_A))[v], sb = ((const float4*)(S + SFTG_SS_B))[v];
+    const float wx = sa.w, wy = sb.x, wz = sb.y;
+    c.w = fma_(wx, VP[3], fma_(wy, VP[7], fma_(wz, VP[11], VP[15])));
+    c.tx = fma_(wx, VP[0], fma_(wy, VP[4], fma_(wz, VP[8], VP[12])));
+    c.ty = fma_(wx, VP[1], fma_(wy, VP[5], fma_(wz, VP[9], VP[13])));
+    c.tz = fma_(wx, VP[2], fma_(wy, VP[6], fma_(wz, VP[10], VP[14])));
+    c.u = at[384 + v]; c.v = at[448 + v]; c.lu = at[512 + v]; c.lv = at[576 + v];
+    c.px = wx; c.py = wy; c.pz = wz;
+    c.nx = sb.z; c.ny = sb.w; c.nz = S[SFTG_SS_C + 4 * v];
+    return c;
+}
+
+/* one output triangle into its slot, with its tile rectangle; widens mr where it is on screen */
+SFTG_D bool clip_store(const sftg_frame* F, uint32_t slot, const cvert& a, const cvert& b, const cvert& c, uint32_t ii, uint32_t m,
+                       sftg_clip_tri* clips, int4* clip_rect, int4& mr) {
+    if (slot >= F->clip_cap) return false;   /* over capacity: the host grows the pool and re-renders */
+    const float hw = F->hw, hh = F->hh;
+    sftg_clip_tri ct;
+    auto put = [&](int q, const cvert& cv) {
+        const float iw = fdiv(1.f, cv.w);
+        ct.sx[q] = (cv.tx * iw + 1.f) * hw + F->vpx;
+        ct.sy[q] = (-cv.ty * iw + 1.f) * hh + F->vpy;
+        ct.iw[q] = iw;
+        ct.u[q] = cv.u; ct.v[q] = cv.v; ct.lu[q] = cv.lu; ct.lv[q] = cv.lv;
+        ct.px[q] = cv.px; ct.py[q] = cv.py; ct.pz[q] = cv.pz;
+        ct.nx[q] = cv.nx; ct.ny[q] = cv.ny; ct.nz[q] = cv.nz;
+    };
+    put(0, a); put(1, b); put(2, c);
+    ct.inst = ii; ct.m = m;
+    clips[slot] = ct;
+    const float area = (ct.sx[1] - ct.sx[0]) * (ct.sy[2] - ct.sy[0]) - (ct.sy[1] - ct.sy[0]) * (ct.sx[2] - ct.sx[0]);
+    int4 rc = make_int4(1, 0, 1, 0);
+    bool grew = false;
+    if (area > 0.1f) {
+        const int x0 = cvtt(floorf(vmin(ct.sx[0], vmin(ct.sx[1], ct.sx[2])))) >> 6;
+        const int x1 = cvtt(ceilf(vmax(ct.sx[0], vmax(ct.sx[1], ct.sx[2])))) >> 6;
+        const int y0 = cvtt(floorf(vmin(ct.sy[0], vmin(ct.sy[1], ct.sy[2])))) >> 6;
+        const int y1 = cvtt(ceilf(vmax(ct.sy[0], vmax(ct.sy[1], ct.sy[2])))) >> 6;
+        if (!(x1 < 0 || x0 > F->cols - 1 || y1 < 0 || y0 > F->rows - 1)) {
+            rc = make_int4(x0, x1, y0, y1);
+            mr.x = min(mr.x, x0); mr.y = max(mr.y, x1); mr.z = min(mr.z, y0); mr.w = max(mr.w, y1);
+            grew = true;
+        }
+    }
+    clip_rect[slot] = rc;
+    return grew;
+}
+
+/* Near-plane clipping (4691-4772, 4264-4349), CLIP_MESHLETS meshlets per CTA of 16 8-lane groups, one
+ * batch of the meshlet per group and one triangle per lane; meshlets that clip nothing cost a look at
+ * their count.  Slots follow the meshlet's base (an exclusive scan of the meshlets' counts), then
+ * the batches before this one, then the batch's earlier triangles: the reference's order.  Bound by
+ * latency: 32 records per warp, four batches at a time, with the vertices in an array indexed by
+ * which of them are in front (local memory) took 24 us on the skinned 1080p frame. */
+#define CLIP_THREADS 128
+__global__ void __launch_bounds__(CLIP_THREADS)
+k_clip(const sftg_frame* __restrict__ frames, uint32_t n_views, const float* __restrict__ ss,
+       const uint32_t* __restrict__ clip_cnt, const uint32_t* __restrict__ clip_tot, const uint32_t* __restrict__ clip_base,
+       sftg_clip_tri* __restrict__ clips, int4* __restrict__ clip_rect, int4* __restrict__ mrect, uint32_t n_meshlets)
 {
-    const int lane = threadIdx.x & 31, gl = lane & 7, gshift = lane & ~7;
+    const int tid = threadIdx.x, lane = tid & 31, tl = lane & 7, gshift = lane & ~7, b = tid >> 3;
     const uint32_t gmask = 0xFFu << gshift;
-    const uint32_t r_lane = blockIdx.x * blockDim.x + threadIdx.x;
-    uint32_t pending = __ballot_sync(0xFFFFFFFFu, r_lane < n_records && clip_cnt[r_lane] != 0);
-    const uint32_t r_base = r_lane - (uint32_t)lane;
-    while (pending) {
-        /* group g takes the g-th pending record */
-        uint32_t pick = pending;
-        for (int g = 0; g < (lane >> 3) && pick; g++) pick &= pick - 1;
-        const bool have = pick != 0;
-        const uint32_t r = r_base + (have ? (uint32_t)(__ffs(pick) - 1) : 0u);
-        for (int g = 0; g < 4 && pending; g++) pending &= pending - 1;
-        if (!have) continue;   /* whole group: the same pick on its 8 lanes */
-        const uint32_t ssi = r / 16, b = r % 16;
+    const uint32_t m0 = blockIdx.x * CLIP_MESHLETS;
+    const uint32_t mine = m0 + (uint32_t)lane;
+    uint32_t pending = __ballot_sync(0xFFFFFFFFu, lane < CLIP_MESHLETS && mine < n_meshlets && clip_tot[mine] != 0);
+    for (; pending; pending &= pending - 1) {
+        const uint32_t ssi = m0 + (uint32_t)(__ffs(pending) - 1);
+        /* the batch's outputs and those of the batches before it */
+        const uint32_t cnt = clip_cnt[(size_t)ssi * 16 + (lane & 15)];
+        uint32_t before = cnt;
+#pragma unroll
+        for (int o = 1; o < 16; o <<= 1) {
+            const uint32_t t = __shfl_up_sync(0xFFFFFFFFu, before, o, 16);
+            if ((lane & 15) >= o) before += t;
+        }
+        before -= cnt;
+        const uint32_t have = __shfl_sync(0xFFFFFFFFu, cnt, b), first = __shfl_sync(0xFFFFFFFFu, before, b);
+        if (!have) continue;   /* whole group */
         /* the view, then the instance, owning this screen-space slot (both laid out in order) */
         uint32_t v = 0;
         for (uint32_t k = 0; k < n_views; k++) if (frames[k].ss_base <= ssi && frames[k].total_ss) v = k;
@@ -251,44 +308,28 @@ __global__ void k_clip(const sftg_frame* __restrict__ frames, uint32_t n_views, 
         const float* S = ss + (size_t)ssi * SFTG_SS_FLOATS;
         const uint8_t* ind = F->ml_inds + (size_t)g * 512;
         const float* VP = F->vp;
-        const float hw = F->hw, hh = F->hh;
-        const int tl = gl;
-        const uint32_t q[3] = { ind[b * 32 + tl], ind[b * 32 + 8 + tl], ind[b * 32 + 16 + tl] };
-        cvert in[3];
-        cvert out[2][3];
+        const uint32_t q0 = ind[b * 32 + tl], q1 = ind[b * 32 + 8 + tl], q2 = ind[b * 32 + 16 + tl];
         int nc = 0;
-        if ((int)(q[0] | q[1] | q[2]) > 0) {
-            for (int k = 0; k < 3; k++) {
-                const uint32_t vv = q[k];
-                const float4 sa = ((const float4*)(S + SFTG_SS_A))[vv], sb = ((const float4*)(S + SFTG_SS_B))[vv];
-                const float wx = sa.w, wy = sb.x, wz = sb.y;
-                in[k].w = fma_(wx, VP[3], fma_(wy, VP[7], fma_(wz, VP[11], VP[15])));
-                in[k].tx = fma_(wx, VP[0], fma_(wy, VP[4], fma_(wz, VP[8], VP[12])));
-                in[k].ty = fma_(wx, VP[1], fma_(wy, VP[5], fma_(wz, VP[9], VP[13])));
-                in[k].tz = fma_(wx, VP[2], fma_(wy, VP[6], fma_(wz, VP[10], VP[14])));
-                in[k].u = at[384 + vv]; in[k].v = at[448 + vv]; in[k].lu = at[512 + vv]; in[k].lv = at[576 + vv];
-                in[k].px = wx; in[k].py = wy; in[k].pz = wz;
-                in[k].nx = sb.z; in[k].ny = sb.w; in[k].nz = S[SFTG_SS_C + 4 * vv];
-            }
-            const bool a = in[0].tz >= 0.f, bb = in[1].tz >= 0.f, c = in[2].tz >= 0.f;
-            const bool ai = a && bb && c, ao = (in[0].tz < 0.f) && (in[1].tz < 0.f) && (in[2].tz < 0.f);
+        cvert v0, v1, v2;      /* one in front: that vertex, the next, the one before; two: the one behind, the one before, the next */
+        if ((int)(q0 | q1 | q2) > 0) {
+            auto depth = [&](uint32_t q) {
+                const float4 sa = ((const float4*)(S + SFTG_SS_A))[q], sb = ((const float4*)(S + SFTG_SS_B))[q];
+                return fma_(sa.w, VP[2], fma_(sb.x, VP[6], fma_(sb.y, VP[10], VP[14])));
+            };
+            const float d0 = depth(q0), d1 = depth(q1), d2 = depth(q2);
+            const bool f0 = d0 >= 0.f, f1 = d1 >= 0.f, f2 = d2 >= 0.f;
+            const bool ai = f0 && f1 && f2, ao = (d0 < 0.f) && (d1 < 0.f) && (d2 < 0.f);
             if (!(ai || ao)) {
                 /* sft__clip_triangle_near_plane (4264-4349) */
-                const int mask = (int)a | ((int)bb << 1) | ((int)c << 2);
-                float d[3] = { in[0].tz, in[1].tz, in[2].tz };
-                if (mask == 1 || mask == 2 || mask == 4) {
-                    const int ia = mask >> 1, ib = (ia == 2) ? 0 : ia + 1, ic = (ia == 0) ? 2 : ia - 1;
-                    const float tab = fdiv(d[ia], d[ia] - d[ib]), tac = fdiv(d[ia], d[ia] - d[ic]);
-                    out[0][0] = in[ia]; out[0][1] = lerp_cv(in[ia], in[ib], tab); out[0][2] = lerp_cv(in[ia], in[ic], tac);
-                    nc = 1;
-                } else {
-                    const int io = (~mask & 7) >> 1, ia = (io == 0) ? 2 : io - 1, ic = (io == 2) ? 0 : io + 1;
-                    const float tab = fdiv(d[ia], d[ia] - d[io]), tcb = fdiv(d[ic], d[ic] - d[io]);
-                    const cvert nab = lerp_cv(in[ia], in[io], tab), ncb = lerp_cv(in[ic], in[io], tcb);
-                    out[0][0] = in[ia]; out[0][1] = nab; out[0][2] = in[ic];
-                    out[1][0] = nab; out[1][1] = ncb; out[1][2] = in[ic];
-                    nc = 2;
-                }
+                const int mask = (int)f0 | ((int)f1 << 1) | ((int)f2 << 2);
+                const bool one = mask == 1 || mask == 2 || mask == 4;
+                const int p = one ? mask >> 1 : (~mask & 7) >> 1;                 /* the pivot's place */
+                const uint32_t qp = p == 0 ? q0 : (p == 1 ? q1 : q2);
+                const uint32_t qn = p == 0 ? q1 : (p == 1 ? q2 : q0), qb = p == 0 ? q2 : (p == 1 ? q0 : q1);   /* next, before */
+                v0 = clip_vertex(S, at, qp, VP);
+                v1 = clip_vertex(S, at, one ? qn : qb, VP);
+                v2 = clip_vertex(S, at, one ? qb : qn, VP);
+                nc = one ? 1 : 2;
             }
         }
         /* exclusive scan of the output counts over the group's 8 triangles */
@@ -296,40 +337,20 @@ __global__ void k_clip(const sftg_frame* __restrict__ frames, uint32_t n_views, 
 #pragma unroll
         for (int o = 1; o < 8; o <<= 1) {
             const int t = __shfl_up_sync(gmask, incl, o, 8);
-            if (gl >= o) incl += t;
+            if (tl >= o) incl += t;
         }
-        uint32_t slot = clip_base[r] + (uint32_t)(incl - nc);
+        const uint32_t slot = clip_base[ssi] + first + (uint32_t)(incl - nc);
         int4 mr = make_int4(0x7FFFFFFF, (int)0x80000000, 0x7FFFFFFF, (int)0x80000000);
         bool grew = false;
-        for (int k = 0; k < nc; k++, slot++) {
-            if (slot >= F->clip_cap) continue;   /* over capacity: the host grows the pool and re-renders */
-            sftg_clip_tri ct;
-            for (int qv = 0; qv < 3; qv++) {
-                const cvert& cv = out[k][qv];
-                const float iw = fdiv(1.f, cv.w);
-                ct.sx[qv] = (cv.tx * iw + 1.f) * hw + F->vpx;
-                ct.sy[qv] = (-cv.ty * iw + 1.f) * hh + F->vpy;
-                ct.iw[qv] = iw;
-                ct.u[qv] = cv.u; ct.v[qv] = cv.v; ct.lu[qv] = cv.lu; ct.lv[qv] = cv.lv;
-                ct.px[qv] = cv.px; ct.py[qv] = cv.py; ct.pz[qv] = cv.pz;
-                ct.nx[qv] = cv.nx; ct.ny[qv] = cv.ny; ct.nz[qv] = cv.nz;
-            }
-            ct.inst = ii; ct.m = m;
-            clips[slot] = ct;
-            const float area = (ct.sx[1] - ct.sx[0]) * (ct.sy[2] - ct.sy[0]) - (ct.sy[1] - ct.sy[0]) * (ct.sx[2] - ct.sx[0]);
-            int4 rc = make_int4(1, 0, 1, 0);
-            if (area > 0.1f) {
-                const int x0 = cvtt(floorf(vmin(ct.sx[0], vmin(ct.sx[1], ct.sx[2])))) >> 6;
-                const int x1 = cvtt(ceilf(vmax(ct.sx[0], vmax(ct.sx[1], ct.sx[2])))) >> 6;
-                const int y0 = cvtt(floorf(vmin(ct.sy[0], vmin(ct.sy[1], ct.sy[2])))) >> 6;
-                const int y1 = cvtt(ceilf(vmax(ct.sy[0], vmax(ct.sy[1], ct.sy[2])))) >> 6;
-                if (!(x1 < 0 || x0 > F->cols - 1 || y1 < 0 || y0 > F->rows - 1)) {
-                    rc = make_int4(x0, x1, y0, y1);
-                    mr.x = min(mr.x, x0); mr.y = max(mr.y, x1); mr.z = min(mr.z, y0); mr.w = max(mr.w, y1);
-                    grew = true;
-                }
-            }
-            clip_rect[slot] = rc;
+        if (nc == 1) {
+            const float tab = fdiv(v0.tz, v0.tz - v1.tz), tac = fdiv(v0.tz, v0.tz - v2.tz);
+            grew = clip_store(F, slot, v0, lerp_cv(v0, v1, tab), lerp_cv(v0, v2, tac), ii, m, clips, clip_rect, mr);
+        } else if (nc == 2) {
+            const float tab = fdiv(v1.tz, v1.tz - v0.tz), tcb = fdiv(v2.tz, v2.tz - v0.tz);
+            const cvert nab = lerp_cv(v1, v0, tab), ncb = lerp_cv(v2, v0, tcb);
+            const bool g0 = clip_store(F, slot, v1, nab, v2, ii, m, clips, clip_rect, mr);
+            const bool g1 = clip_store(F, slot + 1, nab, ncb, v2, ii, m, clips, clip_rect, mr);
+            grew = g0 || g1;
         }
         /* several triangles and batches of one meshlet may clip: widen its rectangle atomically
          * (min / max commute, so the result does not depend on the order) */
@@ -345,42 +366,49 @@ __global__ void k_clip(const sftg_frame* __restrict__ frames, uint32_t n_views, 
 
 SFTG_D bool rect_has(int x0, int x1, int y0, int y1, int tx, int ty) { return x0 <= tx && tx <= x1 && y0 <= ty && ty <= y1; }
 
-/* Payloads of one meshlet that land on tile (tx, ty), counted or written in reference order:
- * for each batch, its clipped triangles (slot order) then its batch payload.  Lanes 0..15 =
- * batches; returns the meshlet total (same on all lanes). */
-SFTG_D uint32_t bin_meshlet(const sftg_batch_rec* recs, const uint32_t* clip_cnt, const uint32_t* clip_base,
-                            const int4* clip_rect, uint32_t clip_cap, uint32_t vclip, uint32_t ssi, int tx, int ty, int lane, uint64_t* out)
+/* Payloads of a meshlet per half warp (lane & 15 = batch) that land on tile (tx, ty), counted or written
+ * in reference order: for each batch, its clipped triangles (slot order) then its batch payload.
+ * Returns the meshlet's total on the half's lanes; `on` is false for a half without a meshlet. */
+SFTG_D uint32_t bin_meshlet(const sftg_batch_rec* recs, const uint32_t* clip_cnt, const uint32_t* clip_tot, const uint32_t* clip_base,
+                            const int4* clip_rect, uint32_t clip_cap, uint32_t vclip, bool on, uint32_t ssi, int tx, int ty, int lane,
+                            uint64_t* out)
 {
+    const int b = lane & 15;
     uint32_t cnt = 0, nclip = 0, cb = 0;
-    sftg_batch_rec r; r.payload = 0;
-    if (lane < 16) {
-        r = recs[(size_t)ssi * 16 + lane];
-        nclip = clip_cnt[(size_t)ssi * 16 + lane];
-        if (nclip) {
-            cb = clip_base[(size_t)ssi * 16 + lane];
-            for (uint32_t k = 0; k < nclip && cb + k < clip_cap; k++) {
-                const int4 q = clip_rect[cb + k];
-                cnt += rect_has(q.x, q.y, q.z, q.w, tx, ty);
-            }
+    sftg_batch_rec r; r.payload = 0; r.x0 = 1; r.x1 = 0; r.y0 = 1; r.y1 = 0;
+    uint32_t clipping = 0;
+    if (on) { r = recs[(size_t)ssi * 16 + b]; clipping = clip_tot[ssi]; }
+    if (__any_sync(0xFFFFFFFFu, clipping != 0)) {
+        if (clipping) { nclip = clip_cnt[(size_t)ssi * 16 + b]; cb = clip_base[ssi]; }
+        uint32_t incl = nclip;   /* the meshlet's clip slots, batch after batch */
+#pragma unroll
+        for (int o = 1; o < 16; o <<= 1) {
+            const uint32_t v = __shfl_up_sync(0xFFFFFFFFu, incl, o, 16);
+            if (b >= o) incl += v;
         }
-        cnt += (r.payload != 0) && rect_has(r.x0, r.x1, r.y0, r.y1, tx, ty);
+        cb += incl - nclip;
+        for (uint32_t k = 0; k < nclip && cb + k < clip_cap; k++) {
+            const int4 q = clip_rect[cb + k];
+            cnt += rect_has(q.x, q.y, q.z, q.w, tx, ty);
+        }
     }
+    const bool whole = r.payload != 0 && rect_has(r.x0, r.x1, r.y0, r.y1, tx, ty);
+    cnt += whole;
     uint32_t incl = cnt;
 #pragma unroll
-    for (int o = 1; o < 32; o <<= 1) {
-        const uint32_t v = __shfl_up_sync(0xFFFFFFFFu, incl, o);
-        if (lane >= o) incl += v;
+    for (int o = 1; o < 16; o <<= 1) {
+        const uint32_t v = __shfl_up_sync(0xFFFFFFFFu, incl, o, 16);
+        if (b >= o) incl += v;
     }
-    const uint32_t total = __shfl_sync(0xFFFFFFFFu, incl, 31);
-    if (out && lane < 16 && cnt) {
+    if (out && cnt) {
         uint64_t* o = out + (incl - cnt);
         for (uint32_t k = 0; k < nclip && cb + k < clip_cap; k++) {
             const int4 q = clip_rect[cb + k];
             if (rect_has(q.x, q.y, q.z, q.w, tx, ty)) *o++ = (uint64_t)(cb + k - vclip);
         }
-        if (r.payload != 0 && rect_has(r.x0, r.x1, r.y0, r.y1, tx, ty)) *o = r.payload;
+        if (whole) *o = r.payload;
     }
-    return total;
+    return __shfl_sync(0xFFFFFFFFu, incl, lane | 15);
 }
 
 #define COARSE_THREADS 1024   /* a super-tile scans its view's meshlet slots 1024 at a time */
@@ -422,36 +450,46 @@ k_coarse(const sftg_frame* __restrict__ frames, const uint16_t* __restrict__ sti
     if (!stile_list && tid == 0) stile_count[gst] = running;
 }
 
+/* One CTA per (tile, segment): the payloads of the segment's share of the tile's candidate meshlets
+ * (all of the view's slots, or its super-tile's list), BIN_CHUNK candidates at a time.  Run once to
+ * count (tile_pay null), once to write.  Bound by latency: with a CTA per tile the few tiles of a small
+ * frame scanned thousands of meshlets one after the other (155x106 over the atrium 0.44 ms for both
+ * passes), and above 1024 slots the super-tile lists, made first, cost three launches, 33 us; now
+ * frames of under 1024 tiles cut the candidates over up to 608 CTAs instead. */
+#define BIN_CHUNK (4 * BIN_THREADS)
 __global__ void __launch_bounds__(BIN_THREADS)
-k_bin(const sftg_frame* __restrict__ frames, const uint16_t* __restrict__ tile_view, const sftg_batch_rec* __restrict__ recs,
-      const uint32_t* __restrict__ clip_cnt, const uint32_t* __restrict__ clip_base, const int4* __restrict__ clip_rect,
-      const int4* __restrict__ mrect, const uint32_t* __restrict__ stile_count, const uint32_t* __restrict__ stile_start,
-      const uint32_t* __restrict__ stile_list, uint32_t* __restrict__ tile_count, const uint32_t* __restrict__ tile_start,
-      uint64_t* __restrict__ tile_pay, const uint32_t* __restrict__ total, float2* __restrict__ vis, uint32_t* __restrict__ raster_done)
+k_bin(const sftg_frame* __restrict__ frames, const uint16_t* __restrict__ tile_view, uint32_t nseg, const sftg_batch_rec* __restrict__ recs,
+      const uint32_t* __restrict__ clip_cnt, const uint32_t* __restrict__ clip_tot, const uint32_t* __restrict__ clip_base,
+      const int4* __restrict__ clip_rect, const int4* __restrict__ mrect, const uint32_t* __restrict__ stile_count,
+      const uint32_t* __restrict__ stile_start, const uint32_t* __restrict__ stile_list, uint32_t* __restrict__ seg_count,
+      const uint32_t* __restrict__ seg_start, const uint32_t* __restrict__ tile_count, uint64_t* __restrict__ tile_pay,
+      const uint32_t* __restrict__ total, float2* __restrict__ vis, uint32_t* __restrict__ raster_done)
 {
-    __shared__ uint32_t s_hits[BIN_THREADS];
-    __shared__ uint32_t s_cnt[BIN_THREADS];
-    __shared__ uint32_t s_wsum[BIN_THREADS / 32];
-    __shared__ uint32_t s_nhits;
-    const int gtile = blockIdx.x;                       /* batch-wide tile index */
+    __shared__ uint32_t s_hits[BIN_CHUNK];
+    __shared__ uint32_t s_cnt[BIN_CHUNK];
+    __shared__ uint32_t s_wsum[4][BIN_THREADS / 32];
+    __shared__ uint32_t s_total;
+    const int gtile = (int)(blockIdx.x / nseg);         /* batch-wide tile index */
+    const uint32_t seg = blockIdx.x - (uint32_t)gtile * nseg;
     const sftg_frame* F = frames + tile_view[gtile];
     const int tile = gtile - (int)F->tile_base;
     const int tx = tile % F->cols, ty = tile / F->cols;
-    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, half = lane >> 4;
     const uint32_t n_ss = F->total_ss;
     /* clipped payloads carry the view's own slot numbers (slots restart at 0 per frame) */
-    const uint32_t vclip = n_ss ? clip_base[(size_t)F->ss_base * 16] : 0u;
+    const uint32_t vclip = n_ss ? clip_base[F->ss_base] : 0u;
     uint64_t* out = nullptr;
     if (tile_pay) {
         if (sftg_raster_parts(tile_count[gtile], *total, F->samples) > 1u) {   /* rastered in parts, merged into a cleared buffer */
             const int n = F->samples * SFTG_TILE_PX / 2;
             float4* v = (float4*)(vis + F->vis_base + (size_t)tile * F->samples * SFTG_TILE_PX);
-            for (int i = tid; i < n; i += BIN_THREADS) v[i] = make_float4(0.f, 0.f, 0.f, 0.f);
-            if (tid < 4) raster_done[gtile * 4 + tid] = 0u;
+            for (int i = (int)seg * BIN_THREADS + tid; i < n; i += (int)nseg * BIN_THREADS) v[i] = make_float4(0.f, 0.f, 0.f, 0.f);
+            if (seg == 0 && tid < 4) raster_done[gtile * 4 + tid] = 0u;
         }
         /* over capacity: the host grows the buffer and re-renders; write nothing */
-        if ((uint64_t)tile_start[gtile] + tile_count[gtile] > F->tile_cap) return;
-        out = tile_pay + tile_start[gtile];
+        if ((uint64_t)seg_start[blockIdx.x] + seg_count[blockIdx.x] > F->tile_cap) return;
+        if (seg_count[blockIdx.x] == 0) return;
+        out = tile_pay + seg_start[blockIdx.x];
     }
     /* the meshlets that can touch this tile: its super-tile's list, in slot order, or every slot
      * of the view when the view has no coarse lists (scols == 0) */
@@ -463,61 +501,86 @@ k_bin(const sftg_frame* __restrict__ frames, const uint16_t* __restrict__ tile_v
         if ((uint64_t)stile_start[gst] + n_cand > F->stile_cap) n_cand = 0;   /* lists overflowed: the host re-renders */
         cand = stile_list + stile_start[gst];
     }
+    const uint32_t share = (n_cand + nseg - 1) / nseg, c0 = min(n_cand, seg * share), c1 = min(n_cand, c0 + share);
     uint32_t running = 0;
-    for (uint32_t base = 0; base < n_cand; base += BIN_THREADS) {
-        uint32_t s = 0;
-        bool hit = false;
-        if (base + tid < n_cand) {
-            s = cand ? cand[base + tid] : F->ss_base + base + tid;
-            const int4 q = mrect[s];
-            hit = rect_has(q.x, q.y, q.z, q.w, tx, ty);
+    for (uint32_t base = c0; base < c1; base += BIN_CHUNK) {
+        /* four candidates per thread, their loads in flight together; candidate order is (j, tid) */
+        uint32_t s[4], bal[4];
+        bool hit[4], any = false;
+#pragma unroll
+        for (int j = 0; j < 4; j++) {
+            const uint32_t i = base + (uint32_t)(j * BIN_THREADS + tid);
+            hit[j] = false; s[j] = 0;
+            if (i < c1) {
+                s[j] = cand ? cand[i] : F->ss_base + i;
+                const int4 q = mrect[s[j]];
+                hit[j] = rect_has(q.x, q.y, q.z, q.w, tx, ty);
+            }
+            any = any || hit[j];
         }
-        if (!__syncthreads_or(hit)) continue;   /* no meshlet of this chunk touches the tile */
+        if (!__syncthreads_or(any)) continue;   /* no meshlet of this chunk touches the tile */
         /* ordered compaction of hit meshlets */
-        const uint32_t bal = __ballot_sync(0xFFFFFFFFu, hit);
-        if (lane == 0) s_wsum[warp] = __popc(bal);
-        __syncthreads();
-        uint32_t off = 0, tot = 0;
-        for (int w = 0; w < BIN_THREADS / 32; w++) { if (w < warp) off += s_wsum[w]; tot += s_wsum[w]; }
-        if (hit) s_hits[off + __popc(bal & ((1u << lane) - 1u))] = s;
-        if (tid == 0) s_nhits = tot;
-        __syncthreads();
-        const uint32_t nh = s_nhits;
-        /* per-hit payload counts */
-        for (uint32_t h = warp; h < nh; h += BIN_THREADS / 32) {
-            const uint32_t c = bin_meshlet(recs, clip_cnt, clip_base, clip_rect, F->clip_cap, vclip, s_hits[h], tx, ty, lane, nullptr);
-            if (lane == 0) s_cnt[h] = c;
+#pragma unroll
+        for (int j = 0; j < 4; j++) {
+            bal[j] = __ballot_sync(0xFFFFFFFFu, hit[j]);
+            if (lane == 0) s_wsum[j][warp] = __popc(bal[j]);
         }
         __syncthreads();
-        if (warp == 0) {   /* exclusive scan of the hit counts (nh <= 256, 8 per lane); total in s_wsum[0] */
-            uint32_t v[BIN_THREADS / 32], local = 0;
+        uint32_t nh = 0;
 #pragma unroll
-            for (int k = 0; k < BIN_THREADS / 32; k++) {
-                const uint32_t h = (uint32_t)lane * (BIN_THREADS / 32) + k;
-                v[k] = h < nh ? s_cnt[h] : 0u;
-                local += v[k];
+        for (int j = 0; j < 4; j++) {
+            uint32_t off = nh;
+            for (int w = 0; w < BIN_THREADS / 32; w++) { if (w < warp) off += s_wsum[j][w]; nh += s_wsum[j][w]; }
+            if (hit[j]) s_hits[off + __popc(bal[j] & ((1u << lane) - 1u))] = s[j];
+        }
+        __syncthreads();
+        /* per-hit payload counts, two meshlets per warp at a time */
+        for (uint32_t h0 = warp * 2; h0 < nh; h0 += BIN_THREADS / 16) {
+            const uint32_t h = h0 + half;
+            const uint32_t c = bin_meshlet(recs, clip_cnt, clip_tot, clip_base, clip_rect, F->clip_cap, vclip, h < nh, h < nh ? s_hits[h] : 0u,
+                                           tx, ty, lane, nullptr);
+            if ((lane & 15) == 0 && h < nh) s_cnt[h] = c;
+        }
+        __syncthreads();
+        if (out) {
+            if (warp == 0) {   /* exclusive scan of the hit counts, 32 per lane; total in s_total */
+                const uint32_t per = (nh + 31) / 32;
+                uint32_t local = 0;
+                for (uint32_t k = 0; k < per; k++) { const uint32_t h = (uint32_t)lane * per + k; local += h < nh ? s_cnt[h] : 0u; }
+                uint32_t incl = local;
+#pragma unroll
+                for (int o = 1; o < 32; o <<= 1) { const uint32_t t = __shfl_up_sync(0xFFFFFFFFu, incl, o); if (lane >= o) incl += t; }
+                uint32_t acc = incl - local;
+                for (uint32_t k = 0; k < per; k++) {
+                    const uint32_t h = (uint32_t)lane * per + k;
+                    if (h < nh) { const uint32_t c = s_cnt[h]; s_cnt[h] = acc; acc += c; }
+                }
+                if (lane == 31) s_total = incl;
             }
-            uint32_t incl = local;
-#pragma unroll
-            for (int o = 1; o < 32; o <<= 1) { const uint32_t t = __shfl_up_sync(0xFFFFFFFFu, incl, o); if (lane >= o) incl += t; }
-            uint32_t acc = incl - local;
-#pragma unroll
-            for (int k = 0; k < BIN_THREADS / 32; k++) {
-                const uint32_t h = (uint32_t)lane * (BIN_THREADS / 32) + k;
-                if (h < nh) s_cnt[h] = acc;
-                acc += v[k];
+            __syncthreads();
+            for (uint32_t h0 = warp * 2; h0 < nh; h0 += BIN_THREADS / 16) {   /* ordered writes */
+                const uint32_t h = h0 + half;
+                bin_meshlet(recs, clip_cnt, clip_tot, clip_base, clip_rect, F->clip_cap, vclip, h < nh, h < nh ? s_hits[h] : 0u, tx, ty, lane,
+                            out + running + (h < nh ? s_cnt[h] : 0u));
             }
-            if (lane == 31) s_wsum[0] = incl;
+            running += s_total;
+        } else {
+            uint32_t mine = 0;
+            for (uint32_t h = tid; h < nh; h += BIN_THREADS) mine += s_cnt[h];
+            running += mine;   /* this thread's share, summed at the end */
         }
-        __syncthreads();
-        if (out) {   /* ordered writes */
-            for (uint32_t h = warp; h < nh; h += BIN_THREADS / 32)
-                bin_meshlet(recs, clip_cnt, clip_base, clip_rect, F->clip_cap, vclip, s_hits[h], tx, ty, lane, out + running + s_cnt[h]);
-        }
-        running += s_wsum[0];
         __syncthreads();
     }
-    if (!out && tid == 0) tile_count[gtile] = running;
+    if (!out && !tile_pay) {
+        const uint32_t w = __reduce_add_sync(0xFFFFFFFFu, running);
+        if (lane == 0) s_wsum[0][warp] = w;
+        __syncthreads();
+        if (tid == 0) {
+            uint32_t all = 0;
+            for (int k = 0; k < BIN_THREADS / 32; k++) all += s_wsum[0][k];
+            seg_count[blockIdx.x] = all;
+        }
+    }
 }
 
 /* ----------------------------------------------------------------------------------------- */

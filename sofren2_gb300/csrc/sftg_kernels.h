@@ -56,7 +56,7 @@ struct sftg_tile_args {
     const uint16_t* tile_view;
     const float* ss;
     const sftg_clip_tri* clips;
-    const uint32_t* clip_base;     /* exclusive scan of clip counts: a view's first slot is clip_base[ss_base * 16] */
+    const uint32_t* clip_base;     /* exclusive scan of the meshlets' clip counts: a view's first slot is clip_base[ss_base] */
     const uint32_t* tile_order;    /* launch order of the tiles (heaviest first within each sample count) */
     const sftg_raster_item* raster_items;   /* heaviest tiles first within each sample count */
     const uint32_t* raster_range;  /* per sample count: first item, then per sample count: items */
@@ -76,16 +76,19 @@ struct sftg_tile_args {
 };
 
 __global__ void k_geometry(const sftg_frame* frames, const sftg_job* jobs, uint32_t n_jobs, float* ss, sftg_batch_rec* recs,
-                           uint32_t* clip_cnt, int4* mrect);
-__global__ void k_clip(const sftg_frame* frames, uint32_t n_views, const float* ss, const uint32_t* clip_cnt,
-                       const uint32_t* clip_base, sftg_clip_tri* clips, int4* clip_rect, int4* mrect, uint32_t n_records);
+                           uint32_t* clip_cnt, uint32_t* clip_tot, int4* mrect);
+#define CLIP_MESHLETS 4   /* meshlets per CTA of k_clip */
+__global__ void k_clip(const sftg_frame* frames, uint32_t n_views, const float* ss, const uint32_t* clip_cnt, const uint32_t* clip_tot,
+                       const uint32_t* clip_base, sftg_clip_tri* clips, int4* clip_rect, int4* mrect, uint32_t n_meshlets);
 #define SFTG_STILE 4   /* tiles per side of a super-tile (coarse binning) */
 __global__ void k_coarse(const sftg_frame* frames, const uint16_t* stile_view, const int4* mrect, uint32_t* stile_count,
                          const uint32_t* stile_start, uint32_t* stile_list);
-__global__ void k_bin(const sftg_frame* frames, const uint16_t* tile_view, const sftg_batch_rec* recs, const uint32_t* clip_cnt,
-                      const uint32_t* clip_base, const int4* clip_rect, const int4* mrect, const uint32_t* stile_count,
-                      const uint32_t* stile_start, const uint32_t* stile_list, uint32_t* tile_count,
-                      const uint32_t* tile_start, uint64_t* tile_pay, const uint32_t* total, float2* vis, uint32_t* raster_done);
+__global__ void k_bin(const sftg_frame* frames, const uint16_t* tile_view, uint32_t nseg, const sftg_batch_rec* recs,
+                      const uint32_t* clip_cnt, const uint32_t* clip_tot, const uint32_t* clip_base, const int4* clip_rect,
+                      const int4* mrect, const uint32_t* stile_count, const uint32_t* stile_start, const uint32_t* stile_list,
+                      uint32_t* seg_count, const uint32_t* seg_start, const uint32_t* tile_count, uint64_t* tile_pay,
+                      const uint32_t* total, float2* vis, uint32_t* raster_done);
+#define SFTG_BIN_CTAS 608u   /* segments over all tiles of a batch of fewer tiles */
 __global__ void k_scan_reduce(const uint32_t* in, uint32_t n, uint32_t* sums);
 __global__ void k_scan_top(uint32_t* sums, uint32_t nb, uint32_t* total_out);
 __global__ void k_scan_down(const uint32_t* in, uint32_t n, const uint32_t* sums, uint32_t* out);
@@ -97,19 +100,27 @@ size_t sftg_packet_bytes();
  * whose items do not fit keeps the rest of its subtree on its own stack. */
 #define SFTG_OCC_ITEMS_PER_PAIR 64
 #define SFTG_OCC_ITEMS_PER_PAIR_NOALLOC 64
-/* packet_view maps a batch-wide shadow packet to its view, prox_view a batch-wide proxy */
+/* packet_view maps a batch-wide shadow packet to its view, prox_view a batch-wide proxy; the counters at
+ * n_pairs (two words) are zero */
 void sftg_launch_occlusion(const sftg_frame* frames, const uint16_t* packet_view, uint32_t n_packets, const uint16_t* prox_view,
                            uint32_t n_proxies, uint32_t max_inst, void* packets, uint2* pairs, uint32_t* n_pairs,
                            uint32_t max_pairs, uint32_t items_per_pair, uint8_t* light_vis, uint32_t* status, int ray_prune,
                            cudaStream_t st);
 cudaError_t sftg_tile_configure(int max_dynamic_smem);
 int sftg_raster_bands(void);   /* most row bands of a 64x64 tile */
-/* order[] = the batch's tiles, heaviest first inside each sample-count range, items[] = the raster's work
- * items in the same order, range[] their first and number per sample count (6 words); total: the
- * batch's payload count; bands: the raster_bands knob; scratch holds 512 words.  Returns the launches. */
-int sftg_launch_tile_order(const sftg_frame* frames, const uint16_t* tile_view, const uint32_t* tile_count, uint32_t n_tiles,
-                           const uint32_t* total, const int* bands, uint32_t* scratch, uint32_t* order, sftg_raster_item* items,
-                           uint32_t* range, cudaStream_t st);
+/* From the payload counts of the tiles' nseg segments: seg_start[] (exclusive scan) and the batch's
+ * total; per tile its count and start (the same arrays where nseg is 1); order[] = the batch's tiles,
+ * heaviest first inside each sample-count range, items[] = the raster's work items in the same order,
+ * range[] their first and number per sample count (6 words).  bands: the raster_bands knob; scratch
+ * holds 512 words, scan_tmp one per SFTG_SCAN_ELEMS_PER_BLOCK segments.  sftg_launch_tile_starts before
+ * the binning's write pass, sftg_launch_tile_order after it where the first returned false; both
+ * add their launches to *launches. */
+bool sftg_launch_tile_starts(const sftg_frame* frames, const uint16_t* tile_view, const uint32_t* seg_count, uint32_t nseg, uint32_t n_tiles,
+                             uint32_t* seg_start, uint32_t* tile_count, uint32_t* tile_start, uint32_t* total, const int* bands,
+                             uint32_t* order, sftg_raster_item* items, uint32_t* range, cudaStream_t st, int* launches);
+void sftg_launch_tile_order(const sftg_frame* frames, const uint16_t* tile_view, const uint32_t* tile_count, uint32_t n_tiles,
+                            const uint32_t* total, const int* bands, uint32_t* scratch, uint32_t* order, sftg_raster_item* items,
+                            uint32_t* range, cudaStream_t st, int* launches);
 uint32_t sftg_raster_items_max(int S, uint32_t tiles, int bands);   /* bound on the items of a sample-count range */
 /* resolve CTAs per tile and where its light lists are made, from the tuning knobs and the tile count */
 int sftg_resolve_split(int knob, uint32_t tiles);

@@ -480,8 +480,8 @@ k_occl_blas_walk(const sftg_frame* __restrict__ frames, const uint16_t* __restri
     }
 }
 
-/* Phase C: light_vis[p][l] = 3 - rays blocked (8169-8276); one thread per (batch-wide proxy,
- * light column); columns at or beyond the view's light count keep the zero they were cleared to. */
+/* Phase C: light_vis[p][l] = 3 - rays blocked (8169-8276), 0 past the view's lights and where it
+ * traces no packets; one thread per (batch-wide proxy, light column). */
 __global__ void k_occl_finalize(const sftg_frame* __restrict__ frames, const uint16_t* __restrict__ prox_view, uint32_t n_proxies,
                                 const sftg_packet* __restrict__ packets, uint8_t* __restrict__ light_vis)
 {
@@ -490,12 +490,15 @@ __global__ void k_occl_finalize(const sftg_frame* __restrict__ frames, const uin
     const uint32_t gp = i >> 6, l = i & 63;
     const sftg_frame* F = frames + prox_view[gp];
     const uint32_t pc = F->n_proxies, lc = min(F->n_point, 64u), nbatch = (pc + 7) / 8;
-    if (l >= lc) return;
-    const uint32_t p = gp - F->prox_base, b = p / 8, k = p % 8;
-    const sftg_packet* P = packets + F->packet_base;
-    int blocked = 0;
-    for (int ray = 0; ray < 3; ray++) blocked += (P[(l * nbatch + b) * 3 + ray].hits >> k) & 1u;
-    light_vis[(size_t)gp * 64 + l] = (uint8_t)(3 - blocked);
+    uint8_t seen = 0;
+    if (l < lc && F->n_packets) {
+        const uint32_t p = gp - F->prox_base, b = p / 8, k = p % 8;
+        const sftg_packet* P = packets + F->packet_base;
+        int blocked = 0;
+        for (int ray = 0; ray < 3; ray++) blocked += (P[(l * nbatch + b) * 3 + ray].hits >> k) & 1u;
+        seen = (uint8_t)(3 - blocked);
+    }
+    light_vis[(size_t)gp * 64 + l] = seen;
 }
 
 size_t sftg_packet_bytes() { return sizeof(sftg_packet); }
@@ -504,7 +507,7 @@ void sftg_launch_occlusion(const sftg_frame* frames, const uint16_t* packet_view
                            uint32_t n_proxies, uint32_t max_inst, void* packets, uint2* pairs, uint32_t* n_pairs,
                            uint32_t max_pairs, uint32_t items_per_pair, uint8_t* light_vis, uint32_t* status, int ray_prune,
                            cudaStream_t st) {
-    cudaMemsetAsync(n_pairs, 0, 8, st);   /* pair and item counters */
+    if (n_proxies && !n_packets) k_occl_finalize<<<(n_proxies * 64 + 255) / 256, 256, 0, st>>>(frames, prox_view, n_proxies, (const sftg_packet*)packets, light_vis);
     if (!n_packets) return;
     k_occl_tlas<<<(n_packets + OCC_WARPS - 1) / OCC_WARPS, OCC_WARPS * 32, 0, st>>>(frames, packet_view, n_packets,
                                                                                    (sftg_packet*)packets, pairs, n_pairs, max_pairs, status);

@@ -298,7 +298,7 @@ SFTG_D void raster_item(const sftg_tile_args& A, int slab_rows, const sftg_raste
     const sftg_frame* F = A.frames + A.tile_view[gtile];
     const int tile = (int)(gtile - F->tile_base);
     const float* ss = A.ss + (size_t)F->ss_base * SFTG_SS_FLOATS;
-    const sftg_clip_tri* clips = A.clips + (F->total_ss ? A.clip_base[(size_t)F->ss_base * 16] : 0u);
+    const sftg_clip_tri* clips = A.clips + (F->total_ss ? A.clip_base[F->ss_base] : 0u);
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
     const int tmx = (tile % F->cols) * SFTG_TILE, tmy = (tile / F->cols) * SFTG_TILE;
     uint32_t count = A.tile_count[gtile];
@@ -639,7 +639,7 @@ SFTG_D void resolve_item(const sftg_tile_args& A, uint32_t tile0, int split, boo
     const sftg_frame* F = A.frames + A.tile_view[gtile];
     const int tile = (int)(gtile - F->tile_base);
     const float* ss = A.ss + (size_t)F->ss_base * SFTG_SS_FLOATS;
-    const sftg_clip_tri* clips = A.clips + (F->total_ss ? A.clip_base[(size_t)F->ss_base * 16] : 0u);
+    const sftg_clip_tri* clips = A.clips + (F->total_ss ? A.clip_base[F->ss_base] : 0u);
     const uint8_t* light_vis = A.light_vis + (size_t)F->prox_base * 64;
     uint32_t* color = F->color_dev;
     const int CP = F->pitch;   /* colour row stride in pixels (the caller's buffer when written directly) */
@@ -1277,45 +1277,76 @@ __global__ void k_order_scatter(const sftg_frame* __restrict__ frames, const uin
     if (t < n_tiles) order_place(t, order_bucket(frames, tile_view, tile_count, t), tile_count[t], *total, K, cursor, order, items);
 }
 
-/* the same in one CTA for small tile counts: histogram, bucket starts and scatter in shared memory */
+/* The whole of it in one CTA for small tile counts: the scan of the segments' counts (each thread a
+ * run of them), every tile's count and start, then histogram, bucket starts and scatter.  One launch
+ * between the binning's passes instead of a scan before and an order after the second. */
 __global__ void __launch_bounds__(1024)
-k_order_small(const sftg_frame* __restrict__ frames, const uint16_t* __restrict__ tile_view, const uint32_t* __restrict__ tile_count,
-              uint32_t n_tiles, const uint32_t* __restrict__ total, const band_knobs K, uint32_t* __restrict__ order,
-              sftg_raster_item* __restrict__ items, uint32_t* __restrict__ range)
+k_tile_starts(const sftg_frame* __restrict__ frames, const uint16_t* __restrict__ tile_view, const uint32_t* seg_count, uint32_t nseg,
+              uint32_t n_tiles, uint32_t* seg_start, uint32_t* tile_count, uint32_t* tile_start, uint32_t* __restrict__ total,
+              const band_knobs K, uint32_t* __restrict__ order, sftg_raster_item* __restrict__ items, uint32_t* __restrict__ range)
 {
-    __shared__ uint32_t h[2 * ORDER_ALL], base[2 * ORDER_ALL];
-    for (int i = threadIdx.x; i < 2 * ORDER_ALL; i += blockDim.x) h[i] = 0;
+    __shared__ uint32_t h[2 * ORDER_ALL], base[2 * ORDER_ALL], s_w[32], s_all;
+    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+    for (int i = tid; i < 2 * ORDER_ALL; i += 1024) h[i] = 0;
+    const uint32_t n = n_tiles * nseg, per = (n + 1023u) / 1024u, i0 = (uint32_t)tid * per;
+    uint32_t sum = 0;
+    for (uint32_t k = 0; k < per; k++) if (i0 + k < n) sum += seg_count[i0 + k];
+    uint32_t incl = sum;
+#pragma unroll
+    for (int o = 1; o < 32; o <<= 1) { const uint32_t t = __shfl_up_sync(0xFFFFFFFFu, incl, o); if (lane >= o) incl += t; }
+    if (lane == 31) s_w[warp] = incl;
     __syncthreads();
-    const uint32_t all = *total;
-    for (uint32_t t = threadIdx.x; t < n_tiles; t += blockDim.x) {
+    if (warp == 0) {
+        const uint32_t w = s_w[lane];
+        uint32_t wi = w;
+#pragma unroll
+        for (int o = 1; o < 32; o <<= 1) { const uint32_t t = __shfl_up_sync(0xFFFFFFFFu, wi, o); if (lane >= o) wi += t; }
+        s_w[lane] = wi - w;
+        if (lane == 31) { s_all = wi; *total = wi; }
+    }
+    __syncthreads();
+    uint32_t at = s_w[warp] + incl - sum;
+    for (uint32_t k = 0; k < per; k++) if (i0 + k < n) { seg_start[i0 + k] = at; at += seg_count[i0 + k]; }
+    __syncthreads();
+    const uint32_t all = s_all;
+    for (uint32_t t = tid; t < n_tiles; t += 1024) {
+        if (nseg > 1) {
+            const uint32_t a = seg_start[t * nseg], e = t + 1 < n_tiles ? seg_start[(t + 1) * nseg] : all;
+            tile_start[t] = a; tile_count[t] = e - a;
+        }
         const uint32_t b = order_bucket(frames, tile_view, tile_count, t);
         atomicAdd(&h[b], 1u);
         atomicAdd(&h[ORDER_ALL + b], order_bands(K, b / ORDER_BUCKETS) * sftg_raster_parts(tile_count[t], all, 1 << (b / ORDER_BUCKETS)));
     }
     __syncthreads();
-    if (threadIdx.x == 0) order_starts(h, base, range);
+    if (tid == 0) order_starts(h, base, range);
     __syncthreads();
-    for (uint32_t t = threadIdx.x; t < n_tiles; t += blockDim.x)
+    for (uint32_t t = tid; t < n_tiles; t += 1024)
         order_place(t, order_bucket(frames, tile_view, tile_count, t), tile_count[t], all, K, base, order, items);
 }
 
-#define ORDER_SMALL 8192u   /* tile counts up to this are ordered by one CTA */
+#define ORDER_SMALL 8192u   /* tile counts up to this are handled by one CTA */
 
-int sftg_launch_tile_order(const sftg_frame* frames, const uint16_t* tile_view, const uint32_t* tile_count, uint32_t n_tiles,
-                           const uint32_t* total, const int* bands, uint32_t* scratch, uint32_t* order, sftg_raster_item* items,
-                           uint32_t* range, cudaStream_t st) {
-    if (!n_tiles) return 0;
+bool sftg_launch_tile_starts(const sftg_frame* frames, const uint16_t* tile_view, const uint32_t* seg_count, uint32_t nseg, uint32_t n_tiles,
+                             uint32_t* seg_start, uint32_t* tile_count, uint32_t* tile_start, uint32_t* total, const int* bands,
+                             uint32_t* order, sftg_raster_item* items, uint32_t* range, cudaStream_t st, int* launches) {
+    if (n_tiles > ORDER_SMALL) return false;
     const band_knobs K = { { bands[0], bands[1], bands[2] } };
-    if (n_tiles <= ORDER_SMALL) {
-        k_order_small<<<1, 1024, 0, st>>>(frames, tile_view, tile_count, n_tiles, total, K, order, items, range);
-        return 1;
-    }
+    k_tile_starts<<<1, 1024, 0, st>>>(frames, tile_view, seg_count, nseg, n_tiles, seg_start, tile_count, tile_start, total, K, order, items, range);
+    *launches += 1;
+    return true;
+}
+
+void sftg_launch_tile_order(const sftg_frame* frames, const uint16_t* tile_view, const uint32_t* tile_count, uint32_t n_tiles,
+                            const uint32_t* total, const int* bands, uint32_t* scratch, uint32_t* order, sftg_raster_item* items,
+                            uint32_t* range, cudaStream_t st, int* launches) {
+    const band_knobs K = { { bands[0], bands[1], bands[2] } };
     cudaMemsetAsync(scratch, 0, 2 * ORDER_ALL * sizeof(uint32_t), st);
     const uint32_t g = (n_tiles + 255) / 256;
     k_order_count<<<g, 256, 0, st>>>(frames, tile_view, tile_count, n_tiles, total, K, scratch);
     k_order_starts<<<1, 256, 0, st>>>(scratch, range);
     k_order_scatter<<<g, 256, 0, st>>>(frames, tile_view, tile_count, n_tiles, total, K, scratch, order, items);
-    return 3;
+    *launches += 3;
 }
 
 uint32_t sftg_raster_items_max(int S, uint32_t tiles, int bands) {

@@ -56,3 +56,32 @@ def test_order_of_many_tiles(renderer):
             assert np.array_equal(c, alone[views[k][2]]), f"view {k}"
     finally:
         renderer.free_scene(h)
+
+
+@pytest.mark.parametrize("w,h", [(64, 64), (200, 140), (640, 360)])
+def test_binning_segments_equal_oracle(renderer, w, h):
+    """Tile lists of a view with more meshlet slots than one segment holds, from one tile (the most
+    segments) up, with triangles clipped at the near plane among them."""
+    sc = scenes.atrium_scene(w, h, seed=52, nx=16, nz=9, levels=3, arch_segments=8, n_tex=3, tex_size=32, lm_size=512, n_lights=2, n_chars=2,
+                             char_tex=32, floor_quads=(60, 30),
+                             views=[(w, h, (0.2, 0.4, 5.0), (0.5, 2.0, 12.0), np.float32(0.3))])
+    blob = sc.to_bytes()
+    o = Oracle(blob)
+    try:
+        ref = o.render_dump(0, 1)
+    finally:
+        o.close()
+    tss, npx = runtime.scene_counts(sc)
+    assert tss > 1024 and ref["clip"].size > 0
+    handle = renderer.load_scene(blob)
+    try:
+        renderer.set_samples(1)
+        out = renderer.render_debug(handle, 0, tss, npx)
+        res = compare_frames(ref, out, 1, len(sc.frames[0].point_lights))
+        assert not {k: v for k, v in res.items() if k not in ("color_max_lsb", "tlas") and v != 0}, res
+        if w == 640:     # in a batch of over 1024 tiles: super-tile lists and no segments
+            alone = renderer.render(handle, 0)
+            for c in renderer.render_batch([(handle, 0, 1)] * 18, [None] * 18):
+                assert np.array_equal(c, alone)
+    finally:
+        renderer.free_scene(handle)
