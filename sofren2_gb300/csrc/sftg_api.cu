@@ -272,7 +272,7 @@ extern "C" int sftg_texture_upload(sftg_ctx* ctx, const uint32_t* texels, uint64
     sftg_tex t;
     memset(&t, 0, sizeof(t));
     t.w = d->width; t.h = d->height; t.levels = d->levels; t.is_pot = d->is_pot;
-    for (int i = 0; i < 14; i++) { t.offs[i] = (uint32_t)(off / 4) + d->level_offset[i]; t.bw[i] = d->blocks_w[i]; t.shift[i] = d->stride_shift[i]; }
+    for (int i = 0; i < 14; i++) { t.lev[i].off = (uint32_t)(off / 4) + d->level_offset[i]; t.lev[i].bw = d->is_pot ? 1u << d->stride_shift[i] : (uint32_t)d->blocks_w[i]; }
     ctx->h_texs.push_back(t);
     ctx->tables_dirty = true;
     *out_index = (int32_t)ctx->h_texs.size() - 1;
@@ -952,6 +952,8 @@ static int launch_batch(sftg_ctx* ctx, sftg_lane& ln, const batch_bufs& B) {
     CK(record_event(ln, ln.ev[3], st, cap));
     if (B.shadow) CK(cudaMemsetAsync(B.shadow, 0, B.color_total * 16 * 4, st));
     sftg_tile_args A;
+    A.texs = (const sftg_tex*)ctx->texs.ptr; A.texels = (const uint32_t*)ctx->texels.ptr; A.mats = (const sftg_mat*)ctx->mats.ptr;
+    A.ml_inds = (const uint8_t*)ctx->ml_inds.ptr; A.ml_info = (const sftg_meshlet_info*)ctx->ml_info.ptr;
     A.frames = B.frames; A.tile_view = B.tile_view; A.ss = B.ss; A.clips = B.clips; A.clip_base = B.clip_base;
     A.tile_order = B.tile_order; A.raster_items = B.raster_items; A.raster_range = B.raster_range; A.raster_done = B.raster_done;
     A.tile_nlights = B.tile_nlights; A.tile_lights = B.tile_lights;
@@ -1029,7 +1031,7 @@ static uint64_t batch_key(const sftg_ctx* ctx, const batch_bufs& B) {
                            B.mrect, B.clips, B.clip_rect, B.tile_count, B.tile_start, B.tile_order, B.order_scratch, B.raster_items,
                            B.raster_range, B.raster_done, B.tile_pay,
                            B.light_vis, B.packets, B.pairs, B.n_pairs, B.scan_tmp, B.status, B.totals, B.vis, B.zrange,
-                           B.vis_depth, B.vis_id, B.shadow };
+                           B.vis_depth, B.vis_id, B.shadow, ctx->texs.ptr, ctx->texels.ptr, ctx->mats.ptr, ctx->ml_inds.ptr, ctx->ml_info.ptr };
     h = fnv(h, ptrs, sizeof(ptrs));
     const uint32_t cnt[] = { B.max_pairs, B.n_views, B.total_ss, B.n_jobs, B.total_tiles, B.total_prox, B.total_packets, B.max_inst,
                              B.total_stiles, B.nseg,

@@ -52,6 +52,12 @@ static __host__ __device__ __forceinline__ uint32_t sftg_raster_parts(uint32_t c
 }
 
 struct sftg_tile_args {
+    /* resident tables, the same for every view: kernel parameters save a load of the pointer each time */
+    const sftg_tex* texs;
+    const uint32_t* texels;
+    const sftg_mat* mats;
+    const uint8_t* ml_inds;
+    const sftg_meshlet_info* ml_info;
     const sftg_frame* frames;
     const uint16_t* tile_view;
     const float* ss;

@@ -102,7 +102,7 @@ SFTG_D float2 tile_zrange(const float2* zr, uint32_t gtile) {
 SFTG_D uint64_t zkey(float z, uint32_t order) { return ((uint64_t)__float_as_uint(z) << 32) | (uint64_t)(0xFFFFFFFFu - order); }
 
 /* vertices of one vis id (sofren2.c:5163-5209, 6199-6278) */
-SFTG_D void fetch_tri(const sftg_frame* F, const float* ss, const sftg_clip_tri* clips, uint32_t vid, tri_verts& t) {
+SFTG_D void fetch_tri(const sftg_tile_args& A, const sftg_inst* inst, const float* ss, const sftg_clip_tri* clips, uint32_t vid, tri_verts& t) {
     if (vid & 0x80000000u) {
         const sftg_clip_tri* c = &clips[vid & 0x7FFFFFFFu];
         const float* src = c->sx; float* dst = t.sx;
@@ -112,10 +112,9 @@ SFTG_D void fetch_tri(const sftg_frame* F, const float* ss, const sftg_clip_tri*
         return;
     }
     const uint32_t ii = (vid >> 25) & 63, m = (vid >> 7) & 0x3FFFF, tri = vid & 127;
-    const sftg_inst* I = &F->inst[ii];
+    const sftg_inst* I = &inst[ii];
     const uint32_t g = I->meshlet_base + m;
-    const uint8_t* ind = F->ml_inds + (size_t)g * 512;
-    const float* at = F->ml_attr + (size_t)g * 640;
+    const uint8_t* ind = A.ml_inds + (size_t)g * 512;
     const float* Sc = ss + (size_t)(I->ss_offset + m) * SFTG_SS_FLOATS;
     const uint32_t b = tri >> 3, l = tri & 7;
     const uint32_t q[3] = { ind[b * 32 + l], ind[b * 32 + 8 + l], ind[b * 32 + 16 + l] };
@@ -222,30 +221,38 @@ SFTG_D void tri_raster(const tri_setup& T, int y0, int y1, int lane, uint32_t gm
 }
 
 /* ---------------------------------------------------------------- texture sampling */
-SFTG_D uint32_t tex_addr(const sftg_tex& t, int lod, int u, int v) {
+/* a texture's header and one level, a 16- and an 8-byte load */
+struct tex_level { int w, h; bool pot; const uint32_t* base; uint32_t bw; };
+SFTG_D tex_level tex_at(const sftg_tile_args& A, int4 head, int ti, int lod) {
+    const uint2 lv = __ldg((const uint2*)&A.texs[ti].lev[lod]);
+    tex_level t;
+    t.w = max(head.x >> lod, 1); t.h = max(head.y >> lod, 1); t.pot = head.w != 0;
+    t.base = A.texels + lv.x; t.bw = lv.y;
+    return t;
+}
+
+SFTG_D uint32_t tex_addr(const tex_level& t, int u, int v) {
     const uint32_t uu = (uint32_t)u, vv = (uint32_t)v;
-    if (t.is_pot) return ((((vv >> 2) << t.shift[lod]) + (uu >> 2)) << 4) + ((vv & 3u) << 2) + (uu & 3u);
-    return ((((vv >> 2) * (uint32_t)t.bw[lod]) + (uu >> 2)) << 4) + ((vv & 3u) << 2) + (uu & 3u);
+    return (((vv >> 2) * t.bw + (uu >> 2)) << 4) + ((vv & 3u) << 2) + (uu & 3u);
 }
 
 /* sft__sample_tex_bilinear (5543-5660) */
-SFTG_D void sample_bilinear(const sftg_frame* F, int ti, int lod, float cu, float cv, float& r, float& g, float& b) {
+SFTG_D void sample_bilinear(const sftg_tile_args& A, int4 head, int ti, int lod, float cu, float cv, float& r, float& g, float& b) {
     if (ti < 0) { r = g = b = 1.f; return; }
-    const sftg_tex& t = F->texs[ti];
-    const int w = max(t.w >> lod, 1), h = max(t.h >> lod, 1);
+    const tex_level t = tex_at(A, head, ti, lod);
+    const int w = t.w, h = t.h;
     const float upx = cu * (float)w - 0.5f, vpx = cv * (float)h - 0.5f;
     const float uf0 = floorf(upx), vf0 = floorf(vpx);
     const float ufr = upx - uf0, vfr = vpx - vf0;
     const int u0 = cvtt(uf0), v0 = cvtt(vf0);
     const int wm = w - 1, hm = h - 1;
     int u0w, v0w, u1, v1;
-    if (t.is_pot) { u1 = (u0 + 1) & wm; v1 = (v0 + 1) & hm; u0w = u0 & wm; v0w = v0 & hm; }
+    if (t.pot) { u1 = (u0 + 1) & wm; v1 = (v0 + 1) & hm; u0w = u0 & wm; v0w = v0 & hm; }
     else {   /* the reference has no lower clamp here (it reads outside the texture); clamp at 0 */
         u1 = max(0, min(u0 + 1, wm)); v1 = max(0, min(v0 + 1, hm)); u0w = max(0, min(u0, wm)); v0w = max(0, min(v0, hm));
     }
-    const uint32_t* base = F->texels + t.offs[lod];
-    const uint32_t c00 = __ldg(&base[tex_addr(t, lod, u0w, v0w)]), c10 = __ldg(&base[tex_addr(t, lod, u1, v0w)]);
-    const uint32_t c01 = __ldg(&base[tex_addr(t, lod, u0w, v1)]), c11 = __ldg(&base[tex_addr(t, lod, u1, v1)]);
+    const uint32_t c00 = __ldg(&t.base[tex_addr(t, u0w, v0w)]), c10 = __ldg(&t.base[tex_addr(t, u1, v0w)]);
+    const uint32_t c01 = __ldg(&t.base[tex_addr(t, u0w, v1)]), c11 = __ldg(&t.base[tex_addr(t, u1, v1)]);
     const float i255 = 1.f / 255.f;
     float out[3];
 #pragma unroll
@@ -260,15 +267,15 @@ SFTG_D void sample_bilinear(const sftg_frame* F, int ti, int lod, float cu, floa
 }
 
 /* sft__sample_tex_nearest (5662-5729) */
-SFTG_D void sample_nearest(const sftg_frame* F, int ti, int lod, float cu, float cv, float& r, float& g, float& b) {
+SFTG_D void sample_nearest(const sftg_tile_args& A, int4 head, int ti, int lod, float cu, float cv, float& r, float& g, float& b) {
     if (ti < 0) { r = g = b = 1.f; return; }
-    const sftg_tex& t = F->texs[ti];
-    const int w = max(t.w >> lod, 1), h = max(t.h >> lod, 1);
+    const tex_level t = tex_at(A, head, ti, lod);
+    const int w = t.w, h = t.h;
     const int u0 = cvtt(floorf(cu * (float)w)), v0 = cvtt(floorf(cv * (float)h));
     const int wm = w - 1, hm = h - 1;
     int uw, vw;
-    if (t.is_pot) { uw = u0 & wm; vw = v0 & hm; } else { uw = max(0, min(u0, wm)); vw = max(0, min(v0, hm)); }
-    const uint32_t c = __ldg(&F->texels[t.offs[lod] + tex_addr(t, lod, uw, vw)]);
+    if (t.pot) { uw = u0 & wm; vw = v0 & hm; } else { uw = max(0, min(u0, wm)); vw = max(0, min(v0, hm)); }
+    const uint32_t c = __ldg(&t.base[tex_addr(t, uw, vw)]);
     const float i255 = 1.f / 255.f;
     r = (float)((c >> 16) & 255u) * i255; g = (float)((c >> 8) & 255u) * i255; b = (float)(c & 255u) * i255;
 }
@@ -343,7 +350,7 @@ SFTG_D void raster_item(const sftg_tile_args& A, int slab_rows, const sftg_raste
                         const uint32_t ii = (uint32_t)(pay & 0xFFFFFF), m = (uint32_t)((pay >> 24) & 0xFFFFFF), b = (uint32_t)((pay >> 48) & 0xFF);
                         const sftg_inst* I = &F->inst[ii];
                         const uint32_t g = I->meshlet_base + m;
-                        const uint8_t* ind = F->ml_inds + (size_t)g * 512;
+                        const uint8_t* ind = A.ml_inds + (size_t)g * 512;
                         const float* Sc = ss + (size_t)(I->ss_offset + m) * SFTG_SS_FLOATS;
                         const uint32_t q[3] = { ind[b * 32 + l], ind[b * 32 + 8 + l], ind[b * 32 + 16 + l] };
 #pragma unroll
@@ -599,7 +606,9 @@ SFTG_D float warp_max(float v) { float r; asm volatile("redux.sync.max.f32 %0, %
  * lane per covered fragment and the proxies selected per 32 fragments instead of per CTA (which
  * also took a second interpolation of every pixel) measured: skinned characters 1080p 2x 0.252 ->
  * 0.172 ms, atrium 1080p 4x 0.541 -> 0.381, atrium 1279x719 1x 0.272 -> 0.103, mixed materials
- * 1333x717 2x 0.213 -> 0.143, skinned 320x180 2x 0.516 -> 0.074, a batch of 48 views 12.3 -> 8.0.
+ * 1333x717 2x 0.213 -> 0.143, skinned 320x180 2x 0.516 -> 0.074, a batch of 48 views 12.3 -> 8.0; with
+ * the resident tables as kernel parameters, a texture's fields in two loads, a light's share of the
+ * chunk's proxy filter computed once and no normals for lightmapped chunks 0.344 and 7.2.
  * Sets of 16 blocks at 2x cost 3-15 %, contiguous sets per CTA at 4x 7 %.
  *
  * One (tile, part) item, run by one CTA.  The CTA makes the tile's light list and proxy cache
@@ -633,6 +642,9 @@ SFTG_D void resolve_item(const sftg_tile_args& A, uint32_t tile0, int split, boo
     __shared__ uint32_t s_meta[RESOLVE_WARPS][plan::cap], s_vid[RESOLVE_WARPS][plan::cap];
     __shared__ float s_acc[RESOLVE_WARPS][S > 1 ? plan::pixels * 3 : 1];
     __shared__ uint32_t s_wm[RESOLVE_WARPS][SFTG_MAX_TILE_LIGHTS / 2];
+    /* per warp and light, of the chunk in hand: its centre minus the light with 1 / |.|^2, the filter's radius */
+    __shared__ float4 s_fd[RESOLVE_WARPS][SFTG_MAX_TILE_LIGHTS];
+    __shared__ float s_fr[RESOLVE_WARPS][SFTG_MAX_TILE_LIGHTS];
 
     const uint32_t gtile = A.tile_order[tile0 + item / (uint32_t)split];   /* batch-wide tile index, heaviest first */
     const int part = (int)(item % (uint32_t)split);
@@ -641,6 +653,7 @@ SFTG_D void resolve_item(const sftg_tile_args& A, uint32_t tile0, int split, boo
     const float* ss = A.ss + (size_t)F->ss_base * SFTG_SS_FLOATS;
     const sftg_clip_tri* clips = A.clips + (F->total_ss ? A.clip_base[F->ss_base] : 0u);
     const uint8_t* light_vis = A.light_vis + (size_t)F->prox_base * 64;
+    const sftg_inst* inst = F->inst;
     uint32_t* color = F->color_dev;
     const int CP = F->pitch;   /* colour row stride in pixels (the caller's buffer when written directly) */
     float* shadow_out = A.shadow_out;
@@ -870,8 +883,8 @@ SFTG_D void resolve_item(const sftg_tile_args& A, uint32_t tile0, int split, boo
             const int gx = x + (pl & 3), gy = y + (pl >> 2);
             const float pxf = ((float)x + 0.5f) + (float)(pl & 3), pyf = ((float)y + 0.5f) + (float)(pl >> 2);
             tri_verts T;
-            fetch_tri(F, ss, clips, vid, T);
-            const sftg_meshlet_info info = F->ml_info[F->inst[T.inst].meshlet_base + T.m];
+            fetch_tri(A, inst, ss, clips, vid, T);
+            const int4 info = __ldg((const int4*)&A.ml_info[inst[T.inst].meshlet_base + T.m]);   /* bone, skin slot, material, lightmap */
             /* D6 barycentrics and perspective-correct interpolation (6282-6347) */
             const float dx1 = T.sx[1] - T.sx[0], dx2 = T.sx[2] - T.sx[0], dy1 = T.sy[1] - T.sy[0], dy2 = T.sy[2] - T.sy[0];
             const float idet = rcpr(dx1 * dy2 - dx2 * dy1);
@@ -893,8 +906,13 @@ SFTG_D void resolve_item(const sftg_tile_args& A, uint32_t tile0, int split, boo
             };
             /* material (6350-6382) */
             uint32_t base = 0xFFFFFFFFu; int ti = -1; float shin = 4.f;
-            if (info.material >= 0) { const sftg_mat mt = F->mats[info.material]; base = mt.base_color; ti = mt.tex; shin = mt.shininess; }
+            if (info.z >= 0) {
+                const int4 mt = __ldg((const int4*)&A.mats[info.z]);
+                ti = mt.x; base = (uint32_t)mt.y; shin = __int_as_float(mt.z);
+            }
             if (F->debug_mode == 5) { ti = F->debug_tex; base = 0xFFFFFFFFu; }   /* checkerboard view (6373-6376) */
+            int4 head = make_int4(0, 0, 0, 0);   /* the texture's width, height, levels, pot */
+            if (ti >= 0) head = __ldg((const int4*)&A.texs[ti]);
 #define INTERP(a) fma_(w0, (a)[0], fma_(w1, (a)[1], w2 * (a)[2]))
             /* D7 LOD from the first covered lane's derivatives (5501-5541): its neighbours' coordinates from
              * their lanes where the triangle covers them, else interpolated here */
@@ -911,7 +929,13 @@ SFTG_D void resolve_item(const sftg_tile_args& A, uint32_t tile0, int split, boo
             weights(pxf, pyf);
             const float cu = INTERP(T.u), cv = INTERP(T.v), clu = INTERP(T.lu), clv = INTERP(T.lv);
             const v3 P = mk3(INTERP(T.px), INTERP(T.py), INTERP(T.pz));
-            const v3 N = vnorm_fast(mk3(INTERP(T.nx), INTERP(T.ny), INTERP(T.nz)));
+            /* normal and view direction: a lightmapped surface uses neither */
+            const bool lm = info.w >= 0;
+            v3 N = mk3(0.f, 0.f, 0.f), V = N;
+            if (__any_sync(0xFFFFFFFFu, !lm)) {
+                N = vnorm_fast(mk3(INTERP(T.nx), INTERP(T.ny), INTERP(T.nz)));
+                V = vnorm_fast(sub3(mk3(F->cam[0], F->cam[1], F->cam[2]), P));
+            }
 #undef INTERP
             if (!full && __any_sync(0xFFFFFFFFu, !(fabsf(P.x) + fabsf(P.y) + fabsf(P.z) <= 1e15f))) { full = true; continue; }
             bool wire = false;
@@ -934,9 +958,8 @@ SFTG_D void resolve_item(const sftg_tile_args& A, uint32_t tile0, int split, boo
                 if (ok_x) { cu_x = su_x; cv_x = sv_x; }
                 if (ok_y) { cu_y = su_y; cv_y = sv_y; }
                 if (ti >= 0) {
-                    const sftg_tex& tx = F->texs[ti];
-                    const float ux = (cu_f - cu_x) * (float)tx.w, vx = (cv_f - cv_x) * (float)tx.h;
-                    const float uy = (cu_f - cu_y) * (float)tx.w, vy = (cv_f - cv_y) * (float)tx.h;
+                    const float ux = (cu_f - cu_x) * (float)head.x, vx = (cv_f - cv_x) * (float)head.y;
+                    const float uy = (cu_f - cu_y) * (float)head.x, vy = (cv_f - cv_y) * (float)head.y;
                     const float a1 = fabsf(ux) > fabsf(vx) ? fabsf(ux) : fabsf(vx);
                     const float a2 = fabsf(uy) > fabsf(vy) ? fabsf(uy) : fabsf(vy);
                     const float rho = a1 > a2 ? a1 : a2;
@@ -944,26 +967,24 @@ SFTG_D void resolve_item(const sftg_tile_args& A, uint32_t tile0, int split, boo
                         const float lf = (float)(31 - __clz((uint32_t)cvtt(rho)));
                         lod = (int)((lf + 0.5f) + (-0.375f));
                     }
-                    lod = lod < 0 ? 0 : (lod > tx.levels - 1 ? tx.levels - 1 : lod);
+                    lod = lod < 0 ? 0 : (lod > head.z - 1 ? head.z - 1 : lod);
                 }
             }
             float out[3];
             {
                 float tr, tg, tb;
-                if (lod > 1) sample_nearest(F, ti, lod, cu, cv, tr, tg, tb);
-                else sample_bilinear(F, ti, lod, cu, cv, tr, tg, tb);
+                if (lod > 1) sample_nearest(A, head, ti, lod, cu, cv, tr, tg, tb);
+                else sample_bilinear(A, head, ti, lod, cu, cv, tr, tg, tb);
                 out[0] = tr * ((float)((base >> 16) & 0xFF) * i255); out[1] = tg * ((float)((base >> 8) & 0xFF) * i255);
                 out[2] = tb * ((float)(base & 0xFF) * i255);
             }
-            const bool lm = info.lightmap_tex >= 0;
             const bool lighted = !(shin < 0.f);
             if (!lighted) { out[0] = out[0] * (-shin); out[1] = out[1] * (-shin); out[2] = out[2] * (-shin); }
             if (__any_sync(0xFFFFFFFFu, lighted)) {
-                const v3 V = vnorm_fast(sub3(mk3(F->cam[0], F->cam[1], F->cam[2]), P));
                 const float sscale = ((shin + 8.f) / 8.f) * 0.04f;
                 float dif[3], spc[3] = { 0.f, 0.f, 0.f }, lms = 1.f;
                 if (lm) {
-                    sample_bilinear(F, info.lightmap_tex, 0, clu, clv, dif[0], dif[1], dif[2]);
+                    sample_bilinear(A, __ldg((const int4*)&A.texs[info.w]), info.w, 0, clu, clv, dif[0], dif[1], dif[2]);
                     dif[0] = dif[0] * F->lightmap_brightness; dif[1] = dif[1] * F->lightmap_brightness; dif[2] = dif[2] * F->lightmap_brightness;
                 } else {
                     dif[0] = F->ambient[0]; dif[1] = F->ambient[1]; dif[2] = F->ambient[2];
@@ -997,17 +1018,23 @@ SFTG_D void resolve_item(const sftg_tile_args& A, uint32_t tile0, int split, boo
                         const v3 he = mk3(hx - bc.x, hy - bc.y, hz - bc.z);
                         const float br = sqrtf(he.x * he.x + he.y * he.y + he.z * he.z) * 1.002f +
                                          1e-6f * (fabsf(bc.x) + fabsf(bc.y) + fabsf(bc.z));
+                        if (lane < ntl) {
+                            const float4 L = s_lp[lane];
+                            const v3 D = mk3(bc.x - L.x, bc.y - L.y, bc.z - L.z);
+                            const float dd = fma_(D.x, D.x, fma_(D.y, D.y, D.z * D.z));
+                            s_fd[warp][lane] = make_float4(D.x, D.y, D.z, dd > 0.f ? __fdividef(1.f, dd) : 0.f);
+                            s_fr[warp][lane] = br + (dd > 0.f ? 2e-3f * dd * rsqrtf(dd) : 0.f);
+                        }
+                        __syncwarp();
                         for (int i0 = 0; i0 < ntl; i0 += 2) {
                             const int i = i0 + (lane >> 4), k = lane & 15;
                             bool keep = false;
                             if (i < ntl && k < s_npc[i]) {
-                                const float4 L = s_lp[i], Wv = s_btw[i * SFTG_MAX_LIGHT_PROXIES + k];
-                                const v3 D = mk3(bc.x - L.x, bc.y - L.y, bc.z - L.z);
-                                const float dd = D.x * D.x + D.y * D.y + D.z * D.z;
-                                const float t = dd > 0.f ? fminf(fmaxf(__fdividef(Wv.x * D.x + Wv.y * D.y + Wv.z * D.z, dd), 0.f), 1.f) : 0.f;
-                                const v3 E = mk3(Wv.x - t * D.x, Wv.y - t * D.y, Wv.z - t * D.z);
-                                const float r = s_rbm[i * SFTG_MAX_LIGHT_PROXIES + k] + br + 2e-3f * sqrtf(dd);
-                                keep = !(E.x * E.x + E.y * E.y + E.z * E.z > r * r);
+                                const float4 D = s_fd[warp][i], Wv = s_btw[i * SFTG_MAX_LIGHT_PROXIES + k];
+                                const float t = __saturatef(fma_(Wv.x, D.x, fma_(Wv.y, D.y, Wv.z * D.z)) * D.w);
+                                const v3 E = mk3(fma_(-t, D.x, Wv.x), fma_(-t, D.y, Wv.y), fma_(-t, D.z, Wv.z));
+                                const float r = s_rbm[i * SFTG_MAX_LIGHT_PROXIES + k] + s_fr[warp][i];
+                                keep = !(fma_(E.x, E.x, fma_(E.y, E.y, E.z * E.z)) > r * r);
                             }
                             const uint32_t bal = __ballot_sync(0xFFFFFFFFu, keep);
                             if (lane == 0) wm[i0 >> 1] = bal;

@@ -6,7 +6,7 @@
  *                     padded to 4x4 and stored 4x4 block-linear (row-major texels inside a
  *                     block, row-major blocks), as sft_texture_create lays it out
  *                     (sofren2.c:9181-9310)
- *   sftg_tex          per texture: size, levels, pot flag, per-level texel offset / blocks_w / shift
+ *   sftg_tex          per texture: size, levels, pot flag, per-level texel offset / blocks per row
  *   sftg_mat          per material: texture index (-1 none), base colour, shininess
  *   meshlet pool      per meshlet g: attr[g] = f32[10][64] (x y z nx ny nz u v lu lv),
  *                     inds[g] = u8[512] (16 batches x [v0 x8, v1 x8, v2 x8, pad x8]),
@@ -49,11 +49,9 @@
 #define SFTG_SS_D 768
 #define SFTG_SS_FLOATS 832         /* floats per record (3328 B) */
 
-typedef struct sftg_tex {
+typedef struct sftg_tex {      /* 128 B, read as one 16-byte and one 8-byte load */
     int32_t w, h, levels, is_pot;
-    uint32_t offs[14];     /* texel offset of each level from the heap base */
-    int32_t bw[14];        /* 4x4 blocks per row */
-    int32_t shift[14];     /* log2(bw) when pot */
+    struct { uint32_t off, bw; } lev[14];   /* per level: texel offset from the heap base, 4x4 blocks per row */
 } sftg_tex;
 
 typedef struct sftg_mat {
