@@ -23,6 +23,7 @@
 #include <stdio.h>
 #include <stdlib.h>
 #include <string.h>
+#include <unistd.h>
 #include <algorithm>
 #include <vector>
 #include <chrono>
@@ -110,6 +111,7 @@ struct sftg_ctx {
     uint32_t blas_items = 0, blas_launches = 0; /* and its triangles and kernels */
     cudaEvent_t ev_blas[2] = { nullptr, nullptr };
     bool use_graphs = true;
+    bool host_tables = false;                  /* the GPU reads and writes pageable host memory through the host's page tables */
     sftg_tuning tuning = { { 16, 16, 16 }, { 8, 8, 8 }, 1, 0, { 0, 0, 0 }, { 0, 0, 0 }, 0 };   /* measured best on the single-view workloads */
     /* transient models (one frame's dynamic meshes): pool marks where they start */
     bool tr_live = false, tr_pinned = false;
@@ -217,6 +219,12 @@ extern "C" int sftg_create(int device, sftg_ctx** out) {
     if (cudaMalloc((void**)&ctx->d_ray_next, 256) != cudaSuccess) { ctx->d_ray_next = nullptr; sftg_destroy(ctx); return SFTG_E_CUDA; }
     sftg_tile_configure(227 * 1024);
     if (noalloc_scratch_setup(device) != cudaSuccess) { sftg_destroy(ctx); return SFTG_E_CUDA; }
+    {
+        int access = 0, tables = 0;
+        cudaDeviceGetAttribute(&access, cudaDevAttrPageableMemoryAccess, device);
+        cudaDeviceGetAttribute(&tables, cudaDevAttrPageableMemoryAccessUsesHostPageTables, device);
+        ctx->host_tables = access && tables;
+    }
     { const char* e = getenv("SFTG_NO_GRAPHS"); if (e && *e && *e != '0') ctx->use_graphs = false; }
     *out = ctx;
     return SFTG_OK;
@@ -507,7 +515,8 @@ struct view_plan {
     uint32_t ss_base, total_ss, tile_base, tiles, prox_base, packet_base, n_packets, stile_base, stiles, scols;
     uint32_t inst_off, bone_off, pl_off, dl_off, tl_off;
     uint64_t vis_base, color_off;
-    uint32_t* direct;   /* the caller's pinned colour buffer, written by the kernels in place; else null */
+    uint32_t* direct;   /* the caller's colour buffer, written by the kernels in place; else null */
+    bool pageable;      /* and it is pageable memory */
     int32_t direct_pitch;   /* its row stride in pixels */
 };
 
@@ -565,18 +574,47 @@ static int sample_slot(int S) { return S == 1 ? 0 : (S == 2 ? 1 : 2); }
  * (screen-space cache, batch records, clip pool, tile lists, light_vis, visibility buffers) are
  * laid out view after view, with tiles numbered by sample count first (1, 2, 4) so that each
  * raster/resolve specialisation covers one contiguous tile range. */
-/* The device-visible address of a caller's colour buffer the kernels can write in place: page-
- * locked host memory (registered or allocated by CUDA) with a clearing view and a pitch of whole
- * pixels.  Writes then reach host memory over the chip-to-chip link as the resolve stores them,
- * and the frame needs no device-to-host copy.  Null for any other buffer (copied as before). */
-static uint32_t* direct_color(const sftg_frame_desc& fd, uint32_t* host, int32_t pitch_bytes) {
-    if (!host || !fd.clear) return nullptr;
+/* The address by which kernels reach a caller's host array in place: page-locked memory (registered or
+ * allocated by CUDA), or, where the GPU shares the host's page tables (Grace), pageable memory.  Null
+ * for any other.  Through pageable copies the driver stages every byte on a host thread: 100
+ * poses took 45 us of which the kernel takes 10, and a 3.8 MB frame kept and returned 95 us. */
+static void* host_visible(const sftg_ctx* ctx, const void* p, bool* pageable = nullptr) {
+    if (pageable) *pageable = false;
+    if (!p || ((uintptr_t)p & 3u)) return nullptr;
+    cudaPointerAttributes at;
+    if (cudaPointerGetAttributes(&at, p) != cudaSuccess) { cudaGetLastError(); return nullptr; }
+    if (at.type == cudaMemoryTypeHost) return at.devicePointer;
+    if (at.type != cudaMemoryTypeUnregistered || !ctx->host_tables) return nullptr;
+    if (pageable) *pageable = true;
+    return const_cast<void*>(p);
+}
+
+/* Populates the pages of a host array before kernels use it (a GPU access to a page the host has never
+ * touched is served by a fault), rows of `bytes` bytes at `pitch`.  Output bytes are touched by an
+ * atomic that leaves them as they are. */
+static void touch_pages(const void* p, size_t bytes, size_t pitch, size_t rows, bool output) {
+    const size_t page = (size_t)sysconf(_SC_PAGESIZE);
+    uintptr_t last = ~(uintptr_t)0;
+    for (size_t r = 0; r < rows && bytes; r++) {
+        const uintptr_t a = (uintptr_t)p + r * pitch, e = a + bytes;
+        for (uintptr_t q = a; q < e; q = (q / page + 1) * page) {
+            if (q / page == last) continue;
+            last = q / page;
+            if (output) __atomic_fetch_or((unsigned char*)q, (unsigned char)0, __ATOMIC_RELAXED);
+            else (void)*(volatile const unsigned char*)q;
+        }
+    }
+}
+
+/* The address of a caller's colour buffer that the kernels write (and, where the frame does not clear,
+ * blend with) in place, its pitch a whole number of pixels; null for any other buffer (copied).
+ * Stores then reach host memory over the chip-to-chip link as the resolve makes them. */
+static uint32_t* direct_color(const sftg_ctx* ctx, const sftg_frame_desc& fd, uint32_t* host, int32_t pitch_bytes, bool& pageable) {
+    pageable = false;
+    if (!host) return nullptr;
     const size_t pitch = pitch_bytes > 0 ? (size_t)pitch_bytes : (size_t)fd.width * 4;
     if (pitch % 4 || pitch < (size_t)fd.width * 4) return nullptr;
-    cudaPointerAttributes at;
-    if (cudaPointerGetAttributes(&at, host) != cudaSuccess) { cudaGetLastError(); return nullptr; }
-    if (at.type != cudaMemoryTypeHost || !at.devicePointer) return nullptr;
-    return (uint32_t*)at.devicePointer;
+    return (uint32_t*)host_visible(ctx, host, &pageable);
 }
 
 static int build_batch(sftg_ctx* ctx, sftg_lane& ln, const sftg_frame_desc* fds, uint32_t nv, bool want_debug, batch_bufs& B,
@@ -656,9 +694,30 @@ static int build_batch(sftg_ctx* ctx, sftg_lane& ln, const sftg_frame_desc* fds,
         if (fd->n_instances > max_inst) max_inst = fd->n_instances;
         n_pl += fd->n_point; n_dl += fd->n_dir; n_tl += fd->tlas_count;
         P.color_off = color_total; color_total += (uint64_t)W * H;
-        P.direct = direct_color(*fd, host_color ? host_color[v] : nullptr, pitch_bytes ? pitch_bytes[v] : 0);
+        P.direct = direct_color(ctx, *fd, host_color ? host_color[v] : nullptr, pitch_bytes ? pitch_bytes[v] : 0, P.pageable);
         P.direct_pitch = P.direct ? (pitch_bytes && pitch_bytes[v] > 0 ? pitch_bytes[v] / 4 : W) : W;
     }
+    if (host_color && nv > 1) {
+        /* views whose buffers share bytes are copied one after the other, in view order; page-locked buffers
+         * of clearing views are written in place all the same (interleaved parts of one picture) */
+        std::vector<std::pair<uintptr_t, uint32_t>> by;
+        for (uint32_t v = 0; v < nv; v++) if (host_color[v]) by.push_back({ (uintptr_t)host_color[v], v });
+        std::sort(by.begin(), by.end());
+        uintptr_t end = 0;
+        uint32_t prev = 0;
+        auto copied = [&](uint32_t v) {
+            if (B.plan[v].pageable || !fds[v].clear) { B.plan[v].direct = nullptr; B.plan[v].pageable = false; B.plan[v].direct_pitch = fds[v].width; }
+        };
+        for (const auto& q : by) {
+            const uint32_t v = q.second;
+            const size_t pitch = pitch_bytes && pitch_bytes[v] > 0 ? (size_t)pitch_bytes[v] : (size_t)fds[v].width * 4;
+            if (end > q.first) { copied(prev); copied(v); }
+            const uintptr_t e = q.first + pitch * (size_t)(fds[v].height - 1) + (size_t)fds[v].width * 4;
+            if (e > end) { end = e; prev = v; }
+        }
+    }
+    for (uint32_t v = 0; v < nv; v++)
+        if (B.plan[v].pageable) touch_pages(host_color[v], (size_t)fds[v].width * 4, (size_t)B.plan[v].direct_pitch * 4, fds[v].height, true);
     if (max_pairs * (1 + SFTG_OCC_ITEMS_PER_PAIR) > 0xFFFFFFF0ull || total_ss > (1u << 26)) return set_err(ctx, SFTG_E_LIMIT, "batch too large for one submission");
     uint32_t total_tiles = 0;
     uint64_t vis_total = 0;
@@ -954,6 +1013,7 @@ static int launch_batch(sftg_ctx* ctx, sftg_lane& ln, const batch_bufs& B) {
     sftg_tile_args A;
     A.texs = (const sftg_tex*)ctx->texs.ptr; A.texels = (const uint32_t*)ctx->texels.ptr; A.mats = (const sftg_mat*)ctx->mats.ptr;
     A.ml_inds = (const uint8_t*)ctx->ml_inds.ptr; A.ml_info = (const sftg_meshlet_info*)ctx->ml_info.ptr;
+    A.totals = B.totals;
     A.frames = B.frames; A.tile_view = B.tile_view; A.ss = B.ss; A.clips = B.clips; A.clip_base = B.clip_base;
     A.tile_order = B.tile_order; A.raster_items = B.raster_items; A.raster_range = B.raster_range; A.raster_done = B.raster_done;
     A.tile_nlights = B.tile_nlights; A.tile_lights = B.tile_lights;
@@ -1390,9 +1450,23 @@ extern "C" int sftg_pose_eval(sftg_ctx* ctx, const sftg_pose_request* reqs, uint
         off[k] = total;
         total += ctx->h_skels[reqs[k].skeleton].bone_count;
     }
+    /* the caller's arrays in place: a request with an out-of-range animation is not written to */
+    bool page_posed = false, page_global = false;
+    const sftg_pose_request* v_req = (const sftg_pose_request*)host_visible(ctx, reqs);
+    const uint32_t* v_off = (const uint32_t*)host_visible(ctx, off.data());
+    float* v_posed = (float*)host_visible(ctx, posed, &page_posed);
+    float* v_global = global ? (float*)host_visible(ctx, global, &page_global) : nullptr;
+    const size_t b_mat = (size_t)total * 64;
+    if (v_req && v_off && v_posed && (!global || v_global)) {
+        if (page_posed) touch_pages(posed, b_mat, 0, 1, true);
+        if (page_global) touch_pages(global, b_mat, 0, 1, true);
+        sftg_launch_pose(pose_tables(ctx), v_req, v_off, n, v_posed, v_global, ctx->stream);
+        CK(cudaGetLastError());
+        CK(cudaStreamSynchronize(ctx->stream));
+        return SFTG_OK;
+    }
     /* device io: requests, offsets, posed, global */
     const size_t b_req = ((size_t)n * sizeof(sftg_pose_request) + 255) & ~(size_t)255, b_off = ((size_t)n * 4 + 255) & ~(size_t)255;
-    const size_t b_mat = (size_t)total * 64;
     int rc = pool_reserve(ctx, ctx->p_pose_io, b_req + b_off + 2 * b_mat + 256);
     if (rc) return rc;
     char* io = (char*)ctx->p_pose_io.ptr;
@@ -1448,14 +1522,24 @@ extern "C" int sftg_raycast(sftg_ctx* ctx, const sftg_ray* rays, uint32_t n, sft
     if (!ctx || (n && (!rays || !hits))) return SFTG_E_ARG;
     if (!n) return SFTG_OK;
     CK(cudaSetDevice(ctx->device));
+    int rc;
+    /* few rays: the caller's arrays in place (the walk of many reads and writes them more than once) */
+    const sftg_ray* v_rays = n <= SFTG_RAY_WIDE_MAX ? (const sftg_ray*)host_visible(ctx, rays) : nullptr;
+    sftg_ray_hit* v_hits = n <= SFTG_RAY_WIDE_MAX ? (sftg_ray_hit*)host_visible(ctx, hits) : nullptr;
+    if (v_rays && v_hits) {
+        touch_pages(rays, (size_t)n * sizeof(sftg_ray), 0, 1, false);
+        touch_pages(hits, (size_t)n * sizeof(sftg_ray_hit), 0, 1, true);
+        if ((rc = sftg_raycast_device(ctx, v_rays, n, v_hits))) return rc;
+    } else {
     const size_t b_ray = ((size_t)n * sizeof(sftg_ray) + 255) & ~(size_t)255;
-    int rc = pool_reserve(ctx, ctx->p_ray_io, b_ray + (size_t)n * sizeof(sftg_ray_hit) + 256);
+    rc = pool_reserve(ctx, ctx->p_ray_io, b_ray + (size_t)n * sizeof(sftg_ray_hit) + 256);
     if (rc) return rc;
     sftg_ray* d_rays = (sftg_ray*)ctx->p_ray_io.ptr;
     sftg_ray_hit* d_hits = (sftg_ray_hit*)((char*)ctx->p_ray_io.ptr + b_ray);
     CK(cudaMemcpyAsync(d_rays, rays, (size_t)n * sizeof(sftg_ray), cudaMemcpyHostToDevice, ctx->stream));
     if ((rc = sftg_raycast_device(ctx, d_rays, n, d_hits))) return rc;
     CK(cudaMemcpyAsync(hits, d_hits, (size_t)n * sizeof(sftg_ray_hit), cudaMemcpyDeviceToHost, ctx->stream));
+    }
     CK(cudaStreamSynchronize(ctx->stream));
     for (uint32_t k = 0; k < n; k++)
         if (hits[k].hit == 2) return set_err(ctx, SFTG_E_DEVICE_STATUS, "ray %u: BLAS walk overflowed its stack", k);

@@ -366,13 +366,12 @@ k_ray_wide(const sftg_ray* __restrict__ rays, uint32_t n, const sftg_model* __re
     if (lane == 0) store_hit(R, hit, overflow, win_t, tris + win, hits + k);
 }
 
-#define RAY_WIDE_MAX 81920u  /* rays up to which a ray gets a whole warp: measured 389 us against 468 at 65536, 5.0 ms against 1.85 at 2^20 */
 #define RAY_GRID (152 * 8)   /* CTAs of the many-ray walk: 8 fit an SM (registers) */
 
 int sftg_launch_raycast(const sftg_ray* rays, uint32_t n, const sftg_model* models, uint32_t n_models, const sftg_wslot* wslots,
                         const sftg_wtri* wtris, uint32_t* next, sftg_ray_hit* hits, cudaStream_t st) {
     if (!n) return 0;
-    if (n <= RAY_WIDE_MAX) {
+    if (n <= SFTG_RAY_WIDE_MAX) {
         k_ray_wide<<<(n + RAY_WARPS - 1) / RAY_WARPS, RAY_WARPS * 32, 0, st>>>(rays, n, models, n_models, wslots, wtris, hits);
         return 0;
     }

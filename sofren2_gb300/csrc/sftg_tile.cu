@@ -572,6 +572,11 @@ k_tile_lights(const sftg_tile_args A, uint32_t tile0)
     }
 }
 
+/* the batch exceeded a capacity: the host grows it and renders the batch again */
+SFTG_D bool over_capacity(const sftg_tile_args& A, const sftg_frame* F) {
+    return A.totals[0] > F->clip_cap || A.totals[1] > F->tile_cap || A.totals[2] > F->stile_cap;
+}
+
 #define TILE_BLOCKS (16 * 32)                 /* 4x2 blocks per 64x64 tile; a CTA resolves 1/split of them */
 #define RESOLVE_WARPS (TILE_THREADS / 32)
 #define LIGHT_SLOTS (SFTG_MAX_TILE_LIGHTS * SFTG_MAX_LIGHT_PROXIES)
@@ -661,6 +666,7 @@ SFTG_D void resolve_item(const sftg_tile_args& A, uint32_t tile0, int split, boo
     const int tmx = (tile % F->cols) * SFTG_TILE, tmy = (tile / F->cols) * SFTG_TILE;
     const float2* vis = A.vis + F->vis_base + (size_t)tile * S * SFTG_TILE_PX;
 
+    if (!F->clear && over_capacity(A, F)) return;   /* the whole CTA: the caller's pixels stay for the next attempt */
     const sftg_tile_lights* TL = A.tile_lights + gtile;
     if (tid == 0) s_odd = shadow_out != nullptr;
     if (records) {   /* D2 and D3's selection come from the tile's record (k_tile_lights) */
@@ -1394,6 +1400,7 @@ __global__ void __launch_bounds__(256) k_debug_overlay(const sftg_tile_args A)
     const sftg_frame* F = A.frames + A.tile_view[gtile];
     const int mode = F->debug_mode;
     if (mode < 2 || mode > 4) return;
+    if (!F->clear && over_capacity(A, F)) return;
     const int tile = (int)(gtile - F->tile_base);
     const int tmx = (tile % F->cols) * SFTG_TILE, tmy = (tile / F->cols) * SFTG_TILE;
     const int sw = (int)(F->hw * 2.f), sh = (int)(F->hh * 2.f);

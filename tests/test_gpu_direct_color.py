@@ -86,3 +86,41 @@ def test_debug_views_into_pinned_buffer(renderer, mode):
         renderer.set_debug_mode(0)
         renderer.set_samples(1)
         renderer.free_scene(h)
+
+
+@pytest.mark.parametrize("samples", [1, 2, 4])
+def test_pageable_buffers_in_place_and_copied(renderer, samples):
+    """Pageable buffers, which the kernels reach in place where the GPU shares the host's page tables: a
+    fresh (never touched) one, one with a padded pitch and guard pixels on both sides, an unaligned
+    one (copied), kept pixels under a frame that does not clear, and interleaved halves of one picture
+    in one batch (copied in view order)."""
+    h, keep = renderer.load_scene(gc.blob("small")), renderer.load_scene(gc.blob("variety_noclear"))
+    try:
+        renderer.set_samples(samples)
+        w, hh = renderer.frame_size(h, 0)
+        t, pinned = _pinned(hh, w, 0)
+        want = renderer.render(h, 0, pinned).copy()
+        assert np.array_equal(renderer.render(h, 0, np.empty((hh, w), np.uint32)), want)
+        room = np.full((hh + 2, w + 11), 0x1234567, np.uint32)
+        renderer.render(h, 0, room[1:-1, 5:5 + w])
+        assert np.array_equal(room[1:-1, 5:5 + w], want)
+        room[1:-1, 5:5 + w] = 0x1234567
+        assert (room == 0x1234567).all()
+        odd = np.zeros(hh * w * 4 + 1, np.uint8)[1:].view(np.uint32).reshape(hh, w)
+        assert np.array_equal(renderer.render(h, 0, odd), want)
+        kw, kh = renderer.frame_size(keep, 0)
+        init = np.random.default_rng(7).integers(0, 1 << 32, size=(kh, kw), dtype=np.uint32)
+        t2, kp = _pinned(kh, kw, 0)
+        kp[:] = init
+        kept = renderer.render(keep, 0, kp)
+        assert np.array_equal(renderer.render(keep, 0, init.copy()), kept)
+        both = np.zeros((hh, 2 * w), np.uint32)
+        renderer.render_batch([(h, 0, samples), (h, 0, samples)], [both[:, :w], both[:, w:]])
+        assert np.array_equal(both[:, :w], want) and np.array_equal(both[:, w:], want)
+        one = np.zeros((hh, w), np.uint32)
+        renderer.render_batch([(h, 0, 1), (h, 0, samples)], [one, one])
+        assert np.array_equal(one, want), "two views into one buffer: the last one's pixels"
+    finally:
+        renderer.set_samples(1)
+        renderer.free_scene(h)
+        renderer.free_scene(keep)
