@@ -175,7 +175,8 @@ typedef struct sftg_tuning {
     int32_t resolve_split[3];     /* most resolve CTAs per 64x64 tile at 1x, 2x, 4x: 1, 2, 4, 8 or 16 (default 16); 8 and
                                      16 are halved, down to 4, where the tiles alone fill the GPU */
     int32_t raster_slab_rows[3];  /* rows per triangle a raster group walks at a time at 1x, 2x, 4x: 4..64 (default 8) */
-    int32_t geom_job_width;       /* meshlets per geometry warp: 1..8 (default 1; the reference's job is 8) */
+    int32_t geom_job_width;       /* meshlets per geometry job: 1..8 (default 1); 8, the reference's, from 4096 meshlets
+                                     in a batch on */
     int32_t occl_ray_prune;       /* 1: also cull BLAS children no unblocked shadow ray reaches (faster; can differ
                                      from the reference only where a ray grazes a triangle's plane); default 0.
                                      The only knob that is not result-neutral: sftg_autotune leaves it as set */

@@ -617,6 +617,20 @@ static uint32_t* direct_color(const sftg_ctx* ctx, const sftg_frame_desc& fd, ui
     return (uint32_t*)host_visible(ctx, host, &pageable);
 }
 
+/* Meshlets per geometry job: the knob's, or the reference's whole group of 8 from SFTG_WIDE_JOBS meshlets
+ * in the batch on. */
+static uint32_t job_width(const sftg_ctx* ctx, const sftg_frame_desc* fds, uint32_t nv) {
+    uint64_t n = 0;
+    for (uint32_t v = 0; v < nv && n < SFTG_WIDE_JOBS; v++) {
+        if (fds[v].n_instances > SFTG_MAX_INSTANCES) break;   /* refused by the caller, as are models out of range */
+        for (uint32_t i = 0; i < fds[v].n_instances && n < SFTG_WIDE_JOBS; i++) {
+            const int32_t m = fds[v].instances[i].model;
+            if (m >= 0 && (size_t)m < ctx->h_models.size()) n += ctx->h_models[m].total_meshlets;
+        }
+    }
+    return n >= SFTG_WIDE_JOBS ? 8u : (uint32_t)ctx->tuning.geom_job_width;
+}
+
 static int build_batch(sftg_ctx* ctx, sftg_lane& ln, const sftg_frame_desc* fds, uint32_t nv, bool want_debug, batch_bufs& B,
                        uint32_t* const* host_color = nullptr, const int32_t* pitch_bytes = nullptr) {
     if (!nv || nv > 65535) return set_err(ctx, SFTG_E_ARG, "a batch holds 1 to 65535 views, not %u", nv);
@@ -629,6 +643,7 @@ static int build_batch(sftg_ctx* ctx, sftg_lane& ln, const sftg_frame_desc* fds,
     std::vector<float> bones;
     uint32_t total_ss = 0, total_prox = 0, total_packets = 0, max_inst = 0, n_pl = 0, n_dl = 0, n_tl = 0;
     uint64_t max_pairs = 0, color_total = 0;
+    const uint32_t jw = job_width(ctx, fds, nv);
     for (uint32_t v = 0; v < nv; v++) {
         const sftg_frame_desc* fd = &fds[v];
         view_plan& P = B.plan[v];
@@ -653,7 +668,6 @@ static int build_batch(sftg_ctx* ctx, sftg_lane& ln, const sftg_frame_desc* fds,
                 I.bones = (int32_t)((bones.size() - P.bone_off) / 16);
                 bones.insert(bones.end(), id.bones, id.bones + (size_t)id.bone_count * 16);
             }
-            const uint32_t jw = (uint32_t)ctx->tuning.geom_job_width;
             if (ctx->h_job_tmpl.size() <= (size_t)id.model) ctx->h_job_tmpl.resize((size_t)id.model + 1);
             sftg_ctx::job_tmpl& T = ctx->h_job_tmpl[id.model];
             if (T.jw != jw || T.meshlet_base != md.meshlet_base || T.total != md.total_meshlets) {
@@ -975,14 +989,16 @@ static int launch_batch(sftg_ctx* ctx, sftg_lane& ln, const batch_bufs& B) {
     }
     CK(record_event(ln, ln.ev_geo, st, cap));
     if (B.n_jobs) {
-        k_geometry<<<(B.n_jobs + 3) / 4, 128, 0, st>>>(B.frames, B.jobs, B.n_jobs, B.ss, B.recs, B.clip_cnt, B.clip_tot, B.mrect);
+        k_geometry<<<(B.n_jobs + 1) / 2, 128, 0, st>>>(B.frames, B.jobs, B.n_jobs, B.ss, B.recs, B.clip_cnt, B.clip_tot, B.mrect);
         ln.launches++;
         CK(cudaGetLastError());
     }
     if (B.total_ss) {
         scan_u32(B.clip_tot, B.clip_base, B.total_ss, B.scan_tmp, B.totals + 0, st, &ln.launches);
-        k_clip<<<(B.total_ss + CLIP_MESHLETS - 1) / CLIP_MESHLETS, 128, 0, st>>>(B.frames, B.n_views, B.ss, B.clip_cnt, B.clip_tot, B.clip_base,
-                                                                                 B.clips, B.clip_rect, B.mrect, B.total_ss);
+        /* meshlets per CTA: one while the CTAs are few (those that clip follow one another in one), else eight */
+        const uint32_t per = B.total_ss <= 2048u ? 1u : 8u;
+        k_clip<<<(B.total_ss + per - 1) / per, 128, 0, st>>>(B.frames, B.n_views, B.ss, B.clip_cnt, B.clip_tot, B.clip_base, B.clips, B.clip_rect,
+                                                             B.mrect, B.total_ss, per);
         ln.launches++;
         CK(cudaGetLastError());
     }

@@ -1,13 +1,12 @@
 /*
  * Geometry, clipping and binning kernels of the sofren2 render path.
  *
- *   k_geometry  one warp per job of up to 8 meshlets (sft__worker_phase_geom, sofren2.c:4901-5145):
+ *   k_geometry  two warps per job of up to 8 meshlets (sft__worker_phase_geom, sofren2.c:4901-5145):
  *               lanes 0-7 run the bounding-sphere frustum test and normal-cone test; each
- *               surviving meshlet is skinned (4 joints, bone matrices staged in shared
- *               memory), transformed and projected two vertices per lane, written to the
- *               screen-space cache, then its 128 triangles are set up four batches at a
- *               time (sft__geom_setup_and_bin_batch, 4775-4884): one 8-lane group per batch,
- *               shuffles build the batch's tile rectangle and lane mask.
+ *               surviving meshlet is skinned (4 joints), transformed and projected a vertex
+ *               per lane, written to the screen-space cache, then its 128 triangles are set
+ *               up eight batches at a time (sft__geom_setup_and_bin_batch, 4775-4884): one
+ *               8-lane group per batch, shuffles build the batch's tile rectangle and lane mask.
  *   k_clip      near-plane clipping of straddling triangles (4691-4772, 4264-4381); clip
  *               slots come from an exclusive scan of the meshlets' clip counts, which numbers
  *               them in the reference's single-worker emission order.
@@ -24,42 +23,42 @@
 #include "sftg_lane.cuh"
 #include "sftg_kernels.h"
 
-#define GEOM_WARPS 4
-#define GEOM_BONES 64
+#define GEOM_TEAMS 2    /* meshlet jobs per CTA, two warps each */
 
 /* ----------------------------------------------------------------------------------------- */
-__global__ void __launch_bounds__(GEOM_WARPS * 32)
+/* Two warps per job, a vertex per lane and two rounds of four triangle batches per warp.  Bound by
+ * latency: a frame's few hundred to few thousand meshlets leave the SMs a few warps each, and a warp's
+ * time is its chain of loads (job, instance, bounds, vertices, indices) and its own instructions.
+ * One warp per job (two vertices per lane in turn, bones staged in 16 KB of shared memory per CTA,
+ * index bytes loaded where they are used) took, with the clipping after it, 39 us on the skinned 1080p
+ * frame (743 meshlets) and 75 on the 1080p 4x atrium, where this takes 27 and 49 (jobs of one meshlet). */
+__global__ void __launch_bounds__(GEOM_TEAMS * 64)
 k_geometry(const sftg_frame* __restrict__ frames, const sftg_job* __restrict__ jobs, uint32_t n_jobs, float* __restrict__ ss,
            sftg_batch_rec* __restrict__ recs, uint32_t* __restrict__ clip_cnt, uint32_t* __restrict__ clip_tot, int4* __restrict__ mrect)
 {
-    __shared__ uint4 s_ind[GEOM_WARPS][32];    /* the meshlet's 512 index bytes */
-    __shared__ float s_bones[GEOM_WARPS][GEOM_BONES * 16];
-    __shared__ float s_v[GEOM_WARPS][6][64];   /* tx ty tz w sx sy */
-    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-    const uint32_t job_i = blockIdx.x * GEOM_WARPS + warp;
-    if (job_i >= n_jobs) return;
+    __shared__ uint4 s_ind[GEOM_TEAMS][32];    /* the meshlet's 512 index bytes */
+    __shared__ float s_v[GEOM_TEAMS][3][64];   /* tz sx sy */
+    __shared__ int4 s_mr[GEOM_TEAMS];          /* the second warp's share of the meshlet's rectangle */
+    __shared__ uint32_t s_clips[GEOM_TEAMS];
+    const int team = threadIdx.x >> 6, tt = threadIdx.x & 63, warp = tt >> 5, lane = tt & 31;
+    const uint32_t job_i = blockIdx.x * GEOM_TEAMS + team;
+    if (job_i >= n_jobs) return;   /* the whole team */
+    auto team_sync = [&]() { asm volatile("bar.sync %0, 64;" ::"r"(team + 1) : "memory"); };
     const sftg_job J = jobs[job_i];
     const sftg_frame* F = frames + J.view;
     const sftg_inst* I = &F->inst[J.inst];
     float T[16];
 #pragma unroll
     for (int k = 0; k < 16; k++) T[k] = I->T[k];
-    const sftg_model Md = F->models[I->model];
-    const float* bones_g = (J.skinned && I->bones >= 0) ? F->bones + (size_t)I->bones * 16 : nullptr;
-    const int nb = (int)Md.bone_count;
-    const bool bones_in_smem = bones_g && nb <= GEOM_BONES;
-    if (bones_in_smem) {
-        for (int k = lane; k < nb * 16; k += 32) s_bones[warp][k] = bones_g[k];
-        __syncwarp();
-    }
-    const float* bones = bones_in_smem ? s_bones[warp] : bones_g;
+    const float* bones = (J.skinned && I->bones >= 0) ? F->bones + (size_t)I->bones * 16 : nullptr;
 
     /* ---- cull (lanes 0..7), 4939-4994 ---- */
     bool inside = false;
     const uint32_t g0 = I->meshlet_base + J.first;
     if (lane < (int)J.count) {
-        const float* cl = F->ml_cull + (size_t)(g0 + lane) * 8;
-        v3 ctr = mk3(cl[0], cl[1], cl[2]), ax = mk3(cl[4], cl[5], cl[6]);
+        const float4* cl = (const float4*)(F->ml_cull + (size_t)(g0 + lane) * 8);
+        const float4 c0 = cl[0], c1 = cl[1];
+        v3 ctr = mk3(c0.x, c0.y, c0.z), ax = mk3(c1.x, c1.y, c1.z);
         if (J.skinned) {
             const int cb = F->ml_info[I->meshlet_base + J.group_first].culling_bone;   /* the group's first bone */
             const float* B = bones + (size_t)cb * 16;
@@ -67,7 +66,7 @@ k_geometry(const sftg_frame* __restrict__ frames, const sftg_job* __restrict__ j
         }
         ctr = xform(ctr, T); ax = xform_dir(ax, T);
         const float sxs = fsqrt(T[0] * T[0] + T[1] * T[1] + T[2] * T[2]);
-        const float rad = cl[3] * sxs;
+        const float rad = c0.w * sxs;
         ax = vnorm(ax);
         bool in = true;
 #pragma unroll
@@ -78,10 +77,10 @@ k_geometry(const sftg_frame* __restrict__ frames, const sftg_job* __restrict__ j
         const v3 vr = sub3(ctr, mk3(F->cam[0], F->cam[1], F->cam[2]));
         const float dd = fsqrt(vdot(vr, vr));
         const float dv = vdot(vr, ax);
-        const float thr = fma_(dd, cl[7], rad);
+        const float thr = fma_(dd, c1.w, rad);
         inside = in && (dv <= thr);
     }
-    const uint32_t alive = __ballot_sync(0xFFFFFFFFu, inside) & 0xFFu;
+    const uint32_t alive = __ballot_sync(0xFFFFFFFFu, inside) & 0xFFu;   /* the same in both warps */
 
     const float hw = F->hw, hh = F->hh;
     const float bias_x = hw + F->vpx, scale_y = -hh, bias_y = hh + F->vpy;
@@ -94,28 +93,31 @@ k_geometry(const sftg_frame* __restrict__ frames, const sftg_job* __restrict__ j
         const uint32_t ssi = F->ss_base + I->ss_offset + m;
         if (!((alive >> ln) & 1u)) {
             /* its records are read only where its rectangle or its clip count says so */
-            if (lane == 0) { mrect[ssi] = make_int4(1, 0, 1, 0); clip_tot[ssi] = 0; }
+            if (tt == 0) { mrect[ssi] = make_int4(1, 0, 1, 0); clip_tot[ssi] = 0; }
             continue;
         }
         const float* at = F->ml_attr + (size_t)g * 640;
         float* S = ss + (size_t)ssi * SFTG_SS_FLOATS;
-        const sftg_meshlet_info info = F->ml_info[g];
-        s_ind[warp][lane] = ((const uint4*)(F->ml_inds + (size_t)g * 512))[lane];
-        /* ---- vertices: lane and lane + 32 (5015-5124) ---- */
-#pragma unroll
-        for (int h = 0; h < 2; h++) {
-            const int v = lane + 32 * h;
+        if (warp == 0) s_ind[team][lane] = ((const uint4*)(F->ml_inds + (size_t)g * 512))[lane];
+        /* ---- vertex tt (5015-5124) ---- */
+        {
+            const int v = tt;
             const v3 p = mk3(at[v], at[64 + v], at[128 + v]);
             const v3 n = mk3(at[192 + v], at[256 + v], at[320 + v]);
+            const float tu = at[384 + v], tv = at[448 + v], tlu = at[512 + v], tlv = at[576 + v];
             v3 pw, nw;
             if (J.skinned) {
-                const uint16_t* js = F->skin_j + (size_t)info.skin_slot * 256;
-                const uint8_t* ws = F->skin_w + (size_t)info.skin_slot * 256;
+                const int slot = F->ml_info[g].skin_slot;
+                const uint16_t* js = F->skin_j + (size_t)slot * 256;
+                const uint8_t* ws = F->skin_w + (size_t)slot * 256;
                 const float inv255 = 1.f / 255.f;
                 v3 vp[4], vn[4]; float wt[4];
 #pragma unroll
                 for (int k = 0; k < 4; k++) {
-                    const float* M = bones + (size_t)js[k * 64 + v] * 16;
+                    float M[16];
+                    const float4* B = (const float4*)(bones + (size_t)js[k * 64 + v] * 16);
+#pragma unroll
+                    for (int q = 0; q < 4; q++) { const float4 r = B[q]; M[4 * q] = r.x; M[4 * q + 1] = r.y; M[4 * q + 2] = r.z; M[4 * q + 3] = r.w; }
                     wt[k] = (float)ws[k * 64 + v] * inv255;
                     vp[k] = xform(p, M); vn[k] = xform_dir(n, M);
                 }
@@ -135,32 +137,32 @@ k_geometry(const sftg_frame* __restrict__ frames, const sftg_job* __restrict__ j
             const float tz = fma_(pw.x, VP[2], fma_(pw.y, VP[6], fma_(pw.z, VP[10], VP[14])));
             const float iw = rcpr(w);
             const float sx = fma_(tx, iw * hw, bias_x), sy = fma_(ty, iw * scale_y, bias_y);
-            /* vertex-major record (sftg_types.h, SFTG_SS_*): two float4 and one float per vertex */
+            s_v[team][0][v] = tz; s_v[team][1][v] = sx; s_v[team][2][v] = sy;
+            /* vertex-major record (sftg_types.h, SFTG_SS_*): three float4 and one float per vertex */
             ((float4*)(S + SFTG_SS_A))[v] = make_float4(x86nan(sx), x86nan(sy), x86nan(iw), pw.x);
             ((float4*)(S + SFTG_SS_B))[v] = make_float4(pw.y, pw.z, nw.x, nw.y);
-            ((float4*)(S + SFTG_SS_C))[v] = make_float4(nw.z, at[384 + v], at[448 + v], at[512 + v]);
-            S[SFTG_SS_D + v] = at[576 + v];
-            s_v[warp][0][v] = tx; s_v[warp][1][v] = ty; s_v[warp][2][v] = tz; s_v[warp][3][v] = w;
-            s_v[warp][4][v] = sx; s_v[warp][5][v] = sy;
+            ((float4*)(S + SFTG_SS_C))[v] = make_float4(nw.z, tu, tv, tlu);
+            S[SFTG_SS_D + v] = tlv;
         }
-        __syncwarp();
-        /* ---- triangle batches: 4 per round, one 8-lane group each (4775-4884) ---- */
-        const uint8_t* ind = (const uint8_t*)s_ind[warp];
+        team_sync();
+        /* ---- triangle batches: 4 per round, one 8-lane group each, warp w the rounds 2w and 2w + 1 (4775-4884) ---- */
+        const uint8_t* ind = (const uint8_t*)s_ind[team];
         const int grp = lane >> 3, tl = lane & 7;
         int4 mr = make_int4(9999, -9999, 9999, -9999);
         uint32_t clips = 0;
-        for (int round = 0; round < 4; round++) {
-            const int b = round * 4 + grp;
+#pragma unroll
+        for (int round = 0; round < 2; round++) {
+            const int b = (warp * 2 + round) * 4 + grp;
             const uint32_t i0 = ind[b * 32 + tl], i1 = ind[b * 32 + 8 + tl], i2 = ind[b * 32 + 16 + tl];
             const bool valid = (int)(i0 | i1 | i2) > 0;
-            const float tz0 = s_v[warp][2][i0], tz1 = s_v[warp][2][i1], tz2 = s_v[warp][2][i2];
+            const float tz0 = s_v[team][0][i0], tz1 = s_v[team][0][i1], tz2 = s_v[team][0][i2];
             const bool ai = (tz0 >= 0.f) && (tz1 >= 0.f) && (tz2 >= 0.f);
             const bool ao = (tz0 < 0.f) && (tz1 < 0.f) && (tz2 < 0.f);
             const bool inter = valid && !(ai || ao);
             uint32_t nclip = inter ? (uint32_t)((tz0 >= 0.f) + (tz1 >= 0.f) + (tz2 >= 0.f)) : 0u;
-            const float sx0 = s_v[warp][4][i0], sy0 = s_v[warp][5][i0];
-            const float sx1 = s_v[warp][4][i1], sy1 = s_v[warp][5][i1];
-            const float sx2 = s_v[warp][4][i2], sy2 = s_v[warp][5][i2];
+            const float sx0 = s_v[team][1][i0], sy0 = s_v[team][2][i0];
+            const float sx1 = s_v[team][1][i1], sy1 = s_v[team][2][i1];
+            const float sx2 = s_v[team][1][i2], sy2 = s_v[team][2][i2];
             const float dx1 = sx1 - sx0, dy1 = sy1 - sy0, dx2 = sx2 - sx0, dy2 = sy2 - sy0;
             const int tx0 = cvtt(vmin(sx0, vmin(sx1, sx2))) >> 6, tx1 = cvtt(vmax(sx0, vmax(sx1, sx2))) >> 6;
             const int ty0 = cvtt(vmin(sy0, vmin(sy1, sy2))) >> 6, ty1 = cvtt(vmax(sy0, vmax(sy1, sy2))) >> 6;
@@ -198,8 +200,13 @@ k_geometry(const sftg_frame* __restrict__ frames, const sftg_job* __restrict__ j
             mr.w = max(mr.w, __shfl_xor_sync(0xFFFFFFFFu, mr.w, o));
             clips += __shfl_xor_sync(0xFFFFFFFFu, clips, o);
         }
-        if (lane == 0) { mrect[ssi] = mr; clip_tot[ssi] = clips; }
-        __syncwarp();
+        if (warp == 1 && lane == 0) { s_mr[team] = mr; s_clips[team] = clips; }
+        team_sync();   /* also: both warps are done with the vertices and indices */
+        if (tt == 0) {
+            const int4 o = s_mr[team];
+            mrect[ssi] = make_int4(min(mr.x, o.x), max(mr.y, o.y), min(mr.z, o.z), max(mr.w, o.w));
+            clip_tot[ssi] = clips + s_clips[team];
+        }
     }
 }
 
@@ -265,23 +272,24 @@ SFTG_D bool clip_store(const sftg_frame* F, uint32_t slot, const cvert& a, const
     return grew;
 }
 
-/* Near-plane clipping (4691-4772, 4264-4349), CLIP_MESHLETS meshlets per CTA of 16 8-lane groups, one
+/* Near-plane clipping (4691-4772, 4264-4349), `per` meshlets per CTA of 16 8-lane groups, one
  * batch of the meshlet per group and one triangle per lane; meshlets that clip nothing cost a look at
  * their count.  Slots follow the meshlet's base (an exclusive scan of the meshlets' counts), then
  * the batches before this one, then the batch's earlier triangles: the reference's order.  Bound by
  * latency: 32 records per warp, four batches at a time, with the vertices in an array indexed by
- * which of them are in front (local memory) took 24 us on the skinned 1080p frame. */
+ * which of them are in front (local memory) took 24 us on the skinned 1080p frame; four meshlets per
+ * CTA there leave most of the GPU idle while two or three of one CTA clip in turn. */
 #define CLIP_THREADS 128
 __global__ void __launch_bounds__(CLIP_THREADS)
 k_clip(const sftg_frame* __restrict__ frames, uint32_t n_views, const float* __restrict__ ss,
        const uint32_t* __restrict__ clip_cnt, const uint32_t* __restrict__ clip_tot, const uint32_t* __restrict__ clip_base,
-       sftg_clip_tri* __restrict__ clips, int4* __restrict__ clip_rect, int4* __restrict__ mrect, uint32_t n_meshlets)
+       sftg_clip_tri* __restrict__ clips, int4* __restrict__ clip_rect, int4* __restrict__ mrect, uint32_t n_meshlets, uint32_t per)
 {
     const int tid = threadIdx.x, lane = tid & 31, tl = lane & 7, gshift = lane & ~7, b = tid >> 3;
     const uint32_t gmask = 0xFFu << gshift;
-    const uint32_t m0 = blockIdx.x * CLIP_MESHLETS;
+    const uint32_t m0 = blockIdx.x * per;
     const uint32_t mine = m0 + (uint32_t)lane;
-    uint32_t pending = __ballot_sync(0xFFFFFFFFu, lane < CLIP_MESHLETS && mine < n_meshlets && clip_tot[mine] != 0);
+    uint32_t pending = __ballot_sync(0xFFFFFFFFu, lane < (int)per && mine < n_meshlets && clip_tot[mine] != 0);
     for (; pending; pending &= pending - 1) {
         const uint32_t ssi = m0 + (uint32_t)(__ffs(pending) - 1);
         /* the batch's outputs and those of the batches before it */

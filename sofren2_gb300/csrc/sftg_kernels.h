@@ -84,9 +84,14 @@ struct sftg_tile_args {
 
 __global__ void k_geometry(const sftg_frame* frames, const sftg_job* jobs, uint32_t n_jobs, float* ss, sftg_batch_rec* recs,
                            uint32_t* clip_cnt, uint32_t* clip_tot, int4* mrect);
-#define CLIP_MESHLETS 4   /* meshlets per CTA of k_clip */
+/* From this many meshlets in a batch on a geometry job is a whole group of eight: there are CTAs enough
+ * without a job per meshlet, the loads at a job's head are paid for once, and the host makes and sends an
+ * eighth of the jobs.  Kernel and whole frame, jobs of 1 / of 8: 1279x719 atrium (8089 meshlets) 38 / 41
+ * and 333 / 290 us, two views of it 54 / 76 and 906 / 847, 48 views 572 / 343 us and 13.6 / 12.2 ms;
+ * below, 743 meshlets (skinned 1080p) 26 / 35 and 337 / 346 us. */
+#define SFTG_WIDE_JOBS 4096
 __global__ void k_clip(const sftg_frame* frames, uint32_t n_views, const float* ss, const uint32_t* clip_cnt, const uint32_t* clip_tot,
-                       const uint32_t* clip_base, sftg_clip_tri* clips, int4* clip_rect, int4* mrect, uint32_t n_meshlets);
+                       const uint32_t* clip_base, sftg_clip_tri* clips, int4* clip_rect, int4* mrect, uint32_t n_meshlets, uint32_t per);
 #define SFTG_STILE 4   /* tiles per side of a super-tile (coarse binning) */
 __global__ void k_coarse(const sftg_frame* frames, const uint16_t* stile_view, const int4* mrect, uint32_t* stile_count,
                          const uint32_t* stile_start, uint32_t* stile_list);
