@@ -236,23 +236,27 @@ SFTG_D uint32_t tex_addr(const tex_level& t, int u, int v) {
     return (((vv >> 2) * t.bw + (uu >> 2)) << 4) + ((vv & 3u) << 2) + (uu & 3u);
 }
 
-/* sft__sample_tex_bilinear (5543-5660) */
-SFTG_D void sample_bilinear(const sftg_tile_args& A, int4 head, int ti, int lod, float cu, float cv, float& r, float& g, float& b) {
+/* sft__sample_tex_bilinear (5543-5660), and sft__sample_tex_nearest (5662-5729) as the bilinear of one
+ * texel: without the half-texel offset the corner is the nearest texel, and with zero fractions
+ * f00 + (f10 - f00) * 0 is f00.  One code path, because a warp's lanes often need both. */
+SFTG_D void sample_tex(const sftg_tile_args& A, int4 head, int ti, int lod, bool nearest, float cu, float cv, float& r, float& g, float& b) {
     if (ti < 0) { r = g = b = 1.f; return; }
     const tex_level t = tex_at(A, head, ti, lod);
     const int w = t.w, h = t.h;
-    const float upx = cu * (float)w - 0.5f, vpx = cv * (float)h - 0.5f;
+    const float half = nearest ? 0.f : 0.5f;
+    const float upx = cu * (float)w - half, vpx = cv * (float)h - half;
     const float uf0 = floorf(upx), vf0 = floorf(vpx);
-    const float ufr = upx - uf0, vfr = vpx - vf0;
+    const float ufr = nearest ? 0.f : upx - uf0, vfr = nearest ? 0.f : vpx - vf0;
     const int u0 = cvtt(uf0), v0 = cvtt(vf0);
     const int wm = w - 1, hm = h - 1;
     int u0w, v0w, u1, v1;
     if (t.pot) { u1 = (u0 + 1) & wm; v1 = (v0 + 1) & hm; u0w = u0 & wm; v0w = v0 & hm; }
-    else {   /* the reference has no lower clamp here (it reads outside the texture); clamp at 0 */
+    else {   /* the reference's bilinear has no lower clamp here (it reads outside the texture); clamp at 0 */
         u1 = max(0, min(u0 + 1, wm)); v1 = max(0, min(v0 + 1, hm)); u0w = max(0, min(u0, wm)); v0w = max(0, min(v0, hm));
     }
-    const uint32_t c00 = __ldg(&t.base[tex_addr(t, u0w, v0w)]), c10 = __ldg(&t.base[tex_addr(t, u1, v0w)]);
-    const uint32_t c01 = __ldg(&t.base[tex_addr(t, u0w, v1)]), c11 = __ldg(&t.base[tex_addr(t, u1, v1)]);
+    const uint32_t c00 = __ldg(&t.base[tex_addr(t, u0w, v0w)]);
+    uint32_t c10 = c00, c01 = c00, c11 = c00;
+    if (!nearest) { c10 = __ldg(&t.base[tex_addr(t, u1, v0w)]); c01 = __ldg(&t.base[tex_addr(t, u0w, v1)]); c11 = __ldg(&t.base[tex_addr(t, u1, v1)]); }
     const float i255 = 1.f / 255.f;
     float out[3];
 #pragma unroll
@@ -264,20 +268,6 @@ SFTG_D void sample_bilinear(const sftg_tile_args& A, int4 head, int ti, int lod,
         out[k] = top + (bot - top) * vfr;
     }
     r = out[0]; g = out[1]; b = out[2];
-}
-
-/* sft__sample_tex_nearest (5662-5729) */
-SFTG_D void sample_nearest(const sftg_tile_args& A, int4 head, int ti, int lod, float cu, float cv, float& r, float& g, float& b) {
-    if (ti < 0) { r = g = b = 1.f; return; }
-    const tex_level t = tex_at(A, head, ti, lod);
-    const int w = t.w, h = t.h;
-    const int u0 = cvtt(floorf(cu * (float)w)), v0 = cvtt(floorf(cv * (float)h));
-    const int wm = w - 1, hm = h - 1;
-    int uw, vw;
-    if (t.pot) { uw = u0 & wm; vw = v0 & hm; } else { uw = max(0, min(u0, wm)); vw = max(0, min(v0, hm)); }
-    const uint32_t c = __ldg(&t.base[tex_addr(t, uw, vw)]);
-    const float i255 = 1.f / 255.f;
-    r = (float)((c >> 16) & 255u) * i255; g = (float)((c >> 8) & 255u) * i255; b = (float)(c & 255u) * i255;
 }
 
 /* ---------------------------------------------------------------- raster */
@@ -582,11 +572,12 @@ SFTG_D bool over_capacity(const sftg_tile_args& A, const sftg_frame* F) {
 #define LIGHT_SLOTS (SFTG_MAX_TILE_LIGHTS * SFTG_MAX_LIGHT_PROXIES)
 
 /* A warp resolves `set` neighbouring 4x2 blocks at a time: up to max_set, fewer where a tile's
- * split leaves its 8 warps less.  Its fragments (covered pixel, distinct triangle) number at most
- * max_set * 8 * S; a chunk of 32 is closed when the next (block, triangle) pair does not fit, so
- * it holds at least 25 of them, which bounds the chunks. */
+ * split leaves its 8 warps less (at 4x sets of 8 leave the L1 60 KB instead of 92: 0.336 ms against
+ * 0.321 on the 1080p atrium, 0.161 against 0.136 at 155x106).  Its fragments (covered pixel, distinct
+ * triangle) number at most max_set * 8 * S; a chunk of 32 is closed when the next (block, triangle)
+ * pair does not fit, so it holds at least 25 of them, which bounds the chunks. */
 template <int S> struct resolve_plan {
-    static constexpr int max_set = S == 1 ? 16 : 8;
+    static constexpr int max_set = S == 1 ? 16 : S == 2 ? 8 : 4;
     static constexpr int pixels = max_set * 8, chunks = pixels * S / 25 + 2, cap = chunks * 32;
 };
 
@@ -613,7 +604,11 @@ SFTG_D float warp_max(float v) { float r; asm volatile("redux.sync.max.f32 %0, %
  * 0.172 ms, atrium 1080p 4x 0.541 -> 0.381, atrium 1279x719 1x 0.272 -> 0.103, mixed materials
  * 1333x717 2x 0.213 -> 0.143, skinned 320x180 2x 0.516 -> 0.074, a batch of 48 views 12.3 -> 8.0; with
  * the resident tables as kernel parameters, a texture's fields in two loads, a light's share of the
- * chunk's proxy filter computed once and no normals for lightmapped chunks 0.344 and 7.2.
+ * chunk's proxy filter computed once and no normals for lightmapped chunks 0.344 (4x) and 7.2.  Then
+ * one issue slot in seven went to waits for instructions and one in three to loads that missed a small
+ * L1: less code (three interpolations in one loop, one sampler, no branches in rcp and rsqrt), sets of 4
+ * blocks at 4x (46 -> 33 KB of shared memory per CTA), sets handed out to the CTA's warps and a round's
+ * places from one ballot gave 4x 0.303, 2x 0.172 -> 0.153 and 6.7 for the 48 views.
  * Sets of 16 blocks at 2x cost 3-15 %, contiguous sets per CTA at 4x 7 %.
  *
  * One (tile, part) item, run by one CTA.  The CTA makes the tile's light list and proxy cache
@@ -642,7 +637,7 @@ SFTG_D void resolve_item(const sftg_tile_args& A, uint32_t tile0, int split, boo
     __shared__ float s_vm[LIGHT_SLOTS], s_rb2[LIGHT_SLOTS], s_rbm[LIGHT_SLOTS];
     __shared__ uint16_t s_lights[SFTG_MAX_TILE_LIGHTS];
     __shared__ float4 s_lp[SFTG_MAX_TILE_LIGHTS], s_lc[SFTG_MAX_TILE_LIGHTS];   /* position with 1/r^2, colour */
-    __shared__ int s_nlights, s_odd;
+    __shared__ int s_nlights, s_odd, s_set;
     __shared__ uint8_t s_npc[SFTG_MAX_TILE_LIGHTS];
     __shared__ uint32_t s_meta[RESOLVE_WARPS][plan::cap], s_vid[RESOLVE_WARPS][plan::cap];
     __shared__ float s_acc[RESOLVE_WARPS][S > 1 ? plan::pixels * 3 : 1];
@@ -668,7 +663,7 @@ SFTG_D void resolve_item(const sftg_tile_args& A, uint32_t tile0, int split, boo
 
     if (!F->clear && over_capacity(A, F)) return;   /* the whole CTA: the caller's pixels stay for the next attempt */
     const sftg_tile_lights* TL = A.tile_lights + gtile;
-    if (tid == 0) s_odd = shadow_out != nullptr;
+    if (tid == 0) { s_odd = shadow_out != nullptr; s_set = RESOLVE_WARPS; }
     if (records) {   /* D2 and D3's selection come from the tile's record (k_tile_lights) */
         if (tid < SFTG_MAX_TILE_LIGHTS) { s_lights[tid] = TL->light[tid]; s_npc[tid] = TL->npc[tid]; }
         if (tid == 0) s_nlights = (int)TL->nlights;
@@ -770,7 +765,9 @@ SFTG_D void resolve_item(const sftg_tile_args& A, uint32_t tile0, int split, boo
     const int set = min(plan::max_set, TILE_BLOCKS / RESOLVE_WARPS / split);   /* 4, 8 or 16: split is at most 16 */
     const int bw = set >= 8 ? 4 : 2, across = 16 / bw, bh = set / bw;
     const int nsets = TILE_BLOCKS / set / split;
-    for (int q0 = warp; q0 < nsets; q0 += RESOLVE_WARPS) {
+    /* sets beyond the first go to whichever warp is free (the 48 views 7.20 -> 7.07 ms) */
+    auto next_set = [&]() { int q = 0; if (lane == 0) q = atomicAdd(&s_set, 1); return __shfl_sync(0xFFFFFFFFu, q, 0); };
+    for (int q0 = warp; q0 < nsets; q0 = next_set()) {
         const int q = S == 4 ? q0 * split + part : part * nsets + q0;
         const int X0 = tmx + (q % across) * bw * 4, Y0 = tmy + (q / across) * bh * 2;
         if (X0 >= lim_x || Y0 >= lim_y) continue;   /* whole warp */
@@ -828,18 +825,24 @@ SFTG_D void resolve_item(const sftg_tile_args& A, uint32_t tile0, int split, boo
                     hits += match;
                 }
                 /* places for the four groups' pairs; a pair does not straddle two chunks */
-                const int n = __popc(mask);
-                int at = 0;
+                const uint32_t cov = __ballot_sync(0xFFFFFFFFu, (mask >> gl) & 1u);
+                int at;
+                if ((cur & 31) + __popc(cov) <= 32) {
+                    at = cur + __popc(cov & ((1u << gshift) - 1u));
+                    cur += __popc(cov);
+                } else {
+                    at = 0;
 #pragma unroll
-                for (int g = 0; g < 4; g++) {
-                    const int ng = __shfl_sync(0xFFFFFFFFu, n, g * 8);
-                    if ((cur & 31) + ng > 32) {
-                        const int nx = (cur + 31) & ~31;
-                        if (cur + lane < nx) metas[cur + lane] = FRAG_NONE;
-                        cur = nx;
+                    for (int g = 0; g < 4; g++) {
+                        const int ng = __popc(cov & (0xFFu << (8 * g)));
+                        if ((cur & 31) + ng > 32) {
+                            const int nx = (cur + 31) & ~31;
+                            if (cur + lane < nx) metas[cur + lane] = FRAG_NONE;
+                            cur = nx;
+                        }
+                        if (g == (lane >> 3)) at = cur;
+                        cur += ng;
                     }
-                    if (g == (lane >> 3)) at = cur;
-                    cur += ng;
                 }
                 if ((mask >> gl) & 1u) {
                     const int pos = at + __popc(mask & ((1u << gl) - 1u));
@@ -887,7 +890,6 @@ SFTG_D void resolve_item(const sftg_tile_args& A, uint32_t tile0, int split, boo
             const int bl = (int)((meta >> 3) & 15u);
             const int x = X0 + (bl % bw) * 4, y = Y0 + (bl / bw) * 2;
             const int gx = x + (pl & 3), gy = y + (pl >> 2);
-            const float pxf = ((float)x + 0.5f) + (float)(pl & 3), pyf = ((float)y + 0.5f) + (float)(pl >> 2);
             tri_verts T;
             fetch_tri(A, inst, ss, clips, vid, T);
             const int4 info = __ldg((const int4*)&A.ml_info[inst[T.inst].meshlet_base + T.m]);   /* bone, skin slot, material, lightmap */
@@ -926,14 +928,15 @@ SFTG_D void resolve_item(const sftg_tile_args& A, uint32_t tile0, int split, boo
             const int fl = __ffs(mask) - 1;
             const bool ok_x = full || ((mask >> (fl ^ 1)) & 1u), ok_y = full || ((mask >> (fl ^ 4)) & 1u);
             float cu_x = 0.f, cv_x = 0.f, cu_y = 0.f, cv_y = 0.f;
-            if (__any_sync(0xFFFFFFFFu, ti >= 0 && !(ok_x && ok_y))) {
-                weights(((float)x + 0.5f) + (float)((fl ^ 1) & 3), ((float)y + 0.5f) + (float)(fl >> 2));
-                cu_x = INTERP(T.u); cv_x = INTERP(T.v);
-                weights(((float)x + 0.5f) + (float)(fl & 3), ((float)y + 0.5f) + (float)((fl ^ 4) >> 2));
-                cu_y = INTERP(T.u); cv_y = INTERP(T.v);
+            float cu = 0.f, cv = 0.f;   /* the last turn leaves the fragment's own, and its weights */
+#pragma unroll 1   /* one copy of the code: unrolled, the kernel's instruction fetches cost 4 % */
+            for (int k = __any_sync(0xFFFFFFFFu, ti >= 0 && !(ok_x && ok_y)) ? 0 : 2; k < 3; k++) {
+                const int at = k == 0 ? fl ^ 1 : k == 1 ? fl ^ 4 : pl;
+                weights(((float)x + 0.5f) + (float)(at & 3), ((float)y + 0.5f) + (float)(at >> 2));
+                cu_x = cu_y; cv_x = cv_y; cu_y = cu; cv_y = cv;
+                cu = INTERP(T.u); cv = INTERP(T.v);
             }
-            weights(pxf, pyf);
-            const float cu = INTERP(T.u), cv = INTERP(T.v), clu = INTERP(T.lu), clv = INTERP(T.lv);
+            const float clu = INTERP(T.lu), clv = INTERP(T.lv);
             const v3 P = mk3(INTERP(T.px), INTERP(T.py), INTERP(T.pz));
             /* normal and view direction: a lightmapped surface uses neither */
             const bool lm = info.w >= 0;
@@ -979,8 +982,7 @@ SFTG_D void resolve_item(const sftg_tile_args& A, uint32_t tile0, int split, boo
             float out[3];
             {
                 float tr, tg, tb;
-                if (lod > 1) sample_nearest(A, head, ti, lod, cu, cv, tr, tg, tb);
-                else sample_bilinear(A, head, ti, lod, cu, cv, tr, tg, tb);
+                sample_tex(A, head, ti, lod, lod > 1, cu, cv, tr, tg, tb);
                 out[0] = tr * ((float)((base >> 16) & 0xFF) * i255); out[1] = tg * ((float)((base >> 8) & 0xFF) * i255);
                 out[2] = tb * ((float)(base & 0xFF) * i255);
             }
@@ -990,7 +992,7 @@ SFTG_D void resolve_item(const sftg_tile_args& A, uint32_t tile0, int split, boo
                 const float sscale = ((shin + 8.f) / 8.f) * 0.04f;
                 float dif[3], spc[3] = { 0.f, 0.f, 0.f }, lms = 1.f;
                 if (lm) {
-                    sample_bilinear(A, __ldg((const int4*)&A.texs[info.w]), info.w, 0, clu, clv, dif[0], dif[1], dif[2]);
+                    sample_tex(A, __ldg((const int4*)&A.texs[info.w]), info.w, 0, false, clu, clv, dif[0], dif[1], dif[2]);
                     dif[0] = dif[0] * F->lightmap_brightness; dif[1] = dif[1] * F->lightmap_brightness; dif[2] = dif[2] * F->lightmap_brightness;
                 } else {
                     dif[0] = F->ambient[0]; dif[1] = F->ambient[1]; dif[2] = F->ambient[2];
@@ -1070,8 +1072,8 @@ SFTG_D void resolve_item(const sftg_tile_args& A, uint32_t tile0, int split, boo
                     v3 Ln = mk3(0.f, 0.f, 0.f);
                     float ndl = 0.f;
                     bool lit = false;
+                    Ln = vnorm_fast(Lr);
                     if (!lm) {
-                        Ln = vnorm_fast(Lr);
                         ndl = vmax(vdot(N, Ln), 0.f);
                         lit = (ndl > 0.f) && alive && in_tri && lighted;
                     }
@@ -1101,7 +1103,6 @@ SFTG_D void resolve_item(const sftg_tile_args& A, uint32_t tile0, int split, boo
                     }
                     float msh = 0.f;
                     if (bmask) {
-                        if (lm) Ln = vnorm_fast(Lr);
                         const float lrl = fsqrt(d2);
                         const float bk = 0.2f, b4 = 0.25f / 0.2f;
                         /* the smooth-max blend over the surviving proxies in index order */
