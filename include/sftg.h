@@ -182,7 +182,8 @@ typedef struct sftg_tuning {
                                      The only knob that is not result-neutral: sftg_autotune leaves it as set */
     int32_t raster_bands[3];      /* row bands a tile's raster is cut into at 1x, 2x, 4x, each a CTA of its own: 1, 2 or 4
                                      (at 4x at least 2); 0 = the least (default).  Apart from that a heavy tile's
-                                     payload list is cut into parts by the batch's payload counts */
+                                     payload list is cut into parts by the batch's payload counts, and the
+                                     other tiles of a batch of under 304 get up to 4 bands */
     int32_t tile_lights[3];       /* where a tile's light list and proxy selection are made at 1x, 2x, 4x: 1 = by each of
                                      its resolve CTAs, 2 = once per tile by a launch before the resolve (its CTAs read
                                      the result), 0 = 2 where the range has at least 128 tiles, else 1 (default) */

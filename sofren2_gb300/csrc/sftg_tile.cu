@@ -1241,12 +1241,23 @@ __device__ __forceinline__ uint32_t order_bucket(const sftg_frame* frames, const
     return si * ORDER_BUCKETS + (ORDER_BUCKETS - 1u - key);
 }
 
-struct band_knobs { int b[3]; };   /* tuning.raster_bands */
+struct band_knobs { int b[3], whole; };   /* tuning.raster_bands; least bands of a list in one part */
 
 /* row bands of a tile at 1x, 2x, 4x (slot si): the knob's, at 4x at least 2 (shared memory) */
-__device__ __forceinline__ uint32_t order_bands(const band_knobs& K, uint32_t si) {
-    const uint32_t b = (uint32_t)K.b[si], least = si == 2u ? 2u : 1u;
+__device__ __forceinline__ uint32_t order_bands(const band_knobs& K, uint32_t si, uint32_t parts) {
+    const uint32_t b = (uint32_t)K.b[si], l = si == 2u ? 2u : 1u, w = parts == 1u ? (uint32_t)K.whole : 1u, least = l > w ? l : w;
     return b > least ? b : least;
+}
+
+/* Least bands of the tiles whose list is not cut, for a batch of few tiles: doubled while the tiles'
+ * bands number fewer than the resident CTAs.  A short list can hold triangles that fill the tile, which
+ * rows divide without the merge that parts need: mixed materials 1333x717 2x (252 tiles, 2 bands) 0.092
+ * -> 0.070 ms, 4 bands 0.097; atrium 1280x720 2x (240 tiles) 0.162 -> 0.148; parts of 4 payloads instead
+ * 0.082, and they cost a 640x360 frame of 60 tiles 0.010 where bands cost nothing. */
+static int whole_bands(uint32_t tiles) {
+    int b = 1;
+    while (b < RASTER_BANDS && tiles * (uint32_t)b < SFTG_RASTER_CTAS) b *= 2;
+    return b;
 }
 
 /* the exclusive starts of both histograms, and the item range of every sample count */
@@ -1264,7 +1275,7 @@ __device__ __forceinline__ void order_starts(const uint32_t* h, uint32_t* base, 
 __device__ __forceinline__ void order_place(uint32_t t, uint32_t b, uint32_t count, uint32_t total, const band_knobs& K, uint32_t* cursor,
                                             uint32_t* order, sftg_raster_item* items) {
     order[atomicAdd(&cursor[b], 1u)] = t;
-    const uint32_t bands = order_bands(K, b / ORDER_BUCKETS), parts = sftg_raster_parts(count, total, 1 << (b / ORDER_BUCKETS));
+    const uint32_t parts = sftg_raster_parts(count, total, 1 << (b / ORDER_BUCKETS)), bands = order_bands(K, b / ORDER_BUCKETS, parts);
     uint32_t at = atomicAdd(&cursor[ORDER_ALL + b], bands * parts);
     for (uint32_t p = 0; p < parts; p++)
         for (uint32_t k = 0; k < bands; k++) {
@@ -1285,7 +1296,8 @@ __global__ void k_order_count(const sftg_frame* __restrict__ frames, const uint1
     if (t < n_tiles) {
         const uint32_t b = order_bucket(frames, tile_view, tile_count, t);
         atomicAdd(&h[b], 1u);
-        atomicAdd(&h[ORDER_ALL + b], order_bands(K, b / ORDER_BUCKETS) * sftg_raster_parts(tile_count[t], *total, 1 << (b / ORDER_BUCKETS)));
+        const uint32_t parts = sftg_raster_parts(tile_count[t], *total, 1 << (b / ORDER_BUCKETS));
+        atomicAdd(&h[ORDER_ALL + b], order_bands(K, b / ORDER_BUCKETS, parts) * parts);
     }
     __syncthreads();
     for (int i = threadIdx.x; i < 2 * ORDER_ALL; i += blockDim.x) if (h[i]) atomicAdd(&hist[i], h[i]);
@@ -1350,7 +1362,8 @@ k_tile_starts(const sftg_frame* __restrict__ frames, const uint16_t* __restrict_
         }
         const uint32_t b = order_bucket(frames, tile_view, tile_count, t);
         atomicAdd(&h[b], 1u);
-        atomicAdd(&h[ORDER_ALL + b], order_bands(K, b / ORDER_BUCKETS) * sftg_raster_parts(tile_count[t], all, 1 << (b / ORDER_BUCKETS)));
+        const uint32_t parts = sftg_raster_parts(tile_count[t], all, 1 << (b / ORDER_BUCKETS));
+        atomicAdd(&h[ORDER_ALL + b], order_bands(K, b / ORDER_BUCKETS, parts) * parts);
     }
     __syncthreads();
     if (tid == 0) order_starts(h, base, range);
@@ -1365,7 +1378,7 @@ bool sftg_launch_tile_starts(const sftg_frame* frames, const uint16_t* tile_view
                              uint32_t* seg_start, uint32_t* tile_count, uint32_t* tile_start, uint32_t* total, const int* bands,
                              uint32_t* order, sftg_raster_item* items, uint32_t* range, cudaStream_t st, int* launches) {
     if (n_tiles > ORDER_SMALL) return false;
-    const band_knobs K = { { bands[0], bands[1], bands[2] } };
+    const band_knobs K = { { bands[0], bands[1], bands[2] }, whole_bands(n_tiles) };
     k_tile_starts<<<1, 1024, 0, st>>>(frames, tile_view, seg_count, nseg, n_tiles, seg_start, tile_count, tile_start, total, K, order, items, range);
     *launches += 1;
     return true;
@@ -1374,7 +1387,7 @@ bool sftg_launch_tile_starts(const sftg_frame* frames, const uint16_t* tile_view
 void sftg_launch_tile_order(const sftg_frame* frames, const uint16_t* tile_view, const uint32_t* tile_count, uint32_t n_tiles,
                             const uint32_t* total, const int* bands, uint32_t* scratch, uint32_t* order, sftg_raster_item* items,
                             uint32_t* range, cudaStream_t st, int* launches) {
-    const band_knobs K = { { bands[0], bands[1], bands[2] } };
+    const band_knobs K = { { bands[0], bands[1], bands[2] }, whole_bands(n_tiles) };
     cudaMemsetAsync(scratch, 0, 2 * ORDER_ALL * sizeof(uint32_t), st);
     const uint32_t g = (n_tiles + 255) / 256;
     k_order_count<<<g, 256, 0, st>>>(frames, tile_view, tile_count, n_tiles, total, K, scratch);
@@ -1385,7 +1398,8 @@ void sftg_launch_tile_order(const sftg_frame* frames, const uint16_t* tile_view,
 
 uint32_t sftg_raster_items_max(int S, uint32_t tiles, int bands) {
     const uint32_t least = S == 4 ? 2u : 1u, b = (uint32_t)bands > least ? (uint32_t)bands : least;
-    return b * (tiles + 2u * SFTG_RASTER_CTAS);   /* parts: one per tile, and one per share of the payloads */
+    const uint32_t w = (uint32_t)whole_bands(tiles), bw = b > w ? b : w;   /* of all the batch's tiles it is no larger */
+    return bw * tiles + b * (tiles + 2u * SFTG_RASTER_CTAS);   /* uncut tiles; parts: one per tile, and one per share of the payloads */
 }
 
 /* ---------------------------------------------------------------- debug overlays

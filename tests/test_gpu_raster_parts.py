@@ -41,6 +41,31 @@ def test_parts_equal_oracle(renderer, w, h, nx, samples):
         renderer.free_scene(handle)
 
 
+@pytest.mark.parametrize("samples", [1, 2, 4])
+@pytest.mark.parametrize("w,h", [(60, 30), (150, 200), (960, 832), (1280, 1024)])
+def test_bands_of_uncut_lists_equal_oracle(renderer, w, h, samples):
+    """1 and 12 tiles (4 bands each), 195 (2), 320 (1) of short lists whose triangles fill them."""
+    sc = scenes.atrium_scene(w, h, seed=53, nx=2, nz=1, levels=1, arch_segments=2, n_tex=2, tex_size=16, lm_size=64, n_lights=2, n_chars=0,
+                             char_tex=16, floor_quads=(3, 2))
+    blob = sc.to_bytes()
+    o = Oracle(blob)
+    try:
+        ref = o.render_dump(0, samples)
+    finally:
+        o.close()
+    assert 0 < int(np.median(ref["tile_counts"])) < 32
+    handle = renderer.load_scene(blob)
+    try:
+        renderer.set_samples(samples)
+        tss, npx = runtime.scene_counts(sc)
+        for _ in range(2):
+            out = renderer.render_debug(handle, 0, tss, npx)
+        res = compare_frames(ref, out, samples, len(sc.frames[0].point_lights))
+        assert not {k: v for k, v in res.items() if k not in ("color_max_lsb", "tlas") and v != 0}, res
+    finally:
+        renderer.free_scene(handle)
+
+
 def test_order_of_many_tiles(renderer):
     h = renderer.load_scene(gc.blob("small"))
     try:
