@@ -282,12 +282,29 @@ SFTG_D bool clip_store(const sftg_frame* F, uint32_t slot, const cvert& a, const
 #define CLIP_THREADS 128
 __global__ void __launch_bounds__(CLIP_THREADS)
 k_clip(const sftg_frame* __restrict__ frames, uint32_t n_views, const float* __restrict__ ss,
-       const uint32_t* __restrict__ clip_cnt, const uint32_t* __restrict__ clip_tot, const uint32_t* __restrict__ clip_base,
-       sftg_clip_tri* __restrict__ clips, int4* __restrict__ clip_rect, int4* __restrict__ mrect, uint32_t n_meshlets, uint32_t per)
+       const uint32_t* __restrict__ clip_cnt, const uint32_t* __restrict__ clip_tot, uint32_t* clip_base,
+       sftg_clip_tri* __restrict__ clips, int4* __restrict__ clip_rect, int4* __restrict__ mrect, uint32_t n_meshlets, uint32_t per,
+       uint32_t* __restrict__ total)
 {
     const int tid = threadIdx.x, lane = tid & 31, tl = lane & 7, gshift = lane & ~7, b = tid >> 3;
     const uint32_t gmask = 0xFFu << gshift;
     const uint32_t m0 = blockIdx.x * per;
+    uint32_t base0 = 0;
+    if (total) {   /* one meshlet per CTA: its base is the sum of the counts before it */
+        __shared__ uint32_t s_sum[CLIP_THREADS / 32];
+        uint32_t sum = 0;
+#pragma unroll 4
+        for (uint32_t i = tid; i < m0; i += CLIP_THREADS) sum += clip_tot[i];
+        sum = __reduce_add_sync(0xFFFFFFFFu, sum);
+        if (lane == 0) s_sum[tid >> 5] = sum;
+        __syncthreads();
+#pragma unroll
+        for (int w = 0; w < CLIP_THREADS / 32; w++) base0 += s_sum[w];
+        if (tid == 0) {
+            clip_base[m0] = base0;
+            if (m0 + 1u == n_meshlets) *total = base0 + clip_tot[m0];
+        }
+    }
     const uint32_t mine = m0 + (uint32_t)lane;
     uint32_t pending = __ballot_sync(0xFFFFFFFFu, lane < (int)per && mine < n_meshlets && clip_tot[mine] != 0);
     for (; pending; pending &= pending - 1) {
@@ -347,7 +364,7 @@ k_clip(const sftg_frame* __restrict__ frames, uint32_t n_views, const float* __r
             const int t = __shfl_up_sync(gmask, incl, o, 8);
             if (tl >= o) incl += t;
         }
-        const uint32_t slot = clip_base[ssi] + first + (uint32_t)(incl - nc);
+        const uint32_t slot = (total ? base0 : clip_base[ssi]) + first + (uint32_t)(incl - nc);
         int4 mr = make_int4(0x7FFFFFFF, (int)0x80000000, 0x7FFFFFFF, (int)0x80000000);
         bool grew = false;
         if (nc == 1) {

@@ -91,7 +91,8 @@ __global__ void k_geometry(const sftg_frame* frames, const sftg_job* jobs, uint3
  * below, 743 meshlets (skinned 1080p) 26 / 35 and 337 / 346 us. */
 #define SFTG_WIDE_JOBS 4096
 __global__ void k_clip(const sftg_frame* frames, uint32_t n_views, const float* ss, const uint32_t* clip_cnt, const uint32_t* clip_tot,
-                       const uint32_t* clip_base, sftg_clip_tri* clips, int4* clip_rect, int4* mrect, uint32_t n_meshlets, uint32_t per);
+                       uint32_t* clip_base, sftg_clip_tri* clips, int4* clip_rect, int4* mrect, uint32_t n_meshlets, uint32_t per,
+                       uint32_t* total);
 #define SFTG_STILE 4   /* tiles per side of a super-tile (coarse binning) */
 __global__ void k_coarse(const sftg_frame* frames, const uint16_t* stile_view, const int4* mrect, uint32_t* stile_count,
                          const uint32_t* stile_start, uint32_t* stile_list);

@@ -10,7 +10,8 @@ from sofren2_gb300 import runtime, scenes
 
 pytestmark = pytest.mark.gpu
 
-WIDE = 4096   # SFTG_WIDE_JOBS
+WIDE = 4096     # SFTG_WIDE_JOBS
+SUMMED = 2048   # most meshlets whose clip slots need no scan
 
 
 def _scene(big):
@@ -41,9 +42,9 @@ def test_jobs_equal_oracle(renderer, big):
             out = renderer.render_debug(handle, 0, tss, npx)
             res = compare_frames(ref, out, 2, len(sc.frames[0].point_lights))
             assert not {k: v for k, v in res.items() if k not in ("color_max_lsb", "tlas") and v != 0}, (width, res)
-            if not big:     # batches just under and over the line
+            if not big:     # batches just under and over the lines
                 alone = renderer.render(handle, 0)
-                for n in ((WIDE - 1) // tss, (WIDE - 1) // tss + 1):
+                for n in (SUMMED // tss, SUMMED // tss + 1, (WIDE - 1) // tss, (WIDE - 1) // tss + 1):
                     for c in renderer.render_batch([(handle, 0, 2)] * n, [None] * n):
                         assert np.array_equal(c, alone), (width, n)
     finally:
