@@ -45,3 +45,32 @@ def test_light_vis_equals_oracle(renderer, slices, bands, lights, chars, lo, hi)
         renderer.free_scene(handle)
     assert np.array_equal(out["light_vis"].reshape(-1, 64)[:, :lights], want)
     assert np.array_equal(out["color"], ref["color"])
+
+
+@pytest.mark.parametrize("balls", [0, 1, 3, 4, 5, 20, 33, 60])
+def test_tlas_sizes_equal_oracle(renderer, balls):
+    """TLAS walks of one node up to the 64 instances a frame can hold, four nodes to a step."""
+    sc = scenes.skinned_characters_scene(160, 96, seed=72, n_chars=3, n_lights=5, tex_size=16, ground_quads=6)
+    rng = np.random.default_rng(balls)
+    ball = sc.add_model(scenes.Model([scenes.build_meshlets(scenes.uv_sphere(10, 6, 0.5))], [0]))
+    for f in sc.frames:
+        for _ in range(balls):
+            t = scenes.mat_mul(scenes.mat_scale(np.float32(rng.uniform(0.3, 1.2))),
+                               scenes.mat_translate(*[np.float32(v) for v in (rng.uniform(-5, 5), rng.uniform(1.0, 4.5), rng.uniform(3, 10))]))
+            f.instances.append((ball, t, None))
+        assert len(f.instances) <= 64
+    blob = sc.to_bytes()
+    o = Oracle(blob)
+    try:
+        ref = o.render_dump(0, 2)
+    finally:
+        o.close()
+    handle = renderer.load_scene(blob)
+    try:
+        renderer.set_samples(2)
+        tss, npx = runtime.scene_counts(sc)
+        out = renderer.render_debug(handle, 0, tss, npx)
+    finally:
+        renderer.free_scene(handle)
+    assert np.array_equal(out["light_vis"].reshape(-1, 64)[:, :5], ref["light_vis"].reshape(-1, 64)[:, :5])
+    assert np.array_equal(out["color"], ref["color"])
