@@ -177,13 +177,26 @@ SFTG_D bool tri_setup_one(float sx0, float sy0, float iw0, float sx1, float sy1,
     return true;
 }
 
+/* the least of three, NaN if one is: one instruction */
+SFTG_D float min3(float a, float b, float c) { float r; asm("min.NaN.f32 %0, %1, %2, %3;" : "=f"(r) : "f"(a), "f"(b), "f"(c)); return r; }
+/* two floats in a register pair: one instruction adds both, each rounded as on its own */
+typedef unsigned long long f32x2;
+SFTG_D f32x2 pack2(float a, float b) { f32x2 r; asm("mov.b64 %0, {%1, %2};" : "=l"(r) : "f"(a), "f"(b)); return r; }
+SFTG_D float lo2(f32x2 v) { float a, b; asm("mov.b64 {%0, %1}, %2;" : "=f"(a), "=f"(b) : "l"(v)); return a; }
+SFTG_D float hi2(f32x2 v) { float a, b; asm("mov.b64 {%0, %1}, %2;" : "=f"(a), "=f"(b) : "l"(v)); return b; }
+SFTG_D f32x2 add2(f32x2 a, f32x2 b) { f32x2 r; asm("add.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(a), "l"(b)); return r; }
+
 /* The incremental edge walk of one triangle's rows y0..y1 (5345-5497) by a group of 8 * S lanes: lane
  * (sample << 3 | l) owns one sample of pixel column l of every aligned 8-pixel chunk.  All lanes of a
  * column perform exactly the reference's adds of the pixel (row start + B per row, + 8A per chunk),
  * then each its own sample's offset.  Bound by issue: with 8 lanes per triangle and the samples in
  * turn, the four groups of a warp diverged over their triangles' sizes (17 of 32 threads) and the 4x
  * raster of the 1080p atrium took 0.287 ms; a warp per triangle 0.258, and 0.228 with slabs of 8 rows,
- * which now balance well enough (4 rows 0.251). */
+ * which now balance well enough (4 rows 0.251).  Of 50 instructions per step of a chunk: the trivial
+ * triangles in a loop of their own, the least of the three edges instead of three comparisons, a vote
+ * instead of a ballot and the step's adds in pairs took it to 0.197 (1279x719 1x 0.074 -> 0.062, skinned
+ * 1080p 2x 0.090 -> 0.080, 48 views 3.41 -> 3.06); the row's adds in pairs too cost registers (2x 80
+ * instead of 64, 48 views 3.9). */
 template <int S>
 SFTG_D void tri_raster(const tri_setup& T, int y0, int y1, int lane, uint32_t gmask, int tmx, int ky0, unsigned long long* keys) {
     const int l = lane & 7, smp = (lane >> 3) & (S - 1);
@@ -201,20 +214,35 @@ SFTG_D void tri_raster(const tri_setup& T, int y0, int y1, int lane, uint32_t gm
     const uint32_t order = T.order;
     unsigned long long* const kp = keys + smp * raster_plan<S>::plane + (T.ax0 - tmx) + l;   /* keys hold the band's rows from ky0 */
     const int width = T.ax1 - T.ax0;
-    for (int y = y0; y <= y1; y++) {
-        float e0 = e0r, e1 = e1r, e2 = e2r, z = zr;
-        unsigned long long* k = kp + (y - ky0) * SFTG_TILE;
-        for (int x = 0; x < width; x += 8, k += 8) {
-            if (T.trivial) {
+    if (T.trivial) {
+        for (int y = y0; y <= y1; y++) {
+            float z = zr;
+            unsigned long long* k = kp + (y - ky0) * SFTG_TILE;
+#pragma unroll 1
+            for (int x = 0; x < width; x += 8, k += 8) {
                 const float zs = (S > 1) ? z + dz : z;
                 if (zs > 0.f) atomicMax(k, zkey(zs, order));
-            } else if (S == 1) {
-                if (e0 >= 0.f && e1 >= 0.f && e2 >= 0.f && z > 0.f) atomicMax(k, zkey(z, order));
-            } else if (__ballot_sync(gmask, e0 >= np0 && e1 >= np1 && e2 >= np2)) {
-                const float a = e0 + de0, b = e1 + de1, c = e2 + de2, zs = z + dz;
-                if (a >= 0.f && b >= 0.f && c >= 0.f && zs > 0.f) atomicMax(k, zkey(zs, order));
+                z = z + zc;
             }
-            e0 = e0 + a0c; e1 = e1 + a1c; e2 = e2 + a2c; z = z + zc;
+            zr = zr + T.dzdy;
+        }
+        return;
+    }
+    const f32x2 xA = pack2(a0c, a1c), xB = pack2(a2c, zc);
+    unsigned long long* krow = kp + (y0 - ky0) * SFTG_TILE;
+    for (int y = y0; y <= y1; y++, krow += SFTG_TILE) {
+        f32x2 eA = pack2(e0r, e1r), eB = pack2(e2r, zr);
+        unsigned long long* k = krow;
+#pragma unroll 1
+        for (int x = 0; x < width; x += 8, k += 8) {
+            const float e0 = lo2(eA), e1 = hi2(eA), e2 = lo2(eB), z = hi2(eB);
+            if (S == 1) {
+                if (min3(e0, e1, e2) >= 0.f && z > 0.f) atomicMax(k, zkey(z, order));
+            } else if (__any_sync(gmask, e0 >= np0 && e1 >= np1 && e2 >= np2)) {
+                const float a = e0 + de0, b = e1 + de1, c = e2 + de2, zs = z + dz;
+                if (min3(a, b, c) >= 0.f && zs > 0.f) atomicMax(k, zkey(zs, order));
+            }
+            eA = add2(eA, xA); eB = add2(eB, xB);
         }
         e0r = e0r + T.B[0]; e1r = e1r + T.B[1]; e2r = e2r + T.B[2]; zr = zr + T.dzdy;
     }
