@@ -636,7 +636,8 @@ SFTG_D float warp_max(float v) { float r; asm volatile("redux.sync.max.f32 %0, %
  * one issue slot in seven went to waits for instructions and one in three to loads that missed a small
  * L1: less code (three interpolations in one loop, one sampler, no branches in rcp and rsqrt), sets of 4
  * blocks at 4x (46 -> 33 KB of shared memory per CTA), sets handed out to the CTA's warps and a round's
- * places from one ballot gave 4x 0.303, 2x 0.172 -> 0.153 and 6.7 for the 48 views.
+ * places from one ballot gave 4x 0.303, 2x 0.172 -> 0.160 and 6.7 for the 48 views; a copy of the shading
+ * of its own for `full` 2x 0.151, 6.5 and mixed materials 0.137 -> 0.131.
  * Sets of 16 blocks at 2x cost 3-15 %, contiguous sets per CTA at 4x 7 %.
  *
  * One (tile, part) item, run by one CTA.  The CTA makes the tile's light list and proxy cache
@@ -654,6 +655,7 @@ SFTG_D float warp_max(float v) { float r; asm volatile("redux.sync.max.f32 %0, %
  * covered pixel's zero attenuation meets a value that is not finite (a light's colour, a proxy of
  * zero size, an interpolated position): such chunks are shaded again 8 lanes per pair, the
  * uncovered pixels among them, as the reference does (`full` below). */
+template <bool B> struct flag_t { static constexpr bool value = B; };
 template <int S>
 SFTG_D void resolve_item(const sftg_tile_args& A, uint32_t tile0, int split, bool records, uint32_t item)
 {
@@ -888,9 +890,11 @@ SFTG_D void resolve_item(const sftg_tile_args& A, uint32_t tile0, int split, boo
         __syncwarp();
 
         /* ---------------- shade ---------------- */
-        bool full = s_odd != 0;   /* 8 lanes per pair, uncovered pixels among them */
-        int pass = 0;             /* with `full`: which four of the chunk's pairs */
-        for (int c0 = 0; c0 < cur; ) {
+        /* One chunk; with `full` four of its pairs, 8 lanes each, uncovered pixels among them.  True where it has
+         * to be called again: with `full`, or for the next four pairs.  Two copies of the code, one of which hardly
+         * ever runs. */
+        auto chunk = [&](auto FULL, int c0, int pass) -> bool {
+            constexpr bool full = decltype(FULL)::value;
             uint32_t meta = metas[c0 + lane];
             uint32_t vid;
             int start, end, pl, npass = 1;
@@ -974,7 +978,7 @@ SFTG_D void resolve_item(const sftg_tile_args& A, uint32_t tile0, int split, boo
                 V = vnorm_fast(sub3(mk3(F->cam[0], F->cam[1], F->cam[2]), P));
             }
 #undef INTERP
-            if (!full && __any_sync(0xFFFFFFFFu, !(fabsf(P.x) + fabsf(P.y) + fabsf(P.z) <= 1e15f))) { full = true; continue; }
+            if (!full && __any_sync(0xFFFFFFFFu, !(fabsf(P.x) + fabsf(P.y) + fabsf(P.z) <= 1e15f))) return true;
             bool wire = false;
             if (F->debug_mode == 1) {   /* wireframe view (6645-6671): edges where a barycentric is under its screen width */
                 const float dbu_dx = (0.f - dy2) * idet, dbu_dy = dx2 * idet;
@@ -1210,8 +1214,12 @@ SFTG_D void resolve_item(const sftg_tile_args& A, uint32_t tile0, int split, boo
                     __syncwarp();
                 }
             }
-            if (!full || ++pass >= npass) { c0 += 32; pass = 0; full = s_odd != 0; }
-        }
+            return full && pass + 1 < npass;
+        };
+        const bool odd = s_odd != 0;
+        for (int c0 = 0; c0 < cur; c0 += 32)
+            if (odd || chunk(flag_t<false>(), c0, 0))
+                for (int pass = 0; chunk(flag_t<true>(), c0, pass); pass++) { }
 
         /* ---------------- store ---------------- */
         if (S > 1) {
