@@ -172,8 +172,8 @@ int sftg_light_vis_noalloc(sftg_ctx* ctx, const sftg_frame_desc* frame, uint8_t*
  * the 64x64 tile stays fixed here too, because the per-tile payload lists are part of the
  * render path's observable output). */
 typedef struct sftg_tuning {
-    int32_t resolve_split[3];     /* most resolve CTAs per 64x64 tile at 1x, 2x, 4x: 1, 2, 4, 8 or 16 (default 16); 8 and
-                                     16 are halved, down to 4, where the tiles alone fill the GPU */
+    int32_t resolve_split[3];     /* most resolve CTAs per 64x64 tile at 1x, 2x, 4x: 1, 2, 4, 8 or 16 (default 16); 4
+                                     to 16 are halved, down to 2, where the tiles alone fill the GPU */
     int32_t raster_slab_rows[3];  /* rows per triangle a raster group walks at a time at 1x, 2x, 4x: 4..64 (default 8) */
     int32_t geom_job_width;       /* meshlets per geometry job: 1..8 (default 1); 8, the reference's, from 4096 meshlets
                                      in a batch on */

@@ -1506,20 +1506,20 @@ int sftg_raster_bands(void) { return RASTER_BANDS; }
 
 /* Resolve CTAs per tile for a launch over `tiles` tiles in all: the knob's number, halved down to 4
  * while the launch would exceed 4096 CTAs, about 7 waves of the 152 SMs x 4 resident ones.  Fewer
- * tiles want the 16 (skinned 320x180 2x, 15 tiles: 0.074 ms against 0.139 with 8; atrium 1279x719
- * 1x, 240 tiles: 0.103 against 0.112); with more, a CTA's light list and proxy cache should serve
- * more blocks (1080p, 510 tiles: 0.172 ms with 8, 0.200 with 16 at 2x, 0.381 and 0.404 at 4x; 48
- * views, 16000 tiles: 8.05 ms with 4, 8.12 with 8, 9.03 with 16).  Below 4 a warp has several sets
- * to itself and the tail grows (1080p 2x 0.249 ms with 2). */
+ * tiles want the 16 (skinned 320x180 2x, 15 tiles: 0.063 ms against 0.115 with 8; static 640x360 1x, 60
+ * tiles: 0.014 against 0.018; atrium 1279x719 1x, 240 tiles: 0.098 against 0.100); with more, a CTA's
+ * light list and proxy cache should serve more blocks (1080p, 510 tiles: 0.150 ms with 8, 0.186 with 16
+ * at 2x, 0.309 and 0.321 at 4x).  Below 4 the tail grows (1080p 2x 0.184 ms with 2), except where the
+ * tiles alone are many waves: 48 views, 16000 tiles: 6.39 ms with 2, 6.54 with 4, 6.86 with 8, 7.77 with 16. */
 int sftg_resolve_split(int knob, uint32_t tiles) {
     while (knob > 4 && (uint64_t)tiles * (uint32_t)knob > 4096u) knob /= 2;
-    return knob;
+    return knob == 4 && tiles > 4096u ? 2 : knob;
 }
 
 /* Whether a range's light lists and proxy selections are made once per tile (k_tile_lights) or by
  * each of its resolve CTAs: from 128 tiles on, the selections saved outweigh one more launch on the
- * critical path (240 tiles 1x 0.103 against 0.111 ms, 510 tiles 4x 0.381 against 0.406; 60 tiles
- * 0.0225 against 0.0205). */
+ * critical path (510 tiles 4x 0.307 against 0.321 ms, 48 views 6.86 against 7.18, both at 8 CTAs per tile;
+ * 240 tiles 1x level; 60 tiles 0.016 against 0.013). */
 bool sftg_resolve_records(int knob, uint32_t tiles) { return knob == 2 || (knob == 0 && tiles >= 128u); }
 
 cudaError_t sftg_tile_configure(int max_dynamic_smem) {
