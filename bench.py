@@ -137,13 +137,12 @@ class ClockSampler:
 # profiles/k_resolve_*.md, same kernel code as the library's): DRAM bytes (dram__bytes_read.sum +
 # dram__bytes_write.sum), warp instructions issued (smsp__inst_executed.sum), and the issue-active
 # and FMA-pipe fractions ncu measured over the kernel's active cycles.
-RESOLVE_PROFILE = {
-    "skinned_1080p_2xmsaa": {"traffic": 38166528 + 65792, "instructions": 150347274, "issue_active": 0.599, "fma_pipe": 0.223,
+RESOLVE_PROFILE = {   # at 1080p the phase is k_tile_lights, then k_resolve
+    "skinned_1080p_2xmsaa": {"traffic": 38249472 + 55552 + 35328, "instructions": 121132366 + 460402, "issue_active": 0.642, "fma_pipe": 0.227,
                              "profile": "profiles/k_resolve_skinned_1080p_2x.md"},
-    # the resolve phase here is k_tile_lights (1528470 instructions, no DRAM traffic to speak of) then k_resolve<4>
-    "atrium_1080p_4xmsaa": {"traffic": 75378432 + 3088384 + 36352, "instructions": 360592456 + 1528470, "issue_active": 0.588,
-                            "fma_pipe": 0.204, "profile": "profiles/k_resolve_atrium_1080p_4x.md"},
-    "static_640x360_1x": {"traffic": 2486528, "instructions": 5135702, "issue_active": 0.312, "fma_pipe": 0.072,
+    "atrium_1080p_4xmsaa": {"traffic": 78059264 + 2968064 + 36352, "instructions": 240482344 + 1528470, "issue_active": 0.685,
+                            "fma_pipe": 0.248, "profile": "profiles/k_resolve_atrium_1080p_4x.md"},
+    "static_640x360_1x": {"traffic": 2480128, "instructions": 5068237, "issue_active": 0.377, "fma_pipe": 0.078,
                           "profile": "profiles/k_resolve_static_640x360_1x.md"},
 }
 
