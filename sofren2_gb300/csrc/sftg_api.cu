@@ -12,11 +12,13 @@
  *   2. k_occl_*           light visibility of every shadow proxy (8163-8280), on a second
  *                         stream beside steps 3-5, joined before the resolve
  *   3. k_geometry         cull, skin, transform, project, batch setup (4901-5145)
- *   4. scan + k_clip      near-plane clipping in emission order (4691-4772)
- *   5. k_bin (count), scan, k_bin (write), tile order   per-tile payload lists (4619-4688)
+ *   4. k_clip             near-plane clipping in emission order (4691-4772), after a scan of the clip
+ *                         counts where the meshlets are many
+ *   5. k_bin (count), k_tile_starts (offsets, tile order, raster items), k_bin (write)
+ *                         per-tile payload lists (4619-4688)
  *   6. k_raster, k_resolve  per-tile raster into a shared-memory visibility buffer, then
  *                         the resolve, several CTAs per tile (6756-6813)
- *   7. D2H of the colour buffer into the caller's pitch
+ *   7. D2H of the colour buffer into the caller's pitch, where the resolve could not write it there
  */
 #include <cuda_runtime.h>
 #include <stdarg.h>

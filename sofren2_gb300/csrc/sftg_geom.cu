@@ -8,8 +8,9 @@
  *               up eight batches at a time (sft__geom_setup_and_bin_batch, 4775-4884): one
  *               8-lane group per batch, shuffles build the batch's tile rectangle and lane mask.
  *   k_clip      near-plane clipping of straddling triangles (4691-4772, 4264-4381); clip
- *               slots come from an exclusive scan of the meshlets' clip counts, which numbers
- *               them in the reference's single-worker emission order.
+ *               slots come from an exclusive scan of the meshlets' clip counts (or, of few
+ *               meshlets, each CTA's own sum), which numbers them in the reference's
+ *               single-worker emission order.
  *   k_coarse    one CTA per super-tile (4 x 4 tiles) lists, in slot order, the meshlets of its
  *               view whose tile rectangle overlaps it; run once to count and once to write.
  *   k_bin       one or more CTAs per tile build that tile's payload list in the reference's order

@@ -11,7 +11,7 @@
  * where order = list position * 8 + lane; only z > 0 ever wins (the buffer starts at 0).
  * Coverage and z are replayed bit-exactly: a group of 8 * S threads takes one triangle's rows, a thread
  * one sample of a pixel column of every aligned 8-pixel chunk (tri_raster), with the reference's
- * trivial-accept / AA guard-band choices; the AA chunk skip is a group ballot.  The decoded visibility buffer
+ * trivial-accept / AA guard-band choices; the AA chunk skip is a group vote.  The decoded visibility buffer
  * (depth, vid) goes to global memory, where it stays L2-resident, with the tile's depth range.
  *
  * k_resolve: 1 to 16 CTAs per tile (sftg_resolve_split), each a share of its 4x2 blocks (the
