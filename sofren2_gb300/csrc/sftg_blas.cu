@@ -31,6 +31,7 @@
  */
 #include "sftg_types.h"
 #include "sftg_kernels.h"
+#include "sftg_walk.h"
 #include "sftg_blas_plan.h"
 #include <vector>
 #include <cstring>
@@ -933,7 +934,7 @@ __global__ void k_blas_walk_forms(const sftg_bvh_node* __restrict__ nodes, uint3
     const uint32_t c = i & 7u;
     sftg_wslot s;
     for (int a = 0; a < 3; a++) { s.mn[a] = nd->mn[a][c]; s.mx[a] = nd->mx[a][c]; }
-    s.child = nd->child[c];
+    s.child = sftg_walk_child(nd, c, count);
     s.flags = (nd->leaf ? 1u : 0u) | (c < nd->count ? 2u : 0u);
     sftg_wtri t;
     for (int a = 0; a < 3; a++) t.v0[a] = t.e1[a] = t.e2[a] = 0.f;

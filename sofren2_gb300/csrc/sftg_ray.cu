@@ -19,6 +19,7 @@
  */
 #include "sftg_types.h"
 #include "sftg_kernels.h"
+#include "sftg_walk.h"
 
 #define RAY_STACK 128
 #define RAY_EPS 1e-6f
@@ -271,7 +272,7 @@ k_ray_records(const sftg_ray* __restrict__ rays, uint32_t n, const sftg_model* _
  * nodes): 250 us with 8 lanes per ray, one node per step, now 115. */
 #define WIDE_STACK 384
 
-struct wide_entry { uint32_t id; float tmin, t; };   /* node, or triangle place | 0x80000000 with its distance */
+struct wide_entry { uint32_t id; float tmin, t; };   /* node, or triangle place | SFTG_WALK_TRI with its distance */
 
 __global__ void __launch_bounds__(RAY_WARPS * 32)
 k_ray_wide(const sftg_ray* __restrict__ rays, uint32_t n, const sftg_model* __restrict__ models, uint32_t n_models,
@@ -287,6 +288,10 @@ k_ray_wide(const sftg_ray* __restrict__ rays, uint32_t n, const sftg_model* __re
         return;
     }
     const sftg_model M = models[R.model];
+    if (M.blas_root >= M.blas_count) {   /* a caller's; a child outside the tree is found when it is taken */
+        if (lane == 0) store_hit(R, false, true, 0.f, nullptr, hits + k);
+        return;
+    }
     const ray_ms r = ray_setup(R);
     float lmax = __fdiv_rn(R.max_dist, r.inv_scale), win_t = 0.f;
     const sftg_wslot* nodes = wslots + (size_t)M.blas_base * 8;
@@ -304,7 +309,7 @@ k_ray_wide(const sftg_ray* __restrict__ rays, uint32_t n, const sftg_model* __re
         wide_entry e{ 0u, 0.f, 0.f };
         const bool seen = top - 1 - lane >= 0;
         if (seen) e = stack[top - 1 - lane];
-        const bool tri = (e.id & 0x80000000u) != 0;
+        const bool tri = (e.id & SFTG_WALK_TRI) != 0;
         const bool live = seen && e.tmin < lmax && (!tri || e.t < lmax);
         uint32_t node_m = __ballot_sync(ALL, live && !tri);
         const uint32_t tri_m = __ballot_sync(ALL, live && tri);
@@ -314,7 +319,7 @@ k_ray_wide(const sftg_ray* __restrict__ rays, uint32_t n, const sftg_model* __re
                 const int s = __ffs(c) - 1;
                 const float tmin_s = __shfl_sync(ALL, e.tmin, s), t_s = __shfl_sync(ALL, e.t, s);
                 const uint32_t id_s = __shfl_sync(ALL, e.id, s);
-                if (tmin_s < lmax && t_s < lmax) { lmax = win_t = t_s; win = id_s & 0x7FFFFFFFu; hit = true; }
+                if (tmin_s < lmax && t_s < lmax) { lmax = win_t = t_s; win = id_s & ~SFTG_WALK_TRI; hit = true; }
             }
             top = first_node < 32 ? top - first_node : max(0, top - 32);
             __syncwarp();
@@ -357,7 +362,7 @@ k_ray_wide(const sftg_ray* __restrict__ rays, uint32_t n, const sftg_model* __re
             const uint32_t mine = (m >> (sub * 8)) & 0xFFu;
             const int under = sub < 3 ? __popc(m >> (sub * 8 + 8)) : 0;
             const int rank = leaf ? __popc(mine >> (gl + 1)) : __popc(mine & ((1u << gl) - 1u));
-            stack[below + under + rank] = leaf ? wide_entry{ 0x80000000u | place, tmin, t }
+            stack[below + under + rank] = leaf ? wide_entry{ SFTG_WALK_TRI | place, tmin, t }
                                                : wide_entry{ __float_as_uint(mn.w), nested ? tmin : far, 0.f };
         }
         top = below + outs;

@@ -1,0 +1,50 @@
+"""Ray queries against trees that a caller gave: a node index outside the tree marks the record of
+every walk that comes to it with hit 2, and both walks (a ray of many, a warp for one of few) give the
+same records."""
+import numpy as np
+import pytest
+
+import caller_trees as ct
+import golden_cases as gc
+from sofren2_gb300 import scenes
+
+pytestmark = pytest.mark.gpu
+
+
+@pytest.fixture(scope="module")
+def atrium(renderer):
+    """The scene's handle, its meshes and rays, and an intact copy of its tree behind it in the pool."""
+    h = renderer.load_scene(gc.blob("atrium_small"))
+    sc = gc.scene("atrium_small")
+    yield h, sc.models[0].meshes, scenes.ray_batch(sc, 4000, seed=902)
+    renderer.free_scene(h)
+
+
+@pytest.mark.parametrize("past", [0, 1, 5, ct.TRI - 1, ct.TRI, ct.TRI | 4, ct.NONE - 1, ct.NONE])
+def test_root_outside_the_tree(renderer, atrium, past):
+    h, meshes, rays = atrium
+    nodes, root = ct.built(renderer, h)
+    bad = len(nodes) + past if past < 6 else past
+    r = rays[:600].copy()
+    r["model"] = ct.upload(renderer, meshes, nodes, bad)
+    ct.upload(renderer, meshes, nodes, root)
+    many, few = ct.cast_both(renderer, r)
+    assert (few["hit"] == 2).all() and many.tobytes() == few.tobytes()
+    assert ct.cast(renderer, r)[0] != 0
+
+
+@pytest.mark.parametrize("past", [0, 1, 5, ct.TRI - 1, ct.TRI, ct.TRI | 4, ct.NONE - 1])
+def test_child_outside_the_tree(renderer, atrium, past):
+    """One slot of the root, around everything, with a child that is no node."""
+    h, meshes, rays = atrium
+    nodes, root = ct.built(renderer, h)
+    nodes = nodes[:9].copy()
+    nodes[0]["mn"], nodes[0]["mx"], nodes[0]["child"] = -1e4, 1e4, ct.NONE
+    nodes[0]["child"][0] = 9 + past if past < 6 else past
+    nodes[0]["count"], nodes[0]["leaf"] = 1, 0
+    r = rays[:600].copy()
+    r["max_dist"] = 1e3
+    r["model"] = ct.upload(renderer, meshes, nodes, 0)
+    ct.upload(renderer, meshes, ct.built(renderer, h)[0], root)
+    many, few = ct.cast_both(renderer, r)
+    assert (few["hit"] == 2).all() and many.tobytes() == few.tobytes()
