@@ -51,7 +51,7 @@ SFTG_D void view_look_at(v3 pos, v3 target, v3 up, float* m) {
 }
 
 /* status bits */
-#define OCC_STACK_OVERFLOW 1u
+#define OCC_STACK_OVERFLOW 1u     /* also: a node index outside its tree */
 #define OCC_UNDEFINED_FRUSTUM 2u
 #define OCC_PAIR_OVERFLOW 4u
 
@@ -186,6 +186,10 @@ k_occl_tlas(const sftg_frame* __restrict__ frames, const uint16_t* __restrict__ 
     if (!packet_frustum(x, y, z, am, lpos, L.radius, lane, plane) && lane == 0) atomicOr(status, OCC_UNDEFINED_FRUSTUM);
     if (lane < 6) { P->f[lane] = plane; s_f[warp][lane] = plane; }
     if (F->tlas_count == 0) return;
+    if (F->tlas_root >= F->tlas_count) {   /* children are checked where they are pushed */
+        if (lane == 0) atomicOr(status, OCC_STACK_OVERFLOW);
+        return;
+    }
     int top = 1;
     if (lane == 0) s_stack[warp][0] = F->tlas_root;
     __syncwarp();
@@ -453,6 +457,10 @@ k_occl_blas_expand(const sftg_frame* __restrict__ frames, const uint16_t* __rest
         if (known == P->active) continue;            /* every ray already blocked */
         const sftg_inst* I = &F->inst[pr.y];
         const sftg_model Md = F->models[I->model];
+        if (Md.blas_root >= Md.blas_count) {   /* a caller's tree */
+            if (lane == 0) atomicOr(status, OCC_STACK_OVERFLOW);
+            continue;
+        }
         occ_walk w;
         occ_pair_setup(I, P, lane, w, s_f[warp]);
         const uint32_t sat = occ_walk_from<true>(F, Md, w, s_f[warp], known, Md.blas_root,
