@@ -224,8 +224,8 @@ k_ray_walks(const sftg_ray* __restrict__ rays, uint32_t n, const sftg_model* __r
             }
             /* slot order against the running limit; a box test that passed with the limit at node entry is
              * re-checked with the current one */
-            const uint32_t bads = __ballot_sync(ALL, bad) >> first & 0xFFu;
-            uint32_t c = bads ? 0u : __ballot_sync(ALL, ok) >> first & 0xFFu;
+            const uint32_t bads = __ballot_sync(ALL, bad) >> first & 0xFFu, oks = __ballot_sync(ALL, ok) >> first & 0xFFu;
+            uint32_t c = bads ? 0u : oks;
             while (__any_sync(ALL, c != 0)) {
                 const int s = first + (c ? __ffs(c) - 1 : 0);
                 const float tmin_s = __shfl_sync(ALL, tmin, s), t_s = __shfl_sync(ALL, t, s);

@@ -53,3 +53,8 @@ def cast_both(renderer, rays):
     many = cast(renderer, np.tile(rays, times))[1][:len(rays)]
     few = np.concatenate([cast(renderer, rays[k:k + 1000])[1] for k in range(0, len(rays), 1000)])
     return many, few
+
+
+def differing(a, b):
+    """Indices of the records that differ in any bit."""
+    return np.flatnonzero((a.view(np.uint8).reshape(len(a), -1) != b.view(np.uint8).reshape(len(b), -1)).any(1)).tolist()

@@ -29,7 +29,7 @@ def test_root_outside_the_tree(renderer, atrium, past):
     r["model"] = ct.upload(renderer, meshes, nodes, bad)
     ct.upload(renderer, meshes, nodes, root)
     many, few = ct.cast_both(renderer, r)
-    assert (few["hit"] == 2).all() and many.tobytes() == few.tobytes()
+    assert (few["hit"] == 2).all() and not ct.differing(many, few)
     assert ct.cast(renderer, r)[0] != 0
 
 
@@ -47,4 +47,25 @@ def test_child_outside_the_tree(renderer, atrium, past):
     r["model"] = ct.upload(renderer, meshes, nodes, 0)
     ct.upload(renderer, meshes, ct.built(renderer, h)[0], root)
     many, few = ct.cast_both(renderer, r)
-    assert (few["hit"] == 2).all() and many.tobytes() == few.tobytes()
+    assert (few["hit"] == 2).all() and not ct.differing(many, few)
+
+
+@pytest.mark.parametrize("what", ["child", "triangle"])
+@pytest.mark.parametrize("every", [2, 3, 7])
+def test_walks_that_end_early_beside_others(renderer, atrium, what, every):
+    """Rays of an intact tree beside rays, in the same warp, whose walk ends at an index outside the
+    model: the former answer as they do alone, the latter are marked."""
+    h, meshes, rays = atrium
+    nodes, root = ct.built(renderer, h)
+    good = rays.copy()
+    good["model"] = ct.upload(renderer, meshes, nodes, root)
+    want, _ = ct.cast_both(renderer, good)
+    one = nodes[:1].copy()
+    one["mn"], one["mx"], one["child"] = -1e4, 1e4, ct.NONE
+    one["count"], one["leaf"] = 1, what == "triangle"
+    one["child"][0, 0] = ct.TRI | sum(m.n for m in meshes) << 7 if what == "triangle" else 1
+    r = good.copy()
+    r["model"][::every], r["max_dist"][::every] = ct.upload(renderer, meshes, one, 0), 1e3
+    for got in ct.cast_both(renderer, r):
+        bad = np.arange(len(r)) % every == 0
+        assert (got["hit"][bad] == 2).all() and not ct.differing(got[~bad], want[~bad])
