@@ -33,6 +33,7 @@
 #include "../../include/sftg.h"
 #include "sftg_types.h"
 #include "sftg_kernels.h"
+#include "sftg_walk.h"
 
 #define TILE_THREADS 256
 #define SETUP_CAP 256
@@ -307,22 +308,6 @@ extern "C" int sftg_material_set(sftg_ctx* ctx, int32_t index, int32_t texture, 
     return SFTG_OK;
 }
 
-/* Whether every node's boxes lie inside the box its parent holds for it (sftg_model.nested): true of
- * a tree built from its triangles, not checked by the loaders of caller-built ones. */
-static uint32_t blas_nested(const sftg_bvh_node* nodes, uint32_t count) {
-    for (uint32_t i = 0; i < count; i++) {
-        if (nodes[i].leaf) continue;
-        for (int c = 0; c < nodes[i].count && c < 8; c++) {
-            const uint32_t ch = nodes[i].child[c];
-            if (ch == SFTG_INVALID || ch >= count) continue;
-            for (int q = 0; q < nodes[ch].count && q < 8; q++)
-                for (int a = 0; a < 3; a++)
-                    if (!(nodes[ch].mn[a][q] >= nodes[i].mn[a][c] && nodes[ch].mx[a][q] <= nodes[i].mx[a][c])) return 0;
-        }
-    }
-    return 1;
-}
-
 static int model_upload(sftg_ctx* ctx, const sftg_model_desc* d, int32_t* out_model, bool transient) {
     if (!ctx || !d || !out_model) return SFTG_E_ARG;
     CK(cudaSetDevice(ctx->device));
@@ -394,7 +379,7 @@ static int model_upload(sftg_ctx* ctx, const sftg_model_desc* d, int32_t* out_mo
         if ((rc = pool_reserve(ctx, ctx->blas, ((size_t)ctx->n_blas + d->blas_count) * 256))) return rc;
         CK(cudaMemcpyAsync((char*)ctx->blas.ptr + (size_t)ctx->n_blas * 256, d->blas_nodes, (size_t)d->blas_count * 256, cudaMemcpyHostToDevice, ctx->stream));
         ctx->blas.size = ((size_t)ctx->n_blas + d->blas_count) * 256;
-        md.nested = blas_nested((const sftg_bvh_node*)d->blas_nodes, d->blas_count);
+        md.nested = sftg_blas_nested((const sftg_bvh_node*)d->blas_nodes, d->blas_count, total);
     } else if (d->build_blas && total) {   /* built from the meshlets just uploaded */
         md.blas_count = 0; md.blas_root = 0;
         sftg_blas_job* job = nullptr;

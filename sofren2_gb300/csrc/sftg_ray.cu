@@ -268,7 +268,7 @@ k_ray_records(const sftg_ray* __restrict__ rays, uint32_t n, const sftg_model* _
  * box distance, which is no nearer than its ancestors': rounding is monotone and every box lies
  * inside the one its parent holds for it (sftg_model.nested; of every tree built here).  For the same
  * reason an entry whose box lies at or beyond the limit is dropped unread.  A tree a caller gave
- * with other boxes is walked one node at a time.  600 rays against the atrium (the longest walk 583
+ * with other boxes, or with indices outside the model, is walked one node at a time.  600 rays against the atrium (the longest walk 583
  * nodes): 250 us with 8 lanes per ray, one node per step, now 115. */
 #define WIDE_STACK 384
 

@@ -73,7 +73,8 @@ typedef struct sftg_model {
     uint32_t blas_base, blas_root, blas_count;
     uint32_t bone_count;
     uint32_t mesh_count;
-    uint32_t nested;       /* 1: every BLAS node's boxes lie inside the box its parent holds for it */
+    uint32_t nested;       /* 1: every BLAS node's boxes lie inside the box its parent holds for it, and
+                              no index leaves the model */
 } sftg_model;
 
 typedef struct sftg_bvh_node {  /* sft_bvh_node, sofren2.c:967-983 */

@@ -1,8 +1,8 @@
 /* Both ray walks (sofren2_gb300/csrc/sftg_ray.cu, its device code in ray_body.inc) on the CPU
- * (warp_sim.h), on a caller's tree.  argv[1]: u32 nodes, root, meshlets, rays, whether the tree is nested;
- * the node images; attr and inds of the meshlets; the rays.  Writes the records of the walk of many rays,
- * then those of a warp per ray, to argv[2].  Built with the address sanitizer: a read outside the
- * tree's arrays ends the program. */
+ * (warp_sim.h), on a caller's tree.  argv[1]: u32 nodes, root, meshlets, rays, whether the tree is nested
+ * (2: as an upload finds); the node images; attr and inds of the meshlets; the rays.  Writes the records of the
+ * walk of many rays, then those of a warp per ray, to argv[2].  Built with the address sanitizer: a read
+ * outside the tree's arrays ends the program. */
 #include "warp_sim.h"
 #include <vector>
 #include "sftg.h"
@@ -35,7 +35,7 @@ int main(int argc, char** argv) {
     for (blockIdx.x = 0; blockIdx.x < nn * 8; blockIdx.x++) k_blas_walk_forms(nodes.data(), nn, attr.data(), inds.data(), nm, slots.data(), tris.data());
     sftg_model M;
     memset(&M, 0, sizeof(M));
-    M.total_meshlets = nm; M.blas_count = nn; M.blas_root = hd[1]; M.nested = hd[4];
+    M.total_meshlets = nm; M.blas_count = nn; M.blas_root = hd[1]; M.nested = hd[4] == 2 ? sftg_blas_nested(nodes.data(), nn, nm) : hd[4];
     for (sftg_ray& r : rays) r.model = 0;
     std::vector<sftg_ray_hit> many(nr), few(nr);
     uint32_t next = 0;

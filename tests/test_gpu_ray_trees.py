@@ -69,3 +69,21 @@ def test_walks_that_end_early_beside_others(renderer, atrium, what, every):
     for got in ct.cast_both(renderer, r):
         bad = np.arange(len(r)) % every == 0
         assert (got["hit"][bad] == 2).all() and not ct.differing(got[~bad], want[~bad])
+
+
+@pytest.mark.parametrize("what,one_in", [("child", 40), ("triangle", 4)])
+def test_indices_outside_the_model_behind_nearer_hits(renderer, atrium, what, one_in):
+    """Some inner children, or leaf triangles, outside the model: the sequential walk skips those that lie
+    behind a nearer hit, so some records are answers and some are marked; both walks mark the same."""
+    h, meshes, rays = atrium
+    nodes, root = ct.built(renderer, h)
+    rng = np.random.default_rng(40)
+    at = (nodes["leaf"][:, None] == (what == "triangle")) & (np.arange(8) < nodes["count"][:, None]) & (rng.random((len(nodes), 8)) < 1 / one_in)
+    at[root] = False
+    total = sum(m.n for m in meshes)
+    nodes["child"][at] = (ct.TRI | (total + 1) << 7) if what == "triangle" else len(nodes) + 2
+    r = rays.copy()
+    r["model"] = ct.upload(renderer, meshes, nodes, root)
+    many, few = ct.cast_both(renderer, r)
+    assert (many["hit"] == 2).sum() > 100 and (many["hit"] == 1).sum() > 100
+    assert not ct.differing(many, few)

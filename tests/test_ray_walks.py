@@ -33,7 +33,7 @@ def walks(tmp_path_factory):
     return exe
 
 
-def run(exe, tmp_path, nodes, root, meshes, rays, nested):
+def run(exe, tmp_path, nodes, root, meshes, rays, nested):   # nested 2: as an upload finds
     path, out = str(tmp_path / "in.bin"), str(tmp_path / "out.bin")
     with open(path, "wb") as f:
         np.array([len(nodes), root, sum(m.n for m in meshes), len(rays), nested], np.uint32).tofile(f)
@@ -67,7 +67,7 @@ def atrium():
 def test_sound_tree_matches_oracle(walks, atrium, tmp_path):
     nodes, root, meshes, rays, want = atrium
     assert (want["hit"] == 1).sum() > 20
-    for nested in (0, 1):
+    for nested in (0, 1, 2):
         for got in run(walks, tmp_path, nodes, root, meshes, rays, nested):
             assert not differing(got, want)
 
@@ -81,7 +81,7 @@ def test_indices_outside_the_model(walks, atrium, tmp_path, what, bad):
     at &= np.random.default_rng(20).random(at.shape) < (1 / 4 if what == "triangle" else 1 / 20)
     at[root] = False
     n["child"][at] = bad or (TRI | sum(m.n for m in meshes) << 7 if what == "triangle" else len(n))
-    many, few = run(walks, tmp_path, n, root, meshes, rays, 0)
+    many, few = run(walks, tmp_path, n, root, meshes, rays, 2)
     assert (many["hit"] == 2).sum() > 3 and (many["hit"] == 1).sum() > 10
     assert not differing(many, few)
 

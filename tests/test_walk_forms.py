@@ -1,5 +1,6 @@
 """A caller's BLAS as the walks see it (sofren2_gb300/csrc/sftg_walk.h, shared by the upload and the
-kernels), on the CPU: child indices outside the tree."""
+kernels), on the CPU: child indices outside the tree, and the trees that may be expanded ahead of the
+sequential walk."""
 import os
 import shutil
 import subprocess
@@ -24,10 +25,10 @@ def walk_tool(tmp_path_factory):
     return exe
 
 
-def run(exe, tmp_path, nodes):
+def run(exe, tmp_path, nodes, meshlets=2):
     path = str(tmp_path / "nodes.bin")
     nodes.tofile(path)
-    return subprocess.run([exe, path], check=True, capture_output=True, text=True).stdout.splitlines()
+    return subprocess.run([exe, path, str(meshlets)], check=True, capture_output=True, text=True).stdout.splitlines()
 
 
 def tree():
@@ -46,7 +47,7 @@ def tree():
 def test_child_outside_the_tree_is_no_node_and_no_triangle(walk_tool, tmp_path, bad, node, slot):
     n = tree()
     n[node]["child"][slot] = bad
-    words = [[int(w) for w in line.split()] for line in run(walk_tool, tmp_path, n)]
+    words = [[int(w) for w in line.split()] for line in run(walk_tool, tmp_path, n)[:-1]]
     for i in range(len(n)):
         for c in range(8):
             if (i, c) == (node, slot):
@@ -57,5 +58,34 @@ def test_child_outside_the_tree_is_no_node_and_no_triangle(walk_tool, tmp_path, 
 
 def test_sound_tree_keeps_its_words(walk_tool, tmp_path):
     n = tree()
-    words = [[int(w) for w in line.split()] for line in run(walk_tool, tmp_path, n)]
+    words = [[int(w) for w in line.split()] for line in run(walk_tool, tmp_path, n)[:-1]]
     assert np.array_equal(np.array(words, np.uint32), n["child"])
+
+
+def nested(*args):
+    return int(run(*args)[-1])
+
+
+def test_sound_tree_is_nested(walk_tool, tmp_path):
+    n = tree()
+    n[4]["child"][5] = TRI | 300     # past the node's count: no slot of it
+    n[1]["child"][2] = 77
+    assert nested(walk_tool, tmp_path, n) == 1
+    n[1]["count"], n[1]["child"][2] = 3, NONE     # counted, but empty
+    assert nested(walk_tool, tmp_path, n) == 1
+
+
+@pytest.mark.parametrize("node,slot,bad", [(0, 1, 5), (0, 0, TRI), (1, 0, TRI | 4), (2, 0, NONE - 1), (3, 1, TRI | 256), (4, 0, TRI | 1 << 20),
+                                           (4, 0, NONE - 1)])
+def test_tree_with_an_index_outside_the_model_is_not_nested(walk_tool, tmp_path, node, slot, bad):
+    n = tree()
+    n[node]["child"][slot] = bad
+    assert nested(walk_tool, tmp_path, n) == 0
+
+
+@pytest.mark.parametrize("field,value", [("mn", -4.5), ("mx", 4.5), ("mn", np.nan), ("mx", np.inf)])
+@pytest.mark.parametrize("node", [1, 4])
+def test_box_outside_its_parents_is_not_nested(walk_tool, tmp_path, node, field, value):
+    n = tree()
+    n[node][field][1, 0] = value
+    assert nested(walk_tool, tmp_path, n) == 0
