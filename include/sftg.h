@@ -238,13 +238,16 @@ int sftg_pose_eval(sftg_ctx* ctx, const sftg_pose_request* requests, uint32_t n,
 int sftg_pose_eval_device(sftg_ctx* ctx, const sftg_pose_request* d_requests, const uint32_t* d_off, uint32_t n, float* d_posed,
                           float* d_global);
 
-/* Ray queries against resident models (sft_raycast_instance, sofren2.c:3733-3837), any number in
- * one launch, one thread per ray.  A ray names a model and its instance transform; results equal
+/* Ray queries against resident models (sft_raycast_instance, sofren2.c:3733-3837), any number at
+ * once.  A ray names a model and its instance transform; results equal
  * the reference's bit for bit, including its treatment of the transform: the ray enters model
  * space through the transposed rotation rows alone (sft_m_mul_vec adds no translation) and the
  * hit position leaves it the same way.  Skinned models are queried in their bind pose, as in the
  * reference.  A ray whose model is not resident, or has no BLAS, gives hit 0 and distance
- * max_dist; hit 2 marks a walk whose stack overflowed (a BLAS deeper than 18 levels). */
+ * max_dist.  hit 2 marks a walk that could not be finished: one that came to a node or triangle
+ * outside its model (of a tree the caller gave), or whose stack overflowed, which no BLAS of up to
+ * 18 levels does; a deeper one may or may not be answered, depending on the number of rays in the
+ * call. */
 typedef struct sftg_ray {
     float transform[16];       /* the instance's transform, row-major sftmat */
     float origin[3], dir[3];   /* world space; dir need not be normalised */

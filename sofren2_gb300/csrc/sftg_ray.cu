@@ -326,9 +326,11 @@ k_ray_wide(const sftg_ray* __restrict__ rays, uint32_t n, const sftg_model* __re
             continue;
         }
         if (!node_m) { top = max(0, top - 32); __syncwarp(); continue; }
-        /* the nodes to expand: up to four, down to the next triangle, one where the stack is nearly full */
+        /* the nodes to expand: up to four, down to the next triangle; one at a time from where the entries left would
+         * not hold, after one more step of four (28 entries), what the sequential walk may stack and a leaf's
+         * triangles: every walk that fits its RAY_STACK entries fits here */
         if (first_tri < 32) node_m &= (1u << first_tri) - 1u;
-        const int most = nested && top + 32 <= WIDE_STACK ? 4 : 1;
+        const int most = nested && top <= WIDE_STACK - RAY_STACK - 28 - 8 ? 4 : 1;
         uint32_t pick = node_m;
         for (int g = 0; g < sub; g++) pick &= pick - 1;
         const bool have = pick != 0 && sub < most;

@@ -58,3 +58,54 @@ def cast_both(renderer, rays):
 def differing(a, b):
     """Indices of the records that differ in any bit."""
     return np.flatnonzero((a.view(np.uint8).reshape(len(a), -1) != b.view(np.uint8).reshape(len(b), -1)).any(1)).tolist()
+
+
+class Plates:
+    """One meshlet of 120 triangles, one behind the other, each across the z axis."""
+
+    def __init__(self):
+        self.n = 1
+        attr, inds = np.zeros((10, 64), np.float32), np.zeros((16, 4, 8), np.uint8)
+        for q in range(60):
+            attr[0:3, q] = ((-9, 9, 0)[q % 3], (-9, -9, 9)[q % 3], 1 + q // 3 / 32)
+        for t in range(120):
+            p = t % 20
+            inds[t >> 3, 0:3, t & 7] = (3 * p, 3 * p + 1, 3 * p + 2) if t // 20 % 2 else (3 * p, 3 * p + 2, 3 * p + 1)
+        self.attr, self.inds = attr.reshape(1, -1), inds.reshape(1, -1)
+        self.cull = np.array([[0, 0, 1, 20, 0, 0, 1, 2]], np.float32)
+
+
+def deep_tree(levels, side, slot):
+    """A chain of `levels` inner nodes of 8 children, all boxes the same: the chain goes on in `slot`, the other
+    children are leaves of 8 triangles or (side "inner") inner nodes of 8 such leaves.  Leaves are shared
+    by no two slots."""
+    nodes, t = [], [0]
+
+    def add(leaf, kids):
+        n = np.zeros(1, NODE)
+        n["mn"], n["mx"], n["child"] = 1e30, -1e30, NONE
+        n["mn"][:, :, :len(kids)], n["mx"][:, :, :len(kids)] = -9, 9
+        n["child"][0, :len(kids)], n["count"], n["leaf"] = kids, len(kids), leaf
+        nodes.append(n)
+        return len(nodes) - 1
+
+    def leaf():
+        t[0] += 1
+        return add(1, [TRI | (8 * t[0] + k * 7) % 120 for k in range(8)])
+
+    node = leaf()
+    for level in range(levels):
+        kids = [leaf() if side == "leaf" else add(0, [leaf() for _ in range(8)]) for _ in range(7)]
+        kids.insert(slot, node)
+        node = add(0, kids)
+    return np.concatenate(nodes), node
+
+
+def plate_rays(n, seed):
+    rng = np.random.default_rng(seed)
+    r = np.zeros(n, runtime.RAY_DTYPE)
+    r["T"] = np.eye(4, dtype=np.float32).reshape(-1)
+    r["o"] = np.concatenate([rng.uniform(-2, 2, (n, 2)), rng.uniform(-3, 3, (n, 1))], 1)
+    r["d"] = np.concatenate([rng.uniform(-.3, .3, (n, 2)), rng.choice([-1, 1], (n, 1))], 1)
+    r["max_dist"] = rng.choice([1.0, 100.0], n)
+    return r

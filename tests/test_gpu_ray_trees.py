@@ -87,3 +87,15 @@ def test_indices_outside_the_model_behind_nearer_hits(renderer, atrium, what, on
     many, few = ct.cast_both(renderer, r)
     assert (many["hit"] == 2).sum() > 100 and (many["hit"] == 1).sum() > 100
     assert not ct.differing(many, few)
+
+
+@pytest.mark.parametrize("levels", [12, 17, 18])
+@pytest.mark.parametrize("slot", [7, 3])
+def test_deep_trees_whose_boxes_are_all_hit(renderer, levels, slot):
+    """Every walk that fits the 128 entries of the walk of many rays fits the one of few."""
+    nodes, root = ct.deep_tree(levels, "leaf", slot)
+    r = ct.plate_rays(600, levels)
+    r["model"] = ct.upload(renderer, [ct.Plates()], nodes, root)
+    many, few = ct.cast_both(renderer, r)
+    assert not (many["hit"] == 2).any() and (many["hit"] == 1).sum() > 100
+    assert not ct.differing(many, few)

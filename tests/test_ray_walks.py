@@ -9,7 +9,7 @@ import numpy as np
 import pytest
 
 import golden_cases as gc
-from caller_trees import NODE, NONE, TRI, differing
+from caller_trees import NODE, NONE, TRI, Plates, deep_tree, differing, plate_rays
 from oracle_lib import Oracle
 from sofren2_gb300 import runtime, scenes
 
@@ -91,3 +91,14 @@ def test_root_outside_the_tree(walks, atrium, tmp_path, root):
     nodes, _, meshes, rays, _ = atrium
     many, few = run(walks, tmp_path, nodes, len(nodes) + root if root < 2 else root, meshes, rays[:40], 0)
     assert (many["hit"] == 2).all() and not differing(many, few)
+
+
+@pytest.mark.parametrize("levels", [1, 12, 16, 17, 18])
+@pytest.mark.parametrize("side,slot", [("leaf", 7), ("leaf", 3), ("inner", 7)])
+def test_deep_trees_whose_boxes_are_all_hit(walks, tmp_path, levels, side, slot):
+    """Every walk that fits the 128 entries of the walk of many rays fits the one of few."""
+    levels -= side == "inner" and levels == 18     # a level more of its own
+    nodes, root = deep_tree(levels, side, slot)
+    many, few = run(walks, tmp_path, nodes, root, [Plates()], plate_rays(8, levels), 2)
+    assert not (many["hit"] == 2).any() and (many["hit"] == 1).any()
+    assert not differing(many, few)
