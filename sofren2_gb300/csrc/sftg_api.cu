@@ -69,6 +69,7 @@ struct sftg_lane {
     int graph_launches = 0;
     float timings[5] = { 0, 0, 0, 0, 0 };
     int launches = 0;
+    uint64_t tile_cap = 0, clip_cap = 0, stile_cap = 0;   /* the capacities its last batch was laid out with */
     /* a batch in flight (sftg_frames_submit): what sftg_lane_wait needs to finish it */
     bool busy = false;
     const sftg_frame_desc* fds = nullptr;
@@ -776,6 +777,7 @@ static int build_batch(sftg_ctx* ctx, sftg_lane& ln, const sftg_frame_desc* fds,
     const size_t stage_bytes = so;
     size_t raster_items = 1;
     for (int si = 0; si < 3; si++) if (B.s_tiles[si]) raster_items += sftg_raster_items_max(1 << si, B.s_tiles[si], ctx->tuning.raster_bands[si]);
+    ln.clip_cap = ctx->clip_cap; ln.tile_cap = ctx->tile_cap; ln.stile_cap = ctx->stile_cap;
     /* device arena layout */
     size_t need = stage_bytes + 4096;
     auto acc = [&](size_t bytes) { need = ((need + 255) & ~(size_t)255) + bytes; };
@@ -1176,7 +1178,8 @@ static int finish_batch(sftg_ctx* ctx, sftg_lane& ln, const sftg_frame_desc* fds
                         const uint32_t** out_dev) {
     CK(cudaEventSynchronize(ln.ev_done));
     const uint32_t clip_total = ln.h_status[2], pay_total = ln.h_status[3], stile_total = ln.h_status[4];
-    if (clip_total > ctx->clip_cap || pay_total > ctx->tile_cap || stile_total > ctx->stile_cap) {   /* capacity exceeded: grow and redo */
+    /* over the batch's own capacities (another lane's batch may have grown the context's since): grow and redo */
+    if (clip_total > ln.clip_cap || pay_total > ln.tile_cap || stile_total > ln.stile_cap) {
         while (ctx->clip_cap < clip_total) ctx->clip_cap *= 2;
         while (ctx->tile_cap < pay_total) ctx->tile_cap *= 2;
         while (ctx->stile_cap < stile_total) ctx->stile_cap *= 2;
