@@ -594,6 +594,11 @@ static void touch_pages(const void* p, size_t bytes, size_t pitch, size_t rows, 
     }
 }
 
+/* Arrays that share bytes: a kernel that reads one while it writes the other, in no order, needs a copy. */
+static bool overlap(const void* a, size_t na, const void* b, size_t nb) {
+    return a && b && (uintptr_t)a < (uintptr_t)b + nb && (uintptr_t)b < (uintptr_t)a + na;
+}
+
 /* The address of a caller's colour buffer that the kernels write (and, where the frame does not clear,
  * blend with) in place, its pitch a whole number of pixels; null for any other buffer (copied).
  * Stores then reach host memory over the chip-to-chip link as the resolve makes them. */
@@ -1465,7 +1470,8 @@ extern "C" int sftg_pose_eval(sftg_ctx* ctx, const sftg_pose_request* reqs, uint
     float* v_posed = (float*)host_visible(ctx, posed, &page_posed);
     float* v_global = global ? (float*)host_visible(ctx, global, &page_global) : nullptr;
     const size_t b_mat = (size_t)total * 64;
-    if (v_req && v_off && v_posed && (!global || v_global)) {
+    if (v_req && v_off && v_posed && (!global || v_global) && !overlap(posed, b_mat, global, b_mat) &&
+        !overlap(reqs, (size_t)n * sizeof(*reqs), posed, b_mat) && !overlap(reqs, (size_t)n * sizeof(*reqs), global, b_mat)) {
         if (page_posed) touch_pages(posed, b_mat, 0, 1, true);
         if (page_global) touch_pages(global, b_mat, 0, 1, true);
         sftg_launch_pose(pose_tables(ctx), v_req, v_off, n, v_posed, v_global, ctx->stream);
@@ -1534,19 +1540,19 @@ extern "C" int sftg_raycast(sftg_ctx* ctx, const sftg_ray* rays, uint32_t n, sft
     /* few rays: the caller's arrays in place (the walk of many reads and writes them more than once) */
     const sftg_ray* v_rays = n <= SFTG_RAY_WIDE_MAX ? (const sftg_ray*)host_visible(ctx, rays) : nullptr;
     sftg_ray_hit* v_hits = n <= SFTG_RAY_WIDE_MAX ? (sftg_ray_hit*)host_visible(ctx, hits) : nullptr;
-    if (v_rays && v_hits) {
+    if (v_rays && v_hits && !overlap(rays, (size_t)n * sizeof(*rays), hits, (size_t)n * sizeof(*hits))) {
         touch_pages(rays, (size_t)n * sizeof(sftg_ray), 0, 1, false);
         touch_pages(hits, (size_t)n * sizeof(sftg_ray_hit), 0, 1, true);
         if ((rc = sftg_raycast_device(ctx, v_rays, n, v_hits))) return rc;
     } else {
-    const size_t b_ray = ((size_t)n * sizeof(sftg_ray) + 255) & ~(size_t)255;
-    rc = pool_reserve(ctx, ctx->p_ray_io, b_ray + (size_t)n * sizeof(sftg_ray_hit) + 256);
-    if (rc) return rc;
-    sftg_ray* d_rays = (sftg_ray*)ctx->p_ray_io.ptr;
-    sftg_ray_hit* d_hits = (sftg_ray_hit*)((char*)ctx->p_ray_io.ptr + b_ray);
-    CK(cudaMemcpyAsync(d_rays, rays, (size_t)n * sizeof(sftg_ray), cudaMemcpyHostToDevice, ctx->stream));
-    if ((rc = sftg_raycast_device(ctx, d_rays, n, d_hits))) return rc;
-    CK(cudaMemcpyAsync(hits, d_hits, (size_t)n * sizeof(sftg_ray_hit), cudaMemcpyDeviceToHost, ctx->stream));
+        const size_t b_ray = ((size_t)n * sizeof(sftg_ray) + 255) & ~(size_t)255;
+        rc = pool_reserve(ctx, ctx->p_ray_io, b_ray + (size_t)n * sizeof(sftg_ray_hit) + 256);
+        if (rc) return rc;
+        sftg_ray* d_rays = (sftg_ray*)ctx->p_ray_io.ptr;
+        sftg_ray_hit* d_hits = (sftg_ray_hit*)((char*)ctx->p_ray_io.ptr + b_ray);
+        CK(cudaMemcpyAsync(d_rays, rays, (size_t)n * sizeof(sftg_ray), cudaMemcpyHostToDevice, ctx->stream));
+        if ((rc = sftg_raycast_device(ctx, d_rays, n, d_hits))) return rc;
+        CK(cudaMemcpyAsync(hits, d_hits, (size_t)n * sizeof(sftg_ray_hit), cudaMemcpyDeviceToHost, ctx->stream));
     }
     CK(cudaStreamSynchronize(ctx->stream));
     for (uint32_t k = 0; k < n; k++)
