@@ -270,8 +270,8 @@ int sftg_raycast_device(sftg_ctx* ctx, const sftg_ray* d_rays, uint32_t n, sftg_
  * the frame descriptions, everything they point at and the colour buffers must stay valid until
  * sftg_lane_wait returns.  sftg_lane_done is 1 once the lane's batch has finished (or the lane is
  * idle) and 0 while it runs; sftg_lane_wait waits for it, re-renders it when a capacity had to
- * grow, and returns its status.  A batch with a view that keeps the caller's pixels (clear off) in
- * memory the GPU cannot reach completes inside sftg_frames_submit.  Each view's pixels are those it would get alone. */
+ * grow, and returns its status.  A batch with a view that keeps the caller's pixels (clear off)
+ * completes inside sftg_frames_submit.  Each view's pixels are those it would get alone. */
 #define SFTG_MAX_LANES 8
 int sftg_frames_submit(sftg_ctx* ctx, uint32_t lane, const sftg_frame_desc* frames, uint32_t n_views, uint32_t* const* colors,
                        const int32_t* pitch_bytes);

@@ -1290,13 +1290,15 @@ extern "C" int sftg_frames_submit(sftg_ctx* ctx, uint32_t lane, const sftg_frame
         if (colors) ln.colors[v] = colors[v];
         if (pitch_bytes) ln.pitch[v] = pitch_bytes[v];
     }
+    bool keeps = false;
+    for (uint32_t v = 0; v < n_views; v++) keeps = keeps || (!fds[v].clear && ln.colors[v]);
     batch_bufs B;
     bool defer = false;
     if ((rc = submit_batch(ctx, ln, fds, n_views, ln.colors.data(), ln.pitch.data(), nullptr, B, defer))) return rc;
     ln.busy = true;
-    if (defer) {   /* a view keeps the caller's pixels: finish now, so that a re-render can start from them */
+    if (keeps) {   /* finish now: a re-render starts from the caller's pixels, and so does the next batch that keeps them */
         ln.busy = false;
-        rc = finish_batch(ctx, ln, fds, n_views, ln.colors.data(), ln.pitch.data(), B, true, nullptr, nullptr);
+        rc = finish_batch(ctx, ln, fds, n_views, ln.colors.data(), ln.pitch.data(), B, defer, nullptr, nullptr);
         for (int attempt = 0; rc == BATCH_REDO && attempt < 4; attempt++) {
             batch_bufs B2;
             if ((rc = submit_batch(ctx, ln, fds, n_views, ln.colors.data(), ln.pitch.data(), nullptr, B2, defer))) return rc;
