@@ -27,6 +27,7 @@
 #include <string.h>
 #include <unistd.h>
 #include <algorithm>
+#include <utility>
 #include <vector>
 #include <chrono>
 
@@ -76,6 +77,7 @@ struct sftg_lane {
     uint32_t nv = 0;
     std::vector<uint32_t*> colors;
     std::vector<int32_t> pitch;
+    std::vector<std::pair<uintptr_t, uintptr_t>> in_place;   /* pageable buffers it writes in place, [start, end), ascending */
 };
 
 struct sftg_ctx {
@@ -1143,6 +1145,28 @@ static int launch_batch_graph(sftg_ctx* ctx, sftg_lane& ln, const batch_bufs& B)
     return 0;
 }
 
+/* Batches over one pageable buffer are drawn in the order they were submitted: waits for those on other
+ * lanes that still write, in place, a buffer of this one (copies returned from their submission when they
+ * were done), and notes this one's. */
+static int wait_shared_buffers(sftg_ctx* ctx, sftg_lane& ln, const sftg_frame_desc* fds, uint32_t nv, uint32_t* const* host_color,
+                               const int32_t* pitch_bytes, const batch_bufs& B) {
+    ln.in_place.clear();
+    for (uint32_t v = 0; v < nv && host_color; v++) {
+        if (!host_color[v]) continue;
+        const size_t pitch = pitch_bytes && pitch_bytes[v] > 0 ? (size_t)pitch_bytes[v] : (size_t)fds[v].width * 4;
+        const uintptr_t a = (uintptr_t)host_color[v], e = a + pitch * (size_t)(fds[v].height - 1) + (size_t)fds[v].width * 4;
+        for (int l = 0; l < SFTG_MAX_LANES; l++) {
+            const sftg_lane& o = ctx->lanes[l];
+            if (&o == &ln || !o.busy || !o.fds || o.in_place.empty()) continue;
+            auto it = std::upper_bound(o.in_place.begin(), o.in_place.end(), std::make_pair(e, (uintptr_t)0));   /* the first from e on */
+            if (it != o.in_place.begin() && (--it)->second > a) CK(cudaEventSynchronize(o.ev_done));
+        }
+        if (B.plan[v].pageable) ln.in_place.push_back({ a, e });
+    }
+    std::sort(ln.in_place.begin(), ln.in_place.end());   /* disjoint: views of one batch that share bytes are copied */
+    return 0;
+}
+
 /* Queues a batch on a lane: the frame block, the caller's pixels for views that keep them, the
  * launches (one graph replay unless debug capture or graphs are off), the status read-back, the
  * colour read-back (deferred to finish_batch when a view keeps the caller's pixels, so that a
@@ -1156,6 +1180,7 @@ static int submit_batch(sftg_ctx* ctx, sftg_lane& ln, const sftg_frame_desc* fds
     }
     int rc;
     if ((rc = build_batch(ctx, ln, fds, nv, dbg != nullptr, B, host_color, pitch_bytes))) return rc;
+    if ((rc = wait_shared_buffers(ctx, ln, fds, nv, host_color, pitch_bytes, B))) return rc;
     defer_colors = false;
     for (uint32_t v = 0; v < nv; v++)   /* the reference blends over / keeps the caller's pixels */
         if (!fds[v].clear && host_color && host_color[v] && !B.plan[v].direct) {

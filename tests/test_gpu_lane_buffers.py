@@ -75,3 +75,38 @@ def test_kept_batches_over_one_buffer_follow_one_another(renderer, kept, pinned)
         assert all(np.array_equal(b, steps[-1]) for b in bufs)
     finally:
         renderer.set_samples(1)
+
+
+@pytest.mark.parametrize("where", ["same", "rows", "corner"])
+@pytest.mark.parametrize("second", ["lane", "call", "kept"])
+def test_later_batches_over_pageable_buffers_win(renderer, kept, where, second):
+    """A long batch on one lane, whose last view goes to a buffer that the next submission, or a call on the
+    synchronous lane, draws over: the buffer ends as if the two had run one after the other."""
+    keep_h, init = kept
+    big, small = renderer.load_scene(gc.blob("atrium_small")), renderer.load_scene(gc.blob("small"))
+    try:
+        renderer.set_samples(1)
+        w, h = renderer.frame_size(big, 0)
+        over = keep_h if second == "kept" else small
+        w2, h2 = renderer.frame_size(over, 0)
+        room = np.zeros((h + h2 + 4, w + w2 + 4), np.uint32)
+        a, at = room[2:2 + h, 2:2 + w], {"same": (2, 2), "rows": (2 + h // 2, 2), "corner": (1 + h, 1 + w)}[where]
+        b = room[at[0]:at[0] + h2, at[1]:at[1] + w2]
+        renderer.render(big, 0, a)
+        renderer.render(over, 0, b)
+        want = room.copy()
+        assert (want[2:2 + h, 2:2 + w] != 0).any()
+        for _ in range(3):
+            room[:] = 0
+            others = [np.zeros((h, w), np.uint32) for _ in range(60)]
+            _submit(renderer, 1, [(big, 0, c) for c in others] + [(big, 0, a)])
+            if second == "call":
+                renderer.render(over, 0, b)
+            else:
+                _submit(renderer, 2, [(over, 0, b)])
+                assert renderer.lib.sft_batch_wait(2) == 0
+            assert renderer.lib.sft_batch_wait(1) == 0
+            assert np.array_equal(room, want)
+    finally:
+        renderer.free_scene(big)
+        renderer.free_scene(small)
