@@ -145,7 +145,8 @@ int sftg_frame_render_device(sftg_ctx* ctx, const sftg_frame_desc* frame, const 
  * Each view's result is identical to rendering it alone with sftg_frame_render.
  * colors (optional) holds one host pointer per view (entries may be null), pitch_bytes
  * (optional) one pitch per view (0 = width*4); out_device_colors (optional) receives one device
- * pointer per view, valid until the next render call.  No counterpart in the reference, which
+ * pointer per view, valid until the next render call: to rows of width pixels, or, for a clearing
+ * view with a page-locked buffer in colors, that buffer, in its own pitch.  No counterpart in the reference, which
  * renders one view per sft_present. */
 int sftg_frames_render(sftg_ctx* ctx, const sftg_frame_desc* frames, uint32_t n_views, uint32_t* const* colors,
                        const int32_t* pitch_bytes, const uint32_t** out_device_colors);

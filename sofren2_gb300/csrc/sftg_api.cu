@@ -626,7 +626,7 @@ static uint32_t job_width(const sftg_ctx* ctx, const sftg_frame_desc* fds, uint3
     return n >= SFTG_WIDE_JOBS ? 8u : (uint32_t)ctx->tuning.geom_job_width;
 }
 
-static int build_batch(sftg_ctx* ctx, sftg_lane& ln, const sftg_frame_desc* fds, uint32_t nv, bool want_debug, batch_bufs& B,
+static int build_batch(sftg_ctx* ctx, sftg_lane& ln, const sftg_frame_desc* fds, uint32_t nv, bool want_debug, bool want_dev, batch_bufs& B,
                        uint32_t* const* host_color = nullptr, const int32_t* pitch_bytes = nullptr) {
     if (!nv || nv > 65535) return set_err(ctx, SFTG_E_ARG, "a batch holds 1 to 65535 views, not %u", nv);
     if (want_debug && nv != 1) return set_err(ctx, SFTG_E_ARG, "debug capture covers single-view submissions only");
@@ -704,6 +704,7 @@ static int build_batch(sftg_ctx* ctx, sftg_lane& ln, const sftg_frame_desc* fds,
         n_pl += fd->n_point; n_dl += fd->n_dir; n_tl += fd->tlas_count;
         P.color_off = color_total; color_total += (uint64_t)W * H;
         P.direct = direct_color(ctx, *fd, host_color ? host_color[v] : nullptr, pitch_bytes ? pitch_bytes[v] : 0, P.pageable);
+        if (want_dev && (P.pageable || !fd->clear)) { P.direct = nullptr; P.pageable = false; }   /* colours on the device are asked for */
         P.direct_pitch = P.direct ? (pitch_bytes && pitch_bytes[v] > 0 ? pitch_bytes[v] / 4 : W) : W;
     }
     if (host_color && nv > 1) {
@@ -1172,14 +1173,14 @@ static int wait_shared_buffers(sftg_ctx* ctx, sftg_lane& ln, const sftg_frame_de
  * colour read-back (deferred to finish_batch when a view keeps the caller's pixels, so that a
  * re-render still starts from them) and the lane's completion event. */
 static int submit_batch(sftg_ctx* ctx, sftg_lane& ln, const sftg_frame_desc* fds, uint32_t nv, uint32_t* const* host_color,
-                        const int32_t* pitch_bytes, sftg_debug_out* dbg, batch_bufs& B, bool& defer_colors) {
+                        const int32_t* pitch_bytes, sftg_debug_out* dbg, bool want_dev, batch_bufs& B, bool& defer_colors) {
     auto pitch_of = [&](uint32_t v) { return (pitch_bytes && pitch_bytes[v] > 0) ? (size_t)pitch_bytes[v] : (size_t)fds[v].width * 4; };
     if (&ln != &ctx->lanes[0]) {   /* after every upload queued so far on lane 0's stream */
         CK(cudaEventRecord(ctx->ev_upload, ctx->stream));
         CK(cudaStreamWaitEvent(ln.stream, ctx->ev_upload, 0));
     }
     int rc;
-    if ((rc = build_batch(ctx, ln, fds, nv, dbg != nullptr, B, host_color, pitch_bytes))) return rc;
+    if ((rc = build_batch(ctx, ln, fds, nv, dbg != nullptr, want_dev, B, host_color, pitch_bytes))) return rc;
     if ((rc = wait_shared_buffers(ctx, ln, fds, nv, host_color, pitch_bytes, B))) return rc;
     defer_colors = false;
     for (uint32_t v = 0; v < nv; v++)   /* the reference blends over / keeps the caller's pixels */
@@ -1265,7 +1266,7 @@ static int finish_batch(sftg_ctx* ctx, sftg_lane& ln, const sftg_frame_desc* fds
 
 /* Renders a batch of views on lane 0 and waits for it.  host_color[v] (optional) receives view
  * v's colour with pitch pitch_bytes[v]; out_dev[v] (optional) its device colour buffer, valid
- * until the next synchronous call. */
+ * until the next synchronous call (of a clearing view with a page-locked buffer, that buffer). */
 static int batch_common(sftg_ctx* ctx, const sftg_frame_desc* fds, uint32_t nv, uint32_t* const* host_color, const int32_t* pitch_bytes,
                         sftg_debug_out* dbg, const uint32_t** out_dev) {
     if (!ctx || !fds) return SFTG_E_ARG;
@@ -1276,7 +1277,7 @@ static int batch_common(sftg_ctx* ctx, const sftg_frame_desc* fds, uint32_t nv, 
     for (int attempt = 0; attempt < 4; attempt++) {
         batch_bufs B;
         bool defer = false;
-        if ((rc = submit_batch(ctx, ln, fds, nv, host_color, pitch_bytes, dbg, B, defer))) return rc;
+        if ((rc = submit_batch(ctx, ln, fds, nv, host_color, pitch_bytes, dbg, out_dev != nullptr, B, defer))) return rc;
         rc = finish_batch(ctx, ln, fds, nv, host_color, pitch_bytes, B, defer, dbg, out_dev);
         if (rc != BATCH_REDO) return rc;
     }
@@ -1319,14 +1320,14 @@ extern "C" int sftg_frames_submit(sftg_ctx* ctx, uint32_t lane, const sftg_frame
     for (uint32_t v = 0; v < n_views; v++) keeps = keeps || (!fds[v].clear && ln.colors[v]);
     batch_bufs B;
     bool defer = false;
-    if ((rc = submit_batch(ctx, ln, fds, n_views, ln.colors.data(), ln.pitch.data(), nullptr, B, defer))) return rc;
+    if ((rc = submit_batch(ctx, ln, fds, n_views, ln.colors.data(), ln.pitch.data(), nullptr, false, B, defer))) return rc;
     ln.busy = true;
     if (keeps) {   /* finish now: a re-render starts from the caller's pixels, and so does the next batch that keeps them */
         ln.busy = false;
         rc = finish_batch(ctx, ln, fds, n_views, ln.colors.data(), ln.pitch.data(), B, defer, nullptr, nullptr);
         for (int attempt = 0; rc == BATCH_REDO && attempt < 4; attempt++) {
             batch_bufs B2;
-            if ((rc = submit_batch(ctx, ln, fds, n_views, ln.colors.data(), ln.pitch.data(), nullptr, B2, defer))) return rc;
+            if ((rc = submit_batch(ctx, ln, fds, n_views, ln.colors.data(), ln.pitch.data(), nullptr, false, B2, defer))) return rc;
             rc = finish_batch(ctx, ln, fds, n_views, ln.colors.data(), ln.pitch.data(), B2, defer, nullptr, nullptr);
         }
         if (rc == BATCH_REDO) return set_err(ctx, SFTG_E_NOMEM, "frame capacities did not converge");
@@ -1361,7 +1362,7 @@ extern "C" int sftg_lane_wait(sftg_ctx* ctx, uint32_t lane) {
     for (int attempt = 0; rc == BATCH_REDO && attempt < 4; attempt++) {
         batch_bufs B;
         bool defer = false;
-        if ((rc = submit_batch(ctx, ln, fds, ln.nv, ln.colors.data(), ln.pitch.data(), nullptr, B, defer))) return rc;
+        if ((rc = submit_batch(ctx, ln, fds, ln.nv, ln.colors.data(), ln.pitch.data(), nullptr, false, B, defer))) return rc;
         rc = finish_batch(ctx, ln, fds, ln.nv, ln.colors.data(), ln.pitch.data(), B, defer, nullptr, nullptr);
     }
     if (rc == BATCH_REDO) return set_err(ctx, SFTG_E_NOMEM, "frame capacities did not converge");
