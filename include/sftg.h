@@ -197,7 +197,8 @@ int sftg_set_tuning(sftg_ctx* ctx, const sftg_tuning* tuning);
 /* Times the given views with each candidate setting (median of reps renders per candidate,
  * coordinate search: job width, then per sample count slab rows, raster bands, and resolve split
  * with where the tile light lists are made, jointly, then the persistent tile queue), keeps the
- * fastest in the context and copies it to *out (optional). */
+ * fastest in the context and copies it to *out (optional).  A knob that the views' size overrules
+ * stays as it is set. */
 int sftg_autotune(sftg_ctx* ctx, const sftg_frame_desc* frames, uint32_t n_views, int32_t reps, sftg_tuning* out);
 
 /* Skeletal animation on the GPU (sft_pose_update, sofren2.c:8952-9108).  A skeleton (bones in

@@ -612,9 +612,9 @@ static uint32_t* direct_color(const sftg_ctx* ctx, const sftg_frame_desc& fd, ui
     return (uint32_t*)host_visible(ctx, host, &pageable);
 }
 
-/* Meshlets per geometry job: the knob's, or the reference's whole group of 8 from SFTG_WIDE_JOBS meshlets
- * in the batch on. */
-static uint32_t job_width(const sftg_ctx* ctx, const sftg_frame_desc* fds, uint32_t nv) {
+/* Whether a batch has SFTG_WIDE_JOBS meshlets or more: a geometry job is then the reference's whole group
+ * of 8, whatever the knob says. */
+static bool wide_jobs(const sftg_ctx* ctx, const sftg_frame_desc* fds, uint32_t nv) {
     uint64_t n = 0;
     for (uint32_t v = 0; v < nv && n < SFTG_WIDE_JOBS; v++) {
         if (fds[v].n_instances > SFTG_MAX_INSTANCES) break;   /* refused by the caller, as are models out of range */
@@ -623,7 +623,7 @@ static uint32_t job_width(const sftg_ctx* ctx, const sftg_frame_desc* fds, uint3
             if (m >= 0 && (size_t)m < ctx->h_models.size()) n += ctx->h_models[m].total_meshlets;
         }
     }
-    return n >= SFTG_WIDE_JOBS ? 8u : (uint32_t)ctx->tuning.geom_job_width;
+    return n >= SFTG_WIDE_JOBS;
 }
 
 static int build_batch(sftg_ctx* ctx, sftg_lane& ln, const sftg_frame_desc* fds, uint32_t nv, bool want_debug, bool want_dev, batch_bufs& B,
@@ -638,7 +638,7 @@ static int build_batch(sftg_ctx* ctx, sftg_lane& ln, const sftg_frame_desc* fds,
     std::vector<float> bones;
     uint32_t total_ss = 0, total_prox = 0, total_packets = 0, max_inst = 0, n_pl = 0, n_dl = 0, n_tl = 0;
     uint64_t max_pairs = 0, color_total = 0;
-    const uint32_t jw = job_width(ctx, fds, nv);
+    const uint32_t jw = wide_jobs(ctx, fds, nv) ? 8u : (uint32_t)ctx->tuning.geom_job_width;
     for (uint32_t v = 0; v < nv; v++) {
         const sftg_frame_desc* fd = &fds[v];
         view_plan& P = B.plan[v];
@@ -1639,7 +1639,7 @@ extern "C" int sftg_autotune(sftg_ctx* ctx, const sftg_frame_desc* fds, uint32_t
     sftg_tuning best = ctx->tuning;
     int rc;
     if ((rc = batch_common(ctx, fds, n_views, nullptr, nullptr, nullptr, nullptr))) return rc;   /* warm: arena, tables */
-    {
+    if (!wide_jobs(ctx, fds, n_views)) {   /* else every width runs as 8 */
         const int widths[4] = { 1, 2, 4, 8 };
         float bt = 1e30f;
         for (int k = 0; k < 4; k++) {
@@ -1670,16 +1670,21 @@ extern "C" int sftg_autotune(sftg_ctx* ctx, const sftg_frame_desc* fds, uint32_t
             if (t < bt) { bt = t; best.raster_bands[si] = bands[k]; }
         }
         /* resolve split and where the tile light lists are made, jointly: per-tile lists take the
-         * split-fold selection work out of every CTA, which favours higher splits */
-        const int splits[5] = { 4, 8, 16, 2, 1 };
+         * split-fold selection work out of every CTA, which favours higher splits.  Of splits that these
+         * views' tiles bring to the same number of CTAs the largest stands: fewer tiles take more of it */
+        const int splits[5] = { 16, 8, 4, 2, 1 };
+        uint32_t tiles = 0;
+        for (const sftg_frame_desc& f : sub) tiles += (uint32_t)((f.width + 63) / 64) * (uint32_t)((f.height + 63) / 64);
         bt = 1e30f;
-        for (int k = 0; k < 5; k++)
+        for (int k = 0; k < 5; k++) {
+            if (k && sftg_resolve_split(splits[k], tiles) >= sftg_resolve_split(splits[k - 1], tiles)) continue;
             for (int m = 1; m <= 2; m++) {
                 ctx->tuning = best; ctx->tuning.resolve_split[si] = splits[k]; ctx->tuning.tile_lights[si] = m;
                 float t;
                 if ((rc = time_phase(ctx, sub.data(), (uint32_t)sub.size(), reps, 4, &t))) { ctx->tuning = best; return rc; }
                 if (t < bt) { bt = t; best.resolve_split[si] = splits[k]; best.tile_lights[si] = m; }
             }
+        }
     }
     {   /* the persistent tile queue, against raster + resolve of all views */
         float bt = 1e30f;
