@@ -260,7 +260,10 @@ typedef struct sftg_ray_hit {  /* sft_ray_hit (sofren2.c:895-900) */
     uint32_t hit;
     float distance, pos[3], normal[3];
 } sftg_ray_hit;
-/* host arrays; returns when hits is filled (SFTG_E_DEVICE_STATUS if a walk overflowed) */
+/* Rays in one call: 2^32 less 2^20 (more than a GPU's memory holds), so that 32-bit counters that run past
+ * the last ray do not wrap; SFTG_E_LIMIT beyond. */
+#define SFTG_RAY_MAX 0xFFF00000u
+/* host arrays; returns when hits is filled (SFTG_E_DEVICE_STATUS if a walk could not be finished) */
 int sftg_raycast(sftg_ctx* ctx, const sftg_ray* rays, uint32_t n, sftg_ray_hit* hits);
 /* device arrays, queued on the context's stream (sftg_stream); returns without waiting */
 int sftg_raycast_device(sftg_ctx* ctx, const sftg_ray* d_rays, uint32_t n, sftg_ray_hit* d_hits);

@@ -1551,6 +1551,7 @@ extern "C" int sftg_pose_eval(sftg_ctx* ctx, const sftg_pose_request* reqs, uint
 extern "C" int sftg_raycast_device(sftg_ctx* ctx, const sftg_ray* d_rays, uint32_t n, sftg_ray_hit* d_hits) {
     if (!ctx || (n && (!d_rays || !d_hits))) return SFTG_E_ARG;
     if (!n) return SFTG_OK;
+    if (n > SFTG_RAY_MAX) return set_err(ctx, SFTG_E_LIMIT, "%u rays in one call (at most %u)", n, SFTG_RAY_MAX);
     CK(cudaSetDevice(ctx->device));
     int rc = sync_tables(ctx);   /* the device model table follows uploads lazily */
     if (rc) return rc;
@@ -1563,6 +1564,7 @@ extern "C" int sftg_raycast_device(sftg_ctx* ctx, const sftg_ray* d_rays, uint32
 extern "C" int sftg_raycast(sftg_ctx* ctx, const sftg_ray* rays, uint32_t n, sftg_ray_hit* hits) {
     if (!ctx || (n && (!rays || !hits))) return SFTG_E_ARG;
     if (!n) return SFTG_OK;
+    if (n > SFTG_RAY_MAX) return set_err(ctx, SFTG_E_LIMIT, "%u rays in one call (at most %u)", n, SFTG_RAY_MAX);
     CK(cudaSetDevice(ctx->device));
     int rc;
     /* few rays: the caller's arrays in place (the walk of many reads and writes them more than once) */

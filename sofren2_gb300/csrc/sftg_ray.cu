@@ -13,9 +13,9 @@
  *                transform, the normal normalised (sft_v_norm)
  * Arithmetic is the reference's scalar C sequence in IEEE single precision: the file is built
  * with -fmad=false, and divisions and square roots are the correctly rounded intrinsics.  The walk
- * of many rays holds RAY_STACK entries (an 8-wide BLAS needs 7 per level); a walk that would
- * overflow its stack, or that meets a node or meshlet index outside its model, stops and marks its
- * record with hit = 2.
+ * of many rays holds RAY_STACK entries (an 8-wide BLAS needs 7 per level), that of few whatever the
+ * former would stack; a walk that would overflow its stack, or that meets a node or meshlet index
+ * outside its model, stops and marks its record with hit = 2.
  */
 #include "sftg_types.h"
 #include "sftg_kernels.h"
@@ -159,7 +159,7 @@ k_ray_walks(const sftg_ray* __restrict__ rays, uint32_t n, const sftg_model* __r
                 uint32_t k0 = 0;
                 if (lane == 0) k0 = atomicAdd(next, 32u);
                 k0 = __shfl_sync(ALL, k0, 0);
-                dry = k0 >= n;   /* the counter passes n by at most 32 a warp: the host bounds n */
+                dry = k0 >= n;   /* the counter passes n by at most 32 a warp: n is at most SFTG_RAY_MAX */
                 const uint32_t mine = k0 + (uint32_t)lane;
                 const bool in = !dry && mine < n;
                 bool walk = false;
@@ -374,6 +374,7 @@ k_ray_wide(const sftg_ray* __restrict__ rays, uint32_t n, const sftg_model* __re
 }
 
 #define RAY_GRID (152 * 8)   /* CTAs of the many-ray walk: 8 fit an SM (registers) */
+static_assert(RAY_GRID * RAY_WARPS * 32u <= 0xFFFFFFFFu - SFTG_RAY_MAX, "the ray counter does not wrap");
 
 int sftg_launch_raycast(const sftg_ray* rays, uint32_t n, const sftg_model* models, uint32_t n_models, const sftg_wslot* wslots,
                         const sftg_wtri* wtris, uint32_t* next, sftg_ray_hit* hits, cudaStream_t st) {
