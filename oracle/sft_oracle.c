@@ -406,6 +406,7 @@ typedef struct {
     u32 invalid_packets;
     f32* depth; u32* vid;        /* per tile buffers, S * 4096 each, all tiles */
     u32* color;
+    const u32* start;            /* the caller's pixels before the frame (sfto_set_pixels); NULL: zeros */
     mat4* inst_T; const mat4** inst_bones;
     int debug_mode;              /* enum sft_debug_mode (sofren2.c:59-67) */
     otex checker;                /* the base material's 256x256 checkerboard (sofren2.c:8062-8080) */
@@ -1662,6 +1663,7 @@ static int render_frame(octx* c, u32 fi, int S, int threads, const char* dump_pa
     c->depth = (f32*)malloc(per * ntiles * 4);
     c->vid = (u32*)malloc(per * ntiles * 4);
     c->color = (u32*)calloc((size_t)c->W * c->H, 4);
+    if (c->start) memcpy(c->color, c->start, (size_t)c->W * c->H * 4);
     if (threads < 1) threads = 1;
     pthread_t th[64]; tile_job jobs[64];
     if (threads > 64) threads = 64;
@@ -2071,6 +2073,10 @@ int sfto_shadow_fp64(void* hp, uint32_t frame, int samples, double* out) {
     out[2] = (double)h->c.fp64_n; out[3] = (double)h->c.fp64_big;
     return rc;
 }
+
+/* Pixels (width * height of the frames rendered from here on) that a frame starts from, read while it is
+ * rendered; NULL: zeros. */
+void sfto_set_pixels(void* hp, const uint32_t* pixels) { ((oracle_handle*)hp)->c.start = pixels; }
 
 /* enum sft_debug_mode for the following renders (0 = none) */
 int sfto_set_debug_mode(void* hp, int mode) {
