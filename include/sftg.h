@@ -29,7 +29,9 @@ extern "C" {
 #define SFTG_E_ARG (-2)           /* invalid argument */
 #define SFTG_E_NOMEM (-3)         /* device allocation failed */
 #define SFTG_E_LIMIT (-4)         /* a reference limit was exceeded (e.g. > 64 instances) */
-#define SFTG_E_DEVICE_STATUS (-5) /* a kernel reported a bounded-walk overflow */
+#define SFTG_E_DEVICE_STATUS (-5) /* a kernel could not finish a walk: its stack overflowed (a frame's occlusion
+                                     holds trees, TLAS or BLAS, of up to 14 levels in any case, ray queries of up
+                                     to 18; deeper ones may fit), or a node index lies outside its tree */
 
 typedef struct sftg_ctx sftg_ctx;
 

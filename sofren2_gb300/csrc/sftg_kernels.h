@@ -168,7 +168,8 @@ struct sftg_pose_tables {
     const float* keys;
     const uint32_t* order;         /* per skeleton: bone | parent << 16 (0xFFFF: a root), parents first */
 };
-/* rays up to which a ray gets a whole warp: 389 us against 468 at 65536, 5.0 ms against 1.85 at 2^20 */
+/* rays up to which a ray gets a whole warp: 400 us at 65536 against 468 of the refilled queue; either side of
+ * the line 481 us (81920, warps) and 489 (81921, queue); 131072 by the queue 602 us; 2^20 5.0 ms against 1.8 */
 #define SFTG_RAY_WIDE_MAX 81920u
 /* next: a device word, the ray counter of a launch of many rays; returns a cudaError_t */
 int sftg_launch_raycast(const sftg_ray* rays, uint32_t n, const sftg_model* models, uint32_t n_models, const sftg_wslot* wslots,

@@ -18,6 +18,7 @@
 #include "sftg_kernels.h"
 
 #define OCC_WARPS 4
+/* entries; one node a step from half on, so trees of up to 14 levels fit whatever is hit (7 entries a level) */
 #define OCC_STACK 256         /* TLAS */
 #define OCC_WALK_STACK 256    /* BLAS */
 #define OCC_ALL 0xFFFFFFFFu

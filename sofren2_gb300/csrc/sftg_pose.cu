@@ -12,8 +12,10 @@
  *              16-byte rows, consecutive over the warp
  * Matrix products follow sft_m_mul (sofren2.c:1668): left-to-right sums of plain products.
  *
- * Bound by issue, most of it the slerps and the local products (a quarter of the time is the
- * 2.8 KB of matrices a request of 22 bones writes, at the copy rate).  One warp per request, lanes
+ * Half of the issue slots are used, most of them for the slerps and the local products, with 23 of 32
+ * threads (bones with and without a rotation sampler share a warp); the waits are for the samplers' keys
+ * and at the two barriers (a quarter of the time is the 2.8 KB of matrices a request of 22 bones
+ * writes, at the copy rate).  One warp per request, lanes
  * on channels and whole matrices stored per lane, took 361 us for 65536 requests of 22 bones: the
  * hierarchy ran level by level with a few lanes, and each store touched 32 lines.  Now 105 us; 1024
  * requests 14.4 -> 12.4 us.

@@ -125,9 +125,9 @@ __device__ __forceinline__ bool has_blas(const sftg_ray& R, const sftg_model* mo
  * and each takes the next ray when its own is done: the warp draws 32 rays at a time from a counter
  * and sets them up a lane per ray.  Finished walks leave (triangle, distance) in their hit record;
  * k_ray_records turns those into records, again a thread per ray.
- * Bound by issue and by the latency of the node loads.  Groups diverging from one another in one
- * warp, with set-up and record by 8 lanes each, ran 9 of 32 threads: 2^20 rays against the atrium
- * took 4.73 ms, now 1.85.  10 and 12 resident CTAs (fewer registers, less L1) took 2.01 and 2.19. */
+ * Bound by issue (65 % of the slots, 27 of 32 threads) and by the latency of the node loads.  Groups
+ * diverging from one another in one warp, with set-up and record by 8 lanes each, ran 9 of 32 threads:
+ * 2^20 rays against the atrium took 4.73 ms, now 1.79.  10 and 12 resident CTAs (fewer registers, less L1) took 2.01 and 2.19. */
 #define RAY_PENDING 4u   /* of a record's hit word: a walk's result, bit 0 hit, bit 1 overflow */
 
 __global__ void __launch_bounds__(RAY_WARPS * 32)
