@@ -1522,27 +1522,29 @@ extern "C" int sftg_pose_eval(sftg_ctx* ctx, const sftg_pose_request* reqs, uint
     CK(cudaGetLastError());
     /* a request with an out-of-range animation leaves its matrices as they were: those are saved,
      * the whole result is copied straight into the caller's arrays, and the saved ones put back */
-    std::vector<uint32_t> keep;
+    struct span { size_t at, count; };   /* floats; the requests may lie under the outputs and are not read again */
+    std::vector<span> keep;
     size_t keep_floats = 0;
     for (uint32_t k = 0; k < n; k++) {
         const sftg_skel_dev& sk = ctx->h_skels[reqs[k].skeleton];
-        if (reqs[k].animation < 0 || (uint32_t)reqs[k].animation >= sk.anim_count) { keep.push_back(k); keep_floats += (size_t)sk.bone_count * 16; }
+        if (reqs[k].animation < 0 || (uint32_t)reqs[k].animation >= sk.anim_count) {
+            keep.push_back({ (size_t)off[k] * 16, (size_t)sk.bone_count * 16 });
+            keep_floats += keep.back().count;
+        }
     }
     std::vector<float> saved(keep_floats * (global ? 2 : 1));
     size_t q = 0;
-    for (uint32_t k : keep) {
-        const size_t c = (size_t)ctx->h_skels[reqs[k].skeleton].bone_count * 16;
-        memcpy(saved.data() + q, posed + (size_t)off[k] * 16, c * 4); q += c;
-        if (global) { memcpy(saved.data() + q, global + (size_t)off[k] * 16, c * 4); q += c; }
+    for (const span& r : keep) {
+        memcpy(saved.data() + q, posed + r.at, r.count * 4); q += r.count;
+        if (global) { memcpy(saved.data() + q, global + r.at, r.count * 4); q += r.count; }
     }
     CK(cudaMemcpyAsync(posed, d_posed, b_mat, cudaMemcpyDeviceToHost, ctx->stream));
     if (global) CK(cudaMemcpyAsync(global, d_global, b_mat, cudaMemcpyDeviceToHost, ctx->stream));
     CK(cudaStreamSynchronize(ctx->stream));
     q = 0;
-    for (uint32_t k : keep) {
-        const size_t c = (size_t)ctx->h_skels[reqs[k].skeleton].bone_count * 16;
-        memcpy(posed + (size_t)off[k] * 16, saved.data() + q, c * 4); q += c;
-        if (global) { memcpy(global + (size_t)off[k] * 16, saved.data() + q, c * 4); q += c; }
+    for (const span& r : keep) {
+        memcpy(posed + r.at, saved.data() + q, r.count * 4); q += r.count;
+        if (global) { memcpy(global + r.at, saved.data() + q, r.count * 4); q += r.count; }
     }
     return SFTG_OK;
 }

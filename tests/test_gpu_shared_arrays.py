@@ -67,3 +67,20 @@ def test_matrices_over_the_requests(renderer, poses, out):
     r[:] = rec
     renderer.pose_eval_host(r, *room)
     assert np.array_equal(room[0], posed) and np.array_equal(room[1], glob)
+
+
+@pytest.mark.parametrize("out", [0, 1])
+def test_matrices_over_requests_some_of_which_leave_them(renderer, poses, out):
+    """A request with an animation out of range leaves its matrices, here the bytes of requests, as they were."""
+    rec, posed, glob = poses
+    bad = rec.copy()
+    bad["animation"][::7] = 1000
+    room = [np.full_like(posed, 3), np.full_like(posed, 4)]
+    r = room[out].view(np.uint8)[:rec.nbytes].view(runtime.POSE_REQUEST_DTYPE)
+    r[:] = bad
+    before = [x.copy() for x in room]
+    renderer.pose_eval_host(r, *room)
+    for got, was, want in zip(room, before, (posed, glob)):
+        got, was, want = (x.view(np.uint32).reshape(len(rec), -1) for x in (got, was, want))
+        left = np.arange(len(rec)) % 7 == 0
+        assert np.array_equal(got[left], was[left]) and np.array_equal(got[~left], want[~left])
